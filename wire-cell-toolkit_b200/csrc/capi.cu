@@ -150,6 +150,8 @@ struct PlaneState {
     DevBuf d_table;        // [G][2npad+1][ldr] floats
     int spec_N{0};
     DevBuf d_spec;         // [G][2npad+1][M] packed spectra for spec_N
+    DevBuf d_wspec;        // their wire spectra (wire_fft.cuh), where the overlap-save form applies
+    bool have_wspec{false};
     // long-range response (ImpactTransform::waveform, gen/src/ImpactTransform.cxx:327-343); empty: none
     std::vector<float> long_wf;
     int long_pad{0};
@@ -435,6 +437,11 @@ static int ensure_spectra(Core& c, PlaneState& ps, int N)
     CUDA_TRY(ps.d_spec.ensure(sizeof(float2) * (size_t)rows * (N / 2)));
     launch_rfft_rows(ps.d_table.as<float>(), ps.ldr, std::min(ps.nresp, N), ps.d_spec.as<float2>(), N / 2, rows, d,
                      c.own_stream);
+    ps.have_wspec = wire_fft_fits(ps.G, ps.npad, N / 2);
+    if (ps.have_wspec) {
+        CUDA_TRY(ps.d_wspec.ensure(sizeof(float2) * wire_spec_count(ps.G, N / 2)));
+        launch_wire_spec(ps.d_spec.as<float2>(), ps.d_wspec.as<float2>(), ps.G, ps.npad, N / 2, c.own_stream);
+    }
     CUDA_TRY(cudaGetLastError());
     CUDA_TRY(cudaStreamSynchronize(c.own_stream));
     ps.spec_N = N;
@@ -538,8 +545,8 @@ static int prepare_event(Core& c, const double* d_depos, size_t ndepos, cudaStre
     Core::StageTimer t_prep(&c, 0, s);
     CUDA_TRY(cudaMemsetAsync(c.d_wcnt.p, 0, sizeof(int) * (nkeys + 1), s));
     CUDA_TRY(c.d_kbound.ensure(sizeof(unsigned long long) * (size_t)nkeys * kTileBlocks));
-    CUDA_TRY(c.d_wide.ensure((size_t)nkeys));
-    CUDA_TRY(cudaMemsetAsync(c.d_wide.p, 0, (size_t)nkeys, s));
+    CUDA_TRY(c.d_wide.ensure((size_t)nkeys + nwt));  // and, behind the keys, a flag per wire (set by the raster)
+    CUDA_TRY(cudaMemsetAsync(c.d_wide.p, 0, (size_t)nkeys + nwt, s));
     CUDA_TRY(cudaMemsetAsync(c.d_kbound.p, 0, sizeof(unsigned long long) * (size_t)nkeys * kTileBlocks, s));
     k_win_init<<<1, 64, 0, s>>>(c.d_win.as<WindowDev>(), np);
     EventTable& et = ev.et;
@@ -738,6 +745,7 @@ static int forward_device(Core& c, const double* d_depos, size_t ndepos, float* 
     const TprofPool pool{c.d_pool.as<float>(), c.d_pool_off.as<int>(), c.d_pool_used.as<unsigned long long>(),
                          wide};
 
+    unsigned char* row_flag = c.d_wide.as<unsigned char>() + ev.nkeys;
     Core::StageTimer t_r(&c, 1, s);
     launch_fill(c.d_rec.as<PatchRec>(), ev.et, ev.nkeys, pset, c.d_wcur.as<int>(), c.d_wlist.as<Visit>(),
                 (long long)std::max(total_visits, 1), s);
@@ -748,13 +756,13 @@ static int forward_device(Core& c, const double* d_depos, size_t ndepos, float* 
                          c.d_fluc.as<FlucRec>(), s);
         launch_raster_fluc(c.d_rec.as<PatchRec>(), c.d_fluc.as<FlucRec>(), ev.fp, ev.et, c.d_wcnt.as<int>(),
                            c.d_woff.as<int>(), c.d_wlist.as<Visit>(), (long long)std::max(total_visits, 1), gset,
-                           c.d_Q.as<float>(), s);
+                           c.d_Q.as<float>(), row_flag, s);
     }
     else
         launch_raster_wires(c.d_rec.as<PatchRec>(), c.d_tprof.as<float>(), pool, c.d_wide.as<unsigned char>(),
                             c.d_wcnt.as<int>(),
                             c.d_woff.as<int>(), c.d_wlist.as<Visit>(), (long long)std::max(total_visits, 1),
-                            c.d_kbound.as<unsigned long long>(), gset, c.d_Q.as<float>(), s);
+                            c.d_kbound.as<unsigned long long>(), gset, c.d_Q.as<float>(), row_flag, s);
     t_r.close((n > 0 ? 1 : 0) + (ev.fp.on_patch && n > 0 ? 1 : 0) + (!ev.fp.on_patch && wide > 0 ? 1 : 0) +
               (rows > 0 ? 1 : 0));
     CUDA_TRY(cudaGetLastError());
@@ -815,13 +823,18 @@ static int forward_device(Core& c, const double* d_depos, size_t ndepos, float* 
                 launch_rfft_rows(Q, N, N, reinterpret_cast<float2*>(Q), M, ps.G * nin, d, ps_s);
                 t_f.close(1);
                 Core::StageTimer t_c(&c, 3, ps_s);
-                launch_wire_conv(reinterpret_cast<const float2*>(Q), ps.d_spec.as<float2>(), V, ps.G, ps.npad, nin,
-                                 nout, M, ps.mirror, ps_s);
+                if (ps.have_wspec && wire_fft_pays(ps.npad, nout))
+                    launch_wire_conv_fft(reinterpret_cast<const float2*>(Q), ps.d_wspec.as<float2>(), V, ps.G,
+                                         ps.npad, nin, nout, M, ps_s);
+                else
+                    launch_wire_conv(reinterpret_cast<const float2*>(Q), ps.d_spec.as<float2>(), V, ps.G, ps.npad,
+                                     nin, nout, M, ps.mirror, ps_s);
                 t_c.close(1);
                 const int wlo = std::max(0, w.m_start_ch), whi = std::min(ps.desc.nwires, w.m_end_ch);
                 Core::StageTimer t_i(&c, 4, ps_s);
                 launch_irfft_rows(V, nout, d, w.start_ch - ps.npad, wlo, whi, w.start_tick, std::min(N, w.nt_ref),
-                                  nticks, d_frame + (size_t)ps.row0 * nticks, ps_s);
+                                  nticks, d_frame + (size_t)ps.row0 * nticks, ps_s, row_flag + pset.p[ip].wire_base,
+                                  ps.desc.nwires, ps.npad);
                 if (!ps.long_wf.empty() && whi > wlo) {
                     rc = long_conv_rows(c, ps, d_frame + ((size_t)ps.row0 + wlo) * nticks, nticks, whi - wlo, nticks,
                                         false, ps_s);
@@ -925,8 +938,12 @@ static int adjoint_device(Core& c, const double* d_depos, size_t ndepos, const f
         t_f.close(2);
         float* dQ = c.d_Q.as<float>() + g.qoff;
         Core::StageTimer t_c(&c, 7, s);
-        launch_wire_conv_adj(reinterpret_cast<const float2*>(Gr), ps.d_spec.as<float2>(),
-                             reinterpret_cast<float2*>(dQ), ps.G, ps.npad, nin, nout, M, s);
+        if (ps.have_wspec && wire_adj_fft_pays(ps.npad))
+            launch_wire_adj_fft(reinterpret_cast<const float2*>(Gr), ps.d_wspec.as<float2>(),
+                                reinterpret_cast<float2*>(dQ), ps.G, ps.npad, nin, nout, M, s);
+        else
+            launch_wire_conv_adj(reinterpret_cast<const float2*>(Gr), ps.d_spec.as<float2>(),
+                                 reinterpret_cast<float2*>(dQ), ps.G, ps.npad, nin, nout, M, s);
         t_c.close(1);
         Core::StageTimer t_i(&c, 8, s);
         launch_irfft_rows(reinterpret_cast<const float2*>(dQ), ps.G * nin, d, 0, 0, ps.G * nin, 0, N, N, dQ, s);
@@ -1039,7 +1056,7 @@ struct BatchState {
     BatchStatic bs{};
     std::vector<std::unique_ptr<FftPlanDev>> cls_plans;
     DevBuf d_descs;
-    std::vector<std::unique_ptr<DevBuf>> spec;  // [plane * ncls + cls]
+    std::vector<std::unique_ptr<DevBuf>> spec;  // [plane * ncls + cls]: taps, then wire spectra where they apply
     DevBuf d_spec_tab;                          // const float2* [plane][ncls]
     int maxM{0}, maxG{0}, nsm{148};
     DevBuf d_Q, d_V, d_rec, d_tprof, d_win, d_wcnt, d_woff, d_wcur, d_kbound, d_wlist, d_plans;
@@ -1134,13 +1151,18 @@ static int batch_setup(Core& c)
     }
     CUDA_TRY(b.d_descs.ensure(sizeof(FftDesc) * descs.size()));
     CUDA_TRY(cudaMemcpy(b.d_descs.p, descs.data(), sizeof(FftDesc) * descs.size(), cudaMemcpyHostToDevice));
+    bs.nwires_total = nwt;
     long long q = 0, v = 0;
+    int wbase = 0;
     b.maxG = 0;
     b.spec.clear();
-    std::vector<const float2*> tab((size_t)np * bs.ncls);
+    std::vector<const float2*> tab(2 * (size_t)np * bs.ncls);  // taps, then wire spectra
     for (int ip = 0; ip < np; ++ip) {
         PlaneState& ps = *c.planes[ip];
         BatchPlaneStatic& pl = bs.pl[ip];
+        pl.wire_base = wbase;
+        wbase += ps.desc.nwires;
+        pl.wire_fft = wire_fft_fits(ps.G, ps.npad, b.maxM) ? 1 : 0;
         pl.G = ps.G;
         pl.npad = ps.npad;
         pl.waveform_pad = ps.waveform_pad;
@@ -1164,6 +1186,14 @@ static int batch_setup(Core& c)
                              b.cls_plans[k]->desc, c.own_stream);
             CUDA_TRY(cudaGetLastError());
             tab[(size_t)ip * bs.ncls + k] = sp->as<float2>();
+            if (pl.wire_fft) {
+                auto ws = std::make_unique<DevBuf>();
+                CUDA_TRY(ws->ensure(sizeof(float2) * wire_spec_count(ps.G, N / 2)));
+                launch_wire_spec(sp->as<float2>(), ws->as<float2>(), ps.G, ps.npad, N / 2, c.own_stream);
+                CUDA_TRY(cudaGetLastError());
+                tab[((size_t)np + ip) * bs.ncls + k] = ws->as<float2>();
+                b.spec.push_back(std::move(ws));
+            }
             b.spec.push_back(std::move(sp));
         }
     }
@@ -1279,7 +1309,7 @@ static int forward_batch_device(Core& c, const double* d_depos, const long long*
         CUDA_TRY(b.d_woff.ensure(sizeof(int) * (size_t)(nkeysK + 1)));
         CUDA_TRY(b.d_wcur.ensure(sizeof(int) * (size_t)(nkeysK + 1 + (nkeysK + 1023) / 1024)));
         CUDA_TRY(b.d_kbound.ensure(sizeof(unsigned long long) * (size_t)nkeysK * kTileBlocks));
-        CUDA_TRY(b.d_wide.ensure((size_t)nkeysK));
+        CUDA_TRY(b.d_wide.ensure((size_t)nkeysK + (size_t)K * bs.nwires_total));  // keys, then wire flags
         CUDA_TRY(b.d_wlist.ensure(sizeof(Visit) * (size_t)b.vcap));
         CUDA_TRY(b.d_plans.ensure(sizeof(BatchPlan) * (size_t)nch));
         CUDA_TRY(b.d_ident.ensure(sizeof(int)));
@@ -1333,7 +1363,8 @@ static int forward_batch_device(Core& c, const double* d_depos, const long long*
                 const double* dep = d_depos ? d_depos + 7 * offsets[c0] : nullptr;
                 cudaMemsetAsync(b.d_wcnt.p, 0, sizeof(int) * (size_t)(nk + 1), s);
                 cudaMemsetAsync(b.d_kbound.p, 0, sizeof(unsigned long long) * (size_t)nk * kTileBlocks, s);
-                cudaMemsetAsync(b.d_wide.p, 0, (size_t)nk, s);
+                cudaMemsetAsync(b.d_wide.p, 0, (size_t)nk + (size_t)ne * bs.nwires_total, s);
+                unsigned char* row_flag = b.d_wide.as<unsigned char>() + nk;
                 k_win_init<<<(ne * np + 63) / 64, 64, 0, s>>>(b.d_win.as<WindowDev>(), ne * np);
                 // random streams keyed by the frame ident of each event: base (a device
                 // value written before every launch of the graph) + c0 + event
@@ -1360,14 +1391,22 @@ static int forward_batch_device(Core& c, const double* d_depos, const long long*
                 launch_raster_batch(plans + ch, bs, pset, b.d_rec.as<PatchRec>(), et.dep0[ne], b.d_tprof.as<float>(),
                                     pool, b.d_wide.as<unsigned char>(), b.d_wcnt.as<int>(), b.d_woff.as<int>(), b.d_wlist.as<Visit>(), b.vcap,
                                     b.d_kbound.as<unsigned long long>(), b.d_Q.as<float>(), nb_r, b.maxG, et, fp,
-                                    b.d_fluc.as<FlucRec>(), s);
+                                    b.d_fluc.as<FlucRec>(), row_flag, s);
                 launch_rfft_batch(plans + ch, b.d_descs.as<FftDesc>(), b.d_Q.as<float>(), nb_f, b.tune.fft_threads,
                                   b.maxM, s);
                 // one launch per run of planes that share the pad and the group pairing
                 // (the launches use one work counter, so they must not overlap: same stream)
                 for (int ip0 = 0; ip0 < np;) {
                     int ip1 = ip0 + 1;
-                    while (ip1 < np && c.planes[ip1]->npad == c.planes[ip0]->npad &&
+                    if (bs.pl[ip0].wire_fft) {
+                        while (ip1 < np && bs.pl[ip1].wire_fft) ++ip1;
+                        launch_conv_fft_batch(plans + ch, bs, ip0, ip1,
+                                              b.d_spec_tab.as<const float2*>() + (size_t)np * bs.ncls,
+                                              b.d_Q.as<float>(), b.d_V.as<float2>(), b.nsm * 2, s);
+                        ip0 = ip1;
+                        continue;
+                    }
+                    while (ip1 < np && !bs.pl[ip1].wire_fft && c.planes[ip1]->npad == c.planes[ip0]->npad &&
                            c.planes[ip1]->mirror == c.planes[ip0]->mirror)
                         ++ip1;
                     launch_conv_batch(plans + ch, bs, ip0, ip1, c.planes[ip0]->mirror,
@@ -1375,7 +1414,7 @@ static int forward_batch_device(Core& c, const double* d_depos, const long long*
                     ip0 = ip1;
                 }
                 launch_irfft_batch(plans + ch, bs, b.d_descs.as<FftDesc>(), b.d_V.as<float2>(), d_frames + c0 * fstride,
-                                   fstride, nb_f, b.tune.fft_threads, b.maxM, s);
+                                   fstride, nb_f, b.tune.fft_threads, b.maxM, row_flag, s);
             }
             cudaError_t ce = cudaStreamEndCapture(s, &graph);
             if (ce != cudaSuccess) {

@@ -137,6 +137,37 @@ __device__ __forceinline__ void bfly8(float2* v)
     v[7] = csub(e3, t3);
 }
 
+// 16 = 4 x 4: n = n1 + 4 n2, k = 4 k1 + k2.
+template <int SIGN>
+__device__ __forceinline__ void bfly16(float2* v)
+{
+    constexpr float c1 = 0.92387953251128674f, s1 = 0.38268343236508977f;  // cos, sin of pi/8
+#pragma unroll
+    for (int n = 0; n < 4; ++n) bfly4<SIGN>(v[n], v[n + 4], v[n + 8], v[n + 12]);  // v[n + 4 k2]
+    const float2 w1 = make_float2(c1, SIGN * s1), w3 = make_float2(s1, SIGN * c1);
+    const float2 w2 = make_float2(kS2, SIGN * kS2), w6 = make_float2(-kS2, SIGN * kS2);
+    v[5] = cmul(v[5], w1);
+    v[6] = cmul(v[6], w2);
+    v[7] = cmul(v[7], w3);
+    v[9] = cmul(v[9], w2);
+    v[10] = cmul_i<SIGN>(v[10]);
+    v[11] = cmul(v[11], w6);
+    v[13] = cmul(v[13], w3);
+    v[14] = cmul(v[14], w6);
+    v[15] = cmul(v[15], make_float2(-c1, -SIGN * s1));
+#pragma unroll
+    for (int k = 0; k < 4; ++k) bfly4<SIGN>(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);  // v[4 k2 + k1]
+    // X[4 k1 + k2] sits at v[4 k2 + k1]: transpose (register renaming only)
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int b = a + 1; b < 4; ++b) {
+            const float2 t = v[4 * a + b];
+            v[4 * a + b] = v[4 * b + a];
+            v[4 * b + a] = t;
+        }
+}
+
 template <int R, int SIGN>
 __device__ __forceinline__ void bfly(float2* v)
 {

@@ -25,6 +25,7 @@
 #include "kernels.cuh"
 #include "gauss.cuh"
 #include "rng.cuh"
+#include "wire_fft.cuh"
 
 #include <algorithm>
 #include <cfloat>
@@ -656,7 +657,8 @@ __device__ __forceinline__ void raster_tile(const GridPlane& P, int row, int kti
                                             const int* __restrict__ wire_cnt, const int* __restrict__ wire_off,
                                             const Visit* __restrict__ visits, long long vcap,
                                             const unsigned long long* __restrict__ key_bound,
-                                            float* __restrict__ Q, int* smem_i, float* scale, float* iscale)
+                                            float* __restrict__ Q, unsigned char* __restrict__ row_flag, int* smem_i,
+                                            float* scale, float* iscale)
 {
     __syncthreads();  // the previous item of a persistent block is done with the shared arrays
     const int w = P.start_ch + row;
@@ -685,6 +687,7 @@ __device__ __forceinline__ void raster_tile(const GridPlane& P, int row, int kti
         }
         return;
     }
+    if (tid == 0) row_flag[P.wire_base + w] = 1;  // the wire holds charge (every block of the row writes the same)
     const bool spread = key >= 0 && wide_key[key];
     {
         int4* g4 = reinterpret_cast<int4*>(grid);
@@ -903,7 +906,8 @@ __global__ void __launch_bounds__(kRasterThreads, 5) k_raster_wires(const PatchR
                                                                  const Visit* __restrict__ visits, long long vcap,
                                                                  const unsigned long long* __restrict__ key_bound,
                                                                  GridSet gs, float* __restrict__ Q, TprofPool pool,
-                                                                 const unsigned char* __restrict__ wide_key)
+                                                                 const unsigned char* __restrict__ wide_key,
+                                                                 unsigned char* __restrict__ row_flag)
 {
     extern __shared__ int smem_i[];
     __shared__ float scale[kTileBlocks], iscale[kTileBlocks];
@@ -914,20 +918,21 @@ __global__ void __launch_bounds__(kRasterThreads, 5) k_raster_wires(const PatchR
     const int row = rel / P.ntile;
     const int ktile = P.ktile0 + (rel - row * P.ntile);  // absolute tick tile
     raster_tile(P, row, ktile, 0, gs.ntiles_abs, rec, tprof, pool, wide_key, wire_cnt, wire_off, visits, vcap,
-                key_bound, Q, smem_i, scale, iscale);
+                key_bound, Q, row_flag, smem_i, scale, iscale);
 }
 
 void launch_raster_wires(const PatchRec* rec, const float* tprof, const TprofPool& pool, const unsigned char* wide_key,
                          const int* wire_cnt,
                          const int* wire_off, const Visit* visits, long long vcap,
-                         const unsigned long long* key_bound, const GridSet& gs, float* Q, cudaStream_t s)
+                         const unsigned long long* key_bound, const GridSet& gs, float* Q, unsigned char* row_flag,
+                         cudaStream_t s)
 {
     if (gs.nrows_total <= 0) return;
     size_t smem = 0;
     for (int i = 0; i < gs.nplanes; ++i) smem = std::max(smem, raster_smem_bytes(gs.p[i].G));
     cudaFuncSetAttribute((const void*)k_raster_wires, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     k_raster_wires<<<gs.nrows_total, kRasterThreads, smem, s>>>(rec, tprof, wire_cnt, wire_off, visits, vcap,
-                                                                    key_bound, gs, Q, pool, wide_key);
+                                                                    key_bound, gs, Q, pool, wide_key, row_flag);
 }
 
 // ---------------------------------------------------------------------------
@@ -1029,7 +1034,8 @@ __device__ __forceinline__ void raster_tile_fluc(const GridPlane& P, int ip, int
                                                  const PatchRec* __restrict__ rec, const FlucRec* __restrict__ fluc,
                                                  const int* __restrict__ wire_cnt, const int* __restrict__ wire_off,
                                                  const Visit* __restrict__ visits, long long vcap,
-                                                 float* __restrict__ Q, long long* grid)
+                                                 float* __restrict__ Q, unsigned char* __restrict__ row_flag,
+                                                 long long* grid)
 {
     __syncthreads();  // the previous item of a persistent block is done with the grid
     __shared__ float s_p[kFlucRasterThreads / 32][16], s_w[kFlucRasterThreads / 32][16];
@@ -1047,6 +1053,7 @@ __device__ __forceinline__ void raster_tile_fluc(const GridPlane& P, int ip, int
         cnt = off < 0 ? 0 : (int)min((long long)wire_cnt[key], max(0ll, vcap - off));
         list = visits + max(off, 0);
     }
+    if (tid == 0 && cnt > 0) row_flag[P.wire_base + w] = 1;
     for (int k = tid; k < G * kTileLd; k += blockDim.x) grid[k] = 0;
     __syncthreads();
     const float pbs = P.pbs, tbs = P.tbs, inv_pbs = 1.0f / pbs;
@@ -1120,7 +1127,8 @@ __global__ void __launch_bounds__(kFlucRasterThreads) k_raster_fluc(const PatchR
                                                                     const int* __restrict__ wire_cnt,
                                                                     const int* __restrict__ wire_off,
                                                                     const Visit* __restrict__ visits, long long vcap,
-                                                                    GridSet gs, float* __restrict__ Q)
+                                                                    GridSet gs, float* __restrict__ Q,
+                                                                    unsigned char* __restrict__ row_flag)
 {
     extern __shared__ long long grid64[];
     int ip = 0;
@@ -1130,19 +1138,19 @@ __global__ void __launch_bounds__(kFlucRasterThreads) k_raster_fluc(const PatchR
     const int row = rel / P.ntile;
     const int ktile = P.ktile0 + (rel - row * P.ntile);
     raster_tile_fluc(P, ip, row, ktile, 0, gs.ntiles_abs, evt, fp, rec, fluc, wire_cnt, wire_off, visits, vcap, Q,
-                     grid64);
+                     row_flag, grid64);
 }
 
 void launch_raster_fluc(const PatchRec* rec, const FlucRec* fluc, const FlucParams& fp, const EventTable& evt,
                         const int* wire_cnt, const int* wire_off, const Visit* visits, long long vcap,
-                        const GridSet& gs, float* Q, cudaStream_t s)
+                        const GridSet& gs, float* Q, unsigned char* row_flag, cudaStream_t s)
 {
     if (gs.nrows_total <= 0) return;
     size_t smem = 0;
     for (int i = 0; i < gs.nplanes; ++i) smem = std::max(smem, raster_fluc_smem_bytes(gs.p[i].G));
     cudaFuncSetAttribute((const void*)k_raster_fluc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     k_raster_fluc<<<gs.nrows_total, kFlucRasterThreads, smem, s>>>(rec, fluc, fp, evt, wire_cnt, wire_off, visits,
-                                                                     vcap, gs, Q);
+                                                                     vcap, gs, Q, row_flag);
 }
 
 // Independent Binomial(n, p) draws: out[i] from the stream of key (seed,
@@ -1454,13 +1462,26 @@ __device__ __forceinline__ void irfft_row(const float2* __restrict__ v, const Ff
     }
 }
 
+// Whether a flagged charge wire lies within pad of wire W (all threads of the
+// block call it): rows out of every charge's reach stay exactly zero, whatever
+// rounding the convolution left in their spectra.
+__device__ __forceinline__ bool row_reached(const unsigned char* __restrict__ flag, int nwires, int W, int pad)
+{
+    int any = 0;
+    const int hi = min(nwires - 1, W + pad);
+    for (int w = max(0, W - pad) + threadIdx.x; w <= hi; w += blockDim.x) any |= flag[w];
+    return __syncthreads_or(any);
+}
+
 __global__ void k_irfft_rows(const float2* __restrict__ Vh, int nrows, FftDesc d, int wire0, int wlo, int whi,
-                             int tick0, int ncols, int nticks, float* __restrict__ frame)
+                             int tick0, int ncols, int nticks, float* __restrict__ frame,
+                             const unsigned char* __restrict__ row_flag, int nwires, int npad)
 {
     extern __shared__ float2 sm[];
     const int row = blockIdx.x;
     const int W = wire0 + row;
     if (row >= nrows || W < wlo || W >= whi) return;
+    if (row_flag && !row_reached(row_flag, nwires, W, npad)) return;
     irfft_row(Vh + (size_t)row * d.M, d, frame + (size_t)W * nticks, tick0, ncols, nticks, sm);
 }
 
@@ -1473,7 +1494,9 @@ __global__ void k_irfft_rows(const float2* __restrict__ Vh, int nrows, FftDesc d
 template <int IT>
 __global__ void __launch_bounds__(256) k_irfft_rows_pf(const float2* __restrict__ Vh, int r0, int r1, FftDesc d,
                                                        int wire0, int tick0, int ncols, int nticks,
-                                                       float* __restrict__ frame)
+                                                       float* __restrict__ frame,
+                                                       const unsigned char* __restrict__ row_flag, int nwires,
+                                                       int npad)
 {
     extern __shared__ float2 sm[];
     const int M = d.M, tid = threadIdx.x, nth = blockDim.x;
@@ -1498,13 +1521,18 @@ __global__ void __launch_bounds__(256) k_irfft_rows_pf(const float2* __restrict_
     const int nR = M / 8;
     const float sc = 1.0f / (float)M;
     while (row < r1) {
+        const int next = row + gridDim.x;
+        if (row_flag && !row_reached(row_flag, nwires, wire0 + row, npad)) {  // uniform over the block
+            if (next < r1) fetch(next);
+            row = next;
+            continue;
+        }
 #pragma unroll
         for (int it = 0; it < IT; ++it) {
             const int k = tid + it * nth;
             if (k < M) b[k] = pv[it];
         }
         __syncthreads();
-        const int next = row + gridDim.x;
         if (next < r1) fetch(next);
         // first stage (radix 8, no twiddles) on the pre-processed bins
         for (int j = tid; j < nR; j += nth) {
@@ -1548,7 +1576,8 @@ __global__ void __launch_bounds__(256) k_irfft_rows_pf(const float2* __restrict_
 
 template <int IT>
 static bool launch_irfft_pf(const float2* Vh, int r0, int r1, const FftDesc& d, int wire0, int tick0, int ncols,
-                            int nticks, float* frame, cudaStream_t s)
+                            int nticks, float* frame, const unsigned char* row_flag, int nwires, int npad,
+                            cudaStream_t s)
 {
     const size_t smem = 4 * (size_t)d.M * sizeof(float2);
     allow_smem((const void*)k_irfft_rows_pf<IT>, smem);
@@ -1558,26 +1587,31 @@ static bool launch_irfft_pf(const float2* Vh, int r0, int r1, const FftDesc& d, 
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_irfft_rows_pf<IT>, 256, smem) != cudaSuccess) return false;
     const int grid = std::min(r1 - r0, per * nsm);
     if (grid <= 0 || r1 - r0 < 2 * grid) return false;  // under two rows per block: one block per row
-    k_irfft_rows_pf<IT><<<grid, 256, smem, s>>>(Vh, r0, r1, d, wire0, tick0, ncols, nticks, frame);
+    k_irfft_rows_pf<IT><<<grid, 256, smem, s>>>(Vh, r0, r1, d, wire0, tick0, ncols, nticks, frame, row_flag, nwires,
+                                                npad);
     return true;
 }
 
 void launch_irfft_rows(const float2* Vh, int nrows, const FftDesc& d, int wire0, int wlo, int whi, int tick0,
-                       int ncols, int nticks, float* frame, cudaStream_t s)
+                       int ncols, int nticks, float* frame, cudaStream_t s, const unsigned char* row_flag, int nwires,
+                       int npad)
 {
     if (nrows <= 0) return;
     if (d.M % 16 == 0 && d.nst >= 2 && d.radix[0] == 8 && 4 * (size_t)d.M * sizeof(float2) <= 128 * 1024) {
         // the rows that are frame wires: wire0 + r in [wlo, whi)
         const int r0 = std::max(0, wlo - wire0), r1 = std::min(nrows, whi - wire0);
         if (r1 <= r0) return;
-        if (d.M <= 1024 && launch_irfft_pf<4>(Vh, r0, r1, d, wire0, tick0, ncols, nticks, frame, s)) return;
-        if (d.M > 1024 && d.M <= 2048 && launch_irfft_pf<8>(Vh, r0, r1, d, wire0, tick0, ncols, nticks, frame, s))
+        if (d.M <= 1024 && launch_irfft_pf<4>(Vh, r0, r1, d, wire0, tick0, ncols, nticks, frame, row_flag, nwires,
+                                               npad, s))
+            return;
+        if (d.M > 1024 && d.M <= 2048 && launch_irfft_pf<8>(Vh, r0, r1, d, wire0, tick0, ncols, nticks, frame,
+                                                                row_flag, nwires, npad, s))
             return;
     }
     allow_smem((const void*)k_irfft_rows, 2 * d.M * sizeof(float2));
     const int nth = d.M >= 2048 ? 512 : 256;
     k_irfft_rows<<<nrows, nth, 2 * d.M * sizeof(float2), s>>>(Vh, nrows, d, wire0, wlo, whi, tick0, ncols, nticks,
-                                                                  frame);
+                                                                  frame, row_flag, nwires, npad);
 }
 
 // ---------------------------------------------------------------------------
@@ -2165,7 +2199,9 @@ __global__ void __launch_bounds__(256) k_plan_batch(BatchPlan* __restrict__ plan
         c_raster[k] = o.nin * o.ntile;
         c_rows[k] = pl.G * o.nin;
         c_orows[k] = o.nout;
-        c_conv[k] = o.nin ? ((o.M + 31) / 32) * ((o.nout + kConvRows - 1) / kConvRows) : 0;
+        c_conv[k] = !o.nin        ? 0
+                    : pl.wire_fft ? wire_fblocks(o.M) * wire_blocks(o.nout, pl.npad)
+                                  : ((o.M + 31) / 32) * ((o.nout + kConvRows - 1) / kConvRows);
         if (st) atomicOr(&s_status, st);
     }
     __syncthreads();
@@ -2243,7 +2279,8 @@ __global__ void __launch_bounds__(kRasterThreads, FLUC ? 1 : 5) k_raster_batch(c
                                                                  const Visit* __restrict__ visits, long long vcap,
                                                                  const unsigned long long* __restrict__ key_bound,
                                                                  float* __restrict__ Q, EventTable evt, FlucParams fp,
-                                                                 const FlucRec* __restrict__ fluc)
+                                                                 const FlucRec* __restrict__ fluc,
+                                                                 unsigned char* __restrict__ row_flag)
 {
     extern __shared__ int smem_i[];
     __shared__ float scale[kTileBlocks], iscale[kTileBlocks];
@@ -2277,10 +2314,12 @@ __global__ void __launch_bounds__(kRasterThreads, FLUC ? 1 : 5) k_raster_batch(c
         const int row = rel / E.ntile;
         if constexpr (FLUC)
             raster_tile_fluc(P, ip, row, E.ktile0 + (rel - row * E.ntile), e * bs.nkeys, bs.ntiles, evt, fp, rec,
-                             fluc, wire_cnt, wire_off, visits, vcap, Q, reinterpret_cast<long long*>(smem_i));
+                             fluc, wire_cnt, wire_off, visits, vcap, Q, row_flag + (size_t)e * bs.nwires_total,
+                             reinterpret_cast<long long*>(smem_i));
         else
             raster_tile(P, row, E.ktile0 + (rel - row * E.ntile), e * bs.nkeys, bs.ntiles, rec, tprof, pool,
-                        wide_key, wire_cnt, wire_off, visits, vcap, key_bound, Q, smem_i, scale, iscale);
+                        wide_key, wire_cnt, wire_off, visits, vcap, key_bound, Q,
+                        row_flag + (size_t)e * bs.nwires_total, smem_i, scale, iscale);
     }
 }
 
@@ -2289,19 +2328,19 @@ void launch_raster_batch(const BatchPlan* plan, const BatchStatic& bs, const Pla
                          const unsigned char* wide_key, const int* wire_cnt, const int* wire_off,
                          const Visit* visits, long long vcap, const unsigned long long* key_bound, float* Q,
                          int nblocks, int maxG, const EventTable& evt, const FlucParams& fp, const FlucRec* fluc,
-                         cudaStream_t s)
+                         unsigned char* row_flag, cudaStream_t s)
 {
     const size_t smem = std::max(raster_smem_bytes(maxG), raster_fluc_smem_bytes(maxG));
     if (fp.on_patch)
         k_raster_batch<true><<<nblocks, kRasterThreads, smem, s>>>(plan, bs, ps, rec, recstride, tprof, pool, wide_key,
                                                                     wire_cnt,
                                                                     wire_off, visits, vcap, key_bound, Q, evt, fp,
-                                                                    fluc);
+                                                                    fluc, row_flag);
     else
         k_raster_batch<false><<<nblocks, kRasterThreads, smem, s>>>(plan, bs, ps, rec, recstride, tprof, pool,
                                                                      wide_key, wire_cnt,
                                                                      wire_off, visits, vcap, key_bound, Q, evt, fp,
-                                                                     fluc);
+                                                                     fluc, row_flag);
 }
 
 // Time FFT of every charge-grid row of the pass, in place (rows of N reals
@@ -2402,6 +2441,44 @@ __global__ void __launch_bounds__(32 * kConvRG) k_conv_batch(const BatchPlan* __
     }
 }
 
+// The same by overlap-save (wire_fft.cuh): items of planes ip0 .. ip1-1, all
+// with wire_fft set.
+__global__ void __launch_bounds__(kWThreads, 2) k_conv_fft_batch(const BatchPlan* __restrict__ plan, BatchStatic bs,
+                                                                 int ip0, int ip1,
+                                                                 const float2* const* __restrict__ wspec,
+                                                                 const float* __restrict__ Q, float2* __restrict__ V)
+{
+    extern __shared__ float2 wsm[];
+    __shared__ int s_item;
+    if (plan->status & kBatchSkip) return;
+    wfft::load_twiddles(wsm + 2 * kWEx, threadIdx.x);
+    const int nev = plan->nev, np = plan->np;
+    int total = 0;
+    for (int ip = ip0; ip < ip1; ++ip) total += plan->pre_conv[ip][nev];
+    int* ctr = const_cast<int*>(&plan->next[3 + ip0]);
+    for (int item = next_item(ctr, &s_item); item < total; item = next_item(ctr, &s_item)) {
+        int ip = ip0, rel = item;
+        while (rel >= plan->pre_conv[ip][nev]) {
+            rel -= plan->pre_conv[ip][nev];
+            ++ip;
+        }
+        const int* pre = plan->pre_conv[ip];
+        const int e = find_entry(pre, nev, rel);
+        const EvPlane& E = plan->ep[e * np + ip];
+        rel -= pre[e];
+        const int nfb = wire_fblocks(E.M);
+        const int oblk = rel / nfb, fblk = rel - oblk * nfb;
+        wfft::conv_tile(reinterpret_cast<const float2*>(Q + E.qoff), wspec[(size_t)ip * bs.ncls + E.cls], V + E.voff,
+                        bs.pl[ip].G, bs.pl[ip].npad, E.nin, E.nout, E.M, fblk, oblk, wsm);
+    }
+}
+
+void launch_conv_fft_batch(const BatchPlan* plan, const BatchStatic& bs, int ip0, int ip1,
+                           const float2* const* wspec, const float* Q, float2* V, int nblocks, cudaStream_t s)
+{
+    k_conv_fft_batch<<<nblocks, kWThreads, kWConvSmem, s>>>(plan, bs, ip0, ip1, wspec, Q, V);
+}
+
 size_t conv_smem_bytes(int npad, bool pair)
 {
     if (npad != 10 && npad != 21) return 0;
@@ -2425,7 +2502,8 @@ void launch_conv_batch(const BatchPlan* plan, const BatchStatic& bs, int ip0, in
 
 // Inverse time FFT of every V row of the pass and the frame write of its event.
 __global__ void k_irfft_batch(const BatchPlan* __restrict__ plan, BatchStatic bs, const FftDesc* __restrict__ descs,
-                              const float2* __restrict__ V, float* __restrict__ frames, long long frame_stride)
+                              const float2* __restrict__ V, float* __restrict__ frames, long long frame_stride,
+                              const unsigned char* __restrict__ row_flag)
 {
     extern __shared__ float2 sm[];
     if (plan->status & kBatchSkip) return;
@@ -2442,6 +2520,7 @@ __global__ void k_irfft_batch(const BatchPlan* __restrict__ plan, BatchStatic bs
         const int W = E.start_ch - pl.npad + o;
         const int wlo = max(0, E.m_start_ch), whi = min(pl.nwires, E.m_end_ch);
         if (W < wlo || W >= whi) continue;  // uniform over the block
+        if (!row_reached(row_flag + (size_t)e * bs.nwires_total + pl.wire_base, pl.nwires, W, pl.npad)) continue;
         const FftDesc d = descs[E.cls];
         irfft_row(V + E.voff + (size_t)o * E.M, d, frames + (size_t)e * frame_stride + (size_t)(pl.row0 + W) * bs.nticks,
                   E.start_tick, min(E.N, E.nt_ref), bs.nticks, sm);
@@ -2449,10 +2528,11 @@ __global__ void k_irfft_batch(const BatchPlan* __restrict__ plan, BatchStatic bs
 }
 
 void launch_irfft_batch(const BatchPlan* plan, const BatchStatic& bs, const FftDesc* descs, const float2* V,
-                        float* frames, long long frame_stride, int nblocks, int nthreads, int maxM, cudaStream_t s)
+                        float* frames, long long frame_stride, int nblocks, int nthreads, int maxM,
+                        const unsigned char* row_flag, cudaStream_t s)
 {
     const size_t smem = 2 * (size_t)maxM * sizeof(float2);
-    k_irfft_batch<<<nblocks, nthreads, smem, s>>>(plan, bs, descs, V, frames, frame_stride);
+    k_irfft_batch<<<nblocks, nthreads, smem, s>>>(plan, bs, descs, V, frames, frame_stride, row_flag);
 }
 
 // Shared-memory opt-ins of the batched kernels, set before a graph capture
@@ -2465,6 +2545,7 @@ void batch_kernel_attributes(int maxG, int maxM)
     cudaFuncSetAttribute((const void*)k_raster_batch<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sr);
     cudaFuncSetAttribute((const void*)k_rfft_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, sf);
     cudaFuncSetAttribute((const void*)k_irfft_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, sf);
+    cudaFuncSetAttribute((const void*)k_conv_fft_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWConvSmem);
     cudaFuncSetAttribute((const void*)k_conv_batch<10, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)conv_smem_bytes(10, true));
     cudaFuncSetAttribute((const void*)k_conv_batch<10, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,

@@ -134,13 +134,15 @@ constexpr int kMaxClasses = 48;  // time-FFT length classes of the batched path
 // charge-grid (Q, floats) and wire-convolution (V, complex) arenas.
 struct BatchPlaneStatic {
     int G, npad, waveform_pad, nwires, imp_nbins, row0, nin_max;
+    int wire_base;    // first entry of the plane's wires in the event's wire flags
+    int wire_fft;     // overlap-save wire convolution (wire_fft.cuh) at every length class
     double imp_min, imp_bs;
     long long qslot;  // offset of the plane's grid within an event slot (floats)
     long long vslot;  // offset of the plane's V rows within an event slot (complex values)
 };
 
 struct BatchStatic {
-    int np, nticks, nkeys, ntiles;
+    int np, nticks, nkeys, ntiles, nwires_total;
     double start_time, tbs;   // tick binning of the window arithmetic (ImpactTransform)
     int ncls;
     int cls_N[kMaxClasses];   // ascending time-FFT lengths
@@ -236,7 +238,7 @@ void launch_fluc_sums(const PatchRec* rec, const EventTable& et, const PlaneSet&
                       const double* fq, FlucRec* fluc, cudaStream_t s);
 void launch_raster_fluc(const PatchRec* rec, const FlucRec* fluc, const FlucParams& fp, const EventTable& evt,
                         const int* wire_cnt, const int* wire_off, const Visit* visits, long long vcap,
-                        const GridSet& gs, float* Q, cudaStream_t s);
+                        const GridSet& gs, float* Q, unsigned char* row_flag, cudaStream_t s);
 void launch_scan(const int* wire_cnt, int nwires_total, int* wire_off, int* wire_cur, cudaStream_t s);
 void launch_tprof_pool(const PatchRec* rec, const EventTable& et, int nplanes, float tbs, const TprofPool& pool,
                        int* status, cudaStream_t s);
@@ -246,16 +248,32 @@ size_t raster_smem_bytes(int G);
 void launch_raster_wires(const PatchRec* rec, const float* tprof, const TprofPool& pool, const unsigned char* wide_key,
                          const int* wire_cnt,
                          const int* wire_off, const Visit* visits, long long vcap,
-                         const unsigned long long* key_bound, const GridSet& gs, float* Q, cudaStream_t s);
+                         const unsigned long long* key_bound, const GridSet& gs, float* Q, unsigned char* row_flag,
+                         cudaStream_t s);  // row_flag[wire_base + wire] = 1 for every wire with a visit
 void launch_rfft_rows(const float* in, long in_ld, int in_len, float2* out, long out_ld, int nrows,
                       const FftDesc& d, cudaStream_t s);
 void launch_wire_conv(const float2* Qh, const float2* Rh, float2* Vh, int ngroups, int npad, int nrows_in,
                       int nrows_out, int M, bool pair, cudaStream_t s);
+// Overlap-save forms (wire_fft.cu): Rw holds wire_spec_count(G, M) values made
+// from the taps by launch_wire_spec; wire_fft_fits says whether they apply,
+// wire_fft_pays and wire_adj_fft_pays where they are the faster form.
+size_t wire_spec_count(int G, int M);
+bool wire_fft_fits(int G, int npad, int M);
+bool wire_fft_pays(int npad, int nout);
+bool wire_adj_fft_pays(int npad);
+void launch_wire_spec(const float2* taps, float2* Rw, int G, int npad, int M, cudaStream_t s);
+void launch_wire_conv_fft(const float2* Qh, const float2* Rw, float2* Vh, int G, int npad, int nin, int nout, int M,
+                          cudaStream_t s);
+void launch_wire_adj_fft(const float2* Gh, const float2* Rw, float2* dQh, int G, int npad, int nin, int nout, int M,
+                         cudaStream_t s);
 // the single-buffered 32-frequency tiles (any alignment; the fallback of launch_wire_conv)
 void launch_wire_conv_tiles(const float2* Qh, const float2* Rh, float2* Vh, int ngroups, int npad, int nrows_in,
                             int nrows_out, int M, bool pair, cudaStream_t s);
+// row_flag (optional): flags of the plane's nwires charge wires; a row further
+// than npad wires from every flagged one is left alone (the caller's zeros)
 void launch_irfft_rows(const float2* Vh, int nrows, const FftDesc& d, int wire0, int wlo, int whi, int tick0,
-                       int ncols, int nticks, float* frame, cudaStream_t s);
+                       int ncols, int nticks, float* frame, cudaStream_t s, const unsigned char* row_flag = nullptr,
+                       int nwires = 0, int npad = 0);
 
 void launch_spec_mul(float2* X, long ldx, int nrows, int M, const float2* R, cudaStream_t s);
 // Waveform::edge of frame rows [r0, r0 + nrows) within ticks [t0, t1) (ld: row
@@ -332,14 +350,17 @@ void launch_raster_batch(const BatchPlan* plan, const BatchStatic& bs, const Pla
                          const unsigned char* wide_key, const int* wire_cnt, const int* wire_off,
                          const Visit* visits, long long vcap, const unsigned long long* key_bound, float* Q,
                          int nblocks, int maxG, const EventTable& evt, const FlucParams& fp, const FlucRec* fluc,
-                         cudaStream_t s);
+                         unsigned char* row_flag, cudaStream_t s);  // row_flag: [event][wire]
 void launch_rfft_batch(const BatchPlan* plan, const FftDesc* descs, float* Q, int nblocks, int nthreads, int maxM,
                        cudaStream_t s);
 // Wire convolution of planes [ip0, ip1) (all with the same pad and pairing) in one launch.
 void launch_conv_batch(const BatchPlan* plan, const BatchStatic& bs, int ip0, int ip1, bool pair,
                        const float2* const* spec, const float* Q, float2* V, int nblocks, cudaStream_t s);
 void launch_irfft_batch(const BatchPlan* plan, const BatchStatic& bs, const FftDesc* descs, const float2* V,
-                        float* frames, long long frame_stride, int nblocks, int nthreads, int maxM, cudaStream_t s);
+                        float* frames, long long frame_stride, int nblocks, int nthreads, int maxM,
+                        const unsigned char* row_flag, cudaStream_t s);
+void launch_conv_fft_batch(const BatchPlan* plan, const BatchStatic& bs, int ip0, int ip1,
+                           const float2* const* wspec, const float* Q, float2* V, int nblocks, cudaStream_t s);
 size_t conv_smem_bytes(int npad, bool pair);
 void batch_kernel_attributes(int maxG, int maxM);
 

@@ -1,0 +1,83 @@
+// Kernels and launchers of the overlap-save wire convolution (wire_fft.cuh).
+#include "kernels.cuh"
+#include "wire_fft.cuh"
+
+namespace wctb200 {
+
+__global__ void __launch_bounds__(kWThreads, 2) k_wire_conv_fft(const float2* __restrict__ Qh,
+                                                                const float2* __restrict__ Rw,
+                                                                float2* __restrict__ Vh, int G, int P, int nin,
+                                                                int nout, int M)
+{
+    extern __shared__ float2 wsm[];
+    wfft::load_twiddles(wsm + 2 * kWEx, threadIdx.x);
+    __syncthreads();
+    wfft::conv_tile(Qh, Rw, Vh, G, P, nin, nout, M, blockIdx.x, blockIdx.y, wsm);
+}
+
+__global__ void __launch_bounds__(kWThreads, 2) k_wire_adj_fft(const float2* __restrict__ Gh,
+                                                               const float2* __restrict__ Rw,
+                                                               float2* __restrict__ dQh, int G, int P, int nin,
+                                                               int nout, int M)
+{
+    extern __shared__ float2 wsm[];
+    wfft::load_twiddles(wsm + kWEx, threadIdx.x);
+    __syncthreads();
+    wfft::adj_tile(Gh, Rw, dQh, G, P, nin, nout, M, blockIdx.x, blockIdx.y, wsm);
+}
+
+__global__ void __launch_bounds__(kWThreads) k_wire_spec(const float2* __restrict__ taps, float2* __restrict__ Rw,
+                                                         int P, int M)
+{
+    extern __shared__ float2 wsm[];
+    wfft::load_twiddles(wsm + kWEx, threadIdx.x);
+    __syncthreads();
+    wfft::spec_tile(taps, Rw, P, M, blockIdx.x, blockIdx.y, wsm);
+}
+
+size_t wire_spec_count(int G, int M) { return (size_t)G * wire_fblocks(M) * kWEx; }
+
+bool wire_fft_fits(int G, int npad, int M)
+{
+    return npad <= kWMaxPad && M % 2 == 0 && wire_spec_count(G, M) <= kWMaxSpec;
+}
+
+// Where the overlap-save form is the faster one (11 groups, M = 1600, times in
+// us, inputs not in L2).  Its time goes by blocks of 256 - 2P rows, the direct
+// forms' by G (2P + 1) a row.  P = 21: ahead at every size (nin = 2: 27 against
+// 31, 300: 37 / 78, 960: 71 / 148; adjoint 31 / 43, 59 / 74, 113 / 195).
+// P = 10: behind while one block holds all the rows (nin = 80: 29 / 21), ahead
+// from two blocks on (300: 37 / 47, 960: 72 / 86); the adjoint, with a
+// transform back per group, stays behind (960: 119 / 113).  Other pads have no
+// direct kernel of their own in the forward (P = 5, nin = 80: 29 / 87).
+bool wire_fft_pays(int npad, int nout)
+{
+    return npad >= 16 || npad != 10 || nout > wire_valid(npad);
+}
+bool wire_adj_fft_pays(int npad) { return npad >= 16; }
+
+void launch_wire_spec(const float2* taps, float2* Rw, int G, int npad, int M, cudaStream_t s)
+{
+    cudaFuncSetAttribute((const void*)k_wire_spec, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWAdjSmem);
+    k_wire_spec<<<dim3(wire_fblocks(M), G), kWThreads, kWAdjSmem, s>>>(taps, Rw, npad, M);
+}
+
+void launch_wire_conv_fft(const float2* Qh, const float2* Rw, float2* Vh, int G, int npad, int nin, int nout, int M,
+                          cudaStream_t s)
+{
+    if (nout <= 0) return;
+    cudaFuncSetAttribute((const void*)k_wire_conv_fft, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWConvSmem);
+    k_wire_conv_fft<<<dim3(wire_fblocks(M), wire_blocks(nout, npad)), kWThreads, kWConvSmem, s>>>(
+        Qh, Rw, Vh, G, npad, nin, nout, M);
+}
+
+void launch_wire_adj_fft(const float2* Gh, const float2* Rw, float2* dQh, int G, int npad, int nin, int nout, int M,
+                         cudaStream_t s)
+{
+    if (nin <= 0) return;
+    cudaFuncSetAttribute((const void*)k_wire_adj_fft, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWAdjSmem);
+    k_wire_adj_fft<<<dim3(wire_fblocks(M), wire_blocks(nin, npad)), kWThreads, kWAdjSmem, s>>>(Gh, Rw, dQh, G, npad,
+                                                                                               nin, nout, M);
+}
+
+}  // namespace wctb200
