@@ -6,14 +6,16 @@ import subprocess
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libwctb200.so")
-SOURCES = ["kernels.cu", "wire_fft.cu", "adjoint.cu", "dft.cu", "splat.cu", "capi.cu", "pir.cpp"]
-HEADERS = ["common.cuh", "fft.cuh", "wire_fft.cuh", "gauss.cuh", "kernels.cuh", "rng.cuh", "fft_lengths.h", "json.hpp", "pir.hpp"]
+SOURCES = ["kernels.cu", "fft3.cu", "fft3_batch.cu", "fft3_c2c.cu", "wire_fft.cu", "adjoint.cu", "dft.cu",
+           "splat.cu", "capi.cu", "pir.cpp"]
+HEADERS = ["common.cuh", "fft.cuh", "fft3.cuh", "wire_fft.cuh", "gauss.cuh", "kernels.cuh", "rng.cuh",
+           "fft_lengths.h", "json.hpp", "pir.hpp"]
 
 NVCC_FLAGS = [
     "-O3", "-std=c++17", "-lineinfo",
     "-gencode", "arch=compute_100a,code=sm_100a",
     "-Xcompiler", "-fPIC", "-Xcompiler", "-ffp-contract=off",
-    "--expt-relaxed-constexpr",
+    "--expt-relaxed-constexpr", "--threads", "0",
     "-shared", "-Xlinker", "-soname=libwctb200.so",
 ]
 

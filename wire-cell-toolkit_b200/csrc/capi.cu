@@ -73,7 +73,7 @@ struct DevBuf {
 // ---------------------------------------------------------------------------
 struct FftPlanDev {
     FftDesc desc{};
-    DevBuf tw, twh;
+    DevBuf tw, twh, t3;
 };
 
 // Radix schedule for M (no heap use); false if M has a prime factor above 7
@@ -131,6 +131,24 @@ static int make_plan(int M, FftPlanDev& p)
     CUDA_TRY(cudaMemcpy(p.twh.p, twh.data(), sizeof(float2) * M, cudaMemcpyHostToDevice));
     p.desc.tw = p.tw.as<float2>();
     p.desc.twh = p.twh.as<float2>();
+    int r[3];
+    if (fft3_radices(M, r)) {
+        // stage twiddles w^(rk) of stages 2 and 3, [r - 1][k], forward order then inverse
+        std::vector<float2> t3;
+        size_t inv = 0;
+        for (int dir = 0; dir < 2; ++dir) {
+            const int R1 = dir ? r[2] : r[0], R2 = r[1], R3 = dir ? r[0] : r[2];
+            if (dir) inv = t3.size();
+            for (int q = 1; q < R2; ++q)
+                for (int k = 0; k < R1; ++k) t3.push_back(tw[(size_t)k * q * R3 % M]);
+            for (int q = 1; q < R3; ++q)
+                for (int k = 0; k < R1 * R2; ++k) t3.push_back(tw[(size_t)k * q % M]);
+        }
+        CUDA_TRY(p.t3.ensure(sizeof(float2) * t3.size()));
+        CUDA_TRY(cudaMemcpy(p.t3.p, t3.data(), sizeof(float2) * t3.size(), cudaMemcpyHostToDevice));
+        p.desc.t3f = p.t3.as<float2>();
+        p.desc.t3i = p.t3.as<float2>() + inv;
+    }
     return WCT_OK;
 }
 
@@ -1059,6 +1077,8 @@ struct BatchState {
     std::vector<std::unique_ptr<DevBuf>> spec;  // [plane * ncls + cls]: taps, then wire spectra where they apply
     DevBuf d_spec_tab;                          // const float2* [plane][ncls]
     int maxM{0}, maxG{0}, nsm{148};
+    int fft3_blocks[kMaxClasses][2]{};  // persistent blocks of each class's time FFT and inverse
+    bool any_rows{false};               // some class takes the generic row transforms
     DevBuf d_Q, d_V, d_rec, d_tprof, d_win, d_wcnt, d_woff, d_wcur, d_kbound, d_wlist, d_plans;
     DevBuf d_fq, d_fluc, d_ident;  // fluctuation: drifted charges, draw sums, first frame ident of the call
     DevBuf d_pool, d_pool_off, d_pool_used;  // time profiles of long patches
@@ -1126,19 +1146,29 @@ static int batch_setup(Core& c)
     bs.tbs = (c.start_time + c.readout_time - c.start_time) / (int)(c.readout_time / c.tick);
     // ladder of time-FFT lengths from the shortest possible window up
     std::vector<int> cls;
-    const int nfirst = gpu_fft_length(std::max(64, (int)fft_best_length((size_t)4 + std::max(minpad, 0), false)));
+    // (each a length with a three-stage plan, while there is one)
+    auto class_length = [](int n) {
+        const int M = fft3_next((n + 1) / 2);
+        return M ? 2 * M : gpu_fft_length(n);
+    };
+    const int nfirst = class_length(std::max(64, (int)fft_best_length((size_t)4 + std::max(minpad, 0), false)));
     for (double ratio = 1.1;; ratio *= 1.05) {
         cls.clear();
         int N = nfirst;
         for (;;) {
             cls.push_back(N);
             if ((size_t)N >= nneed) break;
-            N = gpu_fft_length(std::max((int)std::ceil(N * ratio), N + 4));
+            N = class_length(std::max((int)std::ceil(N * ratio), N + 4));
         }
         if ((int)cls.size() <= kMaxClasses) break;
     }
     bs.ncls = (int)cls.size();
-    for (int k = 0; k < bs.ncls; ++k) bs.cls_N[k] = cls[k];
+    b.any_rows = false;
+    for (int k = 0; k < bs.ncls; ++k) {
+        bs.cls_N[k] = cls[k];
+        bs.cls_fft3[k] = fft3_batch_blocks(cls[k] / 2, b.fft3_blocks[k]) ? 1 : 0;
+        if (!bs.cls_fft3[k]) b.any_rows = true;
+    }
     b.maxM = cls.back() / 2;
     b.cls_plans.clear();
     std::vector<FftDesc> descs;
@@ -1392,8 +1422,13 @@ static int forward_batch_device(Core& c, const double* d_depos, const long long*
                                     pool, b.d_wide.as<unsigned char>(), b.d_wcnt.as<int>(), b.d_woff.as<int>(), b.d_wlist.as<Visit>(), b.vcap,
                                     b.d_kbound.as<unsigned long long>(), b.d_Q.as<float>(), nb_r, b.maxG, et, fp,
                                     b.d_fluc.as<FlucRec>(), row_flag, s);
-                launch_rfft_batch(plans + ch, b.d_descs.as<FftDesc>(), b.d_Q.as<float>(), nb_f, b.tune.fft_threads,
-                                  b.maxM, s);
+                for (int k = 0; k < bs.ncls; ++k)
+                    if (bs.cls_fft3[k])
+                        launch_rfft3_batch(plans + ch, bs, k, b.cls_plans[k]->desc, b.fft3_blocks[k][0],
+                                           b.d_Q.as<float>(), s);
+                if (b.any_rows)
+                    launch_rfft_batch(plans + ch, b.d_descs.as<FftDesc>(), b.d_Q.as<float>(), nb_f,
+                                      b.tune.fft_threads, b.maxM, s);
                 // one launch per run of planes that share the pad and the group pairing
                 // (the launches use one work counter, so they must not overlap: same stream)
                 for (int ip0 = 0; ip0 < np;) {
@@ -1413,8 +1448,13 @@ static int forward_batch_device(Core& c, const double* d_depos, const long long*
                                       b.d_spec_tab.as<const float2*>(), b.d_Q.as<float>(), b.d_V.as<float2>(), nb_c, s);
                     ip0 = ip1;
                 }
-                launch_irfft_batch(plans + ch, bs, b.d_descs.as<FftDesc>(), b.d_V.as<float2>(), d_frames + c0 * fstride,
-                                   fstride, nb_f, b.tune.fft_threads, b.maxM, row_flag, s);
+                for (int k = 0; k < bs.ncls; ++k)
+                    if (bs.cls_fft3[k])
+                        launch_irfft3_batch(plans + ch, bs, k, b.cls_plans[k]->desc, b.fft3_blocks[k][1],
+                                            b.d_V.as<float2>(), d_frames + c0 * fstride, fstride, row_flag, s);
+                if (b.any_rows)
+                    launch_irfft_batch(plans + ch, bs, b.d_descs.as<FftDesc>(), b.d_V.as<float2>(), d_frames + c0 * fstride,
+                                       fstride, nb_f, b.tune.fft_threads, b.maxM, row_flag, s);
             }
             cudaError_t ce = cudaStreamEndCapture(s, &graph);
             if (ce != cudaSuccess) {

@@ -46,6 +46,17 @@ __host__ __device__ __forceinline__ double dkey_inv(unsigned long long k)
 }
 
 #ifdef __CUDACC__
+// Whether a flagged charge wire lies within pad of wire W (all threads of the
+// block call it): rows out of every charge's reach stay exactly zero, whatever
+// rounding the convolution left in their spectra.
+__device__ __forceinline__ bool row_reached(const unsigned char* __restrict__ flag, int nwires, int W, int pad)
+{
+    int any = 0;
+    const int hi = min(nwires - 1, W + pad);
+    for (int w = max(0, W - pad) + threadIdx.x; w <= hi; w += blockDim.x) any |= flag[w];
+    return __syncthreads_or(any);
+}
+
 // Asynchronous 16-byte global -> shared copies (sm_80+ cp.async, no
 // multicast): src_bytes = 0 fills the 16 bytes with zeros and reads nothing.
 __device__ __forceinline__ void cp_async16(void* smem, const void* gmem, int src_bytes)

@@ -240,6 +240,7 @@ void launch_c2c_rows(const float2* in, long ld_in, float2* out, long ld_out, int
                      float scale, cudaStream_t s)
 {
     if (nrows <= 0) return;
+    if (launch_cfft3(in, ld_in, out, ld_out, nrows, d, sign, scale, s)) return;
     const size_t sm = 2 * sizeof(float2) * (size_t)d.M;
     if (sign < 0) {
         cudaFuncSetAttribute((const void*)k_c2c_rows<-1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);

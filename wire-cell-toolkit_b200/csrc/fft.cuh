@@ -24,6 +24,10 @@ struct FftDesc {
     int radix[kFftMaxStages];    // radix of each stage
     const float2* tw;            // [M]  exp(-2 pi i m / M)
     const float2* twh;           // [M]  exp(-2 pi i k / (2M))  (real packing)
+    // stage twiddles of the three-stage plan (fft3.cuh) in forward and inverse
+    // stage order, or null where M has none
+    const float2* t3f;
+    const float2* t3i;
 };
 
 namespace fftk {
@@ -169,6 +173,40 @@ __device__ __forceinline__ void bfly16(float2* v)
 }
 
 template <int R, int SIGN>
+__device__ __forceinline__ void bfly(float2* v);
+
+// R = A B with A, B coprime, by the prime-factor map (I. J. Good, "The
+// interaction algorithm and practical Fourier analysis", J. Roy. Statist. Soc.
+// B 20 (1958) 361-372): n = B n1 + A n2 mod R, k the residue with k = k1 mod A
+// and k = k2 mod B; no twiddles between the two.
+__host__ __device__ constexpr int crt_index(int a, int b, int k1, int k2)
+{
+    for (int k = 0; k < a * b; ++k)
+        if (k % a == k1 && k % b == k2) return k;
+    return 0;
+}
+template <int A, int B, int SIGN>
+__device__ __forceinline__ void bfly_pfa(float2* v)
+{
+    float2 t[A][B];
+#pragma unroll
+    for (int n2 = 0; n2 < B; ++n2) {
+        float2 u[A];
+#pragma unroll
+        for (int n1 = 0; n1 < A; ++n1) u[n1] = v[(B * n1 + A * n2) % (A * B)];
+        bfly<A, SIGN>(u);
+#pragma unroll
+        for (int n1 = 0; n1 < A; ++n1) t[n1][n2] = u[n1];
+    }
+#pragma unroll
+    for (int k1 = 0; k1 < A; ++k1) {
+        bfly<B, SIGN>(t[k1]);
+#pragma unroll
+        for (int k2 = 0; k2 < B; ++k2) v[crt_index(A, B, k1, k2)] = t[k1][k2];
+    }
+}
+
+template <int R, int SIGN>
 __device__ __forceinline__ void bfly(float2* v)
 {
     if constexpr (R == 2) bfly2<SIGN>(v);
@@ -177,6 +215,13 @@ __device__ __forceinline__ void bfly(float2* v)
     else if constexpr (R == 5) bfly_odd<5, SIGN>(v);
     else if constexpr (R == 7) bfly_odd<7, SIGN>(v);
     else if constexpr (R == 8) bfly8<SIGN>(v);
+    else if constexpr (R == 16) bfly16<SIGN>(v);
+    else if constexpr (R == 6) bfly_pfa<2, 3, SIGN>(v);
+    else if constexpr (R == 10) bfly_pfa<2, 5, SIGN>(v);
+    else if constexpr (R == 12) bfly_pfa<4, 3, SIGN>(v);
+    else if constexpr (R == 14) bfly_pfa<2, 7, SIGN>(v);
+    else if constexpr (R == 15) bfly_pfa<3, 5, SIGN>(v);
+    else if constexpr (R == 20) bfly_pfa<4, 5, SIGN>(v);
 }
 
 // Bank swizzle of the intermediate stage buffers (float2 index; used when M

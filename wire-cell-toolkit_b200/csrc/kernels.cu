@@ -1424,6 +1424,7 @@ void launch_rfft_rows(const float* in, long in_ld, int in_len, float2* out, long
                       cudaStream_t s)
 {
     if (nrows <= 0) return;
+    if (launch_rfft3(in, in_ld, in_len, out, out_ld, nrows, d, s)) return;
     const bool aligned = ((reinterpret_cast<uintptr_t>(in) & 7) == 0) && (in_ld % 2 == 0);
     if (aligned && d.M % 16 == 0 && d.nst >= 2 && d.radix[0] == 8 && 4 * (size_t)d.M * sizeof(float2) <= 128 * 1024) {
         if (d.M / 8 <= 256 && launch_rfft_pf<1>(in, in_ld, in_len, out, out_ld, nrows, d, s)) return;
@@ -1460,17 +1461,6 @@ __device__ __forceinline__ void irfft_row(const float2* __restrict__ v, const Ff
         if (c0 < ncols && t0 >= 0 && t0 < nticks) f[t0] = zz.x * sc;
         if (c0 + 1 < ncols && t0 + 1 >= 0 && t0 + 1 < nticks) f[t0 + 1] = zz.y * sc;
     }
-}
-
-// Whether a flagged charge wire lies within pad of wire W (all threads of the
-// block call it): rows out of every charge's reach stay exactly zero, whatever
-// rounding the convolution left in their spectra.
-__device__ __forceinline__ bool row_reached(const unsigned char* __restrict__ flag, int nwires, int W, int pad)
-{
-    int any = 0;
-    const int hi = min(nwires - 1, W + pad);
-    for (int w = max(0, W - pad) + threadIdx.x; w <= hi; w += blockDim.x) any |= flag[w];
-    return __syncthreads_or(any);
 }
 
 __global__ void k_irfft_rows(const float2* __restrict__ Vh, int nrows, FftDesc d, int wire0, int wlo, int whi,
@@ -1596,11 +1586,11 @@ void launch_irfft_rows(const float2* Vh, int nrows, const FftDesc& d, int wire0,
                        int ncols, int nticks, float* frame, cudaStream_t s, const unsigned char* row_flag, int nwires,
                        int npad)
 {
-    if (nrows <= 0) return;
+    // the rows that are frame wires: wire0 + r in [wlo, whi)
+    const int r0 = std::max(0, wlo - wire0), r1 = std::min(nrows, whi - wire0);
+    if (nrows <= 0 || r1 <= r0) return;
+    if (launch_irfft3(Vh, r0, r1, d, wire0, tick0, ncols, nticks, frame, row_flag, nwires, npad, s)) return;
     if (d.M % 16 == 0 && d.nst >= 2 && d.radix[0] == 8 && 4 * (size_t)d.M * sizeof(float2) <= 128 * 1024) {
-        // the rows that are frame wires: wire0 + r in [wlo, whi)
-        const int r0 = std::max(0, wlo - wire0), r1 = std::min(nrows, whi - wire0);
-        if (r1 <= r0) return;
         if (d.M <= 1024 && launch_irfft_pf<4>(Vh, r0, r1, d, wire0, tick0, ncols, nticks, frame, row_flag, nwires,
                                                npad, s))
             return;
@@ -2197,8 +2187,8 @@ __global__ void __launch_bounds__(256) k_plan_batch(BatchPlan* __restrict__ plan
         o.voff = (long long)e * bs.vslot_total + pl.vslot;
         plan->ep[k] = o;
         c_raster[k] = o.nin * o.ntile;
-        c_rows[k] = pl.G * o.nin;
-        c_orows[k] = o.nout;
+        c_rows[k] = bs.cls_fft3[cls] ? 0 : pl.G * o.nin;
+        c_orows[k] = bs.cls_fft3[cls] ? 0 : o.nout;
         c_conv[k] = !o.nin        ? 0
                     : pl.wire_fft ? wire_fblocks(o.M) * wire_blocks(o.nout, pl.npad)
                                   : ((o.M + 31) / 32) * ((o.nout + kConvRows - 1) / kConvRows);

@@ -146,6 +146,7 @@ struct BatchStatic {
     double start_time, tbs;   // tick binning of the window arithmetic (ImpactTransform)
     int ncls;
     int cls_N[kMaxClasses];   // ascending time-FFT lengths
+    unsigned char cls_fft3[kMaxClasses];  // the class has a three-stage plan (launches of its own)
     long long qslot_total, vslot_total;
     BatchPlaneStatic pl[kMaxPlanes];
 };
@@ -254,6 +255,27 @@ void launch_rfft_rows(const float* in, long in_ld, int in_len, float2* out, long
                       const FftDesc& d, cudaStream_t s);
 void launch_wire_conv(const float2* Qh, const float2* Rh, float2* Vh, int ngroups, int npad, int nrows_in,
                       int nrows_out, int M, bool pair, cudaStream_t s);
+// Three-stage row transforms (fft3.cu): false where the length has no plan or
+// the rows are not 16-byte aligned, and nothing was launched.  fft3_radices:
+// the plan's radices in forward order.
+bool fft3_radices(int M, int* r);
+bool launch_rfft3(const float* in, long in_ld, int in_len, float2* out, long out_ld, int nrows, const FftDesc& d,
+                  cudaStream_t s);
+bool launch_irfft3(const float2* Vh, int r0, int r1, const FftDesc& d, int wire0, int tick0, int ncols, int nticks,
+                   float* frame, const unsigned char* row_flag, int nwires, int npad, cudaStream_t s);
+bool launch_cfft3(const float2* in, long ld_in, float2* out, long ld_out, int nrows, const FftDesc& d, int sign,
+                  float scale, cudaStream_t s);
+// The smallest length >= M with a plan, 0 without one.
+int fft3_next(int M);
+// Batched rows of length class cls (d: its plan).  fft3_batch_blocks: the
+// persistent blocks of the forward and the inverse kernel on this device,
+// false where M has no plan; call it before a graph capture.
+bool fft3_batch_blocks(int M, int* blocks);
+void launch_rfft3_batch(const BatchPlan* plan, const BatchStatic& bs, int cls, const FftDesc& d, int nblocks,
+                        float* Q, cudaStream_t s);
+void launch_irfft3_batch(const BatchPlan* plan, const BatchStatic& bs, int cls, const FftDesc& d, int nblocks,
+                         const float2* V, float* frames, long long fstride, const unsigned char* row_flag,
+                         cudaStream_t s);
 // Overlap-save forms (wire_fft.cu): Rw holds wire_spec_count(G, M) values made
 // from the taps by launch_wire_spec; wire_fft_fits says whether they apply,
 // wire_fft_pays and wire_adj_fft_pays where they are the faster form.
