@@ -219,6 +219,7 @@ struct Core {
     DevBuf d_splat;            // DepoFluxSplat accumulator (doubles)
     DevBuf d_gframe, d_gdep, d_gglob;  // adjoint host entry point
     DevBuf d_fq, d_fluc;               // fluctuation: drifted charges, per (plane, depo) draw sums
+    DevBuf d_draws, d_draws_used;            // fluctuation: the cells' draws
     DevBuf d_pool, d_pool_off, d_pool_used;  // time profiles of long patches
     DevBuf d_wide;                           // per visit key: holds a long patch
     // modify_depo charge scale ([depo][plane], wct_dt_set_charge_scale); used
@@ -475,7 +476,7 @@ __global__ void k_win_init(WindowDev* w, int n)
     w[i].pmax = 0ull;
     w[i].tmax = 0ull;
     w[i].nadded = w[i].out_time = w[i].out_pitch = w[i].oversize = w[i].bigcharge = 0;
-    w[i].wide_ticks = w[i].nvisits = 0;
+    w[i].wide_ticks = w[i].nvisits = w[i].ncells = 0;
 }
 
 // Drift, patch records, per-plane windows and charge-grid layout of one event:
@@ -770,9 +771,15 @@ static int forward_device(Core& c, const double* d_depos, size_t ndepos, float* 
     if (!ev.fp.on_patch && wide > 0)
         launch_tprof_pool(c.d_rec.as<PatchRec>(), ev.et, np, (float)ev.tb.bs, pool, nullptr, s);
     if (ev.fp.on_patch) {
+        // room for every cell's draw, as counted by the prep kernel, up to kMaxDrawCells
+        const long long cells = (long long)std::min<unsigned long long>(c.h_win[0].ncells, kMaxDrawCells);
+        CUDA_TRY(c.d_draws.ensure(sizeof(int) * (size_t)std::max<long long>(cells, 1)));
+        CUDA_TRY(c.d_draws_used.ensure(sizeof(unsigned long long)));
+        CUDA_TRY(cudaMemsetAsync(c.d_draws_used.p, 0, sizeof(unsigned long long), s));
+        const DrawPool draws{c.d_draws.as<int>(), c.d_draws_used.as<unsigned long long>(), cells};
         launch_fluc_sums(c.d_rec.as<PatchRec>(), ev.et, pset, (float)ev.tb.bs, ev.fp, c.d_fq.as<double>(),
-                         c.d_fluc.as<FlucRec>(), s);
-        launch_raster_fluc(c.d_rec.as<PatchRec>(), c.d_fluc.as<FlucRec>(), ev.fp, ev.et, c.d_wcnt.as<int>(),
+                         c.d_fluc.as<FlucRec>(), draws, nullptr, s);
+        launch_raster_fluc(c.d_rec.as<PatchRec>(), c.d_fluc.as<FlucRec>(), draws.val, ev.fp, ev.et, c.d_wcnt.as<int>(),
                            c.d_woff.as<int>(), c.d_wlist.as<Visit>(), (long long)std::max(total_visits, 1), gset,
                            c.d_Q.as<float>(), row_flag, s);
     }
@@ -1082,6 +1089,8 @@ struct BatchState {
     DevBuf d_Q, d_V, d_rec, d_tprof, d_win, d_wcnt, d_woff, d_wcur, d_kbound, d_wlist, d_plans;
     DevBuf d_fq, d_fluc, d_ident;  // fluctuation: drifted charges, draw sums, first frame ident of the call
     DevBuf d_pool, d_pool_off, d_pool_used;  // time profiles of long patches
+    DevBuf d_draws, d_draws_used;            // fluctuation: the cells' draws
+    long long draws_cap{0};
     DevBuf d_wide;                           // per key: holds a long patch
     long long pool_cap{0};
     int* h_ident{nullptr};         // pinned source of d_ident
@@ -1100,7 +1109,7 @@ struct BatchState {
     DriftDev g_drift{};
     int g_fluc[2]{0, 0};
     unsigned long long g_seed{0};
-    long long g_pool_cap{0};
+    long long g_pool_cap{0}, g_draws_cap{0};
     std::vector<void*> g_bufs;
     void drop_graph()
     {
@@ -1328,7 +1337,8 @@ static int forward_batch_device(Core& c, const double* d_depos, const long long*
         const long long nkeysK = (long long)K * bs.nkeys;
         std::vector<void*> before = {b.d_Q.p, b.d_V.p, b.d_rec.p, b.d_tprof.p, b.d_win.p, b.d_wcnt.p, b.d_woff.p,
                                      b.d_wcur.p, b.d_kbound.p, b.d_wlist.p, b.d_plans.p, b.d_fq.p, b.d_fluc.p,
-                                     b.d_ident.p, b.d_pool.p, b.d_pool_off.p, b.d_pool_used.p, b.d_wide.p,
+                                     b.d_ident.p, b.d_pool.p, b.d_pool_off.p, b.d_pool_used.p, b.d_wide.p, b.d_draws.p,
+                                     b.d_draws_used.p,
                                      const_cast<double*>(c.qscale())};
         CUDA_TRY(b.d_Q.ensure(sizeof(float) * (size_t)bs.qslot_total * K));
         CUDA_TRY(b.d_V.ensure(sizeof(float2) * (size_t)bs.vslot_total * K));
@@ -1351,11 +1361,16 @@ static int forward_batch_device(Core& c, const double* d_depos, const long long*
         if (c.fluctuate) {
             CUDA_TRY(b.d_fq.ensure(sizeof(double) * (size_t)np * maxdep));
             CUDA_TRY(b.d_fluc.ensure(sizeof(FlucRec) * (size_t)np * maxdep));
+            if (b.draws_cap < 160LL * np * maxdep) b.draws_cap = 160LL * np * maxdep;  // the cells of a track depo
+            b.draws_cap = std::min(b.draws_cap, kMaxDrawCells);
+            CUDA_TRY(b.d_draws.ensure(sizeof(int) * (size_t)b.draws_cap));
+            CUDA_TRY(b.d_draws_used.ensure(sizeof(unsigned long long)));
         }
         if (!b.h_ident) CUDA_TRY(cudaMallocHost(&b.h_ident, sizeof(int)));
         std::vector<void*> after = {b.d_Q.p, b.d_V.p, b.d_rec.p, b.d_tprof.p, b.d_win.p, b.d_wcnt.p, b.d_woff.p,
                                     b.d_wcur.p, b.d_kbound.p, b.d_wlist.p, b.d_plans.p, b.d_fq.p, b.d_fluc.p,
-                                    b.d_ident.p, b.d_pool.p, b.d_pool_off.p, b.d_pool_used.p, b.d_wide.p,
+                                    b.d_ident.p, b.d_pool.p, b.d_pool_off.p, b.d_pool_used.p, b.d_wide.p, b.d_draws.p,
+                                     b.d_draws_used.p,
                                     const_cast<double*>(c.qscale())};
         if (b.h_plans_n < (size_t)nch) {
             if (b.h_plans) cudaFreeHost(b.h_plans);
@@ -1368,7 +1383,7 @@ static int forward_batch_device(Core& c, const double* d_depos, const long long*
                           std::memcmp(&b.g_tune, &b.tune, sizeof(BatchTune)) == 0 &&
                           std::memcmp(&b.g_drift, &c.drifter, sizeof(DriftDev)) == 0 &&
                           b.g_fluc[0] == (int)c.fluctuate && b.g_fluc[1] == (int)c.drift_fluctuate &&
-                          b.g_seed == c.seed && b.g_pool_cap == b.pool_cap &&
+                          b.g_seed == c.seed && b.g_pool_cap == b.pool_cap && b.g_draws_cap == b.draws_cap &&
                           b.g_offsets.size() == (size_t)nev + 1 &&
                           std::equal(b.g_offsets.begin(), b.g_offsets.end(), offsets);
         if (!same) {
@@ -1411,9 +1426,14 @@ static int forward_batch_device(Core& c, const double* d_depos, const long long*
                 cudaMemsetAsync(d_frames + c0 * fstride, 0, sizeof(float) * (size_t)(ne * fstride), s);
                 const TprofPool pool{b.d_pool.as<float>(), b.d_pool_off.as<int>(),
                                      b.d_pool_used.as<unsigned long long>(), b.pool_cap};
-                if (fp.on_patch)
+                if (fp.on_patch) {
+                    cudaMemsetAsync(b.d_draws_used.p, 0, sizeof(unsigned long long), s);
                     launch_fluc_sums(b.d_rec.as<PatchRec>(), et, pset, (float)tb.bs, fp, b.d_fq.as<double>(),
-                                     b.d_fluc.as<FlucRec>(), s);
+                                     b.d_fluc.as<FlucRec>(),
+                                     DrawPool{b.d_draws.as<int>(), b.d_draws_used.as<unsigned long long>(),
+                                              b.draws_cap},
+                                     &plans[ch].status, s);
+                }
                 else {
                     cudaMemsetAsync(b.d_pool_used.p, 0, sizeof(unsigned long long), s);
                     launch_tprof_pool(b.d_rec.as<PatchRec>(), et, np, (float)tb.bs, pool, &plans[ch].status, s);
@@ -1421,7 +1441,7 @@ static int forward_batch_device(Core& c, const double* d_depos, const long long*
                 launch_raster_batch(plans + ch, bs, pset, b.d_rec.as<PatchRec>(), et.dep0[ne], b.d_tprof.as<float>(),
                                     pool, b.d_wide.as<unsigned char>(), b.d_wcnt.as<int>(), b.d_woff.as<int>(), b.d_wlist.as<Visit>(), b.vcap,
                                     b.d_kbound.as<unsigned long long>(), b.d_Q.as<float>(), nb_r, b.maxG, et, fp,
-                                    b.d_fluc.as<FlucRec>(), row_flag, s);
+                                    b.d_fluc.as<FlucRec>(), b.d_draws.as<int>(), row_flag, s);
                 for (int k = 0; k < bs.ncls; ++k)
                     if (bs.cls_fft3[k])
                         launch_rfft3_batch(plans + ch, bs, k, b.cls_plans[k]->desc, b.fft3_blocks[k][0],
@@ -1478,6 +1498,7 @@ static int forward_batch_device(Core& c, const double* d_depos, const long long*
             b.g_fluc[1] = (int)c.drift_fluctuate;
             b.g_seed = c.seed;
             b.g_pool_cap = b.pool_cap;
+            b.g_draws_cap = b.draws_cap;
             b.g_offsets.assign(offsets, offsets + nev + 1);
         }
         *b.h_ident = c.frame_count;
@@ -1496,6 +1517,7 @@ static int forward_batch_device(Core& c, const double* d_depos, const long long*
             st |= b.h_plans[ch].status;
             need = std::max<long long>(need, b.h_plans[ch].total_visits);
         }
+        if (st & kBatchDrawsShort) b.draws_cap = std::min(2 * b.draws_cap, kMaxDrawCells);
         if (st & kBatchPoolShort) b.pool_cap *= 2;  // frames are right; the next call gets more room
         if (st & kBatchTooBig) {  // 2^31 visits in a pass: fewer events per pass
             if (K == 1) return fail(WCT_ERR_SIZE, "an event holds 2^31 or more patch visits; split it");

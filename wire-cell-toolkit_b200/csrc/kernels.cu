@@ -155,6 +155,15 @@ __device__ __forceinline__ int fluc_ident(const FlucParams& fp, int ev)
     return (fp.ident_base ? *fp.ident_base : 0) + fp.ident0 + ev;
 }
 
+// The electrons a drifting depo loses (not inlined: the sampler's registers
+// would be the prep kernel's).
+__device__ __noinline__ int drift_draw(const FlucParams& fp, int ident, int i_ev, int nq, double absorb)
+{
+    Philox g;
+    g.init(fp.key0, fp.key1 + 0x9E3779B9u * (unsigned)ident, (unsigned)i_ev, kRngDriftTag, 0u);
+    return binomial(nq, absorb, g);
+}
+
 // One thread per (depo, plane) of every event of the table (plane =
 // blockIdx.y; each plane's threads drift the depo again, which is cheaper
 // than serialising the planes' FP64 chains in one thread); per-event window
@@ -210,10 +219,7 @@ __global__ void __launch_bounds__(256, 4) k_prep_all(const double* __restrict__ 
                         const double absorb = __dsub_rn(1.0, exp(__ddiv_rn(-dt, dd.lifetime)));
                         if (fp.on_drift) {
                             // Binomial(|Q|, absorb) electrons absorbed (Drifter.cxx:179-185)
-                            Philox g;
-                            g.init(fp.key0, fp.key1 + 0x9E3779B9u * (unsigned)fluc_ident(fp, ev),
-                                   (unsigned)(i - evt.dep0[ev]), kRngDriftTag, 0u);
-                            const int nabs = binomial((int)fabs(q), absorb, g);
+                            const int nabs = drift_draw(fp, fluc_ident(fp, ev), i - evt.dep0[ev], (int)fabs(q), absorb);
                             q = __dsub_rn(q, q < 0 ? -(double)nabs : (double)nabs);
                         }
                         else q = __dsub_rn(q, __dmul_rn(q, absorb));
@@ -267,7 +273,7 @@ __global__ void __launch_bounds__(256, 4) k_prep_all(const double* __restrict__ 
     auto umin = [](unsigned long long a, unsigned long long b) { return a < b ? a : b; };
     auto umax = [](unsigned long long a, unsigned long long b) { return a > b ? a : b; };
     auto iadd = [](int a, int b) { return a + b; };
-    unsigned long long myvis = 0;
+    unsigned long long myvis = 0, mycells = 0;
     {
         const PlaneDev& pl = ps.p[ip];
         unsigned long long kpmin = ~0ull, kpmax = 0ull, ktmin = ~0ull, ktmax = 0ull;
@@ -352,6 +358,7 @@ __global__ void __launch_bounds__(256, 4) k_prep_all(const double* __restrict__ 
         const int kspan = r.np ? (r.toff + r.nt - 1) / kTile - k0 + 1 : 0;
         count_visits(wire_cnt, pl.wire_base, w0, span, k0, kspan, ps.ntiles);
         myvis += (unsigned long long)span * (unsigned long long)kspan;
+        if (fp.on_patch) mycells += (unsigned long long)r.np * (unsigned long long)r.nt;
         if (r.nt > kTprof) {  // keys that hold a long patch: their raster block spreads visits over warps
             unsigned char* wk = wide_all + (size_t)ev * nkeys;
             for (int ww = 0; ww < span; ++ww)
@@ -423,6 +430,11 @@ __global__ void __launch_bounds__(256, 4) k_prep_all(const double* __restrict__ 
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) myvis += __shfl_xor_sync(0xffffffffu, myvis, o);
     if (l == 0 && myvis) atomicAdd(&win[0].nvisits, myvis);
+    if (fp.on_patch) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) mycells += __shfl_xor_sync(0xffffffffu, mycells, o);
+        if (l == 0 && mycells) atomicAdd(&win[0].ncells, mycells);
+    }
 }
 
 void launch_prep_all(const double* depos, const EventTable& et, int nkeys, const DriftDev& dd, int do_drift,
@@ -966,62 +978,255 @@ __device__ __forceinline__ int cell_draw(const FlucParams& fp, int ident, int i_
     return binomial(nq, (double)relval, g);
 }
 
+// The draws of every patch's cells, stored for the raster, and their sums: one
+// warp per (plane, four depos).
+//
+// What bounds it: the arithmetic of the draws.  Cells of a patch differ in the
+// sampler they need (inversion below a mean of 10, BTRS above) and in how far
+// it goes, so a warp that drew its cells in order had 9 of 32 lanes at work, in
+// double precision, and the raster drew all of them a second time (3.3 + 5.1 ms
+// for 100k depos on three planes, 40 M cells).  Here cells are sorted into
+// small queues of the warp -- inversion, BTRS squeeze, BTRS full test -- and a
+// queue is worked off when it holds a whole warp's worth; four patches share
+// the queues, so that few are worked off part full, and the lanes of one pass
+// over their bin integrals.  The transcendentals are in single precision where
+// that decides the draw (rng.cuh).  Now 1.9 ms, and 1.1 ms of raster.
 constexpr int kFlucWarps = 4;
-constexpr int kFlucTab = 1024;  // patches hold at most kMaxPatchT ticks and kMaxPatchP bins
+constexpr int kFlucSlots = 4;      // depos of a warp
+constexpr int kFlucTab = 2048;     // bin integrals of a warp (one patch: at most kMaxPatchP + kMaxPatchT)
+constexpr int kFlucQueue = 64;     // a queue holds at most 31 cells when another 32 come
+constexpr unsigned kNoCell = 0xffffffffu;
+static_assert(kFlucTab >= kMaxPatchP + kMaxPatchT, "one patch fits the tables");
 
-// One warp per (plane, depo): the sum of the cell draws.
-__global__ void __launch_bounds__(kFlucWarps * 32) k_fluc_sums(const PatchRec* __restrict__ rec, EventTable evt,
-                                                               PlaneSet ps, float tbs, FlucParams fp,
-                                                               const double* __restrict__ fq,
-                                                               FlucRec* __restrict__ fluc)
+struct FlucSlot {
+    float invS;
+    int nq, nt, i_ev;
+    unsigned key1;
+    int pbase, tbase;  // its pitch and time integrals in the table
+    int* store;        // its draws, or null
+};
+
+__global__ void __launch_bounds__(kFlucWarps * 32, 6) k_fluc_sums(const PatchRec* __restrict__ rec, EventTable evt,
+                                                                  PlaneSet ps, float tbs, FlucParams fp,
+                                                                  const double* __restrict__ fq,
+                                                                  FlucRec* __restrict__ fluc, DrawPool draws,
+                                                                  int* status)
 {
-    __shared__ float s_p[kFlucWarps][kFlucTab], s_t[kFlucWarps][kFlucTab];
+    __shared__ float s_tab[kFlucWarps][kFlucTab];
+    __shared__ unsigned s_q[kFlucWarps][3][kFlucQueue];
+    __shared__ FlucSlot s_slot[kFlucWarps][kFlucSlots];
+    const unsigned full = 0xffffffffu;
     const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int n = evt.dep0[evt.nev];
+    const int n = evt.dep0[evt.nev], groups = (n + kFlucSlots - 1) / kFlucSlots;
     const long long gw = (long long)blockIdx.x * kFlucWarps + wib;
-    if (gw >= (long long)n * ps.nplanes) return;  // whole warps only; no block barrier follows
-    const int ip = (int)(gw / n), i = (int)(gw - (long long)ip * n);
-    const PatchRec r = rec[(size_t)ip * n + i];
-    FlucRec out{0, 0.f, 0.f, 0};
-    if (r.np > 0 && r.nt > 0) {
-        const float pbs = (float)ps.p[ip].imp_bs;
-        const int np = r.np, nt = r.nt;
-        for (int k = lane; k < np; k += 32) s_p[wib][k] = unit_bin(k, pbs, r.pcr, r.sp);
-        for (int t = lane; t < nt; t += 32) s_t[wib][t] = unit_bin(t, tbs, r.tcr, r.st);
+    if (gw >= (long long)groups * ps.nplanes) return;  // whole warps only; no block barrier follows
+    const int ip = (int)(gw / groups), i0 = (int)(gw - (long long)ip * groups) * kFlucSlots;
+    const float pbs = (float)ps.p[ip].imp_bs;
+    float* const tab = s_tab[wib];
+    FlucSlot* const slot = s_slot[wib];
+    // lanes 0 .. 3 own a depo each: its record, room for its draws, its normalisation
+    const int mine = i0 + lane;
+    const bool own = lane < kFlucSlots && mine < n;
+    PatchRec r{};
+    FlucRec out{0, 0.f, 0.f, -1};
+    double Q = 0.0;
+    int i_ev = 0;
+    unsigned key1 = 0;
+    if (own) {
+        r = rec[(size_t)ip * n + mine];
+        if (r.np > 0 && r.nt > 0) {
+            const long long off = (long long)atomicAdd(draws.used, (unsigned long long)r.np * r.nt);
+            if (off + (long long)r.np * r.nt <= draws.cap) out.off = (int)off;
+            else if (status) atomicOr(status, kBatchDrawsShort);
+            out.invS = patch_inv_norm(r, pbs, tbs);
+            Q = fq[(size_t)ip * n + mine];
+            out.nq = (int)fabs(Q);
+            const int ev = event_of_depo(evt, mine);
+            i_ev = mine - evt.dep0[ev];
+            key1 = fp.key1 + 0x9E3779B9u * (unsigned)fluc_ident(fp, ev);
+        }
+        else
+            r.np = r.nt = 0;
+    }
+    const int size = own ? r.np + r.nt : 0;
+    const unsigned key0 = fp.key0;
+    long long sum_mine = 0;
+    for (int s0 = 0; s0 < kFlucSlots;) {
+        // as many of the slots s0 .. s1-1 as the table holds (one always fits)
+        int s1 = s0, used = 0, pre[kFlucSlots + 1], cells[kFlucSlots + 1], pbase = 0;
+        pre[0] = cells[0] = 0;
+#pragma unroll
+        for (int s = 0; s < kFlucSlots; ++s) {
+            const int sz = __shfl_sync(full, size, s), nc = __shfl_sync(full, (int)r.np * (int)r.nt, s);
+            const bool take = s >= s0 && s == s1 && used + sz <= kFlucTab;
+            if (take) {
+                if (lane == s) pbase = used;
+                used += sz;
+                ++s1;
+            }
+            pre[s + 1] = used;
+            cells[s + 1] = cells[s] + (take ? nc : 0);
+        }
         __syncwarp();
-        const float invS = patch_inv_norm(r, pbs, tbs);
-        const double Q = fq[(size_t)ip * n + i];
-        const int nq = (int)fabs(Q);
-        const int ev = event_of_depo(evt, i);
-        const int ident = fluc_ident(fp, ev), i_ev = i - evt.dep0[ev];
-        long long sum = 0;
-        for (int c = lane; c < np * nt; c += 32) {
-            const int k = c / nt, t = c - k * nt;
-            const float relval = __fmul_rn(__fmul_rn(s_p[wib][k], s_t[wib][t]), invS);
-            sum += cell_draw(fp, ident, i_ev, ip, c, nq, relval);
+        if (lane >= s0 && lane < s1 && own)
+            slot[lane] = FlucSlot{out.invS, out.nq, r.nt, i_ev, key1, pbase, pbase + r.np,
+                                  out.off >= 0 ? draws.val + out.off : nullptr};
+        // unit bin integrals of all the taken patches, over the lanes
+        for (int b0 = 0; b0 < used; b0 += 32) {
+            const int b = b0 + lane;
+            int s = s0;
+#pragma unroll
+            for (int q = 0; q + 1 < kFlucSlots; ++q)
+                if (q >= s0 && q + 1 < s1 && b >= pre[q + 1]) s = q + 1;
+            const int np = __shfl_sync(full, (int)r.np, s);
+            const float pcr = __shfl_sync(full, r.pcr, s), sp = __shfl_sync(full, r.sp, s);
+            const float tcr = __shfl_sync(full, r.tcr, s), st = __shfl_sync(full, r.st, s);
+            int first = 0;
+#pragma unroll
+            for (int q = 0; q < kFlucSlots; ++q)
+                if (q == s) first = pre[q];
+            if (b < used) {
+                const int k = b - first;
+                tab[b] = k < np ? unit_bin(k, pbs, pcr, sp) : unit_bin(k - np, tbs, tcr, st);
+            }
+        }
+        __syncwarp();
+        // a cell: slot, bin and tick in one word
+        long long sum[kFlucSlots] = {0, 0, 0, 0};
+        int cnt[3] = {0, 0, 0};
+        auto rel_of = [&](unsigned e) {
+            const FlucSlot& S = slot[e >> 30];
+            return __fmul_rn(__fmul_rn(tab[S.pbase + ((e >> 15) & 0x7fffu)], tab[S.tbase + (e & 0x7fffu)]), S.invS);
+        };
+        auto cell_of = [&](unsigned e) { return ((e >> 15) & 0x7fffu) * slot[e >> 30].nt + (e & 0x7fffu); };
+        auto put = [&](unsigned e, int N) {
+#pragma unroll
+            for (int s = 0; s < kFlucSlots; ++s)
+                if ((int)(e >> 30) == s) sum[s] += N;
+            int* const st = slot[e >> 30].store;
+            if (st) st[cell_of(e)] = N;
+        };
+        auto block_of = [&](unsigned e, unsigned at) {
+            const FlucSlot& S = slot[e >> 30];
+            return philox_block(key0, S.key1, (unsigned)S.i_ev, (unsigned)ip, cell_of(e), at);
+        };
+        auto again = [&](unsigned e) {  // the double-precision draw
+            const FlucSlot& S = slot[e >> 30];
+            Philox g;
+            g.init(key0, S.key1, (unsigned)S.i_ev, (unsigned)ip, cell_of(e));
+            return binomial_double(S.nq, (double)rel_of(e), g);
+        };
+        auto push = [&](int q, bool on, unsigned e) {
+            const unsigned m = __ballot_sync(full, on);
+            if (on) s_q[wib][q][cnt[q] + __popc(m & ((1u << lane) - 1u))] = e;
+            cnt[q] += __popc(m);
+            __syncwarp();
+        };
+        // the last m cells of queue q, one a lane
+        auto pop = [&](int q, int m, unsigned& e) {
+            cnt[q] -= m;
+            const bool on = lane < m;
+            e = on ? s_q[wib][q][cnt[q] + lane] : 0u;
+            __syncwarp();
+            return on;
+        };
+        const int ncell = cells[kFlucSlots];
+        for (int c0 = 0; c0 < ncell; c0 += 32) {
+            const int c = c0 + lane;
+            int kind = -1;  // 0 inversion, 1 BTRS, 2 the full test's queue; -1 settled here
+            unsigned e = 0;
+            if (c < ncell) {
+                int s = s0, first = 0;
+#pragma unroll
+                for (int q = 0; q < kFlucSlots; ++q)
+                    if (q >= s0 && q < s1 && c >= cells[q]) s = q, first = cells[q];
+                const int nt = slot[s].nt, nq = slot[s].nq;
+                // bin = c / nt: (c - first + 1/2) / nt is 1/(2 nt) or more from an integer
+                const int k = (int)(((float)(c - first) + 0.5f) * __fdividef(1.0f, (float)nt));
+                e = ((unsigned)s << 30) | ((unsigned)k << 15) | (unsigned)(c - first - k * nt);
+                const float rel = rel_of(e);
+                if (nq <= 0 || !(rel > 0.f)) put(e, 0);
+                else if (rel >= 1.f) put(e, nq);
+                else if (rel > 0.5f) kind = 2;
+                else kind = (double)nq * (double)rel < 10.0 ? 0 : 1;
+            }
+            __syncwarp();
+            push(0, kind == 0, e);
+            push(1, kind == 1, e);
+            push(2, kind == 2, e);
+            // work off the full queues, every queue after the last cells (each
+            // sampler stands here once: its code is what fills the instruction cache)
+            const int least = c0 + 32 >= ncell ? 1 : 32;
+            for (;;) {
+                unsigned x, doubt = kNoCell;  // doubt: a cell for the double-precision draw
+                int N;
+                if (cnt[1] >= least && cnt[2] < 32) {
+                    const bool on = pop(1, min(32, cnt[1]), x);
+                    N = 0;
+                    if (on) {
+                        const uint4 o = block_of(x, 0u);
+                        N = draw_btrs<true>(slot[x >> 30].nq, (double)rel_of(x), uniform53(o.x, o.y) - 0.5,
+                                            (float)uniform53(o.z, o.w));
+                        if (N >= 0) put(x, N);
+                    }
+                    push(2, on && N < 0, x);  // open, out of range or in doubt
+                }
+                else if (cnt[2] >= least) {
+                    if (pop(2, min(32, cnt[2]), x)) {
+                        const double p = (double)rel_of(x);
+                        N = p <= 0.5 && (double)slot[x >> 30].nq * p >= 10.0 ? kDrawReject : kDrawDoubt;
+                        for (unsigned at = 0; at < 8 && N == kDrawReject; ++at) {
+                            const uint4 o = block_of(x, at);
+                            N = draw_btrs<false>(slot[x >> 30].nq, p, uniform53(o.x, o.y) - 0.5,
+                                                 (float)uniform53(o.z, o.w));
+                        }
+                        if (N >= 0) put(x, N);
+                        else doubt = x;
+                    }
+                }
+                else if (cnt[0] >= least) {
+                    if (pop(0, min(32, cnt[0]), x)) {
+                        const uint4 o = block_of(x, 0u);
+                        N = draw_inversion(slot[x >> 30].nq, rel_of(x), (float)uniform53(o.x, o.y));
+                        if (N >= 0) put(x, N);
+                        else doubt = x;
+                    }
+                }
+                else
+                    break;
+                if (doubt != kNoCell) put(doubt, again(doubt));  // rare
+                __syncwarp();
+            }
         }
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-        out.nq = nq;
-        out.invS = invS;
-        out.scale = sum > 0 ? (float)(Q / (double)sum) : 0.f;
+        for (int s = 0; s < kFlucSlots; ++s) {
+            if (s < s0 || s >= s1) continue;
+            long long t = sum[s];
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(full, t, o);
+            if (lane == s) sum_mine = t;
+        }
+        s0 = s1;
     }
-    if (lane == 0) fluc[(size_t)ip * n + i] = out;
+    if (own) {
+        out.scale = sum_mine > 0 ? (float)(Q / (double)sum_mine) : 0.f;
+        fluc[(size_t)ip * n + mine] = out;
+    }
 }
 
 void launch_fluc_sums(const PatchRec* rec, const EventTable& et, const PlaneSet& ps, float tbs, const FlucParams& fp,
-                      const double* fq, FlucRec* fluc, cudaStream_t s)
+                      const double* fq, FlucRec* fluc, const DrawPool& draws, int* status, cudaStream_t s)
 {
-    const long long warps = (long long)et.dep0[et.nev] * ps.nplanes;
+    const long long warps = (long long)((et.dep0[et.nev] + kFlucSlots - 1) / kFlucSlots) * ps.nplanes;
     if (warps <= 0) return;
     const long long blocks = (warps + kFlucWarps - 1) / kFlucWarps;
-    k_fluc_sums<<<(unsigned)blocks, kFlucWarps * 32, 0, s>>>(rec, et, ps, tbs, fp, fq, fluc);
+    k_fluc_sums<<<(unsigned)blocks, kFlucWarps * 32, 0, s>>>(rec, et, ps, tbs, fp, fq, fluc, draws, status);
 }
 
 // Fluctuated raster of one (charge row, tick tile) item: one warp per visit,
-// lanes over the visit's ticks in the tile, a loop over the patch bins of the
-// row's wire; cell charges N * Q / sum N split between the two impact groups
-// of the bin by its linear weight (BinnedDiffusion_transform.cxx:296-367).
+// its stored draws spread over the lanes (8, 16 or 32 ticks of a bin side by
+// side); cell charges N * Q / sum N split between the two impact groups of the
+// bin by its linear weight (BinnedDiffusion_transform.cxx:296-367).
 // Accumulation in 64-bit fixed point (2^-16 electron), so the grid does not
 // depend on the order of the adds.
 constexpr int kFlucRasterThreads = 256;
@@ -1029,17 +1234,24 @@ constexpr float kFlucFix = 65536.0f;
 
 size_t raster_fluc_smem_bytes(int G) { return sizeof(long long) * (size_t)G * kTileLd; }
 
+// A cell of a patch whose draws were not stored: the same draw again.
+__device__ __noinline__ int redraw_cell(const FlucParams& fp, int ident, int i_ev, int ip, const PatchRec& r,
+                                        const FlucRec& fr, int k, int t, float pbs, float tbs)
+{
+    const float relval = __fmul_rn(__fmul_rn(unit_bin(k, pbs, r.pcr, r.sp), unit_bin(t, tbs, r.tcr, r.st)), fr.invS);
+    return cell_draw(fp, ident, i_ev, ip, k * r.nt + t, fr.nq, relval);
+}
+
 __device__ __forceinline__ void raster_tile_fluc(const GridPlane& P, int ip, int row, int ktile, int key_base,
                                                  int ntiles_abs, const EventTable& evt, const FlucParams& fp,
                                                  const PatchRec* __restrict__ rec, const FlucRec* __restrict__ fluc,
-                                                 const int* __restrict__ wire_cnt, const int* __restrict__ wire_off,
-                                                 const Visit* __restrict__ visits, long long vcap,
-                                                 float* __restrict__ Q, unsigned char* __restrict__ row_flag,
-                                                 long long* grid)
+                                                 const int* __restrict__ draws, const int* __restrict__ wire_cnt,
+                                                 const int* __restrict__ wire_off, const Visit* __restrict__ visits,
+                                                 long long vcap, float* __restrict__ Q,
+                                                 unsigned char* __restrict__ row_flag, long long* grid)
 {
     __syncthreads();  // the previous item of a persistent block is done with the grid
-    __shared__ float s_p[kFlucRasterThreads / 32][16], s_w[kFlucRasterThreads / 32][16];
-    __shared__ float s_tv[kFlucRasterThreads / 32][kTile];  // unit time bins of the current visit
+    __shared__ float s_w[kFlucRasterThreads / 32][16];
     const int w = P.start_ch + row;
     const int G = P.G, nimp = P.nimp;
     const int tick_lo = ktile * kTile;
@@ -1053,7 +1265,15 @@ __device__ __forceinline__ void raster_tile_fluc(const GridPlane& P, int ip, int
         cnt = off < 0 ? 0 : (int)min((long long)wire_cnt[key], max(0ll, vcap - off));
         list = visits + max(off, 0);
     }
-    if (tid == 0 && cnt > 0) row_flag[P.wire_base + w] = 1;
+    const int qc0 = tick_lo - P.col0;
+    if (cnt == 0) {  // no visit (block-uniform): the tile's G rows are zero
+        for (int k = tid; k < G * kTile; k += blockDim.x) {
+            const int g = k / kTile, qc = qc0 + k - g * kTile;
+            if (qc >= 0 && qc < P.N) Q[P.qoff + ((size_t)g * P.nin + row) * P.N + qc] = 0.f;
+        }
+        return;
+    }
+    if (tid == 0) row_flag[P.wire_base + w] = 1;
     for (int k = tid; k < G * kTileLd; k += blockDim.x) grid[k] = 0;
     __syncthreads();
     const float pbs = P.pbs, tbs = P.tbs, inv_pbs = 1.0f / pbs;
@@ -1069,9 +1289,9 @@ __device__ __forceinline__ void raster_tile_fluc(const GridPlane& P, int ip, int
         const int k0 = wlo + l_lo - r.poff;  // first patch bin on this wire
         if (lane < nb) {
             const int k = k0 + lane;
-            const float p = unit_bin(k, pbs, r.pcr, r.sp);
             float wt;
             if (r.sp > 0.f) {
+                const float p = unit_bin(k, pbs, r.pcr, r.sp);
                 const float isg = __frcp_rn(r.sp);
                 const float x1 = (float)k * pbs - r.pcr, x2 = (float)(k + 1) * pbs - r.pcr;
                 const float g1 = __expf(-0.5f * (x1 * isg) * (x1 * isg)), g2 = __expf(-0.5f * (x2 * isg) * (x2 * isg));
@@ -1079,38 +1299,42 @@ __device__ __forceinline__ void raster_tile_fluc(const GridPlane& P, int ip, int
                 wt = p > 0.f ? fmaf(c0 * (g2 - g1), __frcp_rn(p), x2 * inv_pbs) : 0.f;
             }
             else wt = (pbs - r.pcr) * inv_pbs;
-            s_p[wid][lane] = p;
             s_w[wid][lane] = wt;
         }
         __syncwarp();
-        const int ev = event_of_depo(evt, d);
-        const int ident = fluc_ident(fp, ev), i_ev = d - evt.dep0[ev];
         const int cb = r.toff - tick_lo;
         const int tstart = max(0, -cb), tend = min(rnt, kTile - cb);
         const int ntt = tend - tstart;
-        if (ntt <= 0) continue;  // warp-uniform
-        for (int t = lane; t < ntt; t += 32) s_tv[wid][t] = unit_bin(tstart + t, tbs, r.tcr, r.st);
-        __syncwarp();
-        // cells (bin b, tick t) of the visit in this tile, spread over the lanes
-        for (int cell = lane; cell < nb * ntt; cell += 32) {
-            const int b = cell / ntt, tt = cell - b * ntt;
-            const int t = tstart + tt;
-            const int k = k0 + b;
-            const float relval = __fmul_rn(__fmul_rn(s_p[wid][b], s_tv[wid][tt]), fr.invS);
-            const int N = cell_draw(fp, ident, i_ev, ip, k * rnt + t, fr.nq, relval);
-            if (N) {
-                const float c = (float)N * fr.scale;
-                const float a = c * s_w[wid][b];
-                long long* dst = grid + (size_t)(l_lo + b) * kTileLd + cb + t;
-                atomicAdd(reinterpret_cast<unsigned long long*>(dst), (unsigned long long)__float2ll_rn(a * kFlucFix));
-                atomicAdd(reinterpret_cast<unsigned long long*>(dst + kTileLd),
-                          (unsigned long long)__float2ll_rn((c - a) * kFlucFix));
+        if (ntt > 0) {  // warp-uniform
+            int ident = 0, i_ev = 0;
+            if (fr.off < 0) {
+                const int ev = event_of_depo(evt, d);
+                ident = fluc_ident(fp, ev);
+                i_ev = d - evt.dep0[ev];
+            }
+            const int lg = ntt <= 8 ? 3 : (ntt <= 16 ? 4 : 5);  // ticks side by side: 8, 16 or 32
+            const int sub = lane >> lg, tl = lane & ((1 << lg) - 1), nsub = 32 >> lg;
+            for (int b = sub; b < nb; b += nsub) {
+                const float wb = s_w[wid][b];
+                for (int tt = tl; tt < ntt; tt += 32) {
+                    const int t = tstart + tt, k = k0 + b;
+                    const int N = fr.off >= 0 ? __ldg(draws + fr.off + k * rnt + t)
+                                              : redraw_cell(fp, ident, i_ev, ip, r, fr, k, t, pbs, tbs);
+                    if (N) {
+                        const float c = (float)N * fr.scale;
+                        const float a = c * wb;
+                        long long* dst = grid + (size_t)(l_lo + b) * kTileLd + cb + t;
+                        atomicAdd(reinterpret_cast<unsigned long long*>(dst),
+                                  (unsigned long long)__float2ll_rn(a * kFlucFix));
+                        atomicAdd(reinterpret_cast<unsigned long long*>(dst + kTileLd),
+                                  (unsigned long long)__float2ll_rn((c - a) * kFlucFix));
+                    }
+                }
             }
         }
         __syncwarp();
     }
     __syncthreads();
-    const int qc0 = tick_lo - P.col0;
     for (int k = tid; k < G * kTile; k += blockDim.x) {
         const int g = k / kTile, c = k - g * kTile;
         const int qc = qc0 + c;
@@ -1121,8 +1345,9 @@ __device__ __forceinline__ void raster_tile_fluc(const GridPlane& P, int ip, int
     }
 }
 
-__global__ void __launch_bounds__(kFlucRasterThreads) k_raster_fluc(const PatchRec* __restrict__ rec,
-                                                                    const FlucRec* __restrict__ fluc, FlucParams fp,
+__global__ void __launch_bounds__(kFlucRasterThreads, 4) k_raster_fluc(const PatchRec* __restrict__ rec,
+                                                                    const FlucRec* __restrict__ fluc,
+                                                                    const int* __restrict__ draws, FlucParams fp,
                                                                     EventTable evt,
                                                                     const int* __restrict__ wire_cnt,
                                                                     const int* __restrict__ wire_off,
@@ -1137,11 +1362,12 @@ __global__ void __launch_bounds__(kFlucRasterThreads) k_raster_fluc(const PatchR
     const int rel = blockIdx.x - P.row_base;
     const int row = rel / P.ntile;
     const int ktile = P.ktile0 + (rel - row * P.ntile);
-    raster_tile_fluc(P, ip, row, ktile, 0, gs.ntiles_abs, evt, fp, rec, fluc, wire_cnt, wire_off, visits, vcap, Q,
+    raster_tile_fluc(P, ip, row, ktile, 0, gs.ntiles_abs, evt, fp, rec, fluc, draws, wire_cnt, wire_off, visits, vcap, Q,
                      row_flag, grid64);
 }
 
-void launch_raster_fluc(const PatchRec* rec, const FlucRec* fluc, const FlucParams& fp, const EventTable& evt,
+void launch_raster_fluc(const PatchRec* rec, const FlucRec* fluc, const int* draws, const FlucParams& fp,
+                        const EventTable& evt,
                         const int* wire_cnt, const int* wire_off, const Visit* visits, long long vcap,
                         const GridSet& gs, float* Q, unsigned char* row_flag, cudaStream_t s)
 {
@@ -1149,7 +1375,7 @@ void launch_raster_fluc(const PatchRec* rec, const FlucRec* fluc, const FlucPara
     size_t smem = 0;
     for (int i = 0; i < gs.nplanes; ++i) smem = std::max(smem, raster_fluc_smem_bytes(gs.p[i].G));
     cudaFuncSetAttribute((const void*)k_raster_fluc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k_raster_fluc<<<gs.nrows_total, kFlucRasterThreads, smem, s>>>(rec, fluc, fp, evt, wire_cnt, wire_off, visits,
+    k_raster_fluc<<<gs.nrows_total, kFlucRasterThreads, smem, s>>>(rec, fluc, draws, fp, evt, wire_cnt, wire_off, visits,
                                                                      vcap, gs, Q, row_flag);
 }
 
@@ -2259,7 +2485,7 @@ __device__ __forceinline__ int find_entry(const int* __restrict__ pre, int n, in
 }
 
 template <bool FLUC>
-__global__ void __launch_bounds__(kRasterThreads, FLUC ? 1 : 5) k_raster_batch(const BatchPlan* __restrict__ plan, BatchStatic bs,
+__global__ void __launch_bounds__(kRasterThreads, FLUC ? 4 : 5) k_raster_batch(const BatchPlan* __restrict__ plan, BatchStatic bs,
                                                                  PlaneSet ps, const PatchRec* __restrict__ rec,
                                                                  long long recstride,
                                                                  const float* __restrict__ tprof, TprofPool pool,
@@ -2270,6 +2496,7 @@ __global__ void __launch_bounds__(kRasterThreads, FLUC ? 1 : 5) k_raster_batch(c
                                                                  const unsigned long long* __restrict__ key_bound,
                                                                  float* __restrict__ Q, EventTable evt, FlucParams fp,
                                                                  const FlucRec* __restrict__ fluc,
+                                                                 const int* __restrict__ draws,
                                                                  unsigned char* __restrict__ row_flag)
 {
     extern __shared__ int smem_i[];
@@ -2304,7 +2531,7 @@ __global__ void __launch_bounds__(kRasterThreads, FLUC ? 1 : 5) k_raster_batch(c
         const int row = rel / E.ntile;
         if constexpr (FLUC)
             raster_tile_fluc(P, ip, row, E.ktile0 + (rel - row * E.ntile), e * bs.nkeys, bs.ntiles, evt, fp, rec,
-                             fluc, wire_cnt, wire_off, visits, vcap, Q, row_flag + (size_t)e * bs.nwires_total,
+                             fluc, draws, wire_cnt, wire_off, visits, vcap, Q, row_flag + (size_t)e * bs.nwires_total,
                              reinterpret_cast<long long*>(smem_i));
         else
             raster_tile(P, row, E.ktile0 + (rel - row * E.ntile), e * bs.nkeys, bs.ntiles, rec, tprof, pool,
@@ -2318,19 +2545,19 @@ void launch_raster_batch(const BatchPlan* plan, const BatchStatic& bs, const Pla
                          const unsigned char* wide_key, const int* wire_cnt, const int* wire_off,
                          const Visit* visits, long long vcap, const unsigned long long* key_bound, float* Q,
                          int nblocks, int maxG, const EventTable& evt, const FlucParams& fp, const FlucRec* fluc,
-                         unsigned char* row_flag, cudaStream_t s)
+                         const int* draws, unsigned char* row_flag, cudaStream_t s)
 {
     const size_t smem = std::max(raster_smem_bytes(maxG), raster_fluc_smem_bytes(maxG));
     if (fp.on_patch)
         k_raster_batch<true><<<nblocks, kRasterThreads, smem, s>>>(plan, bs, ps, rec, recstride, tprof, pool, wide_key,
                                                                     wire_cnt,
                                                                     wire_off, visits, vcap, key_bound, Q, evt, fp,
-                                                                    fluc, row_flag);
+                                                                    fluc, draws, row_flag);
     else
         k_raster_batch<false><<<nblocks, kRasterThreads, smem, s>>>(plan, bs, ps, rec, recstride, tprof, pool,
                                                                      wide_key, wire_cnt,
                                                                      wire_off, visits, vcap, key_bound, Q, evt, fp,
-                                                                     fluc, row_flag);
+                                                                     fluc, draws, row_flag);
 }
 
 // Time FFT of every charge-grid row of the pass, in place (rows of N reals

@@ -68,6 +68,7 @@ struct WindowDev {
     // (plane 0 entry of an event only) 64-bit totals of the event: ticks of
     // its patches longer than kTprof, and raster visits of all its patches
     unsigned long long wide_ticks, nvisits;
+    unsigned long long ncells;  // (plane 0 entry) patch cells of the event, counted when patches fluctuate
     int nadded, out_time, out_pitch, oversize;
     int bigcharge;  // patches whose raster bound exceeds kMaxVisitBound
 };
@@ -183,6 +184,7 @@ constexpr int kBatchOversize = 2;
 constexpr int kBatchBigCharge = 4;
 constexpr int kBatchNoClass = 8;
 constexpr int kBatchPoolShort = 16;  // not an error: some time profiles were computed in the raster
+constexpr int kBatchDrawsShort = 64;  // not an error: some fluctuated patches were drawn twice
 constexpr int kBatchTooBig = 32;     // a pass holds 2^31 or more visits: fewer events per pass
 constexpr int kBatchSkip = kBatchVisitOverflow | kBatchTooBig;  // the raster and later stages skip the pass
 
@@ -211,8 +213,17 @@ struct FlucRec {
     int nq;          // (int)|Q|, the binomial trial count of every cell
     float scale;     // Q / (sum of the cell draws), 0 when every draw is 0
     float invS;      // 1 / (sum of unit bin integrals in pitch * in time)
-    int pad;
+    int off;         // the patch's draws in the DrawPool (cell k * nt + t), -1: not stored
 };
+
+// The draws of the pass, written by k_fluc_sums and read by the raster.  A
+// patch that finds no room is drawn again there: the same numbers.
+struct DrawPool {
+    int* val;
+    unsigned long long* used;  // allocation counter (64-bit: no wrap)
+    long long cap;             // cells, at most kMaxDrawCells
+};
+constexpr long long kMaxDrawCells = 1LL << 28;  // 1 GB
 
 // Time profiles of patches longer than kTprof ticks, computed once per depo
 // (the raster would otherwise recompute them on every wire it visits).
@@ -236,8 +247,9 @@ void launch_prep_all(const double* depos, const EventTable& et, int nkeys, const
 void launch_binomial_samples(unsigned long long seed, int ident, int n, double p, long long count, int* out,
                              cudaStream_t s);
 void launch_fluc_sums(const PatchRec* rec, const EventTable& et, const PlaneSet& ps, float tbs, const FlucParams& fp,
-                      const double* fq, FlucRec* fluc, cudaStream_t s);
-void launch_raster_fluc(const PatchRec* rec, const FlucRec* fluc, const FlucParams& fp, const EventTable& evt,
+                      const double* fq, FlucRec* fluc, const DrawPool& draws, int* status, cudaStream_t s);
+void launch_raster_fluc(const PatchRec* rec, const FlucRec* fluc, const int* draws, const FlucParams& fp,
+                        const EventTable& evt,
                         const int* wire_cnt, const int* wire_off, const Visit* visits, long long vcap,
                         const GridSet& gs, float* Q, unsigned char* row_flag, cudaStream_t s);
 void launch_scan(const int* wire_cnt, int nwires_total, int* wire_off, int* wire_cur, cudaStream_t s);
@@ -372,7 +384,7 @@ void launch_raster_batch(const BatchPlan* plan, const BatchStatic& bs, const Pla
                          const unsigned char* wide_key, const int* wire_cnt, const int* wire_off,
                          const Visit* visits, long long vcap, const unsigned long long* key_bound, float* Q,
                          int nblocks, int maxG, const EventTable& evt, const FlucParams& fp, const FlucRec* fluc,
-                         unsigned char* row_flag, cudaStream_t s);  // row_flag: [event][wire]
+                         const int* draws, unsigned char* row_flag, cudaStream_t s);  // row_flag: [event][wire]
 void launch_rfft_batch(const BatchPlan* plan, const FftDesc* descs, float* Q, int nblocks, int nthreads, int maxM,
                        cudaStream_t s);
 // Wire convolution of planes [ip0, ip1) (all with the same pad and pairing) in one launch.

@@ -24,56 +24,61 @@
 
 namespace wctb200 {
 
-struct Philox {
-    uint32_t c[4];
-    uint32_t k[2];
-    uint32_t out[4];
-    int used;  // 64-bit words taken from out (0..2)
-
-    __device__ __forceinline__ void block()
-    {
-        uint32_t x0 = c[0], x1 = c[1], x2 = c[2], x3 = c[3];
-        uint32_t k0 = k[0], k1 = k[1];
+// One block of Philox-4x32-10.
+__device__ __forceinline__ uint4 philox_block(uint32_t k0, uint32_t k1, uint32_t x0, uint32_t x1, uint32_t x2,
+                                              uint32_t x3)
+{
 #pragma unroll
-        for (int r = 0; r < 10; ++r) {
-            const uint32_t lo0 = 0xD2511F53u * x0, hi0 = __umulhi(0xD2511F53u, x0);
-            const uint32_t lo1 = 0xCD9E8D57u * x2, hi1 = __umulhi(0xCD9E8D57u, x2);
-            const uint32_t y0 = hi1 ^ x1 ^ k0, y2 = hi0 ^ x3 ^ k1;
-            x0 = y0;
-            x1 = lo1;
-            x2 = y2;
-            x3 = lo0;
-            k0 += 0x9E3779B9u;
-            k1 += 0xBB67AE85u;
-        }
-        out[0] = x0;
-        out[1] = x1;
-        out[2] = x2;
-        out[3] = x3;
-        ++c[3];  // the last counter word numbers the blocks of one stream
-        used = 0;
+    for (int r = 0; r < 10; ++r) {
+        const uint32_t lo0 = 0xD2511F53u * x0, hi0 = __umulhi(0xD2511F53u, x0);
+        const uint32_t lo1 = 0xCD9E8D57u * x2, hi1 = __umulhi(0xCD9E8D57u, x2);
+        const uint32_t y0 = hi1 ^ x1 ^ k0, y2 = hi0 ^ x3 ^ k1;
+        x0 = y0;
+        x1 = lo1;
+        x2 = y2;
+        x3 = lo0;
+        k0 += 0x9E3779B9u;
+        k1 += 0xBB67AE85u;
     }
+    return make_uint4(x0, x1, x2, x3);
+}
 
-    // Stream (key0, key1) x (ctr0, ctr1, ctr2); the fourth counter word counts blocks.
+// Uniform double in the open interval (0, 1), 53 random bits.
+__device__ __forceinline__ double uniform53(uint32_t hi, uint32_t lo)
+{
+    const uint64_t x = (((uint64_t)hi << 32) | lo) >> 11;
+    return ((double)x + 0.5) * 1.1102230246251565404e-16;  // 2^-53
+}
+
+// The uniforms of the stream (key0, key1) x (ctr0, ctr1, ctr2) in order, two a
+// block; the fourth counter word numbers the blocks.
+struct Philox {
+    uint32_t k0, k1, c0, c1, c2, c3;
+    uint32_t hi, lo;  // the block's second pair, while have is set
+    bool have;
+
     __device__ __forceinline__ void init(uint32_t key0, uint32_t key1, uint32_t ctr0, uint32_t ctr1, uint32_t ctr2)
     {
-        k[0] = key0;
-        k[1] = key1;
-        c[0] = ctr0;
-        c[1] = ctr1;
-        c[2] = ctr2;
-        c[3] = 0;
-        used = 2;
+        k0 = key0;
+        k1 = key1;
+        c0 = ctr0;
+        c1 = ctr1;
+        c2 = ctr2;
+        c3 = 0;
+        have = false;
     }
 
-    // Uniform double in the open interval (0, 1), 53 random bits.
     __device__ __forceinline__ double uniform()
     {
-        if (used == 2) block();
-        const uint64_t hi = out[2 * used], lo = out[2 * used + 1];
-        ++used;
-        const uint64_t x = ((hi << 32) | lo) >> 11;
-        return ((double)x + 0.5) * 1.1102230246251565404e-16;  // 2^-53
+        if (have) {
+            have = false;
+            return uniform53(hi, lo);
+        }
+        const uint4 o = philox_block(k0, k1, c0, c1, c2, c3++);
+        hi = o.z;
+        lo = o.w;
+        have = true;
+        return uniform53(o.x, o.y);
     }
 };
 
@@ -146,13 +151,115 @@ __device__ __forceinline__ int binomial_low(int n, double p, Philox& g)
     return m;  // not reached in practice (acceptance probability per try is above 0.5)
 }
 
-// Binomial(n, p); p >= 1 gives n (GaussianDiffusion.cxx:196-198), p <= 0 gives 0.
-__device__ __forceinline__ int binomial(int n, double p, Philox& g)
+// Binomial(n, p) in double precision throughout, drawing from the stream g.
+static __device__ __noinline__ int binomial_double(int n, double p, Philox g)
+{
+    if (p <= 0.5) return binomial_low(n, p, g);
+    return n - binomial_low(n, 1.0 - p, g);
+}
+
+// log x! correction of stirling_fc in single precision.
+__device__ __forceinline__ float stirling_fcf(int x)
+{
+    if (x < 10) {
+        const float t[10] = {0.08106147f,  0.04134070f,  0.02767793f,  0.02079067f,  0.01664469f,
+                             0.01387613f,  0.01189671f,  0.01041127f,  0.009255462f, 0.008330563f};
+        return t[x];
+    }
+    const float r = __fdividef(1.0f, (float)x + 1.0f), r2 = r * r;
+    return r * (0.083333333f - r2 * (0.0027777778f - r2 * 0.00079365079f));
+}
+
+// The draws of binomial_low for 0 < p <= 1/2 with the transcendentals in
+// single precision: the same uniforms, and every comparison that decides the
+// draw is answered "in doubt" when its two sides are closer than a bound on the
+// single-precision error; the caller then runs the double-precision draw.  So
+// the result, where there is one, is the double-precision draw.
+constexpr int kDrawDoubt = -1;    // take the double-precision draw
+constexpr int kDrawReject = -2;   // BTRS: next attempt
+constexpr int kDrawOpen = -3;     // BTRS: the squeeze did not decide
+
+// Inversion, n p < 10.  The cumulated probabilities are below 1; each of at
+// most about 30 terms is known to (|n log(1-p)| + 4 x) 3e-7 of itself and a
+// sum of them to 1e-5 (margin 2e-5).
+__device__ __forceinline__ int draw_inversion(int n, float p, float u)
+{
+    const float s = __fdividef(p, 1.0f - p);
+    float f = expf((float)n * log1pf(-p));
+    float c = f, left = (float)n;
+    for (int x = 0;; ++x) {
+        if (fabsf(u - c) < 2e-5f) return kDrawDoubt;
+        if (u < c || x == n) return x;
+        f *= s * __fdividef(left, (float)(x + 1));
+        left -= 1.0f;
+        c += f;
+    }
+}
+
+// BTRS, n p >= 10: one attempt with the uniforms u (less one half) and v.  The
+// proposal k = floor(y) needs y to 5e-7 of its distance from the mode; the
+// acceptance ratio's logarithms are taken as log1p of (m - k) / (k + 1) and the
+// like, differences that do not cancel, good to 3e-7 (|k - m| + 20).
+template <bool SQUEEZE_ONLY>
+__device__ __forceinline__ int draw_btrs(int n, double p, double u, float v)
+{
+    const double np = (double)n * p;
+    const float pf = (float)p, qf = 1.0f - pf;
+    const float spq = sqrtf((float)np * qf);
+    const float b = 1.15f + 2.53f * spq;
+    const float a = -0.0873f + 0.0248f * b + 0.01f * pf;
+    const float ib = __fdividef(1.0f, b);
+    const float us = (float)(0.5 - fabs(u));
+    const double dy = (double)(__fdividef(2.0f * a, us) + b) * u;
+    const double y = dy + (np + 0.5), yk = floor(y);
+    const float frac = (float)(y - yk), tol = 2e-6f * (1.0f + fabsf((float)dy));
+    if (frac < tol || frac > 1.0f - tol) return kDrawDoubt;
+    if (!(yk >= 0.0 && yk <= (double)n)) return kDrawReject;
+    const int k = (int)yk;
+    if (fabsf(us - 0.07f) < 1e-6f) return kDrawDoubt;
+    if (us > 0.07f) {
+        const float vr = 0.92f - 4.2f * ib;
+        if (fabsf(v - vr) < 1e-5f) return kDrawDoubt;
+        if (v < vr) return k;
+    }
+    if (SQUEEZE_ONLY) return kDrawOpen;
+    const int m = (int)floor((double)(n + 1) * p);
+    const float alpha = (2.83f + 5.1f * ib) * spq;
+    const float lv = logf(__fdividef(v * alpha, __fdividef(a, us * us) + b));
+    const float dk = (float)(k - m), k1 = (float)k + 1.0f, nk1 = (float)(n - k) + 1.0f;
+    const float lr = ((float)m + 0.5f) * log1pf(__fdividef(-dk, k1)) +
+                     ((float)(n - m) + 0.5f) * log1pf(__fdividef(dk, nk1)) +
+                     dk * logf(__fdividef(nk1, k1) * __fdividef(pf, qf)) + (stirling_fcf(m) - stirling_fcf(k)) +
+                     (stirling_fcf(n - m) - stirling_fcf(n - k));
+    if (!(fabsf(lv - lr) > 4e-5f + 3e-6f * fabsf(dk))) return kDrawDoubt;
+    return lv < lr ? k : kDrawReject;
+}
+
+// binomial_low's draw from the stream g, or kDrawDoubt.
+__device__ __forceinline__ int binomial_low_single(int n, double p, Philox& g)
+{
+    if ((double)n * p < 10.0) return draw_inversion(n, (float)p, (float)g.uniform());
+    for (int attempt = 0; attempt < 8; ++attempt) {
+        const double u = g.uniform() - 0.5;
+        const float v = (float)g.uniform();
+        const int k = draw_btrs<false>(n, p, u, v);
+        if (k != kDrawReject) return k;
+    }
+    return kDrawDoubt;
+}
+
+// Binomial(n, p) from the stream g, just initialised; p >= 1 gives n
+// (GaussianDiffusion.cxx:196-198), p <= 0 gives 0.
+__device__ __forceinline__ int binomial(int n, double p, const Philox& g)
 {
     if (n <= 0 || !(p > 0.0)) return 0;
     if (p >= 1.0) return n;
-    if (p <= 0.5) return binomial_low(n, p, g);
-    return n - binomial_low(n, 1.0 - p, g);
+    int k = kDrawDoubt;
+    if (p <= 0.5) {
+        Philox h = g;
+        k = binomial_low_single(n, p, h);
+    }
+    return k >= 0 ? k : binomial_double(n, p, g);
 }
 
 // Counter-stream tags (first counter word's top bits are the plane, the
