@@ -150,9 +150,18 @@ void launch_wire_conv_adj(const float2* Gh, const float2* Rh, float2* dQh, int G
 
 // ---------------------------------------------------------------------------
 // Per depo: gather the patch cells of dL/dQ on every plane and form the
-// gradients.  One warp per depo; the patch is tabulated in shared memory in
-// chunks (impact bins x ticks) and the chunk's cells are spread over the 32
-// lanes, so every lane is busy whatever the patch shape.
+// gradients.  One warp per depo; the patch's rows are tabulated in shared
+// memory in chunks of impact bins, then each lane takes a tick (8 or 16 ticks
+// and several rows side by side for short patches) and walks down the rows.
+//
+// What bounds it: the reads of dL/dQ, one value a cell, mostly from L2.  Two
+// bins of a wire share the impact group between them, so the bins' factors
+// are summed per group row first (as the raster does): a cell costs one load
+// and three multiply-adds, and the tick factors enter once a lane at the end.
+// Cells spread over the lanes, with both groups loaded and five sums a cell,
+// took 5.1 ms for 500k depos (half in showers of 100 ticks x 30 impacts, three
+// planes); this takes 3.7 ms, at half the issue slots and 20 warps an SM (96
+// registers; 72 spill and take 4.8 ms).
 //
 // With x_k = edge_k - c (c the pitch centre, k = 0..np), u_k = x_k / s,
 // phi the unit normal density and bs the impact bin size:
@@ -165,19 +174,21 @@ void launch_wire_conv_adj(const float2* Gh, const float2* Rh, float2* dQh, int G
 // and the same bin integrals and derivatives in time.  The patch adds
 // qn t_tau a_k to group l and qn t_tau (p_k - a_k) to group l + 1 of its wire,
 // qn = q / (sum_k p_k * sum_tau t_tau) (sums over the clipped patch).  Every
-// accumulated quantity is a sum over cells (k, tau) of a bin factor times a
-// tick factor times dL/dQ, e.g. dL/dqn = sum tv_tau (a_k D0 + (p_k - a_k) D1).
+// accumulated quantity is a sum over rows and ticks of a row factor times a
+// tick factor times dL/dQ, e.g. dL/dqn = sum_tau tv_tau sum_rows A_row D, with
+// A_row = a_k + (p_{k-1} - a_{k-1}) for the row that bins k - 1 and k share.
 // ---------------------------------------------------------------------------
 constexpr int kGatherWarps = 4;
 constexpr int kChunkP = 128;  // impact bins per table chunk
 constexpr int kChunkT = 128;  // ticks per table chunk
-constexpr int kUnroll = 4;    // cells per lane with loads in flight together
+constexpr int kChunkRows = kChunkP + kChunkP / 2 + 2;  // + one row a wire (at least two impacts each)
 
-struct __align__(16) BinTab {
-    float a, p, dadc, dpdc;
-    float dads, dpds;
-    int base;  // offset of (group l, charge row) of this bin in the plane grid, plus the patch's first column
-    int pad;
+// One impact-group row of a patch chunk: the sums of the bin factors of
+// dL/dqn, dL/dc and dL/dsigma, and where the row's first tick lies in the
+// plane's grid.
+struct __align__(16) RowTab {
+    float a, dc, ds;
+    int base;
 };
 
 __device__ __forceinline__ double warp_sum_d(double v)
@@ -185,6 +196,14 @@ __device__ __forceinline__ double warp_sum_d(double v)
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
+}
+
+// s += v, the rounding error added to e (D. E. Knuth's two-sum).
+__device__ __forceinline__ void add_carried(float& s, float& e, float v)
+{
+    const float t = __fadd_rn(s, v), b = __fsub_rn(t, s);
+    e += __fadd_rn(__fsub_rn(s, __fsub_rn(t, b)), __fsub_rn(v, b));
+    s = t;
 }
 
 // Quantities of one bin edge at distance x from the centre (sigma s > 0,
@@ -212,7 +231,7 @@ __global__ void __launch_bounds__(kGatherWarps * 32, 5) k_adj_gather(int n, Plan
                                                                      double* __restrict__ grad,
                                                                      const double* __restrict__ qscale)
 {
-    __shared__ BinTab s_p[kGatherWarps][kChunkP];
+    __shared__ RowTab s_r[kGatherWarps][kChunkRows];
     __shared__ float4 s_t[kGatherWarps][kChunkT];
     const unsigned full = 0xffffffffu;
     const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -221,6 +240,9 @@ __global__ void __launch_bounds__(kGatherWarps * 32, 5) k_adj_gather(int n, Plan
     // per-depo sums over planes: dL/dt', dL/dq', dL/dsL, dL/dsT, dL/d(x', y, z) through the pitch
     double s_ct = 0.0, s_qf = 0.0, s_sL = 0.0, s_sT = 0.0, s_px = 0.0, s_py = 0.0, s_pz = 0.0;
     bool any = false;
+    // the tick table and its sums are the same on every plane unless the patch is cut differently
+    int t_nt = -1;
+    float t_cr = 0.f, t_st = 0.f, tS = 0.f, tSc = 0.f, tSs = 0.f;
     for (int ip = 0; ip < ps.nplanes; ++ip) {
         const PatchRec r = rec[(size_t)ip * n + i];
         const AdjPlane& A = as.p[ip];
@@ -232,15 +254,23 @@ __global__ void __launch_bounds__(kGatherWarps * 32, 5) k_adj_gather(int n, Plan
         const float isp = sp > 0.f ? 1.0f / sp : 0.f, invp = 0.70710678118654752f * isp;
         const float ist = st > 0.f ? 1.0f / st : 0.f, invt = 0.70710678118654752f * ist;
         // lane partial sums of the bin integrals and their derivatives (normalisation)
-        float pS = 0.f, pSc = 0.f, pSs = 0.f, tS = 0.f, tSc = 0.f, tSs = 0.f;
+        float pS = 0.f, pSc = 0.f, pSs = 0.f;
         double acc_qn = 0.0, acc_cp = 0.0, acc_sp = 0.0, acc_ct = 0.0, acc_st = 0.0;
-        const size_t gstride = (size_t)A.nin * A.N;
         const float* dQp = dQ + A.qoff;
         const int col = r.toff - A.col0;
+        const bool have_t = nt <= kChunkT && t_nt == nt && t_cr == r.tcr && t_st == st;
+        if (!have_t) {
+            tS = tSc = tSs = 0.f;
+            t_nt = nt;
+            t_cr = r.tcr;
+            t_st = st;
+        }
         for (int t0 = 0; t0 < nt; t0 += kChunkT) {
             const int ntc = min(kChunkT, nt - t0);
             __syncwarp();
-            if (st > 0.f) {
+            if (have_t) {
+            }
+            else if (st > 0.f) {
                 // one edge per lane, bins from neighbouring lanes (31 bins per round)
                 for (int tb = t0; tb < t0 + ntc; tb += 31) {
                     const int e = tb + lane;
@@ -266,90 +296,94 @@ __global__ void __launch_bounds__(kGatherWarps * 32, 5) k_adj_gather(int n, Plan
             }
             for (int k0 = 0; k0 < np; k0 += kChunkP) {
                 const int nk = min(kChunkP, np - k0);
+                const int wire0 = (r.poff + k0) / A.nimp;
+                int nrows = 0;
                 __syncwarp();
-                for (int kb = k0; kb < k0 + nk; kb += 31) {
-                    const int e = kb + lane;
+                // 30 bins a round: lane 0 holds the bin before (its upper share goes to this round's first row)
+                for (int kb = k0 - 1; kb < k0 + nk - 1; kb += 30) {
+                    const int e = kb + lane;  // lanes 0 .. 30: bins kb .. kb + 30; lane 31: the last one's upper edge
                     float E = 0.f, f = 0.f, uf = 0.f, uuf = 0.f;
-                    if (sp > 0.f && e <= np) edge_terms((float)e * pbs - r.pcr, isp, invp, E, f, uf, uuf);
+                    if (sp > 0.f && e >= 0 && e <= np) edge_terms((float)e * pbs - r.pcr, isp, invp, E, f, uf, uuf);
                     const float E2 = __shfl_down_sync(full, E, 1), f2 = __shfl_down_sync(full, f, 1);
                     const float uf2 = __shfl_down_sync(full, uf, 1), uuf2 = __shfl_down_sync(full, uuf, 1);
-                    if (lane < 31 && e < k0 + nk) {
-                        BinTab b;
+                    float bp = 0.f, ba = 0.f, dpdc = 0.f, dpds = 0.f, dadc = 0.f, dads = 0.f;
+                    const bool real = lane < 31 && e >= k0 && e < k0 + nk;
+                    if (real) {
                         if (sp > 0.f) {
                             const float x2 = (float)(e + 1) * pbs - r.pcr;
-                            b.p = bin_from_edges(E, E2);
-                            b.dpdc = -(f2 - f) * isp;
-                            b.dpds = -(uf2 - uf) * isp;
-                            b.a = fmaf(sp, f2 - f, x2 * b.p) * ipbs;
-                            b.dadc = (((uf2 - uf) - b.p) + x2 * b.dpdc) * ipbs;
-                            b.dads = (((f2 - f) + (uuf2 - uuf)) + x2 * b.dpds) * ipbs;
+                            bp = bin_from_edges(E, E2);
+                            dpdc = -(f2 - f) * isp;
+                            dpds = -(uf2 - uf) * isp;
+                            ba = fmaf(sp, f2 - f, x2 * bp) * ipbs;
+                            dadc = (((uf2 - uf) - bp) + x2 * dpdc) * ipbs;
+                            dads = (((f2 - f) + (uuf2 - uuf)) + x2 * dpds) * ipbs;
                         }
                         else {  // point in pitch: one bin, weight (edge_{k+1} - c) / bs
-                            b.p = 1.f;
-                            b.a = (pbs - r.pcr) * ipbs;
-                            b.dpdc = b.dpds = b.dads = 0.f;
-                            b.dadc = -ipbs;
+                            bp = 1.f;
+                            ba = (pbs - r.pcr) * ipbs;
+                            dadc = -ipbs;
                         }
+                    }
+                    // what the bin below leaves for this bin's lower row
+                    const float ub = bp - ba, ubc = dpdc - dadc, ubs = dpds - dads;
+                    const float lb = __shfl_up_sync(full, ub, 1), lbc = __shfl_up_sync(full, ubc, 1);
+                    const float lbs = __shfl_up_sync(full, ubs, 1);
+                    if (real && lane > 0) {
                         const int kabs = r.poff + e;
                         const int wire = kabs / A.nimp;
                         const int l = kabs - wire * A.nimp;
-                        b.base = (l * A.nin + (wire - A.start_ch)) * A.N + col + t0;
-                        b.pad = 0;
-                        s_p[wib][e - k0] = b;
+                        const bool below = l > 0 && e > k0;  // bin e - 1 shares the row
+                        const int row = e - k0 + (wire - wire0);
+                        const int base = (l * A.nin + (wire - A.start_ch)) * A.N + col + t0;
+                        s_r[wib][row] = RowTab{below ? ba + lb : ba, below ? dadc + lbc : dadc,
+                                               below ? dads + lbs : dads, base};
+                        if (l == A.nimp - 1 || e == k0 + nk - 1)  // the wire's (or the chunk's) last row
+                            s_r[wib][row + 1] = RowTab{ub, ubc, ubs, base + A.nin * A.N};
                         if (t0 == 0) {
-                            pS += b.p;
-                            pSc += b.dpdc;
-                            pSs += b.dpds;
+                            pS += bp;
+                            pSc += dpdc;
+                            pSs += dpds;
                         }
                     }
                 }
+                nrows = nk + (r.poff + k0 + nk - 1) / A.nimp - wire0 + 1;
                 __syncwarp();
-                // cells c = lane + 32 m of the nk x ntc chunk, (k, tau) advanced
-                // incrementally; kUnroll cells per lane have their loads in flight at once
-                const int ncell = nk * ntc;
-                const int dk = 32 / ntc, dt = 32 - dk * ntc;
-                int k = lane / ntc, tau = lane - k * ntc;
-                for (int c0 = 0; c0 < ncell; c0 += 32 * kUnroll) {
-                    float D0[kUnroll], D1[kUnroll];
-                    int kk[kUnroll], tt[kUnroll];
+                const int lg = ntc <= 8 ? 3 : (ntc <= 16 ? 4 : 5);  // ticks side by side: 8, 16 or 32
+                const int sub = lane >> lg, tl = lane & ((1 << lg) - 1), nsub = 32 >> lg;
+                for (int tc = 0; tc < ntc; tc += 32) {
+                    const int tau = tc + tl;
+                    if (tau >= ntc) continue;
+                    const float* q = dQp + tau;
+                    // eight rows a step, their loads in flight together; the steps' sums are
+                    // added with their rounding errors carried along
+                    float U = 0.f, Vc = 0.f, Vs = 0.f, Ue = 0.f, Vce = 0.f, Vse = 0.f;
+                    for (int row = sub; row < nrows; row += 8 * nsub) {
+                        float u[2] = {0.f, 0.f}, vc[2] = {0.f, 0.f}, vs[2] = {0.f, 0.f}, D[8];
 #pragma unroll
-                    for (int u = 0; u < kUnroll; ++u) {
-                        kk[u] = min(k, nk - 1);
-                        tt[u] = tau;
-                        D0[u] = D1[u] = 0.f;
-                        if (c0 + lane + 32 * u < ncell) {
-                            const float* q = dQp + s_p[wib][k].base + tau;
-                            D0[u] = __ldg(q);
-                            D1[u] = __ldg(q + gstride);
+                        for (int m = 0; m < 8; ++m) {
+                            const int rm = row + m * nsub;
+                            D[m] = rm < nrows ? __ldg(q + s_r[wib][rm].base) : 0.f;
                         }
-                        tau += dt;
-                        k += dk;
-                        if (tau >= ntc) {
-                            tau -= ntc;
-                            ++k;
-                        }
-                    }
-                    // cells past the end loaded zeros and add nothing
-                    float pq = 0.f, pc = 0.f, pss = 0.f, pct = 0.f, pst = 0.f;
 #pragma unroll
-                    for (int u = 0; u < kUnroll; ++u) {
-                        const BinTab b = s_p[wib][kk[u]];
-                        const float4 tq = s_t[wib][tt[u]];
-                        const float dd0 = D0[u] - D1[u];
-                        const float uu = fmaf(b.a, dd0, b.p * D1[u]);
-                        const float vc = fmaf(b.dadc, dd0, b.dpdc * D1[u]);
-                        const float vs = fmaf(b.dads, dd0, b.dpds * D1[u]);
-                        pq = fmaf(tq.x, uu, pq);
-                        pc = fmaf(tq.x, vc, pc);
-                        pss = fmaf(tq.x, vs, pss);
-                        pct = fmaf(tq.y, uu, pct);
-                        pst = fmaf(tq.z, uu, pst);
+                        for (int m = 0; m < 8; ++m) {
+                            const RowTab R = s_r[wib][min(row + m * nsub, nrows - 1)];
+                            u[m & 1] = fmaf(R.a, D[m], u[m & 1]);
+                            vc[m & 1] = fmaf(R.dc, D[m], vc[m & 1]);
+                            vs[m & 1] = fmaf(R.ds, D[m], vs[m & 1]);
+                        }
+                        add_carried(U, Ue, u[0] + u[1]);
+                        add_carried(Vc, Vce, vc[0] + vc[1]);
+                        add_carried(Vs, Vse, vs[0] + vs[1]);
                     }
-                    acc_qn += (double)pq;
-                    acc_cp += (double)pc;
-                    acc_sp += (double)pss;
-                    acc_ct += (double)pct;
-                    acc_st += (double)pst;
+                    U += Ue;
+                    Vc += Vce;
+                    Vs += Vse;
+                    const float4 tq = s_t[wib][tau];
+                    acc_qn += (double)(tq.x * U);
+                    acc_cp += (double)(tq.x * Vc);
+                    acc_sp += (double)(tq.x * Vs);
+                    acc_ct += (double)(tq.y * U);
+                    acc_st += (double)(tq.z * U);
                 }
             }
         }
