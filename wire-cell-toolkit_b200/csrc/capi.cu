@@ -220,6 +220,7 @@ struct Core {
     DevBuf d_gframe, d_gdep, d_gglob;  // adjoint host entry point
     DevBuf d_fq, d_fluc;               // fluctuation: drifted charges, per (plane, depo) draw sums
     DevBuf d_draws, d_draws_used;            // fluctuation: the cells' draws
+    DevBuf d_heavy;                          // the raster's heavy tiles
     DevBuf d_pool, d_pool_off, d_pool_used;  // time profiles of long patches
     DevBuf d_wide;                           // per visit key: holds a long patch
     // modify_depo charge scale ([depo][plane], wct_dt_set_charge_scale); used
@@ -508,6 +509,10 @@ static FlucParams fluc_params(const Core& c, bool fluct, int ident0, const int* 
     return fp;
 }
 
+// The d_wide buffer: a byte per key, one per wire, then two counters.
+static size_t wide_counters(size_t nkeys, size_t nwires) { return (nkeys + nwires + 15) & ~(size_t)15; }
+static size_t wide_bytes(size_t nkeys, size_t nwires) { return wide_counters(nkeys, nwires) + 2 * sizeof(int); }
+
 // h_depos (optional): the depos in host memory, uploaded into d_depos here
 // in chunks on the copy stream, each chunk's prep blocks launched as soon as
 // it has arrived.
@@ -564,8 +569,9 @@ static int prepare_event(Core& c, const double* d_depos, size_t ndepos, cudaStre
     Core::StageTimer t_prep(&c, 0, s);
     CUDA_TRY(cudaMemsetAsync(c.d_wcnt.p, 0, sizeof(int) * (nkeys + 1), s));
     CUDA_TRY(c.d_kbound.ensure(sizeof(unsigned long long) * (size_t)nkeys * kTileBlocks));
-    CUDA_TRY(c.d_wide.ensure((size_t)nkeys + nwt));  // and, behind the keys, a flag per wire (set by the raster)
-    CUDA_TRY(cudaMemsetAsync(c.d_wide.p, 0, (size_t)nkeys + nwt, s));
+    // behind the keys: a flag per wire (set by the raster), the heavy-tile counters
+    CUDA_TRY(c.d_wide.ensure(wide_bytes(nkeys, nwt)));
+    CUDA_TRY(cudaMemsetAsync(c.d_wide.p, 0, wide_bytes(nkeys, nwt), s));
     CUDA_TRY(cudaMemsetAsync(c.d_kbound.p, 0, sizeof(unsigned long long) * (size_t)nkeys * kTileBlocks, s));
     k_win_init<<<1, 64, 0, s>>>(c.d_win.as<WindowDev>(), np);
     EventTable& et = ev.et;
@@ -765,6 +771,18 @@ static int forward_device(Core& c, const double* d_depos, size_t ndepos, float* 
                          wide};
 
     unsigned char* row_flag = c.d_wide.as<unsigned char>() + ev.nkeys;
+    HeavyList heavy{};
+    int heavy_blocks = 0;
+    if (!ev.fp.on_patch && (wide > 0 || total_visits > 2 * kHeavyPart)) {
+        const size_t parts = heavy_items(total_visits, ev.nkeys);
+        CUDA_TRY(c.d_heavy.ensure(sizeof(int4) * parts + sizeof(int) * (size_t)ev.nkeys));
+        int nsm = 0;
+        CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c.device));
+        heavy_blocks = kHeavyBlocks * nsm;
+        heavy.count = reinterpret_cast<int*>(c.d_wide.as<char>() + wide_counters(ev.nkeys, pset.nwires_total));
+        heavy.item = c.d_heavy.as<int4>();
+        heavy.done = reinterpret_cast<int*>(heavy.item + parts);
+    }
     Core::StageTimer t_r(&c, 1, s);
     launch_fill(c.d_rec.as<PatchRec>(), ev.et, ev.nkeys, pset, c.d_wcur.as<int>(), c.d_wlist.as<Visit>(),
                 (long long)std::max(total_visits, 1), s);
@@ -787,7 +805,7 @@ static int forward_device(Core& c, const double* d_depos, size_t ndepos, float* 
         launch_raster_wires(c.d_rec.as<PatchRec>(), c.d_tprof.as<float>(), pool, c.d_wide.as<unsigned char>(),
                             c.d_wcnt.as<int>(),
                             c.d_woff.as<int>(), c.d_wlist.as<Visit>(), (long long)std::max(total_visits, 1),
-                            c.d_kbound.as<unsigned long long>(), gset, c.d_Q.as<float>(), row_flag, s);
+                            c.d_kbound.as<unsigned long long>(), gset, c.d_Q.as<float>(), row_flag, heavy, heavy_blocks, s);
     t_r.close((n > 0 ? 1 : 0) + (ev.fp.on_patch && n > 0 ? 1 : 0) + (!ev.fp.on_patch && wide > 0 ? 1 : 0) +
               (rows > 0 ? 1 : 0));
     CUDA_TRY(cudaGetLastError());
@@ -1090,6 +1108,7 @@ struct BatchState {
     DevBuf d_fq, d_fluc, d_ident;  // fluctuation: drifted charges, draw sums, first frame ident of the call
     DevBuf d_pool, d_pool_off, d_pool_used;  // time profiles of long patches
     DevBuf d_draws, d_draws_used;            // fluctuation: the cells' draws
+    DevBuf d_heavy;                          // the raster's heavy tiles
     long long draws_cap{0};
     DevBuf d_wide;                           // per key: holds a long patch
     long long pool_cap{0};
@@ -1338,7 +1357,7 @@ static int forward_batch_device(Core& c, const double* d_depos, const long long*
         std::vector<void*> before = {b.d_Q.p, b.d_V.p, b.d_rec.p, b.d_tprof.p, b.d_win.p, b.d_wcnt.p, b.d_woff.p,
                                      b.d_wcur.p, b.d_kbound.p, b.d_wlist.p, b.d_plans.p, b.d_fq.p, b.d_fluc.p,
                                      b.d_ident.p, b.d_pool.p, b.d_pool_off.p, b.d_pool_used.p, b.d_wide.p, b.d_draws.p,
-                                     b.d_draws_used.p,
+                                     b.d_draws_used.p, b.d_heavy.p,
                                      const_cast<double*>(c.qscale())};
         CUDA_TRY(b.d_Q.ensure(sizeof(float) * (size_t)bs.qslot_total * K));
         CUDA_TRY(b.d_V.ensure(sizeof(float2) * (size_t)bs.vslot_total * K));
@@ -1349,7 +1368,9 @@ static int forward_batch_device(Core& c, const double* d_depos, const long long*
         CUDA_TRY(b.d_woff.ensure(sizeof(int) * (size_t)(nkeysK + 1)));
         CUDA_TRY(b.d_wcur.ensure(sizeof(int) * (size_t)(nkeysK + 1 + (nkeysK + 1023) / 1024)));
         CUDA_TRY(b.d_kbound.ensure(sizeof(unsigned long long) * (size_t)nkeysK * kTileBlocks));
-        CUDA_TRY(b.d_wide.ensure((size_t)nkeysK + (size_t)K * bs.nwires_total));  // keys, then wire flags
+        CUDA_TRY(b.d_wide.ensure(wide_bytes((size_t)nkeysK, (size_t)K * bs.nwires_total)));
+        const size_t parts = heavy_items(b.vcap, nkeysK);
+        CUDA_TRY(b.d_heavy.ensure(sizeof(int4) * parts + sizeof(int) * (size_t)nkeysK));
         CUDA_TRY(b.d_wlist.ensure(sizeof(Visit) * (size_t)b.vcap));
         CUDA_TRY(b.d_plans.ensure(sizeof(BatchPlan) * (size_t)nch));
         CUDA_TRY(b.d_ident.ensure(sizeof(int)));
@@ -1370,7 +1391,7 @@ static int forward_batch_device(Core& c, const double* d_depos, const long long*
         std::vector<void*> after = {b.d_Q.p, b.d_V.p, b.d_rec.p, b.d_tprof.p, b.d_win.p, b.d_wcnt.p, b.d_woff.p,
                                     b.d_wcur.p, b.d_kbound.p, b.d_wlist.p, b.d_plans.p, b.d_fq.p, b.d_fluc.p,
                                     b.d_ident.p, b.d_pool.p, b.d_pool_off.p, b.d_pool_used.p, b.d_wide.p, b.d_draws.p,
-                                     b.d_draws_used.p,
+                                     b.d_draws_used.p, b.d_heavy.p,
                                     const_cast<double*>(c.qscale())};
         if (b.h_plans_n < (size_t)nch) {
             if (b.h_plans) cudaFreeHost(b.h_plans);
@@ -1408,7 +1429,11 @@ static int forward_batch_device(Core& c, const double* d_depos, const long long*
                 const double* dep = d_depos ? d_depos + 7 * offsets[c0] : nullptr;
                 cudaMemsetAsync(b.d_wcnt.p, 0, sizeof(int) * (size_t)(nk + 1), s);
                 cudaMemsetAsync(b.d_kbound.p, 0, sizeof(unsigned long long) * (size_t)nk * kTileBlocks, s);
-                cudaMemsetAsync(b.d_wide.p, 0, (size_t)nk + (size_t)ne * bs.nwires_total, s);
+                const size_t nflags = (size_t)ne * bs.nwires_total;
+                cudaMemsetAsync(b.d_wide.p, 0, wide_bytes((size_t)nk, nflags), s);
+                const HeavyList heavy{reinterpret_cast<int*>(b.d_wide.as<char>() + wide_counters((size_t)nk, nflags)),
+                                      b.d_heavy.as<int4>(),
+                                      reinterpret_cast<int*>(b.d_heavy.as<int4>() + parts)};
                 unsigned char* row_flag = b.d_wide.as<unsigned char>() + nk;
                 k_win_init<<<(ne * np + 63) / 64, 64, 0, s>>>(b.d_win.as<WindowDev>(), ne * np);
                 // random streams keyed by the frame ident of each event: base (a device
@@ -1441,7 +1466,7 @@ static int forward_batch_device(Core& c, const double* d_depos, const long long*
                 launch_raster_batch(plans + ch, bs, pset, b.d_rec.as<PatchRec>(), et.dep0[ne], b.d_tprof.as<float>(),
                                     pool, b.d_wide.as<unsigned char>(), b.d_wcnt.as<int>(), b.d_woff.as<int>(), b.d_wlist.as<Visit>(), b.vcap,
                                     b.d_kbound.as<unsigned long long>(), b.d_Q.as<float>(), nb_r, b.maxG, et, fp,
-                                    b.d_fluc.as<FlucRec>(), b.d_draws.as<int>(), row_flag, s);
+                                    b.d_fluc.as<FlucRec>(), b.d_draws.as<int>(), row_flag, heavy, kHeavyBlocks * b.nsm, s);
                 for (int k = 0; k < bs.ncls; ++k)
                     if (bs.cls_fft3[k])
                         launch_rfft3_batch(plans + ch, bs, k, b.cls_plans[k]->desc, b.fft3_blocks[k][0],

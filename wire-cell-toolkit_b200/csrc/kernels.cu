@@ -96,14 +96,17 @@ __device__ __forceinline__ void count_visits(int* cnt, int wbase, int w0, int ws
     }
 }
 
+// Bound of the fraction of a Gaussian of width s (0: a point) in one bin.
+__device__ __forceinline__ float peak_fraction(float bs, float s)
+{
+    return s > 0.f ? fminf(1.0f, 0.39894228040143268f * bs / s) : 1.0f;  // 1/sqrt(2 pi)
+}
+
 // Magnitude bound of one visit's contribution to any cell: |q| * max bin
 // fraction in pitch * max bin fraction in time * 2 (two bracketing groups).
 __device__ __forceinline__ float visit_bound(float qn, float sp, float st, float pbs, float tbs)
 {
-    const float k = 0.39894228040143268f;  // 1/sqrt(2 pi)
-    const float pm = sp > 0.f ? fminf(1.0f, k * pbs / sp) : 1.0f;
-    const float tm = st > 0.f ? fminf(1.0f, k * tbs / st) : 1.0f;
-    return 2.0f * fabsf(qn) * pm * tm * 1.0001f;
+    return 2.0f * fabsf(qn) * peak_fraction(pbs, sp) * peak_fraction(tbs, st) * 1.0001f;
 }
 
 // Unit bin integral of bin k of a patch (edges at k*bs - cr and (k+1)*bs - cr
@@ -157,10 +160,10 @@ __device__ __forceinline__ int fluc_ident(const FlucParams& fp, int ev)
 
 // The electrons a drifting depo loses (not inlined: the sampler's registers
 // would be the prep kernel's).
-__device__ __noinline__ int drift_draw(const FlucParams& fp, int ident, int i_ev, int nq, double absorb)
+__device__ __noinline__ int drift_draw(unsigned key0, unsigned key1, int i_ev, int nq, double absorb)
 {
     Philox g;
-    g.init(fp.key0, fp.key1 + 0x9E3779B9u * (unsigned)ident, (unsigned)i_ev, kRngDriftTag, 0u);
+    g.init(key0, key1, (unsigned)i_ev, kRngDriftTag, 0u);
     return binomial(nq, absorb, g);
 }
 
@@ -219,7 +222,9 @@ __global__ void __launch_bounds__(256, 4) k_prep_all(const double* __restrict__ 
                         const double absorb = __dsub_rn(1.0, exp(__ddiv_rn(-dt, dd.lifetime)));
                         if (fp.on_drift) {
                             // Binomial(|Q|, absorb) electrons absorbed (Drifter.cxx:179-185)
-                            const int nabs = drift_draw(fp, fluc_ident(fp, ev), i - evt.dep0[ev], (int)fabs(q), absorb);
+                            const int nabs = drift_draw(
+                                fp.key0, fp.key1 + 0x9E3779B9u * (unsigned)fluc_ident(fp, ev), i - evt.dep0[ev],
+                                (int)fabs(q), absorb);
                             q = __dsub_rn(q, q < 0 ? -(double)nabs : (double)nabs);
                         }
                         else q = __dsub_rn(q, __dmul_rn(q, absorb));
@@ -240,6 +245,7 @@ __global__ void __launch_bounds__(256, 4) k_prep_all(const double* __restrict__ 
     if (fq && in) fq[(size_t)ip * n + i] = q;  // the plane's charge: trial count of its fluctuated patch
     // The time profile depends on the depo only (GaussianDiffusion.cxx:124-136):
     // compute it once here for every plane's raster.
+    unsigned long long mywide = 0;
     if (ok && ip == 0) {
         const double st = __ddiv_rn(el, drift_speed);
         const double tlo = __dsub_rn(t, __dmul_rn(st, nsigma));
@@ -247,7 +253,7 @@ __global__ void __launch_bounds__(256, 4) k_prep_all(const double* __restrict__ 
         const int t0 = max(bin_of(tlo, tb.tmin, tb.bs), 0);
         const int t1 = min(bin_of(thi, tb.tmin, tb.bs) + 1, tb.nbins);
         const int nt = t1 - t0;
-        if (nt > kTprof) atomicAdd(&win[0].wide_ticks, (unsigned long long)nt);
+        if (nt > kTprof) mywide = nt;
         if (nt > 0 && nt <= kTprof) {
             float* tp = tprof + (size_t)i * kTprof;
             if (st > 0) {
@@ -358,7 +364,7 @@ __global__ void __launch_bounds__(256, 4) k_prep_all(const double* __restrict__ 
         const int kspan = r.np ? (r.toff + r.nt - 1) / kTile - k0 + 1 : 0;
         count_visits(wire_cnt, pl.wire_base, w0, span, k0, kspan, ps.ntiles);
         myvis += (unsigned long long)span * (unsigned long long)kspan;
-        if (fp.on_patch) mycells += (unsigned long long)r.np * (unsigned long long)r.nt;
+        mycells += (unsigned long long)r.np * (unsigned long long)r.nt;
         if (r.nt > kTprof) {  // keys that hold a long patch: their raster block spreads visits over warps
             unsigned char* wk = wide_all + (size_t)ev * nkeys;
             for (int ww = 0; ww < span; ++ww)
@@ -426,14 +432,24 @@ __global__ void __launch_bounds__(256, 4) k_prep_all(const double* __restrict__ 
             if (l == 0 && nbig) atomicAdd(&wd->bigcharge, nbig);
         }
     }
-    // 64-bit visit total of the event (the visit lists use int offsets)
+    // 64-bit totals of the event (visits: the lists use int offsets), one
+    // atomic per block and quantity: they all go to one address, where a
+    // thread's own atomics queue up (500k depos, half with long patches: 484 us
+    // with one per thread and long patch)
+    __shared__ unsigned long long s_tot[3][8];
+    unsigned long long tot[3] = {myvis, mycells, mywide};
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) myvis += __shfl_xor_sync(0xffffffffu, myvis, o);
-    if (l == 0 && myvis) atomicAdd(&win[0].nvisits, myvis);
-    if (fp.on_patch) {
+    for (int k = 0; k < 3; ++k) {
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) mycells += __shfl_xor_sync(0xffffffffu, mycells, o);
-        if (l == 0 && mycells) atomicAdd(&win[0].ncells, mycells);
+        for (int o = 16; o > 0; o >>= 1) tot[k] += __shfl_xor_sync(0xffffffffu, tot[k], o);
+        if (l == 0) s_tot[k][w] = tot[k];
+    }
+    __syncthreads();
+    if (threadIdx.x < 3) {
+        unsigned long long v = 0;
+        for (int k = 0; k < (int)(blockDim.x >> 5); ++k) v += s_tot[threadIdx.x][k];
+        unsigned long long* to = threadIdx.x == 0 ? &win[0].nvisits : (threadIdx.x == 1 ? &win[0].ncells : &win[0].wide_ticks);
+        if (v) atomicAdd(to, v);
     }
 }
 
@@ -531,31 +547,41 @@ void launch_scan(const int* wire_cnt, int nwires_total, int* wire_off, int* wire
 }
 
 // Time profiles of the long patches, one warp per depo (its first plane with a
-// patch: the time profile does not depend on the plane).
+// patch: the time profile does not depend on the plane); room for a block's
+// depos is taken in one go (one address: see k_prep_all).
 __global__ void __launch_bounds__(256) k_tprof_pool(const PatchRec* __restrict__ rec, EventTable evt, int nplanes,
                                                    float tbs, TprofPool pool, int* status)
 {
-    const int lane = threadIdx.x & 31;
+    __shared__ int s_nt[8];
+    __shared__ long long s_off;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int n = evt.dep0[evt.nev];
-    const int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (i >= n) return;  // whole warps
+    const int i = blockIdx.x * 8 + w;
     PatchRec r{};
-    for (int ip = 0; ip < nplanes; ++ip) {
+    for (int ip = 0; ip < nplanes && i < n; ++ip) {
         r = rec[(size_t)ip * n + i];
         if (r.np) break;
     }
+    const int nt = r.np && r.nt > kTprof ? r.nt : 0;
+    if (lane == 0) s_nt[w] = nt;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        int tot = 0;
+        for (int k = 0; k < 8; ++k) tot += s_nt[k];
+        s_off = tot ? (long long)atomicAdd(pool.used, (unsigned long long)tot) : 0;
+    }
+    __syncthreads();
+    if (i >= n) return;
     int off = -1;
-    if (r.np && r.nt > kTprof) {
-        long long off64 = 0;
-        if (lane == 0) off64 = (long long)atomicAdd(pool.used, (unsigned long long)r.nt);
-        off64 = __shfl_sync(0xffffffffu, off64, 0);
-        off = off64 + r.nt > pool.cap ? -1 : (int)off64;  // 64-bit counter: no wrap
+    if (nt) {
+        long long off64 = s_off;
+        for (int k = 0; k < w; ++k) off64 += s_nt[k];
+        off = off64 + nt > pool.cap ? -1 : (int)off64;  // 64-bit counter: no wrap
         if (off < 0) {
-            off = -1;
             if (lane == 0 && status) atomicOr(status, kBatchPoolShort);
         }
         else
-            for (int t = lane; t < r.nt; t += 32) pool.val[off + t] = unit_bin(t, tbs, r.tcr, r.st);
+            for (int t = lane; t < nt; t += 32) pool.val[off + t] = unit_bin(t, tbs, r.tcr, r.st);
     }
     if (lane == 0) pool.off[i] = off;
 }
@@ -644,9 +670,8 @@ void launch_fill(const PatchRec* rec, const EventTable& et, int nkeys, const Pla
 // the grid is bit-reproducible.
 // ---------------------------------------------------------------------------
 constexpr int kRasterThreads = 256;
-// staged per visit: 12 group coefficients, q, and 16 scaled tick values (odd stride: no bank conflicts)
-constexpr int kStageQ = 12;
-constexpr int kStageT = 13;
+// staged per visit: 12 group coefficients and 16 scaled tick values (odd stride: no bank conflicts)
+constexpr int kStageT = 12;
 constexpr int kStageStride = 29;
 constexpr int kTileLd = kTile + 8;  // fluctuated raster: row stride with an 8-word skew between groups
 // Forward raster grid row stride: 4 words of skew, so eight visits scattering
@@ -658,19 +683,53 @@ size_t raster_smem_bytes(int G)
     return sizeof(int) * (size_t)G * kGridLd + sizeof(float) * (size_t)kRasterThreads * kStageStride +
            sizeof(int4) * (size_t)kRasterThreads;
 }
+// Long visits of a heavy part, behind that: their integer coefficients by group
+// (three int4) and one of (column | length, profile offset, scaled charge, depo).
+constexpr int kLongQuads = 4;
+static size_t raster_heavy_smem_bytes(int G)
+{
+    return raster_smem_bytes(G) + sizeof(int4) * (size_t)kRasterThreads * kLongQuads;
+}
+
+// The first launch rasterises the light tiles, a block each, and lists the
+// heavy ones -- those with long patches (over kTprof ticks; a shower's run over
+// a hundred) or with more visits than kHeavyVisits -- for the second, whose
+// blocks take 256 visits of a tile each: the heaviest tile of an event (a
+// shower's core, a track along a wire) holds thousands of visits and ran on
+// long after the others.  The parts of a tile are added in the grid itself as
+// integers, and the block that finishes a tile turns it into charges.
+//
+// Long patches are taken a column at a time there: a warp takes 32 tick columns
+// of the tile, a lane each, and 32 of the staged visits, and adds those that
+// cross its columns to the groups' sums in registers, one shared atomic a group
+// at the end (warps that owned their columns waited for the fullest ones at the
+// chunk's barrier).  Their cells are the high words of integer products, group coefficient times scaled tick
+// value, so no float-to-int conversion a cell (a quarter of a warp a cycle).
+// 500k depos, half with patches of 100 ticks x 30 impacts, three planes: 2.8 ->
+// 2.1 ms (heavy parts 1.85, at 43 % of the issue slots and 24 warps an SM).
+constexpr int kWideG = 12;         // impact groups (wct_dt_set_response_table takes no more)
+constexpr int kWideAhead = 4;      // visits whose tick values are loaded together
+// (full APA, 520k track depos, fullest tile 3300: 478 us whole; 549 us with tiles
+// over 1024 in parts, 744 us over 512: a part pays for its grid again)
+constexpr int kHeavyVisits = 4096;
+static_assert(kRasterThreads == kHeavyPart, "a part is a block's chunk");
 
 // One raster work item: charge row `row` (wire start_ch + row) of plane P and
 // absolute tick tile ktile.  Visit keys are key_base + wire * ntiles_abs +
-// tile; at most vcap visits exist.  Called by all threads of the block;
-// smem_i holds the dynamic shared memory of raster_smem_bytes(P.G).
+// tile; at most vcap visits exist.  HEAVY: part `seg` of the nseg parts of a
+// heavy tile (slot: its entry of heavy.done); otherwise the whole tile, or its
+// listing under tile_id.  Called by all threads of the block; smem_i holds the
+// dynamic shared memory of raster_smem_bytes(P.G).
+template <bool HEAVY>
 __device__ __forceinline__ void raster_tile(const GridPlane& P, int row, int ktile, int key_base, int ntiles_abs,
                                             const PatchRec* __restrict__ rec, const float* __restrict__ tprof,
                                             const TprofPool& pool, const unsigned char* __restrict__ wide_key,
                                             const int* __restrict__ wire_cnt, const int* __restrict__ wire_off,
                                             const Visit* __restrict__ visits, long long vcap,
                                             const unsigned long long* __restrict__ key_bound,
-                                            float* __restrict__ Q, unsigned char* __restrict__ row_flag, int* smem_i,
-                                            float* scale, float* iscale)
+                                            float* __restrict__ Q, unsigned char* __restrict__ row_flag,
+                                            const HeavyList& heavy, int tile_id, int seg, int nseg, int slot,
+                                            int* smem_i, float* scale, float* iscale)
 {
     __syncthreads();  // the previous item of a persistent block is done with the shared arrays
     const int w = P.start_ch + row;
@@ -680,6 +739,7 @@ __device__ __forceinline__ void raster_tile(const GridPlane& P, int row, int kti
     int* grid = smem_i;                                       // [G][kGridLd], column = tick - tick_lo
     float* stage = reinterpret_cast<float*>(smem_i + (size_t)G * kGridLd);
     int4* stagei = reinterpret_cast<int4*>(stage + (size_t)kRasterThreads * kStageStride);
+    int4* longq = stagei + kRasterThreads;  // heavy parts only
     int cnt = 0;
     const Visit* list = nullptr;
     int key = -1;
@@ -689,8 +749,20 @@ __device__ __forceinline__ void raster_tile(const GridPlane& P, int row, int kti
         cnt = off < 0 ? 0 : (int)min((long long)wire_cnt[key], max(0ll, vcap - off));  // no reads past the list
         list = visits + max(off, 0);
     }
-    if (cnt == 0) {
-        // no visit (block-uniform): the tile's G rows are zero
+    const bool spread = cnt > 0 && wide_key[key];
+    const bool longs = HEAVY && spread;  // the tile holds long patches
+    const bool listed = !HEAVY && (spread || cnt > kHeavyVisits);
+    if (listed) {
+        const int parts = (cnt + kHeavyPart - 1) / kHeavyPart;
+        if (tid == 0) {
+            const int sl = atomicAdd(heavy.count + 1, 1), at = atomicAdd(heavy.count, parts);
+            heavy.done[sl] = 0;
+            for (int k = 0; k < parts; ++k) heavy.item[at + k] = make_int4(tile_id, k, parts, sl);
+        }
+        if (parts == 1) return;  // written whole by its only part
+    }
+    if (cnt == 0 || listed) {
+        // no visit (block-uniform), or parts to come: the tile's G rows are zero
         const int qc0 = tick_lo - P.col0;
         for (int k = tid; k < G * kTile; k += kRasterThreads) {
             const int g = k / kTile, c = k - g * kTile;
@@ -700,8 +772,13 @@ __device__ __forceinline__ void raster_tile(const GridPlane& P, int row, int kti
         return;
     }
     if (tid == 0) row_flag[P.wire_base + w] = 1;  // the wire holds charge (every block of the row writes the same)
-    const bool spread = key >= 0 && wide_key[key];
+    if (HEAVY) {
+        list += (size_t)seg * kHeavyPart;
+        cnt = min(cnt - seg * kHeavyPart, kHeavyPart);
+    }
+    __shared__ int s_unit[1];
     {
+        if (HEAVY && tid == 0) *s_unit = 0;
         int4* g4 = reinterpret_cast<int4*>(grid);
         const int n4 = G * kGridLd / 4;
         for (int k = tid; k < n4; k += kRasterThreads) g4[k] = make_int4(0, 0, 0, 0);
@@ -730,7 +807,7 @@ __device__ __forceinline__ void raster_tile(const GridPlane& P, int row, int kti
         // would otherwise pile up on a few warps); elsewhere visits stay in
         // list order (coalesced reads, alike neighbours along a track)
         const int e = ch * kRasterThreads +
-                      (spread ? (lane >> 1) * (kRasterThreads / 16) + wid * 2 + (lane & 1) : tid);
+                      (longs ? (lane >> 1) * (kRasterThreads / 16) + wid * 2 + (lane & 1) : tid);
         const bool valid = e < cnt;
         int4 si = make_int4(0, 0, 0, 0);  // d, l_lo, ng, (cb << 11) | nt  (cb = toff - tick_lo, ng = 0: none)
         if (valid) {
@@ -774,7 +851,25 @@ __device__ __forceinline__ void raster_tile(const GridPlane& P, int row, int kti
                 }
                 const int cb = r.toff - tick_lo;  // may be negative for patches starting in the previous tile
                 si = make_int4(d, l_lo, ng, ((cb + 1024) << 11) | rnt);
-                my[kStageQ] = r.qn;
+                if (longs && rnt > kTprof) {
+                    // the coefficients by impact group as integers, in units of 2^-30 of the peak
+                    // bin fraction (a group's is below twice that), four times the charge times
+                    // that fraction (the scaled tick values stay below 2^31: the bound behind
+                    // the scale holds twice this product), and where the profile is
+                    const float pm = peak_fraction(pbs, r.sp);
+                    const float unit = __fdividef(1073741824.0f, pm);
+                    int ci[kWideG];
+#pragma unroll
+                    for (int g = 0; g < kWideG; ++g) {
+                        const int lb = g - l_lo;
+                        ci[g] = lb >= 0 && lb < ng ? __float2int_rn(my[max(lb, 0)] * unit) : 0;
+                    }
+                    int4* lq = longq + tid * kLongQuads;
+                    lq[0] = make_int4(si.w, __ldg(pool.off + d), __float_as_int(4.0f * r.qn * pm), d);
+                    lq[1] = make_int4(ci[0], ci[1], ci[2], ci[3]);
+                    lq[2] = make_int4(ci[4], ci[5], ci[6], ci[7]);
+                    lq[3] = make_int4(ci[8], ci[9], ci[10], ci[11]);
+                }
                 if (rnt <= 16) {
                     // tick values scaled to the fixed point of their 64-tick block (0 outside the tile);
                     // the whole 16-value profile row in four 128-bit loads (one L1 wavefront per
@@ -801,7 +896,8 @@ __device__ __forceinline__ void raster_tile(const GridPlane& P, int row, int kti
             }
         }
         stagei[tid] = si;
-        __syncwarp();
+        if (longs) __syncthreads();
+        else __syncwarp();
         // lanes 0 .. nv-1 of this warp hold visits (e grows with the lane)
         const int nv = __popc(__ballot_sync(0xffffffffu, valid));
         // eight visits at a time: four lanes per visit, each lane four ticks (hl + 4k)
@@ -810,90 +906,146 @@ __device__ __forceinline__ void raster_tile(const GridPlane& P, int row, int kti
             const int v = v0 + qv;
             int4 vi = make_int4(0, 0, 0, 0);
             if (v < nv) vi = stagei[wbase + v];
-            const int nt = vi.w & 2047;
-            const bool wide = __any_sync(0xffffffffu, nt > 16);
-            if (!wide) {
-                const int ng = vi.z;
-                const int c0 = (vi.w >> 11) - 1024 + hl;  // tile column of this lane's first tick
-                const float* vc = stage + (size_t)(wbase + min(v, 31)) * kStageStride;
-                float tq[4];
-                int gl[4];  // groups this lane adds at tick hl + 4k (0: tick outside the patch or tile)
-                int mgl = 0;
+            int nt = vi.w & 2047;
+            if (longs && nt > kTprof) nt = 0;  // below
+            const int ng = vi.z;
+            const int c0 = (vi.w >> 11) - 1024 + hl;  // tile column of this lane's first tick
+            const float* vc = stage + (size_t)(wbase + min(v, 31)) * kStageStride;
+            float tq[4];
+            int gl[4];  // groups this lane adds at tick hl + 4k (0: tick outside the patch or tile)
+            int mgl = 0;
 #pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    const int c = c0 + 4 * k;
-                    const bool on = hl + 4 * k < nt && c >= 0 && c < kTile;
-                    tq[k] = on ? vc[kStageT + hl + 4 * k] : 0.f;
-                    gl[k] = on ? ng : 0;
-                    mgl = max(mgl, gl[k]);
-                }
-                const int mg = __reduce_max_sync(0xffffffffu, mgl);
-                // the eight visits start at spread-out groups and wrap around
-                // (visit slot qv at group qv*ng/8): visits of one track share
-                // their columns and would otherwise hit the same words together
-                int gg = (qv * ng) >> 3;
-                int* dst = grid + (vi.y + gg) * kGridLd + c0;
-                int* const wrap = grid + vi.y * kGridLd + c0;
-                int* const last = wrap + (ng - 1) * kGridLd;
-                float cf = vc[gg];
-                for (int g = 0; g < mg; ++g) {
-                    const bool w = dst == last;
-                    const int gn = w ? 0 : gg + 1;
-                    const float cfn = vc[gn];  // next group's coefficient, loaded ahead
-                    int v4[4];
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) v4[k] = __float2int_rn(cf * tq[k]);
-#pragma unroll
-                    for (int k = 0; k < 4; ++k)
-                        if (g < gl[k]) atomicAdd(dst + 4 * k, v4[k]);
-                    dst = w ? wrap : dst + kGridLd;
-                    gg = gn;
-                    cf = cfn;
-                }
+            for (int k = 0; k < 4; ++k) {
+                const int c = c0 + 4 * k;
+                const bool on = hl + 4 * k < nt && c >= 0 && c < kTile;
+                tq[k] = on ? vc[kStageT + hl + 4 * k] : 0.f;
+                gl[k] = on ? ng : 0;
+                mgl = max(mgl, gl[k]);
             }
-            else {
-                // at least one of the eight has more than 16 ticks: whole warp per visit
-                for (int hv = 0; hv < 8; ++hv) {
-                    const int vv = v0 + hv;
-                    if (vv >= nv) break;
-                    const int4 wi = stagei[wbase + vv];
-                    const int ng = wi.z;
-                    if (ng == 0) continue;
-                    const int wnt = wi.w & 2047;
-                    const int cb = (wi.w >> 11) - 1024;
-                    const float* vc = stage + (size_t)(wbase + vv) * kStageStride;
-                    const float qn = vc[kStageQ];
-                    const int tstart = max(0, -cb), tend = min(wnt, kTile - cb);  // ticks inside the tile
-                    const int poff = wnt > kTprof ? __ldg(pool.off + wi.x) : -1;
-                    float rtcr = 0.f, rst = 0.f;
-                    if (wnt > kTprof && poff < 0) {
-                        const PatchRec r = rec[P.recoff + wi.x];
-                        rtcr = r.tcr;
-                        rst = r.st;
-                    }
-                    for (int tc = tstart; tc < tend; tc += 32) {
-                        const int it = tc + lane;
-                        const bool on = it < tend;
-                        float tq = 0.f;
-                        if (on) {
-                            float tv;
-                            if (wnt <= kTprof) tv = __ldg(tprof + (size_t)wi.x * kTprof + it);
-                            else if (poff >= 0) tv = __ldg(pool.val + poff + it);
-                            else tv = unit_bin(it, tbs, rtcr, rst);
-                            tq = tv * qn * scale[(cb + it) / kScaleBlock];
-                        }
-                        int* dst = grid + wi.y * kGridLd + cb + it;
-                        for (int g = 0; g < ng; ++g) {
-                            if (on) atomicAdd(dst, __float2int_rn(vc[g] * tq));
-                            dst += kGridLd;
-                        }
-                    }
-                }
+            const int mg = __reduce_max_sync(0xffffffffu, mgl);
+            // the eight visits start at spread-out groups and wrap around
+            // (visit slot qv at group qv*ng/8): visits of one track share
+            // their columns and would otherwise hit the same words together
+            int gg = (qv * ng) >> 3;
+            int* dst = grid + (vi.y + gg) * kGridLd + c0;
+            int* const wrap = grid + vi.y * kGridLd + c0;
+            int* const last = wrap + (ng - 1) * kGridLd;
+            float cf = vc[gg];
+            for (int g = 0; g < mg; ++g) {
+                const bool w = dst == last;
+                const int gn = w ? 0 : gg + 1;
+                const float cfn = vc[gn];  // next group's coefficient, loaded ahead
+                int v4[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) v4[k] = __float2int_rn(cf * tq[k]);
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    if (g < gl[k]) atomicAdd(dst + 4 * k, v4[k]);
+                dst = w ? wrap : dst + kGridLd;
+                gg = gn;
+                cf = cfn;
             }
         }
-        __syncwarp();
+        if (longs) {
+            // units of 32 columns x 32 staged visits, taken in turn by whichever warp is free
+            for (;;) {
+                int unit = 0;
+                if (lane == 0) unit = atomicAdd(s_unit, 1);
+                unit = __shfl_sync(0xffffffffu, unit, 0);
+                if (unit >= (kTile / 32) * (kRasterThreads / 32)) break;
+                const int slab = unit & (kTile / 32 - 1), b0 = (unit / (kTile / 32)) * 32;
+                const int c = slab * 32 + lane;  // this lane's column
+                const float sc = scale[c / kScaleBlock];
+                const int4 si0 = stagei[b0 + lane];
+                const int cb0 = (si0.w >> 11) - 1024, nt0 = si0.w & 2047;
+                unsigned m = __ballot_sync(0xffffffffu, si0.z > 0 && nt0 > kTprof && cb0 < slab * 32 + 32 &&
+                                                            cb0 + nt0 > slab * 32);
+                if (!m) continue;
+                int acc[kWideG];
+#pragma unroll
+                for (int g = 0; g < kWideG; ++g) acc[g] = 0;
+                // tick values of the next few visits, asked for while the last few are added
+                int vn[kWideAhead];
+                float tn[kWideAhead];
+                auto ask = [&]() {
+#pragma unroll
+                    for (int a = 0; a < kWideAhead; ++a) {
+                        vn[a] = m ? b0 + __ffs(m) - 1 : -1;
+                        m &= m - 1;
+                        tn[a] = 0.f;
+                        if (vn[a] >= 0) {
+                            const int4 lv = longq[vn[a] * kLongQuads];
+                            const int it = c - ((lv.x >> 11) - 1024);
+                            if (it >= 0 && it < (lv.x & 2047)) {
+                                if (lv.y >= 0) tn[a] = __ldg(pool.val + lv.y + it);
+                                else {
+                                    const PatchRec r = rec[P.recoff + lv.w];
+                                    tn[a] = unit_bin(it, tbs, r.tcr, r.st);
+                                }
+                            }
+                        }
+                    }
+                };
+                ask();
+                while (vn[0] >= 0) {
+                    int vs[kWideAhead];
+                    float tv[kWideAhead];
+#pragma unroll
+                    for (int a = 0; a < kWideAhead; ++a) {
+                        vs[a] = vn[a];
+                        tv[a] = tn[a];
+                    }
+                    ask();
+#pragma unroll
+                    for (int a = 0; a < kWideAhead; ++a) {
+                        if (vs[a] < 0) break;
+                        const int4* lq = longq + vs[a] * kLongQuads;
+                        const int tq = __float2int_rn(tv[a] * __int_as_float(lq[0].z) * sc);
+#pragma unroll
+                        for (int q = 0; q < kWideG / 4; ++q) {
+                            const int4 ci = lq[1 + q];
+                            // rounded high words of the products
+                            acc[4 * q] += (int)(((long long)ci.x * tq + 0x80000000ll) >> 32);
+                            acc[4 * q + 1] += (int)(((long long)ci.y * tq + 0x80000000ll) >> 32);
+                            acc[4 * q + 2] += (int)(((long long)ci.z * tq + 0x80000000ll) >> 32);
+                            acc[4 * q + 3] += (int)(((long long)ci.w * tq + 0x80000000ll) >> 32);
+                        }
+                    }
+                }
+#pragma unroll
+                for (int g = 0; g < kWideG; ++g)
+                    if (g < G) atomicAdd(grid + g * kGridLd + c, acc[g]);
+            }
+            __syncthreads();  // the stage is rewritten by the next chunk
+        }
+        else
+            __syncwarp();
     }
     __syncthreads();
+    if (HEAVY && nseg > 1) {
+        // this part into the tile's rows, as integers; the last part to arrive makes them charges
+        const int qc0 = tick_lo - P.col0;
+        int* const Qi = reinterpret_cast<int*>(Q) + P.qoff + (size_t)row * P.N;
+        for (int k = tid; k < G * kTile; k += kRasterThreads) {
+            const int g = k / kTile, c = k - g * kTile, q = qc0 + c;
+            const int v = grid[g * kGridLd + c];
+            if (v && q >= 0 && q < min(P.N, P.ncols)) atomicAdd(Qi + (size_t)g * P.nin * P.N + q, v);
+        }
+        __threadfence();
+        __syncthreads();
+        __shared__ int s_last;
+        if (tid == 0) s_last = atomicAdd(heavy.done + slot, 1) == nseg - 1;
+        __syncthreads();
+        if (!s_last) return;
+        __threadfence();
+        for (int k = tid; k < G * kTile; k += kRasterThreads) {
+            const int g = k / kTile, c = k - g * kTile, q = qc0 + c;
+            if (q < 0 || q >= min(P.N, P.ncols)) continue;
+            int* const at = Qi + (size_t)g * P.nin * P.N + q;
+            *reinterpret_cast<float*>(at) = (float)__ldcg(at) * iscale[c / kScaleBlock];
+        }
+        return;
+    }
     // write the tile's G rows, four columns per thread: grid column c is plane
     // column tick_lo + c - col0 (zero at or past the window's ncols)
     const int qc0 = tick_lo - P.col0;
@@ -911,40 +1063,70 @@ __device__ __forceinline__ void raster_tile(const GridPlane& P, int row, int kti
     }
 }
 
-__global__ void __launch_bounds__(kRasterThreads, 5) k_raster_wires(const PatchRec* __restrict__ rec,
-                                                                 const float* __restrict__ tprof,
-                                                                 const int* __restrict__ wire_cnt,
-                                                                 const int* __restrict__ wire_off,
-                                                                 const Visit* __restrict__ visits, long long vcap,
-                                                                 const unsigned long long* __restrict__ key_bound,
-                                                                 GridSet gs, float* __restrict__ Q, TprofPool pool,
-                                                                 const unsigned char* __restrict__ wide_key,
-                                                                 unsigned char* __restrict__ row_flag)
+// The plane and the (row, tile) of a block of the tile grid.
+__device__ __forceinline__ int grid_tile(const GridSet& gs, int tile, int& row, int& ktile)
+{
+    int ip = 0;
+    while (ip + 1 < gs.nplanes && tile >= gs.p[ip + 1].row_base) ++ip;
+    const GridPlane& P = gs.p[ip];
+    const int rel = tile - P.row_base;
+    row = rel / P.ntile;
+    ktile = P.ktile0 + (rel - row * P.ntile);  // absolute tick tile
+    return ip;
+}
+
+__global__ void __launch_bounds__(kRasterThreads, 5)
+    k_raster_wires(const PatchRec* __restrict__ rec, const float* __restrict__ tprof,
+                   const int* __restrict__ wire_cnt, const int* __restrict__ wire_off,
+                   const Visit* __restrict__ visits, long long vcap, const unsigned long long* __restrict__ key_bound,
+                   GridSet gs, float* __restrict__ Q, TprofPool pool, const unsigned char* __restrict__ wide_key,
+                   unsigned char* __restrict__ row_flag, HeavyList heavy)
 {
     extern __shared__ int smem_i[];
     __shared__ float scale[kTileBlocks], iscale[kTileBlocks];
-    int ip = 0;
-    while (ip + 1 < gs.nplanes && (int)blockIdx.x >= gs.p[ip + 1].row_base) ++ip;
-    const GridPlane& P = gs.p[ip];
-    const int rel = blockIdx.x - P.row_base;
-    const int row = rel / P.ntile;
-    const int ktile = P.ktile0 + (rel - row * P.ntile);  // absolute tick tile
-    raster_tile(P, row, ktile, 0, gs.ntiles_abs, rec, tprof, pool, wide_key, wire_cnt, wire_off, visits, vcap,
-                key_bound, Q, row_flag, smem_i, scale, iscale);
+    int row, ktile;
+    const int ip = grid_tile(gs, blockIdx.x, row, ktile);
+    raster_tile<false>(gs.p[ip], row, ktile, 0, gs.ntiles_abs, rec, tprof, pool, wide_key, wire_cnt, wire_off, visits,
+                       vcap, key_bound, Q, row_flag, heavy, blockIdx.x, 0, 1, 0, smem_i, scale, iscale);
+}
+
+__global__ void __launch_bounds__(kRasterThreads, kHeavyBlocks)
+    k_raster_heavy(const PatchRec* __restrict__ rec, const float* __restrict__ tprof,
+                   const int* __restrict__ wire_cnt, const int* __restrict__ wire_off,
+                   const Visit* __restrict__ visits, long long vcap, const unsigned long long* __restrict__ key_bound,
+                   GridSet gs, float* __restrict__ Q, TprofPool pool, const unsigned char* __restrict__ wide_key,
+                   unsigned char* __restrict__ row_flag, HeavyList heavy)
+{
+    extern __shared__ int smem_i[];
+    __shared__ float scale[kTileBlocks], iscale[kTileBlocks];
+    const int total = heavy.count[0];
+    for (int k = blockIdx.x; k < total; k += gridDim.x) {
+        const int4 it = heavy.item[k];
+        int row, ktile;
+        const int ip = grid_tile(gs, it.x, row, ktile);
+        raster_tile<true>(gs.p[ip], row, ktile, 0, gs.ntiles_abs, rec, tprof, pool, wide_key, wire_cnt, wire_off,
+                          visits, vcap, key_bound, Q, row_flag, heavy, it.x, it.y, it.z, it.w, smem_i, scale, iscale);
+    }
 }
 
 void launch_raster_wires(const PatchRec* rec, const float* tprof, const TprofPool& pool, const unsigned char* wide_key,
                          const int* wire_cnt,
                          const int* wire_off, const Visit* visits, long long vcap,
                          const unsigned long long* key_bound, const GridSet& gs, float* Q, unsigned char* row_flag,
-                         cudaStream_t s)
+                         const HeavyList& heavy, int heavy_blocks, cudaStream_t s)
 {
     if (gs.nrows_total <= 0) return;
     size_t smem = 0;
     for (int i = 0; i < gs.nplanes; ++i) smem = std::max(smem, raster_smem_bytes(gs.p[i].G));
     cudaFuncSetAttribute((const void*)k_raster_wires, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     k_raster_wires<<<gs.nrows_total, kRasterThreads, smem, s>>>(rec, tprof, wire_cnt, wire_off, visits, vcap,
-                                                                    key_bound, gs, Q, pool, wide_key, row_flag);
+                                                                key_bound, gs, Q, pool, wide_key, row_flag, heavy);
+    if (heavy_blocks <= 0) return;  // no tile can be heavy
+    smem = 0;
+    for (int i = 0; i < gs.nplanes; ++i) smem = std::max(smem, raster_heavy_smem_bytes(gs.p[i].G));
+    cudaFuncSetAttribute((const void*)k_raster_heavy, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    k_raster_heavy<<<heavy_blocks, kRasterThreads, smem, s>>>(rec, tprof, wire_cnt, wire_off, visits, vcap, key_bound,
+                                                              gs, Q, pool, wide_key, row_flag, heavy);
 }
 
 // ---------------------------------------------------------------------------
@@ -1035,9 +1217,6 @@ __global__ void __launch_bounds__(kFlucWarps * 32, 6) k_fluc_sums(const PatchRec
     if (own) {
         r = rec[(size_t)ip * n + mine];
         if (r.np > 0 && r.nt > 0) {
-            const long long off = (long long)atomicAdd(draws.used, (unsigned long long)r.np * r.nt);
-            if (off + (long long)r.np * r.nt <= draws.cap) out.off = (int)off;
-            else if (status) atomicOr(status, kBatchDrawsShort);
             out.invS = patch_inv_norm(r, pbs, tbs);
             Q = fq[(size_t)ip * n + mine];
             out.nq = (int)fabs(Q);
@@ -1047,6 +1226,23 @@ __global__ void __launch_bounds__(kFlucWarps * 32, 6) k_fluc_sums(const PatchRec
         }
         else
             r.np = r.nt = 0;
+    }
+    {  // room for the warp's draws in one go (one address: see k_prep_all)
+        const long long mycells = (long long)r.np * r.nt;
+        long long before = 0, all = 0;
+#pragma unroll
+        for (int s = 0; s < kFlucSlots; ++s) {
+            const long long c = __shfl_sync(full, mycells, s);
+            if (s < lane) before += c;
+            all += c;
+        }
+        long long off = 0;
+        if (lane == 0 && all) off = (long long)atomicAdd(draws.used, (unsigned long long)all);
+        off = __shfl_sync(full, off, 0) + before;
+        if (mycells) {
+            if (off + mycells <= draws.cap) out.off = (int)off;
+            else if (status) atomicOr(status, kBatchDrawsShort);
+        }
     }
     const int size = own ? r.np + r.nt : 0;
     const unsigned key0 = fp.key0;
@@ -2484,59 +2680,87 @@ __device__ __forceinline__ int find_entry(const int* __restrict__ pre, int n, in
     return lo;
 }
 
+// The raster parameters of work item `item` of a pass: its event, plane, row and tile.
+__device__ __forceinline__ GridPlane batch_tile(const BatchPlan* __restrict__ plan, const BatchStatic& bs,
+                                                const PlaneSet& ps, long long recstride, int item, int& e, int& ip,
+                                                int& row, int& ktile)
+{
+    const int k = find_entry(plan->pre_raster, plan->nev * plan->np, item);
+    e = k / plan->np;
+    ip = k - e * plan->np;
+    const EvPlane& E = plan->ep[k];
+    GridPlane P;
+    P.nimp = ps.p[ip].nimp;
+    P.G = bs.pl[ip].G;
+    P.nwires = ps.p[ip].nwires;
+    P.wire_base = ps.p[ip].wire_base;
+    P.start_ch = E.start_ch;
+    P.nin = E.nin;
+    P.col0 = E.start_tick;
+    P.ncols = E.ncols;
+    P.N = E.N;
+    P.tbs = (float)bs.tbs;
+    P.pbs = (float)ps.p[ip].imp_bs;
+    P.qoff = E.qoff;
+    P.recoff = (long long)ip * recstride;
+    P.row_base = 0;
+    P.ktile0 = E.ktile0;
+    P.ntile = E.ntile;
+    const int rel = item - plan->pre_raster[k];
+    row = rel / E.ntile;
+    ktile = E.ktile0 + (rel - row * E.ntile);
+    return P;
+}
+
 template <bool FLUC>
-__global__ void __launch_bounds__(kRasterThreads, FLUC ? 4 : 5) k_raster_batch(const BatchPlan* __restrict__ plan, BatchStatic bs,
-                                                                 PlaneSet ps, const PatchRec* __restrict__ rec,
-                                                                 long long recstride,
-                                                                 const float* __restrict__ tprof, TprofPool pool,
-                                                                 const unsigned char* __restrict__ wide_key,
-                                                                 const int* __restrict__ wire_cnt,
-                                                                 const int* __restrict__ wire_off,
-                                                                 const Visit* __restrict__ visits, long long vcap,
-                                                                 const unsigned long long* __restrict__ key_bound,
-                                                                 float* __restrict__ Q, EventTable evt, FlucParams fp,
-                                                                 const FlucRec* __restrict__ fluc,
-                                                                 const int* __restrict__ draws,
-                                                                 unsigned char* __restrict__ row_flag)
+__global__ void __launch_bounds__(kRasterThreads, FLUC ? 4 : 5)
+    k_raster_batch(const BatchPlan* __restrict__ plan, BatchStatic bs, PlaneSet ps, const PatchRec* __restrict__ rec,
+                   long long recstride, const float* __restrict__ tprof, TprofPool pool,
+                   const unsigned char* __restrict__ wide_key, const int* __restrict__ wire_cnt,
+                   const int* __restrict__ wire_off, const Visit* __restrict__ visits, long long vcap,
+                   const unsigned long long* __restrict__ key_bound, float* __restrict__ Q, EventTable evt,
+                   FlucParams fp, const FlucRec* __restrict__ fluc, const int* __restrict__ draws,
+                   unsigned char* __restrict__ row_flag, HeavyList heavy)
 {
     extern __shared__ int smem_i[];
     __shared__ float scale[kTileBlocks], iscale[kTileBlocks];
     if (plan->status & kBatchSkip) return;
     __shared__ int s_item;
-    const int ne = plan->nev * plan->np;
-    const int total = plan->pre_raster[ne];
+    const int total = plan->pre_raster[plan->nev * plan->np];
     int* ctr = const_cast<int*>(&plan->next[0]);
     for (int item = next_item(ctr, &s_item); item < total; item = next_item(ctr, &s_item)) {
-        const int k = find_entry(plan->pre_raster, ne, item);
-        const int e = k / plan->np, ip = k - e * plan->np;
-        const EvPlane& E = plan->ep[k];
-        GridPlane P;
-        P.nimp = ps.p[ip].nimp;
-        P.G = bs.pl[ip].G;
-        P.nwires = ps.p[ip].nwires;
-        P.wire_base = ps.p[ip].wire_base;
-        P.start_ch = E.start_ch;
-        P.nin = E.nin;
-        P.col0 = E.start_tick;
-        P.ncols = E.ncols;
-        P.N = E.N;
-        P.tbs = (float)bs.tbs;
-        P.pbs = (float)ps.p[ip].imp_bs;
-        P.qoff = E.qoff;
-        P.recoff = (long long)ip * recstride;
-        P.row_base = 0;
-        P.ktile0 = E.ktile0;
-        P.ntile = E.ntile;
-        const int rel = item - plan->pre_raster[k];
-        const int row = rel / E.ntile;
+        int e, ip, row, ktile;
+        const GridPlane P = batch_tile(plan, bs, ps, recstride, item, e, ip, row, ktile);
+        unsigned char* flags = row_flag + (size_t)e * bs.nwires_total;
         if constexpr (FLUC)
-            raster_tile_fluc(P, ip, row, E.ktile0 + (rel - row * E.ntile), e * bs.nkeys, bs.ntiles, evt, fp, rec,
-                             fluc, draws, wire_cnt, wire_off, visits, vcap, Q, row_flag + (size_t)e * bs.nwires_total,
-                             reinterpret_cast<long long*>(smem_i));
+            raster_tile_fluc(P, ip, row, ktile, e * bs.nkeys, bs.ntiles, evt, fp, rec, fluc, draws, wire_cnt, wire_off,
+                             visits, vcap, Q, flags, reinterpret_cast<long long*>(smem_i));
         else
-            raster_tile(P, row, E.ktile0 + (rel - row * E.ntile), e * bs.nkeys, bs.ntiles, rec, tprof, pool,
-                        wide_key, wire_cnt, wire_off, visits, vcap, key_bound, Q,
-                        row_flag + (size_t)e * bs.nwires_total, smem_i, scale, iscale);
+            raster_tile<false>(P, row, ktile, e * bs.nkeys, bs.ntiles, rec, tprof, pool, wide_key, wire_cnt, wire_off,
+                               visits, vcap, key_bound, Q, flags, heavy, item, 0, 1, 0, smem_i, scale, iscale);
+    }
+}
+
+__global__ void __launch_bounds__(kRasterThreads, kHeavyBlocks)
+    k_raster_heavy_batch(const BatchPlan* __restrict__ plan, BatchStatic bs, PlaneSet ps,
+                         const PatchRec* __restrict__ rec, long long recstride, const float* __restrict__ tprof,
+                         TprofPool pool, const unsigned char* __restrict__ wide_key,
+                         const int* __restrict__ wire_cnt, const int* __restrict__ wire_off,
+                         const Visit* __restrict__ visits, long long vcap,
+                         const unsigned long long* __restrict__ key_bound, float* __restrict__ Q,
+                         unsigned char* __restrict__ row_flag, HeavyList heavy)
+{
+    extern __shared__ int smem_i[];
+    __shared__ float scale[kTileBlocks], iscale[kTileBlocks];
+    if (plan->status & kBatchSkip) return;
+    const int total = heavy.count[0];
+    for (int k = blockIdx.x; k < total; k += gridDim.x) {
+        const int4 it = heavy.item[k];
+        int e, ip, row, ktile;
+        const GridPlane P = batch_tile(plan, bs, ps, recstride, it.x, e, ip, row, ktile);
+        raster_tile<true>(P, row, ktile, e * bs.nkeys, bs.ntiles, rec, tprof, pool, wide_key, wire_cnt, wire_off,
+                          visits, vcap, key_bound, Q, row_flag + (size_t)e * bs.nwires_total, heavy, it.x, it.y, it.z,
+                          it.w, smem_i, scale, iscale);
     }
 }
 
@@ -2545,19 +2769,22 @@ void launch_raster_batch(const BatchPlan* plan, const BatchStatic& bs, const Pla
                          const unsigned char* wide_key, const int* wire_cnt, const int* wire_off,
                          const Visit* visits, long long vcap, const unsigned long long* key_bound, float* Q,
                          int nblocks, int maxG, const EventTable& evt, const FlucParams& fp, const FlucRec* fluc,
-                         const int* draws, unsigned char* row_flag, cudaStream_t s)
+                         const int* draws, unsigned char* row_flag, const HeavyList& heavy, int heavy_blocks,
+                         cudaStream_t s)
 {
     const size_t smem = std::max(raster_smem_bytes(maxG), raster_fluc_smem_bytes(maxG));
-    if (fp.on_patch)
+    if (fp.on_patch) {
         k_raster_batch<true><<<nblocks, kRasterThreads, smem, s>>>(plan, bs, ps, rec, recstride, tprof, pool, wide_key,
-                                                                    wire_cnt,
-                                                                    wire_off, visits, vcap, key_bound, Q, evt, fp,
-                                                                    fluc, draws, row_flag);
-    else
-        k_raster_batch<false><<<nblocks, kRasterThreads, smem, s>>>(plan, bs, ps, rec, recstride, tprof, pool,
-                                                                     wide_key, wire_cnt,
-                                                                     wire_off, visits, vcap, key_bound, Q, evt, fp,
-                                                                     fluc, draws, row_flag);
+                                                                    wire_cnt, wire_off, visits, vcap, key_bound, Q,
+                                                                    evt, fp, fluc, draws, row_flag, heavy);
+        return;
+    }
+    k_raster_batch<false><<<nblocks, kRasterThreads, smem, s>>>(plan, bs, ps, rec, recstride, tprof, pool, wide_key,
+                                                                 wire_cnt, wire_off, visits, vcap, key_bound, Q, evt,
+                                                                 fp, fluc, draws, row_flag, heavy);
+    k_raster_heavy_batch<<<heavy_blocks, kRasterThreads, raster_heavy_smem_bytes(maxG), s>>>(plan, bs, ps, rec, recstride, tprof, pool,
+                                                                     wide_key, wire_cnt, wire_off, visits, vcap,
+                                                                     key_bound, Q, row_flag, heavy);
 }
 
 // Time FFT of every charge-grid row of the pass, in place (rows of N reals
@@ -2760,6 +2987,8 @@ void batch_kernel_attributes(int maxG, int maxM)
     const int sf = (int)(2 * (size_t)maxM * sizeof(float2));
     cudaFuncSetAttribute((const void*)k_raster_batch<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, sr);
     cudaFuncSetAttribute((const void*)k_raster_batch<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sr);
+    cudaFuncSetAttribute((const void*)k_raster_heavy_batch, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)raster_heavy_smem_bytes(maxG));
     cudaFuncSetAttribute((const void*)k_rfft_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, sf);
     cudaFuncSetAttribute((const void*)k_irfft_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, sf);
     cudaFuncSetAttribute((const void*)k_conv_fft_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWConvSmem);
