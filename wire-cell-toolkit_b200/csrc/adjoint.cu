@@ -379,11 +379,11 @@ __global__ void __launch_bounds__(kGatherWarps * 32, 5) k_adj_gather(int n, Plan
                     Vc += Vce;
                     Vs += Vse;
                     const float4 tq = s_t[wib][tau];
-                    acc_qn += (double)(tq.x * U);
-                    acc_cp += (double)(tq.x * Vc);
-                    acc_sp += (double)(tq.x * Vs);
-                    acc_ct += (double)(tq.y * U);
-                    acc_st += (double)(tq.z * U);
+                    acc_qn = fma((double)tq.x, (double)U, acc_qn);
+                    acc_cp = fma((double)tq.x, (double)Vc, acc_cp);
+                    acc_sp = fma((double)tq.x, (double)Vs, acc_sp);
+                    acc_ct = fma((double)tq.y, (double)U, acc_ct);
+                    acc_st = fma((double)tq.z, (double)U, acc_st);
                 }
             }
         }
