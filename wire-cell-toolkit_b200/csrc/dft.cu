@@ -13,6 +13,7 @@
 // Inverse transforms use inv(x) = conj(fwd(conj(x))) / N.
 #include <algorithm>
 
+#include "fft3.cuh"
 #include "kernels.cuh"
 #include "rng.cuh"
 
@@ -378,14 +379,80 @@ void launch_digitize(const float* in, long ld_in, float* out, long ld_out, int n
 // group's (coherent, so every channel of a group gets the same waveform).
 // One row per block; N even, N/2 a supported FFT length.
 // ---------------------------------------------------------------------------
+// Box-Muller, sqrt(-2 log u1) cos(2 pi u2), in double precision to about 1e-11
+// and rounded to float.  The series are Taylor's, on the ranges that exact
+// reductions leave: the logarithm as e log 2 + 2 atanh((m - 1) / (m + 1)) with m
+// in [sqrt(1/2), sqrt(2)), sine and cosine within pi / 4 of a quarter turn; the
+// root starts from the single-precision one and takes one Newton step.
+// Integers become doubles by additions: conversions run at a quarter of their
+// rate.  (The library's log, sincospi and sqrt, to the last bit of a double, took
+// four times the operations: 248 us for the noise of a 2560 x 6000 frame, 15 M
+// normals, with the generic transform; now 194 us: half the FP64 chains, a quarter each Philox
+// and transform.)
 __device__ __forceinline__ float noise_normal(unsigned k0, unsigned k1, unsigned stream, unsigned model, int i)
 {
-    Philox g;
-    g.init(k0, k1, stream, model, (unsigned)i);
-    const double u1 = g.uniform(), u2 = g.uniform();
-    double sn, cs;
-    sincospi(2.0 * u2, &sn, &cs);
-    return (float)(sqrt(-2.0 * log(u1)) * cs);  // Box-Muller
+    const uint4 o = philox_block(k0, k1, stream, model, (unsigned)i, 0u);
+    const double u1 = uniform53(o.x, o.y), u2 = uniform53(o.z, o.w);
+    // u1 = m 2^e
+    long long bits = __double_as_longlong(u1);
+    int e = (int)(bits >> 52) - 1023;
+    double m = __longlong_as_double((bits & 0x000fffffffffffffll) | 0x3ff0000000000000ll);
+    if (m > 1.4142135623730951) {
+        m *= 0.5;
+        ++e;
+    }
+    // 1 / d on [1.7, 2.42]: a parabola good to 0.16 %, and two Newton steps
+    const double d = m + 1.0;
+    double r = fma(fma(0.1175, d, -0.7253), d, 1.4810);
+    r = r * fma(-d, r, 2.0);
+    r = r * fma(-d, r, 2.0);
+    const double s = (m - 1.0) * r, s2 = s * s;
+    double p = 1.0 / 13.0;
+    p = fma(p, s2, 1.0 / 11.0);
+    p = fma(p, s2, 1.0 / 9.0);
+    p = fma(p, s2, 1.0 / 7.0);
+    p = fma(p, s2, 1.0 / 5.0);
+    p = fma(p, s2, 1.0 / 3.0);
+    p = fma(p * s2, s, s);  // atanh s
+    const double ed = __hiloint2double(0x43300000, e ^ 0x80000000) - 4503601774854144.0;  // e + 2^31 + 2^52
+    const double x = -2.0 * fma(ed, 0.69314718055994531, 2.0 * p);
+    double y = (double)rsqrtf((float)x);
+    y = y * fma(-0.5 * x * y, y, 1.5);
+    // 4 u2 = q + f, f in [-1/2, 1/2]
+    const double v = 4.0 * u2, w = v + 6755399441055744.0;  // 1.5 2^52: rounds, the quarter in the low bits
+    const double f = (v - (w - 6755399441055744.0)) * 1.5707963267948966, f2 = f * f;
+    double c = 1.0 / 479001600.0, z = 1.0 / 6227020800.0;  // 12!, 13!
+    c = fma(c, f2, -1.0 / 3628800.0);
+    c = fma(c, f2, 1.0 / 40320.0);
+    c = fma(c, f2, -1.0 / 720.0);
+    c = fma(c, f2, 1.0 / 24.0);
+    c = fma(c, f2, -0.5);
+    c = fma(c, f2, 1.0);
+    z = fma(z, f2, -1.0 / 39916800.0);
+    z = fma(z, f2, 1.0 / 362880.0);
+    z = fma(z, f2, -1.0 / 5040.0);
+    z = fma(z, f2, 1.0 / 120.0);
+    z = fma(z, f2, -1.0 / 6.0);
+    z = fma(z * f2, f, f);
+    const int turn = __double2loint(w) & 3;
+    const double t = (turn & 1) ? z : c;
+    return (float)(x * y * (turn == 1 || turn == 2 ? -t : t));
+}
+
+// Bin k of a row's packed noise spectrum: bin 0 = (|X_0|, |X_M|), then X_k (Sk = S[k]).
+__device__ __forceinline__ float2 noise_bin(const float* __restrict__ S, float Sk, int M, int k, unsigned k0,
+                                            unsigned k1, unsigned stream, unsigned model, float s2opi)
+{
+    if (k == 0) {
+        const float m0 = S[0] * s2opi, mh = S[M] * s2opi;
+        const float2 x0 = make_float2(m0 * noise_normal(k0, k1, stream, model, 0),
+                                      m0 * noise_normal(k0, k1, stream, model, M));
+        const float2 xh = make_float2(mh * noise_normal(k0, k1, stream, model, M),
+                                      mh * noise_normal(k0, k1, stream, model, 2 * M));
+        return make_float2(sqrtf(x0.x * x0.x + x0.y * x0.y), sqrtf(xh.x * xh.x + xh.y * xh.y));
+    }
+    const float m = Sk * s2opi;
+    return make_float2(m * noise_normal(k0, k1, stream, model, k), m * noise_normal(k0, k1, stream, model, k + M));
 }
 
 __global__ void k_add_noise(float* frame, long ld, int ncols, const float* __restrict__ spectra, int nspec,
@@ -398,29 +465,12 @@ __global__ void k_add_noise(float* frame, long ld, int ncols, const float* __res
     if (sp < 0) return;
     const unsigned stream = (unsigned)row_stream[row];
     const float* S = spectra + (size_t)sp * nspec;
-    const int M = d.M, N = 2 * M, nhalf = M;
+    const int M = d.M, N = 2 * M;
     const int tid = threadIdx.x, nth = blockDim.x;
     const float s2opi = sqrtf(2.0f / 3.141592f);
     float2* a = nsm;
     float2* b = nsm + M;
-    // packed half spectrum: bin 0 = (|X_0|, |X_M|), bins 1 .. M-1 = X_k
-    for (int k = tid; k < M; k += nth) {
-        float2 v;
-        if (k == 0) {
-            const float m0 = S[0] * s2opi, mh = S[nhalf] * s2opi;
-            const float2 x0 = make_float2(m0 * noise_normal(k0, k1, stream, model, 0),
-                                          m0 * noise_normal(k0, k1, stream, model, nhalf));
-            const float2 xh = make_float2(mh * noise_normal(k0, k1, stream, model, nhalf),
-                                          mh * noise_normal(k0, k1, stream, model, 2 * nhalf));
-            v = make_float2(sqrtf(x0.x * x0.x + x0.y * x0.y), sqrtf(xh.x * xh.x + xh.y * xh.y));
-        }
-        else {
-            const float m = S[k] * s2opi;
-            v = make_float2(m * noise_normal(k0, k1, stream, model, k),
-                            m * noise_normal(k0, k1, stream, model, k + nhalf));
-        }
-        b[k] = v;
-    }
+    for (int k = tid; k < M; k += nth) b[k] = noise_bin(S, S[k], M, k, k0, k1, stream, model, s2opi);
     __syncthreads();
     for (int k = tid; k < M; k += nth) a[k] = c2r_bin(b, k, M, d.twh);
     __syncthreads();
@@ -434,11 +484,79 @@ __global__ void k_add_noise(float* frame, long ld, int ncols, const float* __res
     }
 }
 
+// The same at the lengths with a three-stage transform (fft3.cuh), a persistent
+// block per slot over the rows.
+template <class P>
+struct NoiseShape {  // more resident blocks than the inverse alone asks for: the normals are chains of FP64
+    static constexpr int kBlocks = P::cmax(1, 65536 / (IrfftShape<P>::kThreads * 80));
+};
+
+template <class P>
+__global__ void __launch_bounds__(IrfftShape<P>::kThreads, NoiseShape<P>::kBlocks)
+    k_add_noise3(float* frame, long ld, int nrows, int ncols, const float* __restrict__ spectra, int nspec,
+                 const int* __restrict__ row_spec, const int* __restrict__ row_stream, unsigned k0, unsigned k1,
+                 unsigned model, const float2* __restrict__ t3, const float2* __restrict__ twh)
+{
+    extern __shared__ __align__(16) float2 nsm[];
+    const int tid = threadIdx.x, nth = IrfftShape<P>::kThreads;
+    const float s2opi = sqrtf(2.0f / 3.141592f);
+    const int n = min(ncols, 2 * P::M);
+    for (int row = blockIdx.x; row < nrows; row += gridDim.x) {
+        const int sp = row_spec[row];
+        if (sp < 0) continue;  // uniform
+        const float* S = spectra + (size_t)sp * nspec;
+        const unsigned stream = (unsigned)row_stream[row];
+        float Sk = S[tid];  // M has more bins than the block threads; a bin ahead from here on
+        for (int k = tid; k < P::M; k += nth) {
+            const float Sn = k + nth < P::M ? S[k + nth] : 0.f;
+            nsm[k] = noise_bin(S, Sk, P::M, k, k0, k1, stream, model, s2opi);
+            Sk = Sn;
+        }
+        __syncthreads();
+        float* f = frame + (size_t)row * ld;
+        const bool vec = (reinterpret_cast<uintptr_t>(f) & 7) == 0;
+        const bool staged = (reinterpret_cast<uintptr_t>(f) & 15) == 0;
+        irfft3_row<P, true>(nsm, nsm + P::M, f, 0, n, n, vec, t3, twh, tid, staged,
+                            reinterpret_cast<const float2*>(f));
+        __syncthreads();  // the exchange buffer and the staged row are written again
+    }
+}
+
+template <class P>
+static bool go_add_noise3(float* frame, long ld, int nrows, int ncols, const float* spectra, int nspec,
+                          const int* row_spec, const int* row_stream, unsigned k0, unsigned k1, unsigned model,
+                          const FftDesc& d, cudaStream_t s)
+{
+    static std::atomic<int> cache[kFft3Devices];
+    const int nb = persistent_blocks((const void*)k_add_noise3<P>, IrfftShape<P>::kThreads, P::kSmem, cache);
+    if (nb <= 0) return false;
+    k_add_noise3<P><<<std::min(nrows, nb), IrfftShape<P>::kThreads, P::kSmem, s>>>(
+        frame, ld, nrows, ncols, spectra, nspec, row_spec, row_stream, k0, k1, model, d.t3i, d.twh);
+    return true;
+}
+
+static bool launch_add_noise3(float* frame, long ld, int nrows, int ncols, const float* spectra, int nspec,
+                              const int* row_spec, const int* row_stream, unsigned k0, unsigned k1, unsigned model,
+                              const FftDesc& d, cudaStream_t s)
+{
+    if (!d.t3i) return false;
+    switch (d.M) {
+#define X(A, B, C)                                                                                     \
+    WCT_CASE(A, B, C,                                                                                  \
+             return go_add_noise3<I>(frame, ld, nrows, ncols, spectra, nspec, row_spec, row_stream, k0, k1, model, d, \
+                                     s))
+        WCT_FFT3_PLANS(X)
+#undef X
+        default: return false;
+    }
+}
+
 void launch_add_noise(float* frame, long ld, int nrows, int ncols, const float* spectra, int nspec,
                       const int* row_spec, const int* row_stream, unsigned k0, unsigned k1, unsigned model,
                       const FftDesc& d, cudaStream_t s)
 {
     if (nrows <= 0) return;
+    if (launch_add_noise3(frame, ld, nrows, ncols, spectra, nspec, row_spec, row_stream, k0, k1, model, d, s)) return;
     const size_t sm = 2 * sizeof(float2) * (size_t)d.M;
     cudaFuncSetAttribute((const void*)k_add_noise, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     k_add_noise<<<nrows, dft_threads(d.M), sm, s>>>(frame, ld, ncols, spectra, nspec, row_spec, row_stream, k0, k1,

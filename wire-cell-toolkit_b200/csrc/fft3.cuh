@@ -187,7 +187,10 @@ struct IrfftShape {
     static constexpr int kBlocks = P::cmax(1, 65536 / (kThreads * kRegs));
 };
 
-template <class P>
+// ADD: onto the frame's values (tick0 0, ncols = nticks), which `next` then
+// points to where they are 16-byte aligned (more): they arrive while the row is
+// transformed.
+template <class P, bool ADD = false>
 __device__ __forceinline__ void irfft3_row(const float2* sm_row, float2* ex, float* __restrict__ f, int tick0,
                                            int ncols, int nticks, bool vec, const float2* __restrict__ t3,
                                            const float2* __restrict__ twh, int tid, bool more, const float2* next)
@@ -230,9 +233,10 @@ __device__ __forceinline__ void irfft3_row(const float2* sm_row, float2* ex, flo
         }
     }
     __syncthreads();
-    if (more) fft3::copy_row<P::M>(const_cast<float2*>(sm_row), reinterpret_cast<const float*>(next), 2 * P::M, tid,
-                                   IrfftShape<P>::kThreads);
+    if (more) fft3::copy_row<P::M>(const_cast<float2*>(sm_row), reinterpret_cast<const float*>(next),
+                                   ADD ? ncols : 2 * P::M, tid, IrfftShape<P>::kThreads);
     fft3::stage2<P, +1>(e1, e2, t3, tid);
+    if (ADD) cp_async_wait<0>();
     __syncthreads();
     if (tid < P::NS) {
         float2 v[P::R3];
@@ -241,7 +245,12 @@ __device__ __forceinline__ void irfft3_row(const float2* sm_row, float2* ex, flo
 #pragma unroll
         for (int r = 0; r < P::R3; ++r) {
             const int c0 = 2 * (tid + r * P::NS), t0 = tick0 + c0;
-            const float2 z = make_float2(v[r].x * sc, v[r].y * sc);
+            float2 z = make_float2(v[r].x * sc, v[r].y * sc);
+            if (ADD) {
+                const float* was = more ? reinterpret_cast<const float*>(sm_row) : f;
+                if (c0 < ncols) z.x += was[c0];
+                if (c0 + 1 < ncols) z.y += was[c0 + 1];
+            }
             if (vec && c0 + 1 < ncols && t0 >= 0 && t0 + 1 < nticks) *reinterpret_cast<float2*>(f + t0) = z;
             else {
                 if (c0 < ncols && t0 >= 0 && t0 < nticks) f[t0] = z.x;

@@ -43,11 +43,18 @@ __device__ __forceinline__ uint4 philox_block(uint32_t k0, uint32_t k1, uint32_t
     return make_uint4(x0, x1, x2, x3);
 }
 
-// Uniform double in the open interval (0, 1), 53 random bits.
+// A 32-bit unsigned integer as a double: the low word of 2^52 + w (an addition,
+// where a conversion has a quarter of its rate).
+__device__ __forceinline__ double u32_double(uint32_t w)
+{
+    return __hiloint2double(0x43300000, (int)w) - 4503599627370496.0;
+}
+
+// Uniform double in the open interval (0, 1), 53 random bits: (x + 1/2) 2^-53.
 __device__ __forceinline__ double uniform53(uint32_t hi, uint32_t lo)
 {
-    const uint64_t x = (((uint64_t)hi << 32) | lo) >> 11;
-    return ((double)x + 0.5) * 1.1102230246251565404e-16;  // 2^-53
+    const double x = fma(u32_double(hi), 2097152.0, u32_double(lo >> 11));  // exact
+    return (x + 0.5) * 1.1102230246251565404e-16;
 }
 
 // The uniforms of the stream (key0, key1) x (ctr0, ctr1, ctr2) in order, two a
