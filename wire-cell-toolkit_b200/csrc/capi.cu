@@ -43,15 +43,74 @@ static int fail(int code, const std::string& msg) { return fail(code, msg.c_str(
     } while (0)
 
 // ---------------------------------------------------------------------------
-// Device buffer that only grows.
+// Device memory comes from a pool of the library's own, one per device.  What is
+// freed stays mapped up to kPoolKeep bytes and goes back to the device beyond
+// that: mapping and unmapping was most of a call that takes scratch and waits (a
+// 2560 x 6000 2-D transform by itself: 1.9 ms, 0.2 ms of it kernels; the default
+// pool gives everything back at each synchronisation) and of a new component's
+// first event.  The pool may be used from several threads and streams; calls
+// with scratch take and give it back in the order of their stream.
+// ---------------------------------------------------------------------------
+constexpr unsigned long long kPoolKeep = 1ull << 30;
+constexpr size_t kPoolLargest = 512u << 20;  // larger buffers by cudaMalloc: the pool would not keep them
+constexpr int kPoolDevices = 64;
+static std::mutex g_pool_mtx;
+static cudaMemPool_t g_pools[kPoolDevices] = {};
+
+static cudaError_t device_pool(int dev, cudaMemPool_t& pool)
+{
+    if (dev < 0 || dev >= kPoolDevices) return cudaErrorInvalidDevice;
+    std::lock_guard<std::mutex> lk(g_pool_mtx);
+    if (!g_pools[dev]) {
+        cudaMemPoolProps props{};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = dev;
+        cudaMemPool_t made = nullptr;
+        cudaError_t e = cudaMemPoolCreate(&made, &props);
+        if (e != cudaSuccess) return e;
+        unsigned long long keep = kPoolKeep;
+        e = cudaMemPoolSetAttribute(made, cudaMemPoolAttrReleaseThreshold, &keep);
+        if (e != cudaSuccess) {
+            cudaMemPoolDestroy(made);
+            return e;
+        }
+        g_pools[dev] = made;
+    }
+    pool = g_pools[dev];
+    return cudaSuccess;
+}
+
+// Scratch on the current device, in the order of stream s (freed with cudaFreeAsync).
+static cudaError_t pool_alloc(void** p, size_t bytes, cudaStream_t s)
+{
+    int dev = 0;
+    cudaMemPool_t pool = nullptr;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = device_pool(dev, pool);
+    if (e == cudaSuccess) e = cudaMallocFromPoolAsync(p, bytes, pool, s);
+    return e;
+}
+
+// ---------------------------------------------------------------------------
+// Device buffer that only grows, usable on any stream once ensure() returns.
 // ---------------------------------------------------------------------------
 struct DevBuf {
     void* p{nullptr};
     size_t n{0};
+    int dev{0};
     ~DevBuf() { release(); }
     void release()
     {
-        if (p) cudaFree(p);
+        if (p) {
+            // freeing pool memory waits for nothing: let the device finish with it first
+            int now = 0;
+            cudaGetDevice(&now);
+            if (now != dev) cudaSetDevice(dev);
+            cudaDeviceSynchronize();
+            cudaFree(p);
+            if (now != dev) cudaSetDevice(now);
+        }
         p = nullptr;
         n = 0;
     }
@@ -60,8 +119,16 @@ struct DevBuf {
         if (bytes <= n) return cudaSuccess;
         release();
         size_t b = std::max<size_t>(bytes, 256);
-        cudaError_t e = cudaMalloc(&p, b);
+        cudaError_t e = cudaGetDevice(&dev);
+        if (e == cudaSuccess) {
+            if (b > kPoolLargest) e = cudaMalloc(&p, b);
+            else {
+                e = pool_alloc(&p, b, cudaStreamPerThread);
+                if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamPerThread);
+            }
+        }
         if (e == cudaSuccess) n = b;
+        else p = nullptr;
         return e;
     }
     template <typename T>
@@ -1099,7 +1166,7 @@ struct BatchState {
     BatchStatic bs{};
     std::vector<std::unique_ptr<FftPlanDev>> cls_plans;
     DevBuf d_descs;
-    std::vector<std::unique_ptr<DevBuf>> spec;  // [plane * ncls + cls]: taps, then wire spectra where they apply
+    DevBuf d_spec;                              // response spectra of every plane and length class
     DevBuf d_spec_tab;                          // const float2* [plane][ncls]
     int maxM{0}, maxG{0}, nsm{148};
     int fft3_blocks[kMaxClasses][2]{};  // persistent blocks of each class's time FFT and inverse
@@ -1213,7 +1280,6 @@ static int batch_setup(Core& c)
     long long q = 0, v = 0;
     int wbase = 0;
     b.maxG = 0;
-    b.spec.clear();
     std::vector<const float2*> tab(2 * (size_t)np * bs.ncls);  // taps, then wire spectra
     for (int ip = 0; ip < np; ++ip) {
         PlaneState& ps = *c.planes[ip];
@@ -1235,24 +1301,37 @@ static int batch_setup(Core& c)
         q += (long long)ps.G * pl.nin_max * cls.back();
         v += (long long)(pl.nin_max + 2 * ps.npad) * b.maxM;
         b.maxG = std::max(b.maxG, ps.G);
+    }
+    // every plane's response spectra at every length, in one allocation: the wire
+    // spectra where the overlap-save form applies (their taps are scratch), else the taps
+    size_t total = 0, scratch = 0;
+    auto taps_count = [&](int ip, int k) {
+        return (size_t)c.planes[ip]->G * (2 * c.planes[ip]->npad + 1) * (cls[k] / 2);
+    };
+    for (int ip = 0; ip < np; ++ip)
+        for (int k = 0; k < bs.ncls; ++k) {
+            total += bs.pl[ip].wire_fft ? wire_spec_count(c.planes[ip]->G, cls[k] / 2) : taps_count(ip, k);
+            total = (total + 15) & ~(size_t)15;
+            if (bs.pl[ip].wire_fft) scratch = std::max(scratch, taps_count(ip, k));
+        }
+    DevBuf taps_scratch;
+    CUDA_TRY(b.d_spec.ensure(sizeof(float2) * std::max<size_t>(total, 1)));
+    CUDA_TRY(taps_scratch.ensure(sizeof(float2) * std::max<size_t>(scratch, 1)));
+    float2* at = b.d_spec.as<float2>();
+    for (int ip = 0; ip < np; ++ip) {
+        PlaneState& ps = *c.planes[ip];
         const int rows = ps.G * (2 * ps.npad + 1);
         for (int k = 0; k < bs.ncls; ++k) {
             const int N = cls[k];
-            auto sp = std::make_unique<DevBuf>();
-            CUDA_TRY(sp->ensure(sizeof(float2) * (size_t)rows * (N / 2)));
-            launch_rfft_rows(ps.d_table.as<float>(), ps.ldr, std::min(ps.nresp, N), sp->as<float2>(), N / 2, rows,
+            const bool wire = bs.pl[ip].wire_fft;
+            float2* taps = wire ? taps_scratch.as<float2>() : at;
+            launch_rfft_rows(ps.d_table.as<float>(), ps.ldr, std::min(ps.nresp, N), taps, N / 2, rows,
                              b.cls_plans[k]->desc, c.own_stream);
+            if (wire) launch_wire_spec(taps, at, ps.G, ps.npad, N / 2, c.own_stream);
             CUDA_TRY(cudaGetLastError());
-            tab[(size_t)ip * bs.ncls + k] = sp->as<float2>();
-            if (pl.wire_fft) {
-                auto ws = std::make_unique<DevBuf>();
-                CUDA_TRY(ws->ensure(sizeof(float2) * wire_spec_count(ps.G, N / 2)));
-                launch_wire_spec(sp->as<float2>(), ws->as<float2>(), ps.G, ps.npad, N / 2, c.own_stream);
-                CUDA_TRY(cudaGetLastError());
-                tab[((size_t)np + ip) * bs.ncls + k] = ws->as<float2>();
-                b.spec.push_back(std::move(ws));
-            }
-            b.spec.push_back(std::move(sp));
+            tab[((wire ? (size_t)np : 0) + ip) * bs.ncls + k] = at;
+            const size_t used = wire ? wire_spec_count(ps.G, N / 2) : taps_count(ip, k);
+            at += (used + 15) & ~(size_t)15;
         }
     }
     bs.qslot_total = q;
@@ -1804,7 +1883,7 @@ static int four_step_rows(const float2* in, float2* out, int nrows, int N, int s
     const int chunk = std::max(1, std::min(65535, (int)std::min<long long>(nrows, (1LL << 28) / N)));
     AsyncBuf w;
     w.s = s;
-    CUDA_TRY(cudaMallocAsync(&w.p, sizeof(float2) * (size_t)chunk * N, s));
+    CUDA_TRY(pool_alloc(&w.p, sizeof(float2) * (size_t)chunk * N, s));
     float2* W = static_cast<float2*>(w.p);
     for (int r0 = 0; r0 < nrows; r0 += chunk) {
         const int nb = std::min(chunk, nrows - r0);
@@ -1855,7 +1934,7 @@ static int dft_rows(const float2* in, long ld_in, float2* out, long ld_out, int 
             const int chunk = std::max(1, std::min(nrows, (int)std::min<long long>(65535, (1LL << 28) / P)));
             AsyncBuf z;
             z.s = s;
-            CUDA_TRY(cudaMallocAsync(&z.p, sizeof(float2) * (size_t)chunk * P, s));
+            CUDA_TRY(pool_alloc(&z.p, sizeof(float2) * (size_t)chunk * P, s));
             float2* Z = static_cast<float2*>(z.p);
             for (int r0 = 0; r0 < nrows; r0 += chunk) {
                 const int nb = std::min(chunk, nrows - r0);
@@ -1897,7 +1976,7 @@ static int dft_1b_dev(const float2* in, float2* out, int nrows, int ncols, int a
     if (rc0) return rc0;
     AsyncBuf t;
     t.s = s;
-    CUDA_TRY(cudaMallocAsync(&t.p, sizeof(float2) * (size_t)nrows * ncols, s));
+    CUDA_TRY(pool_alloc(&t.p, sizeof(float2) * (size_t)nrows * ncols, s));
     float2* tp = static_cast<float2*>(t.p);
     launch_transpose_c(in, tp, nrows, ncols, s);
     int rc = dft_rows(tp, nrows, tp, nrows, ncols, nrows, sign, s);
@@ -1924,7 +2003,7 @@ static int dft_transpose_dev(const float* in, float* out, int nrows, int ncols, 
     t.s = s;
     void* dst = out;
     if (in == out) {  // through scratch
-        CUDA_TRY(cudaMallocAsync(&t.p, bytes, s));
+        CUDA_TRY(pool_alloc(&t.p, bytes, s));
         dst = t.p;
     }
     if (cplx)
@@ -1948,7 +2027,7 @@ static int dft_host(const float* in, float* out, int nrows, int ncols, int kind,
     {
         AsyncBuf d;
         d.s = s;
-        CUDA_TRY(cudaMallocAsync(&d.p, bytes, s));
+        CUDA_TRY(pool_alloc(&d.p, bytes, s));
         CUDA_TRY(cudaMemcpyAsync(d.p, in, bytes, cudaMemcpyHostToDevice, s));
         float2* dp = static_cast<float2*>(d.p);
         if (kind == 0) rc = dft_1b_dev(dp, dp, nrows, ncols, axis, sign, s);
@@ -2202,7 +2281,7 @@ int wct_convolve_rows_device(const float* in, long ld_in, int nrows, int n_in, c
     cudaStream_t s = (cudaStream_t)stream;
     const int M = nfft / 2;
     float2* scratch = nullptr;
-    CUDA_TRY(cudaMallocAsync(&scratch, sizeof(float2) * (size_t)M * (nrows + 1), s));
+    CUDA_TRY(pool_alloc(reinterpret_cast<void**>(&scratch), sizeof(float2) * (size_t)M * (nrows + 1), s));
     rc = convolve_on(in, ld_in, nrows, n_in, resp, n_resp, nfft, out, ld_out, n_out, d, scratch + M, scratch, s);
     cudaError_t e = cudaFreeAsync(scratch, s);
     if (rc) return rc;
@@ -2998,10 +3077,10 @@ int wct_add_noise(float* frame, int nrows, int ncols, const float* spectra, int 
     {
         AsyncBuf f, sp, rs, rt;
         f.s = sp.s = rs.s = rt.s = s;
-        CUDA_TRY(cudaMallocAsync(&f.p, fb, s));
-        CUDA_TRY(cudaMallocAsync(&sp.p, sb, s));
-        CUDA_TRY(cudaMallocAsync(&rs.p, sizeof(int) * (size_t)nrows, s));
-        CUDA_TRY(cudaMallocAsync(&rt.p, sizeof(int) * (size_t)nrows, s));
+        CUDA_TRY(pool_alloc(&f.p, fb, s));
+        CUDA_TRY(pool_alloc(&sp.p, sb, s));
+        CUDA_TRY(pool_alloc(&rs.p, sizeof(int) * (size_t)nrows, s));
+        CUDA_TRY(pool_alloc(&rt.p, sizeof(int) * (size_t)nrows, s));
         CUDA_TRY(cudaMemcpyAsync(f.p, frame, fb, cudaMemcpyHostToDevice, s));
         if (nspectra)
             CUDA_TRY(cudaMemcpyAsync(sp.p, spectra, sizeof(float) * (size_t)nspectra * nspec, cudaMemcpyHostToDevice,
@@ -3053,8 +3132,8 @@ int wct_digitize(const float* frame, int nrows, int ncols, const float* row_base
     {
         AsyncBuf d, b;
         d.s = b.s = s;
-        CUDA_TRY(cudaMallocAsync(&d.p, bytes, s));
-        CUDA_TRY(cudaMallocAsync(&b.p, sizeof(float) * (size_t)nrows, s));
+        CUDA_TRY(pool_alloc(&d.p, bytes, s));
+        CUDA_TRY(pool_alloc(&b.p, sizeof(float) * (size_t)nrows, s));
         CUDA_TRY(cudaMemcpyAsync(d.p, frame, bytes, cudaMemcpyHostToDevice, s));
         CUDA_TRY(cudaMemcpyAsync(b.p, row_baseline, sizeof(float) * (size_t)nrows, cudaMemcpyHostToDevice, s));
         float* dp = static_cast<float*>(d.p);
@@ -3157,10 +3236,10 @@ int wct_dt_splat(wct_depotransform* h, const wct_splat_config* cfg, const double
     AsyncBuf dd, df;
     dd.s = df.s = s;
     if (ndepos) {
-        CUDA_TRY(cudaMallocAsync(&dd.p, sizeof(double) * 7 * ndepos, s));
+        CUDA_TRY(pool_alloc(&dd.p, sizeof(double) * 7 * ndepos, s));
         CUDA_TRY(cudaMemcpyAsync(dd.p, depos, sizeof(double) * 7 * ndepos, cudaMemcpyHostToDevice, s));
     }
-    CUDA_TRY(cudaMallocAsync(&df.p, fbytes, s));
+    CUDA_TRY(pool_alloc(&df.p, fbytes, s));
     rc = wct_dt_splat_device(h, cfg, static_cast<const double*>(dd.p), ndepos, static_cast<float*>(df.p), s);
     if (rc) return rc;
     CUDA_TRY(cudaMemcpyAsync(frame, df.p, fbytes, cudaMemcpyDeviceToHost, s));
