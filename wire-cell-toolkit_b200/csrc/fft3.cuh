@@ -275,7 +275,7 @@ inline int persistent_blocks(const void* f, int threads, size_t smem, std::atomi
         if (n > 0) return n;
     }
     int nsm = 0, per = 0;
-    if (smem > 48 * 1024 &&
+    if (smem > 40 * 1024 &&  // (a kernel's own static arrays count towards the 48 KB too)
         cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
         return 0;
     if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
