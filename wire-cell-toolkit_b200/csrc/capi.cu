@@ -605,6 +605,7 @@ static int prepare_event(Core& c, const double* d_depos, size_t ndepos, cudaStre
     tb.tmin = c.start_time;
     tb.tmax = c.start_time + c.readout_time;
     tb.bs = (tb.tmax - tb.tmin) / tb.nbins;
+    tb.rbs = 1.0 / tb.bs;
 
     PlaneSet& pset = ev.pset;
     pset = PlaneSet{};
@@ -1431,6 +1432,7 @@ static int forward_batch_device(Core& c, const double* d_depos, const long long*
     tb.tmin = c.start_time;
     tb.tmax = c.start_time + c.readout_time;
     tb.bs = (tb.tmax - tb.tmin) / tb.nbins;
+    tb.rbs = 1.0 / tb.bs;
     for (int attempt = 0; attempt < 8; ++attempt) {
         const long long nkeysK = (long long)K * bs.nkeys;
         std::vector<void*> before = {b.d_Q.p, b.d_V.p, b.d_rec.p, b.d_tprof.p, b.d_win.p, b.d_wcnt.p, b.d_woff.p,
@@ -2402,6 +2404,7 @@ int wct_dt_add_plane(wct_depotransform* h, int face, const wct_plane_desc* d, in
     pd.imp_max = d->pitchmax + 0.5 * regionsize;
     pd.imp_nbins = d->nwires * d->nimpacts;
     pd.imp_bs = (pd.imp_max - pd.imp_min) / pd.imp_nbins;
+    pd.imp_rbs = 1.0 / pd.imp_bs;
     const FaceState& f = c.faces[face];
     pd.have_bb = f.have_bb ? 1 : 0;
     for (int i = 0; i < 3; ++i) {
@@ -3160,6 +3163,7 @@ static int splat_setup(const wct_depotransform* h, const wct_splat_config* cfg, 
     sp.tb.tmin = cfg->window_start;
     sp.tb.tmax = cfg->window_start + nbins * cfg->tick;
     sp.tb.bs = (sp.tb.tmax - sp.tb.tmin) / nbins;
+    sp.tb.rbs = 1.0 / sp.tb.bs;
     sp.nsigma = cfg->nsigma;
     sp.speed = cfg->drift_speed;
     sp.time_shift = cfg->response_plane / cfg->drift_speed;

@@ -36,9 +36,16 @@ namespace wctb200 {
 // ---------------------------------------------------------------------------
 // helpers
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ int bin_of(double v, double lo, double bs)
+// Binning::bin (Binning.h:75), the truncated quotient. The product with the
+// width's reciprocal is within 3 parts in 2^53 of the quotient, so away from a
+// whole number both truncate to the same bin; next to one (and for NaN and
+// out-of-range values) the division decides.
+__device__ __forceinline__ int bin_of(double v, double lo, double bs, double rbs)
 {
-    return __double2int_rz(__ddiv_rn(__dsub_rn(v, lo), bs));  // Binning::bin, Binning.h:75
+    const double d = __dsub_rn(v, lo);
+    const double a = __dmul_rn(d, rbs);
+    if (fabs(a) < 1e8 && fabs(a - rint(a)) > 1e-6) return __double2int_rz(a);
+    return __double2int_rz(__ddiv_rn(d, bs));
 }
 __device__ __forceinline__ double edge_of(int i, double lo, double bs)
 {
@@ -48,6 +55,25 @@ __device__ __forceinline__ double gdistance(double x, double c, double s)
 {
     return s != 0.0 ? __ddiv_rn(__dsub_rn(x, c), s) : __dsub_rn(x, c);  // GaussianDiffusion.h:34-44
 }
+
+// gdistance(x, c, s) > eff or, with below, < -eff. The product eff * s is far
+// closer to the border than 1e-12 of the two sides, so away from it the sign
+// of the difference decides; next to it the division does.
+__device__ __forceinline__ bool beyond(double x, double c, double s, double eff, bool below)
+{
+    const double d = below ? __dsub_rn(c, x) : __dsub_rn(x, c);
+    const double m = eff * s;
+    const double diff = d - m;
+    if (s > 1e-200 && fabs(diff) > 1e-12 * (fabs(d) + fabs(m))) return diff > 0.0;
+    return below ? gdistance(x, c, s) < -eff : gdistance(x, c, s) > eff;
+}
+
+__device__ __forceinline__ unsigned long long warp_min_u64(unsigned long long v)
+{
+    const unsigned hi = (unsigned)(v >> 32), mh = __reduce_min_sync(0xffffffffu, hi);
+    return ((unsigned long long)mh << 32) | __reduce_min_sync(0xffffffffu, hi == mh ? (unsigned)v : 0xffffffffu);
+}
+__device__ __forceinline__ unsigned long long warp_max_u64(unsigned long long v) { return ~warp_min_u64(~v); }
 
 template <typename T, typename Op>
 __device__ __forceinline__ T warp_reduce(T v, Op op)
@@ -74,24 +100,26 @@ __device__ __forceinline__ T warp_reduce(T v, Op op)
 // ---------------------------------------------------------------------------
 // Visit keys of one patch: (wire, tick tile) pairs for the wires
 // [w0, w0 + wspan) and tiles [k0, k0 + kspan); key = wire * ntiles + tile.
-// Warp-aggregated increment of the per-key visit counters.
-__device__ __forceinline__ void count_visits(int* cnt, int wbase, int w0, int wspan, int k0, int kspan, int ntiles)
+// Warp-aggregated increment of the per-key visit counters; keys that hold a
+// long patch are marked (their raster block spreads visits over warps).
+__device__ __forceinline__ void count_visits(int* cnt, unsigned char* wide, bool lng, int wbase, int w0, int wspan,
+                                             int k0, int kspan, int ntiles)
 {
     const int span = wspan * kspan;
-    int maxspan = span;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) maxspan = max(maxspan, __shfl_xor_sync(0xffffffffu, maxspan, o));
+    const int maxspan = __reduce_max_sync(0xffffffffu, span);
     const int lane = threadIdx.x & 31;
+    const unsigned longs = __ballot_sync(0xffffffffu, lng);
+    int key = (wbase + w0) * ntiles + k0, left = kspan;
     for (int k = 0; k < maxspan; ++k) {
-        int key = -1;
-        if (k < span) {
-            const int dw = k / kspan, dk = k - dw * kspan;
-            key = (wbase + w0 + dw) * ntiles + k0 + dk;
+        const unsigned m = __match_any_sync(0xffffffffu, k < span ? key : -1);
+        if (k < span && lane == __ffs(m) - 1) {
+            atomicAdd(cnt + key, __popc(m));
+            if (m & longs) wide[key] = 1;
         }
-        const unsigned act = __ballot_sync(0xffffffffu, key >= 0);
-        if (key >= 0) {
-            const unsigned m = __match_any_sync(act, key);
-            if (lane == __ffs(m) - 1) atomicAdd(cnt + key, __popc(m));
+        ++key;
+        if (--left == 0) {  // next wire
+            left = kspan;
+            key += ntiles - kspan;
         }
     }
 }
@@ -167,6 +195,9 @@ __device__ __noinline__ int drift_draw(unsigned key0, unsigned key1, int i_ev, i
     return binomial(nq, absorb, g);
 }
 
+// Depo counters of a plane in one word, six bits each: a warp's sum fits.
+constexpr unsigned kAdded = 1u, kOutTime = 1u << 6, kOutPitch = 1u << 12, kOversize = 1u << 18, kBig = 1u << 24;
+
 // One thread per (depo, plane) of every event of the table (plane =
 // blockIdx.y; each plane's threads drift the depo again, which is cheaper
 // than serialising the planes' FP64 chains in one thread); per-event window
@@ -174,6 +205,18 @@ __device__ __noinline__ int drift_draw(unsigned key0, unsigned key1, int i_ev, i
 // records [plane][depo]; plane 0's threads also write the drifted charge and
 // the time profiles indexed by the depo's position in the concatenated depo
 // array.
+//
+// Issue-bound at size (520k depos: 1460 instructions a warp, 70% of the issue
+// slots), a chain of FP64 operations when small. Quotients that only place a
+// patch or cut a depo are products away from the border (bin_of, beyond),
+// warp sums are redux instructions with the counters packed in one word, the
+// time window is found once, and profiles leave in 16-byte stores: 520k depos
+// x 3 planes 113 -> 85 us, 20k x 3 12.0 -> 9.1, 2k 13.8 -> 8.6, 500k on tracks
+// with long patches 484 -> 375 (there the bounds' atomics on shared wires; a
+// warp's adding up per block first: no gain, and 9 -> 20 us at 20k).
+// FLUC: charges fluctuate as they drift (kept apart: the sampler's call costs
+// the other case 0.2 KB of spills).
+template <bool FLUC>
 __global__ void __launch_bounds__(256, 4) k_prep_all(const double* __restrict__ dep, EventTable evt, int nkeys,
                                                   DriftDev dd, int do_drift, PlaneSet ps, TimeDev tb,
                                                   double drift_speed, double nsigma, PatchRec* __restrict__ rec,
@@ -220,7 +263,7 @@ __global__ void __launch_bounds__(256, 4) k_prep_all(const double* __restrict__ 
                     const double dt = fabs(__ddiv_rn(__dsub_rn(respx, x), dd.speed));
                     if (dir > 0) {
                         const double absorb = __dsub_rn(1.0, exp(__ddiv_rn(-dt, dd.lifetime)));
-                        if (fp.on_drift) {
+                        if (FLUC) {
                             // Binomial(|Q|, absorb) electrons absorbed (Drifter.cxx:179-185)
                             const int nabs = drift_draw(
                                 fp.key0, fp.key1 + 0x9E3779B9u * (unsigned)fluc_ident(fp, ev), i - evt.dep0[ev],
@@ -245,27 +288,36 @@ __global__ void __launch_bounds__(256, 4) k_prep_all(const double* __restrict__ 
     if (fq && in) fq[(size_t)ip * n + i] = q;  // the plane's charge: trial count of its fluctuated patch
     // The time profile depends on the depo only (GaussianDiffusion.cxx:124-136):
     // compute it once here for every plane's raster.
-    unsigned long long mywide = 0;
-    if (ok && ip == 0) {
-        const double st = __ddiv_rn(el, drift_speed);
-        const double tlo = __dsub_rn(t, __dmul_rn(st, nsigma));
-        const double thi = __dadd_rn(t, __dmul_rn(st, nsigma));
-        const int t0 = max(bin_of(tlo, tb.tmin, tb.bs), 0);
-        const int t1 = min(bin_of(thi, tb.tmin, tb.bs) + 1, tb.nbins);
+    // its window is every plane's.
+    unsigned mywide = 0;
+    double st = 0, tlo = 0, thi = 0;
+    int t0 = 0, t1 = 0;
+    float tcr = 0.f;
+    if (ok) {
+        st = __ddiv_rn(el, drift_speed);  // DepoTransform.cxx:185
+        tlo = __dsub_rn(t, __dmul_rn(st, nsigma));
+        thi = __dadd_rn(t, __dmul_rn(st, nsigma));
+        t0 = max(bin_of(tlo, tb.tmin, tb.bs, tb.rbs), 0);
+        t1 = min(bin_of(thi, tb.tmin, tb.bs, tb.rbs) + 1, tb.nbins);
+        tcr = (float)__dsub_rn(t, edge_of(t0, tb.tmin, tb.bs));
         const int nt = t1 - t0;
-        if (nt > kTprof) mywide = nt;
-        if (nt > 0 && nt <= kTprof) {
+        if (ip == 0 && nt > kTprof) mywide = nt;
+        if (ip == 0 && nt > 0 && nt <= kTprof) {
             float* tp = tprof + (size_t)i * kTprof;
             if (st > 0) {
                 const float fst = (float)st;
-                const float tcr = (float)__dsub_rn(t, edge_of(t0, tb.tmin, tb.bs));
                 const float inv = 1.0f / (1.41421356237309505f * fst);
                 const float tbs = (float)tb.bs;
                 float e1 = edge_erfc(0.f, tbs, tcr, inv);
-                for (int k = 0; k < nt; ++k) {
-                    const float e2 = edge_erfc((float)(k + 1), tbs, tcr, inv);
-                    tp[k] = bin_from_edges(e1, e2);
-                    e1 = e2;
+                for (int k = 0; k < nt; k += 4) {  // (a row is 64 bytes; past the patch: not read)
+                    float v[4];
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const float e2 = edge_erfc((float)(k + j + 1), tbs, tcr, inv);
+                        v[j] = bin_from_edges(e1, e2);
+                        e1 = e2;
+                    }
+                    *reinterpret_cast<float4*>(tp + k) = make_float4(v[0], v[1], v[2], v[3]);
                 }
             }
             else {
@@ -274,16 +326,12 @@ __global__ void __launch_bounds__(256, 4) k_prep_all(const double* __restrict__ 
         }
     }
     __shared__ unsigned long long s_k[4][8];
-    __shared__ int s_c[5][8];
+    __shared__ unsigned s_c[4][8];
     const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-    auto umin = [](unsigned long long a, unsigned long long b) { return a < b ? a : b; };
-    auto umax = [](unsigned long long a, unsigned long long b) { return a > b ? a : b; };
-    auto iadd = [](int a, int b) { return a + b; };
-    unsigned long long myvis = 0, mycells = 0;
     {
         const PlaneDev& pl = ps.p[ip];
         unsigned long long kpmin = ~0ull, kpmax = 0ull, ktmin = ~0ull, ktmax = 0ull;
-        int nadd = 0, nout_t = 0, nout_p = 0, nover = 0, nbig = 0;
+        unsigned flags = 0;  // six bits for each of kAdd ...: a warp's sum stays apart
         PatchRec r;
         r.toff = r.poff = 0;
         r.nt = r.np = 0;
@@ -300,42 +348,37 @@ __global__ void __launch_bounds__(256, 4) k_prep_all(const double* __restrict__ 
         }
         if (inbb) {
             const double ct = t;
-            const double st = __ddiv_rn(el, drift_speed);                         // DepoTransform.cxx:185
             const double rx = __dsub_rn(x, pl.ox), ry = __dsub_rn(y, pl.oy), rz = __dsub_rn(z, pl.oz);
             const double cp = __dadd_rn(__dadd_rn(__dmul_rn(pl.ax, rx), __dmul_rn(pl.ay, ry)),
                                         __dmul_rn(pl.az, rz));                  // Pimpos.cxx:58
             const double sp = et;
             const double eff_t = st > 0 ? nsigma : 0.0;
             const double eff_p = sp > 0 ? nsigma : 0.0;
-            if (gdistance(tb.tmin, ct, st) > eff_t || gdistance(tb.tmax, ct, st) < -eff_t) {
-                nout_t = 1;
+            if (beyond(tb.tmin, ct, st, eff_t, false) || beyond(tb.tmax, ct, st, eff_t, true)) {
+                flags = kOutTime;
             }
-            else if (gdistance(pl.imp_min, cp, sp) > eff_p || gdistance(pl.imp_max, cp, sp) < -eff_p) {
-                nout_p = 1;
+            else if (beyond(pl.imp_min, cp, sp, eff_p, false) || beyond(pl.imp_max, cp, sp, eff_p, true)) {
+                flags = kOutPitch;
             }
             else {
-                nadd = 1;
-                const double tlo = __dsub_rn(ct, __dmul_rn(st, nsigma));
-                const double thi = __dadd_rn(ct, __dmul_rn(st, nsigma));
+                flags = kAdded;
                 const double plo = __dsub_rn(cp, __dmul_rn(sp, nsigma));
                 const double phi = __dadd_rn(cp, __dmul_rn(sp, nsigma));
                 ktmin = dkey(tlo); ktmax = dkey(thi);
                 kpmin = dkey(plo); kpmax = dkey(phi);
-                const int t0 = max(bin_of(tlo, tb.tmin, tb.bs), 0);
-                const int t1 = min(bin_of(thi, tb.tmin, tb.bs) + 1, tb.nbins);
-                const int p0 = max(bin_of(plo, pl.imp_min, pl.imp_bs), 0);
-                const int p1 = min(bin_of(phi, pl.imp_min, pl.imp_bs) + 1, pl.imp_nbins);
+                const int p0 = max(bin_of(plo, pl.imp_min, pl.imp_bs, pl.imp_rbs), 0);
+                const int p1 = min(bin_of(phi, pl.imp_min, pl.imp_bs, pl.imp_rbs) + 1, pl.imp_nbins);
                 if (t1 > t0 && p1 > p0) {
                     const int nt = t1 - t0, np = p1 - p0;
                     if (nt > kMaxPatchT || np > kMaxPatchP || (st == 0.0 && nt != 1) || (sp == 0.0 && np != 1)) {
-                        nover = 1;
+                        flags += kOversize;
                     }
                     else {
                         r.toff = t0;
                         r.poff = p0;
                         r.nt = (unsigned short)nt;
                         r.np = (unsigned short)np;
-                        r.tcr = (float)__dsub_rn(ct, edge_of(t0, tb.tmin, tb.bs));
+                        r.tcr = tcr;
                         r.pcr = (float)__dsub_rn(cp, edge_of(p0, pl.imp_min, pl.imp_bs));
                         r.st = (float)st;
                         r.sp = (float)sp;
@@ -352,30 +395,30 @@ __global__ void __launch_bounds__(256, 4) k_prep_all(const double* __restrict__ 
                             sum_p = bin_from_edges(edge_erfc(0.f, (float)pl.imp_bs, r.pcr, inv),
                                                    edge_erfc((float)np, (float)pl.imp_bs, r.pcr, inv));
                         }
-                        r.qn = (float)(q / ((double)sum_t * (double)sum_p));
+                        // the quotient by a Newton step on the float reciprocal (2^-46, far
+                        // below the float that is kept)
+                        const double sn = (double)sum_t * (double)sum_p;
+                        if (sn > 1e-30) {
+                            const double r0 = (double)__frcp_rn((float)sn);
+                            r.qn = (float)(q * fma(r0, fma(-sn, r0, 1.0), r0));
+                        }
+                        else r.qn = (float)(q / sn);
                     }
                 }
             }
         }
         if (in) rec[(size_t)ip * n + i] = r;
-        const int w0 = r.np ? r.poff / pl.nimp : 0;
-        const int span = r.np ? (r.poff + r.np - 1) / pl.nimp - w0 + 1 : 0;
+        const int w0 = r.np ? (int)((unsigned)r.poff / (unsigned)pl.nimp) : 0;
+        const int span = r.np ? (int)((unsigned)(r.poff + r.np - 1) / (unsigned)pl.nimp) - w0 + 1 : 0;
         const int k0 = r.toff / kTile;
         const int kspan = r.np ? (r.toff + r.nt - 1) / kTile - k0 + 1 : 0;
-        count_visits(wire_cnt, pl.wire_base, w0, span, k0, kspan, ps.ntiles);
-        myvis += (unsigned long long)span * (unsigned long long)kspan;
-        mycells += (unsigned long long)r.np * (unsigned long long)r.nt;
-        if (r.nt > kTprof) {  // keys that hold a long patch: their raster block spreads visits over warps
-            unsigned char* wk = wide_all + (size_t)ev * nkeys;
-            for (int ww = 0; ww < span; ++ww)
-                for (int kk = 0; kk < kspan; ++kk) wk[(pl.wire_base + w0 + ww) * ps.ntiles + k0 + kk] = 1;
-        }
+        count_visits(wire_cnt, wide_all + (size_t)ev * nkeys, r.nt > kTprof, pl.wire_base, w0, span, k0, kspan, ps.ntiles);
         // fixed-point bounds of the raster: per (wire, tile, 64-tick block), summed
         // as integers in units of 2^-16 (each term rounded up), so the bound --
         // and with it the raster's scale -- does not depend on the order of the adds
         if (r.np) {
             const float b = visit_bound(r.qn, r.sp, r.st, (float)pl.imp_bs, (float)tb.bs);
-            if (b > kMaxVisitBound) nbig = 1;
+            if (b > kMaxVisitBound) flags += kBig;
             const unsigned long long bu = __float2ull_ru(fminf(b, kMaxVisitBound) * 65536.0f);
             const int b0 = r.toff / kScaleBlock, b1 = (r.toff + r.nt - 1) / kScaleBlock;
             for (int ww = 0; ww < span; ++ww) {
@@ -383,73 +426,53 @@ __global__ void __launch_bounds__(256, 4) k_prep_all(const double* __restrict__ 
                 for (int bb = b0; bb <= b1; ++bb) atomicAdd(kb + bb, bu);
             }
         }
-        // block reduction, one atomic per block per quantity
-        kpmin = warp_reduce(kpmin, umin);
-        ktmin = warp_reduce(ktmin, umin);
-        kpmax = warp_reduce(kpmax, umax);
-        ktmax = warp_reduce(ktmax, umax);
-        nadd = warp_reduce(nadd, iadd);
-        nout_t = warp_reduce(nout_t, iadd);
-        nout_p = warp_reduce(nout_p, iadd);
-        nover = warp_reduce(nover, iadd);
-        nbig = warp_reduce(nbig, iadd);
+        // block reduction, one atomic per block per quantity (the totals all go
+        // to one address, where a thread's own atomics queue up: 500k depos,
+        // half with long patches, 484 us with one per thread and long patch).
+        // 32 bits hold a block's totals: a patch has at most 2^20 cells.
+        kpmin = warp_min_u64(kpmin);
+        ktmin = warp_min_u64(ktmin);
+        kpmax = warp_max_u64(kpmax);
+        ktmax = warp_max_u64(ktmax);
+        flags = __reduce_add_sync(0xffffffffu, flags);
+        const unsigned vis = __reduce_add_sync(0xffffffffu, (unsigned)(span * kspan));
+        const unsigned cells = __reduce_add_sync(0xffffffffu, (unsigned)r.np * r.nt);
+        if (ip == 0) mywide = __reduce_add_sync(0xffffffffu, mywide);
         if (l == 0) {
             s_k[0][w] = kpmin; s_k[1][w] = kpmax; s_k[2][w] = ktmin; s_k[3][w] = ktmax;
-            s_c[0][w] = nadd; s_c[1][w] = nout_t; s_c[2][w] = nout_p; s_c[3][w] = nover; s_c[4][w] = nbig;
+            s_c[0][w] = flags; s_c[1][w] = vis; s_c[2][w] = cells; s_c[3][w] = mywide;
         }
         __syncthreads();
-        if (w == 0) {
-            const int nw = blockDim.x >> 5;
-            kpmin = l < nw ? s_k[0][l] : ~0ull;
-            kpmax = l < nw ? s_k[1][l] : 0ull;
-            ktmin = l < nw ? s_k[2][l] : ~0ull;
-            ktmax = l < nw ? s_k[3][l] : 0ull;
-            nadd = l < nw ? s_c[0][l] : 0;
-            nout_t = l < nw ? s_c[1][l] : 0;
-            nout_p = l < nw ? s_c[2][l] : 0;
-            nover = l < nw ? s_c[3][l] : 0;
-            nbig = l < nw ? s_c[4][l] : 0;
-            kpmin = warp_reduce(kpmin, umin);
-            ktmin = warp_reduce(ktmin, umin);
-            kpmax = warp_reduce(kpmax, umax);
-            ktmax = warp_reduce(ktmax, umax);
-            nadd = warp_reduce(nadd, iadd);
-            nout_t = warp_reduce(nout_t, iadd);
-            nout_p = warp_reduce(nout_p, iadd);
-            nover = warp_reduce(nover, iadd);
-            nbig = warp_reduce(nbig, iadd);
-            WindowDev* wd = win + ip;
-            if (l == 0 && nadd) {
-                atomicMin(&wd->pmin, kpmin);
-                atomicMax(&wd->pmax, kpmax);
-                atomicMin(&wd->tmin, ktmin);
-                atomicMax(&wd->tmax, ktmax);
-                atomicAdd(&wd->nadded, nadd);
+        // a thread a quantity over the block's warps
+        const int nw = blockDim.x >> 5;
+        WindowDev* wd = win + ip;
+        if (threadIdx.x < 4) {
+            const int k = threadIdx.x;
+            unsigned long long v = s_k[k][0];
+            for (int j = 1; j < nw; ++j) v = k & 1 ? max(v, s_k[k][j]) : min(v, s_k[k][j]);
+            if (v != (k & 1 ? 0ull : ~0ull)) {
+                if (k == 0) atomicMin(&wd->pmin, v);
+                else if (k == 1) atomicMax(&wd->pmax, v);
+                else if (k == 2) atomicMin(&wd->tmin, v);
+                else atomicMax(&wd->tmax, v);
             }
-            if (l == 0 && nout_t) atomicAdd(&wd->out_time, nout_t);
-            if (l == 0 && nout_p) atomicAdd(&wd->out_pitch, nout_p);
-            if (l == 0 && nover) atomicAdd(&wd->oversize, nover);
-            if (l == 0 && nbig) atomicAdd(&wd->bigcharge, nbig);
         }
-    }
-    // 64-bit totals of the event (visits: the lists use int offsets), one
-    // atomic per block and quantity: they all go to one address, where a
-    // thread's own atomics queue up (500k depos, half with long patches: 484 us
-    // with one per thread and long patch)
-    __shared__ unsigned long long s_tot[3][8];
-    unsigned long long tot[3] = {myvis, mycells, mywide};
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) tot[k] += __shfl_xor_sync(0xffffffffu, tot[k], o);
-        if (l == 0) s_tot[k][w] = tot[k];
-    }
-    __syncthreads();
-    if (threadIdx.x < 3) {
-        unsigned long long v = 0;
-        for (int k = 0; k < (int)(blockDim.x >> 5); ++k) v += s_tot[threadIdx.x][k];
-        unsigned long long* to = threadIdx.x == 0 ? &win[0].nvisits : (threadIdx.x == 1 ? &win[0].ncells : &win[0].wide_ticks);
-        if (v) atomicAdd(to, v);
+        else if (threadIdx.x >= 32 && threadIdx.x < 32 + 5) {
+            const int k = threadIdx.x - 32;
+            unsigned v = 0;
+            for (int j = 0; j < nw; ++j) v += (s_c[0][j] >> (6 * k)) & 63u;
+            int* to = k == 0 ? &wd->nadded : k == 1 ? &wd->out_time : k == 2 ? &wd->out_pitch
+                                                   : k == 3 ? &wd->oversize : &wd->bigcharge;
+            if (v) atomicAdd(to, (int)v);
+        }
+        else if (threadIdx.x >= 64 && threadIdx.x < 64 + 3) {
+            // 64-bit totals of the event (visits: the lists use int offsets)
+            const int k = threadIdx.x - 64;
+            unsigned long long v = 0;
+            for (int j = 0; j < nw; ++j) v += s_c[1 + k][j];
+            unsigned long long* to = k == 0 ? &win[0].nvisits : (k == 1 ? &win[0].ncells : &win[0].wide_ticks);
+            if (v) atomicAdd(to, v);
+        }
     }
 }
 
@@ -462,9 +485,9 @@ void launch_prep_all(const double* depos, const EventTable& et, int nkeys, const
     const int nb = et.blk0[et.nev];
     const int b0 = std::max(0, blk_begin), b1 = blk_end < 0 ? nb : std::min(blk_end, nb);
     if (b1 <= b0) return;
-    k_prep_all<<<dim3(b1 - b0, ps.nplanes), 256, 0, s>>>(depos, et, nkeys, dd, do_drift, ps, tb, drift_speed,
-                                                         nsigma, rec, win, wire_cnt, tprof, key_bound, fp, fq, wide,
-                                                         b0, qscale);
+    auto* k = fp.on_drift ? k_prep_all<true> : k_prep_all<false>;
+    k<<<dim3(b1 - b0, ps.nplanes), 256, 0, s>>>(depos, et, nkeys, dd, do_drift, ps, tb, drift_speed, nsigma, rec, win,
+                                                wire_cnt, tprof, key_bound, fp, fq, wide, b0, qscale);
 }
 
 // Exclusive scan of the per-key visit counts: block sums, a scan of the

@@ -27,6 +27,7 @@ struct PlaneDev {
     int nwires, nimp;
     int imp_nbins;
     double imp_min, imp_max, imp_bs;
+    double imp_rbs;           // 1 / imp_bs
     int have_bb;
     double bb_lo[3], bb_hi[3];
     int wire_base;            // first entry of this plane in per-wire arrays
@@ -43,6 +44,7 @@ struct PlaneSet {
 struct TimeDev {
     int nbins;
     double tmin, tmax, bs;
+    double rbs;  // 1 / bs
 };
 
 // Per (plane, depo) patch description, written by the prep kernel.
