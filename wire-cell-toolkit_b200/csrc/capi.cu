@@ -742,6 +742,14 @@ static int prepare_event(Core& c, const double* d_depos, size_t ndepos, cudaStre
     if (qfloats >= (size_t)1 << 40) return fail(WCT_ERR_SIZE, "charge grid too large");
     CUDA_TRY(c.d_Q.ensure(sizeof(float) * std::max<size_t>(qfloats, 1)));
     CUDA_TRY(c.d_V.ensure(sizeof(float2) * std::max<size_t>(vcomplex, 1)));
+    for (int ip = 0; ip < np; ++ip) {
+        GridPlane& g = gset.p[ip];
+        if (!g.nin) continue;
+        FftDesc d;
+        int rc = c.plan_for(g.N / 2, d);
+        if (rc) return rc;
+        g.sparse = rfft3_takes(c.d_Q.as<float>() + g.qoff, g.N, d);
+    }
     return WCT_OK;
 }
 
@@ -931,7 +939,11 @@ static int forward_device(Core& c, const double* d_depos, size_t ndepos, float* 
                 float* Q = c.d_Q.as<float>() + g.qoff;
                 float2* V = c.d_V.as<float2>() + ev.voff[ip];
                 Core::StageTimer t_f(&c, 2, ps_s);
-                launch_rfft_rows(Q, N, N, reinterpret_cast<float2*>(Q), M, ps.G * nin, d, ps_s);
+                launch_rfft_rows(Q, N, N, reinterpret_cast<float2*>(Q), M, ps.G * nin, d, ps_s,
+                                 g.sparse ? TileMap{c.d_wcnt.as<int>() + (size_t)g.wire_base * gset.ntiles_abs,
+                                                    g.nwires, gset.ntiles_abs, g.start_ch, g.nin, g.col0, g.ktile0,
+                                                    g.ntile}
+                                          : TileMap{});
                 t_f.close(1);
                 Core::StageTimer t_c(&c, 3, ps_s);
                 if (ps.have_wspec && wire_fft_pays(ps.npad, nout))
@@ -1551,7 +1563,7 @@ static int forward_batch_device(Core& c, const double* d_depos, const long long*
                 for (int k = 0; k < bs.ncls; ++k)
                     if (bs.cls_fft3[k])
                         launch_rfft3_batch(plans + ch, bs, k, b.cls_plans[k]->desc, b.fft3_blocks[k][0],
-                                           b.d_Q.as<float>(), s);
+                                           b.d_Q.as<float>(), b.d_wcnt.as<int>(), s);
                 if (b.any_rows)
                     launch_rfft_batch(plans + ch, b.d_descs.as<FftDesc>(), b.d_Q.as<float>(), nb_f,
                                       b.tune.fft_threads, b.maxM, s);

@@ -64,6 +64,12 @@ __device__ __forceinline__ void cp_async16(void* smem, const void* gmem, int src
     const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(sa), "l"(gmem), "r"(src_bytes) : "memory");
 }
+// The 4-byte form.
+__device__ __forceinline__ void cp_async4(void* smem, const void* gmem)
+{
+    const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(sa), "l"(gmem) : "memory");
+}
 // The 8-byte form (cached in L1 on the way, the only cache operator it has).
 __device__ __forceinline__ void cp_async8(void* smem, const void* gmem, int src_bytes)
 {

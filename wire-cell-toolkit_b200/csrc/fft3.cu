@@ -8,20 +8,42 @@ namespace wctb200 {
 
 template <class P>
 __global__ void __launch_bounds__(RfftShape<P>::kThreads, RfftShape<P>::kBlocks) k_rfft3(const float* in, long in_ld, int in_len,
-                                                                  float2* out, long out_ld, int nrows,
+                                                                  float2* out, long out_ld, int nrows, TileMap tiles,
                                                                   const float2* __restrict__ t3,
                                                                   const float2* __restrict__ twh)
 {
     extern __shared__ __align__(16) float2 f3sm[];
+    __shared__ int s_cnt[2][kMaxRowTiles];  // a sparse grid's counts, a row ahead of its copy
     const int tid = threadIdx.x;
+    const bool sparse = tiles.cnt != nullptr;
+    const int off = tiles.col0 - tiles.ktile0 * kTile;
     int row = blockIdx.x;
-    if (row < nrows) fft3::copy_row<P::M>(f3sm, in + (size_t)row * in_ld, in_len, tid, RfftShape<P>::kThreads);
-    for (; row < nrows; row += gridDim.x) {
+    if (row >= nrows) return;
+    auto counts = [&](int buf, int r) {
+        if (sparse && r < nrows) fft3::ask_counts(s_cnt[buf], tiles, tiles.start_ch + r % tiles.nin, tid);
+    };
+    auto copy = [&](int buf, int r) {
+        const float* x = in + (size_t)r * in_ld;
+        if (sparse) fft3::copy_tiles<P::M>(f3sm, x, s_cnt[buf], off, tid, RfftShape<P>::kThreads);
+        else fft3::copy_row<P::M>(f3sm, x, in_len, tid, RfftShape<P>::kThreads);
+    };
+    if (sparse) {
+        counts(0, row);
+        cp_async_commit();
+        cp_async_wait<0>();
+        __syncthreads();
+    }
+    counts(1, row + gridDim.x);
+    copy(0, row);
+    for (int buf = 0; row < nrows; row += gridDim.x, buf ^= 1) {
         cp_async_wait<0>();
         __syncthreads();
         const int next = row + gridDim.x;
-        rfft3_row<P>(f3sm, f3sm + P::M, out + (size_t)row * out_ld, t3, twh, tid, next < nrows,
-                     in + (size_t)next * in_ld, in_len);
+        rfft3_row<P>(f3sm, f3sm + P::M, out + (size_t)row * out_ld, t3, twh, tid, [&] {
+            if (next >= nrows) return;
+            counts(buf, next + gridDim.x);
+            copy(buf ^ 1, next);
+        });
     }
 }
 
@@ -56,13 +78,14 @@ __global__ void __launch_bounds__(IrfftShape<P>::kThreads, IrfftShape<P>::kBlock
 
 template <class P>
 static bool go_rfft3(const float* in, long in_ld, int in_len, float2* out, long out_ld, int nrows, const FftDesc& d,
-                     cudaStream_t s)
+                     const TileMap& tiles, cudaStream_t s)
 {
     static std::atomic<int> cache[kFft3Devices];
     const int nb = persistent_blocks((const void*)k_rfft3<P>, RfftShape<P>::kThreads, P::kSmem, cache);
     if (nb <= 0) return false;
-    k_rfft3<P><<<std::min(nrows, nb), RfftShape<P>::kThreads, P::kSmem, s>>>(in, in_ld, in_len, out, out_ld, nrows,
-                                                                            d.t3f, d.twh);
+    if (nrows > 0)
+        k_rfft3<P><<<std::min(nrows, nb), RfftShape<P>::kThreads, P::kSmem, s>>>(in, in_ld, in_len, out, out_ld, nrows,
+                                                                                tiles, d.t3f, d.twh);
     return true;
 }
 
@@ -99,16 +122,21 @@ int fft3_next(int M)
 }
 
 bool launch_rfft3(const float* in, long in_ld, int in_len, float2* out, long out_ld, int nrows, const FftDesc& d,
-                  cudaStream_t s)
+                  const TileMap& tiles, cudaStream_t s)
 {
     // whole 16-byte pieces of every row
     if (!d.t3f || (reinterpret_cast<uintptr_t>(in) & 15) || in_ld % 4) return false;
     switch (d.M) {
-#define X(A, B, C) WCT_CASE(A, B, C, return go_rfft3<P>(in, in_ld, in_len, out, out_ld, nrows, d, s))
+#define X(A, B, C) WCT_CASE(A, B, C, return go_rfft3<P>(in, in_ld, in_len, out, out_ld, nrows, d, tiles, s))
         WCT_FFT3_PLANS(X)
 #undef X
         default: return false;
     }
+}
+
+bool rfft3_takes(const float* in, long in_ld, const FftDesc& d)
+{
+    return launch_rfft3(in, in_ld, 0, nullptr, 0, 0, d, TileMap{}, nullptr);
 }
 
 bool launch_irfft3(const float2* Vh, int r0, int r1, const FftDesc& d, int wire0, int tick0, int ncols, int nticks,

@@ -28,6 +28,7 @@
 #include <atomic>
 
 #include "fft.cuh"
+#include "kernels.cuh"
 
 namespace wctb200 {
 
@@ -115,11 +116,37 @@ __device__ __forceinline__ void copy_row(float2* s, const float* __restrict__ x,
     cp_async_commit();
 }
 
+// The same for a row of 2 M values of a charge grid: tiles without visits
+// (s_cnt, per tile of the row) were not written and count as zero. A piece
+// that two tiles share is read if one of them has visits; the raster zeroes
+// the other's part of it.
+template <int M>
+__device__ __forceinline__ void copy_tiles(float2* s, const float* __restrict__ x, const int* s_cnt, int off, int tid,
+                                           int nth)
+{
+    for (int p = tid; p < M / 2; p += nth) {
+        const int q = 4 * p + off;  // tick past the first tile's first
+        const bool live = s_cnt[q / kTile] | s_cnt[(q + 3) / kTile];
+        cp_async16(s + 2 * p, x + 4 * p, live ? 16 : 0);
+    }
+    cp_async_commit();
+}
+
+// Asks for the visit counts of a row's tiles (wire w; outside the plane or
+// the readout: as if visited, the raster writes those); the caller commits.
+__device__ __forceinline__ void ask_counts(int* s_cnt, const TileMap& t, int w, int tid)
+{
+    if (tid >= t.ntile) return;
+    const int k = t.ktile0 + tid;
+    if (w >= 0 && w < t.nwires && k >= 0 && k < t.ntiles_abs) cp_async4(s_cnt + tid, t.cnt + w * t.ntiles_abs + k);
+    else s_cnt[tid] = 1;
+}
+
 }  // namespace fft3
 
 // ---------------------------------------------------------------------------
 // Real rows (in_len values, zeros beyond) -> M packed bins, in place allowed:
-// one row, staged in sm_row; the next one is asked for once it is taken.
+// one row, staged in sm_row; ask() copies the next one there once it is taken.
 // ---------------------------------------------------------------------------
 template <class P>
 struct RfftShape {
@@ -129,10 +156,10 @@ struct RfftShape {
     static constexpr int kBlocks = P::cmax(1, 65536 / (kThreads * kRegs));
 };
 
-template <class P>
+template <class P, class Ask>
 __device__ __forceinline__ void rfft3_row(const float2* sm_row, float2* ex, float2* __restrict__ o,
                                           const float2* __restrict__ t3, const float2* __restrict__ twh, int tid,
-                                          bool more, const float* next, int len)
+                                          Ask ask)
 {
     float2* e1 = ex;
     float2* e2 = P::kShare ? ex : ex + P::E1;
@@ -145,7 +172,7 @@ __device__ __forceinline__ void rfft3_row(const float2* sm_row, float2* ex, floa
         for (int r = 0; r < P::R1; ++r) e1[r * P::S1 + tid] = v[r];
     }
     __syncthreads();  // the staged row has been taken too
-    if (more) fft3::copy_row<P::M>(const_cast<float2*>(sm_row), next, len, tid, RfftShape<P>::kThreads);
+    ask();
     fft3::stage2<P, -1>(e1, e2, t3, tid);
     __syncthreads();
     const int a = tid;

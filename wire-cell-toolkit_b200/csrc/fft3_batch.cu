@@ -57,28 +57,49 @@ __device__ __forceinline__ int entry_of(const int* pre, int n, int item)
 template <class P>
 __global__ void __launch_bounds__(RfftShape<P>::kThreads, RfftShape<P>::kBlocks)
     k_rfft3_batch(const BatchPlan* __restrict__ plan, BatchStatic bs, int cls, float* Q,
-                  const float2* __restrict__ t3, const float2* __restrict__ twh)
+                  const int* __restrict__ wire_cnt, const float2* __restrict__ t3, const float2* __restrict__ twh)
 {
     extern __shared__ __align__(16) float2 f3sm[];
     __shared__ int s_pre[kMaxBatch * kMaxPlanes + 1];
     if (plan->status & kBatchSkip) return;
     const int tid = threadIdx.x;
     const int ne = plan->nev * plan->np, total = class_rows<false>(plan, bs, cls, s_pre);
-    auto at = [&](int row) {
-        const int k = entry_of(s_pre, ne, row);
-        return Q + plan->ep[k].qoff + (size_t)(row - s_pre[k]) * (2 * P::M);
-    };
+    __shared__ int s_cnt[2][kMaxRowTiles];
     int row = blockIdx.x;
     if (row >= total) return;
-    float* x = at(row);
-    fft3::copy_row<P::M>(f3sm, x, 2 * P::M, tid, RfftShape<P>::kThreads);
-    for (; row < total; row += gridDim.x) {
-        const int next = row + gridDim.x;
-        float* xn = next < total ? at(next) : x;
+    // visit counts of row r's tiles; its address and the offset of its first column in its first tile
+    auto ask = [&](int buf, int r, float*& x, int& off) {
+        if (r >= total) return;
+        const int k = entry_of(s_pre, ne, r), e = k / plan->np, ip = k - e * plan->np;
+        const EvPlane& E = plan->ep[k];
+        const int rel = r - s_pre[k];
+        const TileMap t{wire_cnt + (size_t)e * bs.nkeys + (size_t)bs.pl[ip].wire_base * bs.ntiles, bs.pl[ip].nwires,
+                        bs.ntiles, E.start_ch, E.nin, E.start_tick, E.ktile0, E.ntile};
+        fft3::ask_counts(s_cnt[buf], t, E.start_ch + rel % E.nin, tid);
+        x = Q + E.qoff + (size_t)rel * (2 * P::M);
+        off = E.start_tick - E.ktile0 * kTile;
+    };
+    float *x = nullptr, *xn = nullptr;
+    int off = 0, offn = 0;
+    ask(0, row, x, off);
+    cp_async_commit();
+    cp_async_wait<0>();
+    __syncthreads();
+    ask(1, row + gridDim.x, xn, offn);
+    fft3::copy_tiles<P::M>(f3sm, x, s_cnt[0], off, tid, RfftShape<P>::kThreads);
+    for (int buf = 0; row < total; row += gridDim.x, buf ^= 1) {
         cp_async_wait<0>();
         __syncthreads();
-        rfft3_row<P>(f3sm, f3sm + P::M, reinterpret_cast<float2*>(x), t3, twh, tid, next < total, xn, 2 * P::M);
+        const int next = row + gridDim.x;
+        float* xnn = nullptr;
+        rfft3_row<P>(f3sm, f3sm + P::M, reinterpret_cast<float2*>(x), t3, twh, tid, [&] {
+            if (next >= total) return;
+            const int o = offn;
+            ask(buf, next + gridDim.x, xnn, offn);
+            fft3::copy_tiles<P::M>(f3sm, xn, s_cnt[buf ^ 1], o, tid, RfftShape<P>::kThreads);
+        });
         x = xn;
+        xn = xnn;
     }
 }
 
@@ -149,12 +170,12 @@ bool fft3_batch_blocks(int M, int* blocks)
 }
 
 void launch_rfft3_batch(const BatchPlan* plan, const BatchStatic& bs, int cls, const FftDesc& d, int nblocks,
-                        float* Q, cudaStream_t s)
+                        float* Q, const int* wire_cnt, cudaStream_t s)
 {
     switch (d.M) {
 #define X(A, B, C)                                                                                     \
     WCT_CASE(A, B, C,                                                                                  \
-             k_rfft3_batch<P><<<nblocks, RfftShape<P>::kThreads, P::kSmem, s>>>(plan, bs, cls, Q, d.t3f, d.twh); \
+             k_rfft3_batch<P><<<nblocks, RfftShape<P>::kThreads, P::kSmem, s>>>(plan, bs, cls, Q, wire_cnt, d.t3f, d.twh); \
              return)
         WCT_FFT3_PLANS(X)
 #undef X

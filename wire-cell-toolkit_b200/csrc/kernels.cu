@@ -743,6 +743,27 @@ static_assert(kRasterThreads == kHeavyPart, "a part is a block's chunk");
 // heavy tile (slot: its entry of heavy.done); otherwise the whole tile, or its
 // listing under tile_id.  Called by all threads of the block; smem_i holds the
 // dynamic shared memory of raster_smem_bytes(P.G).
+// A tile without work in this launch: its G rows are zero. Of one without
+// visits in a sparse grid the transform reads only the 16-byte pieces that it
+// shares with a neighbour.
+__device__ __forceinline__ void zero_tile(const GridPlane& P, int row, int qc0, bool unread, float* __restrict__ Q)
+{
+    if (unread) {
+        const int o = qc0 & 3;
+        if (o == 0) return;
+        for (int k = threadIdx.x; k < P.G * 4; k += blockDim.x) {
+            const int g = k >> 2, j = k & 3;
+            const int qc = j < 4 - o ? qc0 + j : qc0 + kTile - 4 + j;
+            if (qc >= 0 && qc < P.N) Q[P.qoff + ((size_t)g * P.nin + row) * P.N + qc] = 0.f;
+        }
+        return;
+    }
+    for (int k = threadIdx.x; k < P.G * kTile; k += blockDim.x) {
+        const int g = k / kTile, qc = qc0 + k - g * kTile;
+        if (qc >= 0 && qc < P.N) Q[P.qoff + ((size_t)g * P.nin + row) * P.N + qc] = 0.f;
+    }
+}
+
 template <bool HEAVY>
 __device__ __forceinline__ void raster_tile(const GridPlane& P, int row, int ktile, int key_base, int ntiles_abs,
                                             const PatchRec* __restrict__ rec, const float* __restrict__ tprof,
@@ -763,13 +784,14 @@ __device__ __forceinline__ void raster_tile(const GridPlane& P, int row, int kti
     float* stage = reinterpret_cast<float*>(smem_i + (size_t)G * kGridLd);
     int4* stagei = reinterpret_cast<int4*>(stage + (size_t)kRasterThreads * kStageStride);
     int4* longq = stagei + kRasterThreads;  // heavy parts only
-    int cnt = 0;
+    int cnt = 0, held = 1;
     const Visit* list = nullptr;
     int key = -1;
     if (w >= 0 && w < P.nwires && ktile >= 0 && ktile < ntiles_abs) {
         key = key_base + (P.wire_base + w) * ntiles_abs + ktile;
         const int off = wire_off[key];
-        cnt = off < 0 ? 0 : (int)min((long long)wire_cnt[key], max(0ll, vcap - off));  // no reads past the list
+        held = wire_cnt[key];
+        cnt = off < 0 ? 0 : (int)min((long long)held, max(0ll, vcap - off));  // no reads past the list
         list = visits + max(off, 0);
     }
     const bool spread = cnt > 0 && wide_key[key];
@@ -785,13 +807,7 @@ __device__ __forceinline__ void raster_tile(const GridPlane& P, int row, int kti
         if (parts == 1) return;  // written whole by its only part
     }
     if (cnt == 0 || listed) {
-        // no visit (block-uniform), or parts to come: the tile's G rows are zero
-        const int qc0 = tick_lo - P.col0;
-        for (int k = tid; k < G * kTile; k += kRasterThreads) {
-            const int g = k / kTile, c = k - g * kTile;
-            const int qc = qc0 + c;
-            if (qc >= 0 && qc < P.N) Q[P.qoff + ((size_t)g * P.nin + row) * P.N + qc] = 0.f;
-        }
+        zero_tile(P, row, tick_lo - P.col0, P.sparse && held == 0, Q);  // no visit (block-uniform), or parts to come
         return;
     }
     if (tid == 0) row_flag[P.wire_base + w] = 1;  // the wire holds charge (every block of the row writes the same)
@@ -1476,20 +1492,18 @@ __device__ __forceinline__ void raster_tile_fluc(const GridPlane& P, int ip, int
     const int tick_lo = ktile * kTile;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const int nwarps = blockDim.x >> 5;
-    int cnt = 0;
+    int cnt = 0, held = 1;
     const Visit* list = nullptr;
     if (w >= 0 && w < P.nwires && ktile >= 0 && ktile < ntiles_abs) {
         const int key = key_base + (P.wire_base + w) * ntiles_abs + ktile;
         const int off = wire_off[key];
-        cnt = off < 0 ? 0 : (int)min((long long)wire_cnt[key], max(0ll, vcap - off));
+        held = wire_cnt[key];
+        cnt = off < 0 ? 0 : (int)min((long long)held, max(0ll, vcap - off));
         list = visits + max(off, 0);
     }
     const int qc0 = tick_lo - P.col0;
-    if (cnt == 0) {  // no visit (block-uniform): the tile's G rows are zero
-        for (int k = tid; k < G * kTile; k += blockDim.x) {
-            const int g = k / kTile, qc = qc0 + k - g * kTile;
-            if (qc >= 0 && qc < P.N) Q[P.qoff + ((size_t)g * P.nin + row) * P.N + qc] = 0.f;
-        }
+    if (cnt == 0) {  // no visit (block-uniform)
+        zero_tile(P, row, qc0, P.sparse && held == 0, Q);
         return;
     }
     if (tid == 0) row_flag[P.wire_base + w] = 1;
@@ -1866,10 +1880,10 @@ static bool launch_rfft_pf(const float* in, long in_ld, int in_len, float2* out,
 }
 
 void launch_rfft_rows(const float* in, long in_ld, int in_len, float2* out, long out_ld, int nrows, const FftDesc& d,
-                      cudaStream_t s)
+                      cudaStream_t s, const TileMap& tiles)
 {
     if (nrows <= 0) return;
-    if (launch_rfft3(in, in_ld, in_len, out, out_ld, nrows, d, s)) return;
+    if (launch_rfft3(in, in_ld, in_len, out, out_ld, nrows, d, tiles, s)) return;
     const bool aligned = ((reinterpret_cast<uintptr_t>(in) & 7) == 0) && (in_ld % 2 == 0);
     if (aligned && d.M % 16 == 0 && d.nst >= 2 && d.radix[0] == 8 && 4 * (size_t)d.M * sizeof(float2) <= 128 * 1024) {
         if (d.M / 8 <= 256 && launch_rfft_pf<1>(in, in_ld, in_len, out, out_ld, nrows, d, s)) return;
@@ -2729,6 +2743,7 @@ __device__ __forceinline__ GridPlane batch_tile(const BatchPlan* __restrict__ pl
     P.row_base = 0;
     P.ktile0 = E.ktile0;
     P.ntile = E.ntile;
+    P.sparse = bs.cls_fft3[E.cls];  // taken by k_rfft3_batch
     const int rel = item - plan->pre_raster[k];
     row = rel / E.ntile;
     ktile = E.ktile0 + (rel - row * E.ntile);

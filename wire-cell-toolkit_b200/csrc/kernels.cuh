@@ -97,7 +97,19 @@ struct GridPlane {
     long long recoff;         // offset of this plane's PatchRecs
     int row_base;             // first block of this plane in the raster grid
     int ktile0, ntile;        // absolute tick tiles covering grid columns [0, N)
+    bool sparse;              // the row transform skips tiles without visits: the raster leaves them unwritten
 };
+
+// The visit counts of a plane's grid rows, for a row transform that does not
+// read tiles without visits (cnt null: every tile is read). Row i of a group
+// is wire start_ch + i, column c tick col0 + c.
+struct TileMap {
+    const int* cnt;           // [nwires][ntiles_abs]
+    int nwires, ntiles_abs;
+    int start_ch, nin;
+    int col0, ktile0, ntile;
+};
+constexpr int kMaxRowTiles = 64;  // tiles of a row: planned lengths have at most 12000 columns
 
 struct GridSet {
     int nplanes;
@@ -281,7 +293,7 @@ void launch_raster_wires(const PatchRec* rec, const float* tprof, const TprofPoo
 // (row_flag[wire_base + wire] = 1 for every wire with a visit; heavy_blocks 0:
 // the event has neither patches over kTprof ticks nor enough visits for a heavy tile)
 void launch_rfft_rows(const float* in, long in_ld, int in_len, float2* out, long out_ld, int nrows,
-                      const FftDesc& d, cudaStream_t s);
+                      const FftDesc& d, cudaStream_t s, const TileMap& tiles = TileMap{});
 void launch_wire_conv(const float2* Qh, const float2* Rh, float2* Vh, int ngroups, int npad, int nrows_in,
                       int nrows_out, int M, bool pair, cudaStream_t s);
 // Three-stage row transforms (fft3.cu): false where the length has no plan or
@@ -289,7 +301,9 @@ void launch_wire_conv(const float2* Qh, const float2* Rh, float2* Vh, int ngroup
 // the plan's radices in forward order.
 bool fft3_radices(int M, int* r);
 bool launch_rfft3(const float* in, long in_ld, int in_len, float2* out, long out_ld, int nrows, const FftDesc& d,
-                  cudaStream_t s);
+                  const TileMap& tiles, cudaStream_t s);
+// launch_rfft3 takes rows at this address (a grid may then be sparse).
+bool rfft3_takes(const float* in, long in_ld, const FftDesc& d);
 bool launch_irfft3(const float2* Vh, int r0, int r1, const FftDesc& d, int wire0, int tick0, int ncols, int nticks,
                    float* frame, const unsigned char* row_flag, int nwires, int npad, cudaStream_t s);
 bool launch_cfft3(const float2* in, long ld_in, float2* out, long ld_out, int nrows, const FftDesc& d, int sign,
@@ -301,7 +315,7 @@ int fft3_next(int M);
 // false where M has no plan; call it before a graph capture.
 bool fft3_batch_blocks(int M, int* blocks);
 void launch_rfft3_batch(const BatchPlan* plan, const BatchStatic& bs, int cls, const FftDesc& d, int nblocks,
-                        float* Q, cudaStream_t s);
+                        float* Q, const int* wire_cnt, cudaStream_t s);
 void launch_irfft3_batch(const BatchPlan* plan, const BatchStatic& bs, int cls, const FftDesc& d, int nblocks,
                          const float2* V, float* frames, long long fstride, const unsigned char* row_flag,
                          cudaStream_t s);
