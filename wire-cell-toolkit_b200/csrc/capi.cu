@@ -578,7 +578,7 @@ static FlucParams fluc_params(const Core& c, bool fluct, int ident0, const int* 
 
 // The d_wide buffer: a byte per key, one per wire, then two counters.
 static size_t wide_counters(size_t nkeys, size_t nwires) { return (nkeys + nwires + 15) & ~(size_t)15; }
-static size_t wide_bytes(size_t nkeys, size_t nwires) { return wide_counters(nkeys, nwires) + 2 * sizeof(int); }
+static size_t wide_bytes(size_t nkeys, size_t nwires) { return wide_counters(nkeys, nwires) + 4 * sizeof(int); }
 
 // h_depos (optional): the depos in host memory, uploaded into d_depos here
 // in chunks on the copy stream, each chunk's prep blocks launched as soon as
@@ -848,16 +848,15 @@ static int forward_device(Core& c, const double* d_depos, size_t ndepos, float* 
 
     unsigned char* row_flag = c.d_wide.as<unsigned char>() + ev.nkeys;
     HeavyList heavy{};
-    int heavy_blocks = 0;
+    int nsm = 0;
     if (!ev.fp.on_patch && (wide > 0 || total_visits > 2 * kHeavyPart)) {
         const size_t parts = heavy_items(total_visits, ev.nkeys);
-        CUDA_TRY(c.d_heavy.ensure(sizeof(int4) * parts + sizeof(int) * (size_t)ev.nkeys));
-        int nsm = 0;
+        CUDA_TRY(c.d_heavy.ensure(sizeof(int4) * parts + 2 * sizeof(int) * (size_t)ev.nkeys));
         CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c.device));
-        heavy_blocks = kHeavyBlocks * nsm;
         heavy.count = reinterpret_cast<int*>(c.d_wide.as<char>() + wide_counters(ev.nkeys, pset.nwires_total));
         heavy.item = c.d_heavy.as<int4>();
         heavy.done = reinterpret_cast<int*>(heavy.item + parts);
+        heavy.mid = heavy.done + ev.nkeys;
     }
     Core::StageTimer t_r(&c, 1, s);
     launch_fill(c.d_rec.as<PatchRec>(), ev.et, ev.nkeys, pset, c.d_wcur.as<int>(), c.d_wlist.as<Visit>(),
@@ -881,7 +880,7 @@ static int forward_device(Core& c, const double* d_depos, size_t ndepos, float* 
         launch_raster_wires(c.d_rec.as<PatchRec>(), c.d_tprof.as<float>(), pool, c.d_wide.as<unsigned char>(),
                             c.d_wcnt.as<int>(),
                             c.d_woff.as<int>(), c.d_wlist.as<Visit>(), (long long)std::max(total_visits, 1),
-                            c.d_kbound.as<unsigned long long>(), gset, c.d_Q.as<float>(), row_flag, heavy, heavy_blocks, s);
+                            c.d_kbound.as<unsigned long long>(), gset, c.d_Q.as<float>(), row_flag, heavy, nsm, s);
     t_r.close((n > 0 ? 1 : 0) + (ev.fp.on_patch && n > 0 ? 1 : 0) + (!ev.fp.on_patch && wide > 0 ? 1 : 0) +
               (rows > 0 ? 1 : 0));
     CUDA_TRY(cudaGetLastError());
@@ -1463,7 +1462,7 @@ static int forward_batch_device(Core& c, const double* d_depos, const long long*
         CUDA_TRY(b.d_kbound.ensure(sizeof(unsigned long long) * (size_t)nkeysK * kTileBlocks));
         CUDA_TRY(b.d_wide.ensure(wide_bytes((size_t)nkeysK, (size_t)K * bs.nwires_total)));
         const size_t parts = heavy_items(b.vcap, nkeysK);
-        CUDA_TRY(b.d_heavy.ensure(sizeof(int4) * parts + sizeof(int) * (size_t)nkeysK));
+        CUDA_TRY(b.d_heavy.ensure(sizeof(int4) * parts + 2 * sizeof(int) * (size_t)nkeysK));
         CUDA_TRY(b.d_wlist.ensure(sizeof(Visit) * (size_t)b.vcap));
         CUDA_TRY(b.d_plans.ensure(sizeof(BatchPlan) * (size_t)nch));
         CUDA_TRY(b.d_ident.ensure(sizeof(int)));
@@ -1526,7 +1525,8 @@ static int forward_batch_device(Core& c, const double* d_depos, const long long*
                 cudaMemsetAsync(b.d_wide.p, 0, wide_bytes((size_t)nk, nflags), s);
                 const HeavyList heavy{reinterpret_cast<int*>(b.d_wide.as<char>() + wide_counters((size_t)nk, nflags)),
                                       b.d_heavy.as<int4>(),
-                                      reinterpret_cast<int*>(b.d_heavy.as<int4>() + parts)};
+                                      reinterpret_cast<int*>(b.d_heavy.as<int4>() + parts),
+                                      reinterpret_cast<int*>(b.d_heavy.as<int4>() + parts) + nkeysK};
                 unsigned char* row_flag = b.d_wide.as<unsigned char>() + nk;
                 k_win_init<<<(ne * np + 63) / 64, 64, 0, s>>>(b.d_win.as<WindowDev>(), ne * np);
                 // random streams keyed by the frame ident of each event: base (a device
@@ -1559,7 +1559,7 @@ static int forward_batch_device(Core& c, const double* d_depos, const long long*
                 launch_raster_batch(plans + ch, bs, pset, b.d_rec.as<PatchRec>(), et.dep0[ne], b.d_tprof.as<float>(),
                                     pool, b.d_wide.as<unsigned char>(), b.d_wcnt.as<int>(), b.d_woff.as<int>(), b.d_wlist.as<Visit>(), b.vcap,
                                     b.d_kbound.as<unsigned long long>(), b.d_Q.as<float>(), nb_r, b.maxG, et, fp,
-                                    b.d_fluc.as<FlucRec>(), b.d_draws.as<int>(), row_flag, heavy, kHeavyBlocks * b.nsm, s);
+                                    b.d_fluc.as<FlucRec>(), b.d_draws.as<int>(), row_flag, heavy, b.nsm, s);
                 for (int k = 0; k < bs.ncls; ++k)
                     if (bs.cls_fft3[k])
                         launch_rfft3_batch(plans + ch, bs, k, b.cls_plans[k]->desc, b.fft3_blocks[k][0],

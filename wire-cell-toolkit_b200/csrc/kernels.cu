@@ -693,6 +693,8 @@ void launch_fill(const PatchRec* rec, const EventTable& et, int nkeys, const Pla
 // the grid is bit-reproducible.
 // ---------------------------------------------------------------------------
 constexpr int kRasterThreads = 256;
+constexpr int kLightThreads = 64;  // of the launch over all tiles, most of them with few visits or none
+constexpr int kLightBlocks = 11;
 // staged per visit: 12 group coefficients and 16 scaled tick values (odd stride: no bank conflicts)
 constexpr int kStageT = 12;
 constexpr int kStageStride = 29;
@@ -701,11 +703,11 @@ constexpr int kTileLd = kTile + 8;  // fluctuated raster: row stride with an 8-w
 // to eight consecutive group rows at the same four columns hit 32 distinct banks.
 constexpr int kGridLd = kTile + 4;
 
-size_t raster_smem_bytes(int G)
+static size_t raster_smem(int G, int threads)
 {
-    return sizeof(int) * (size_t)G * kGridLd + sizeof(float) * (size_t)kRasterThreads * kStageStride +
-           sizeof(int4) * (size_t)kRasterThreads;
+    return sizeof(int) * (size_t)G * kGridLd + (sizeof(float) * kStageStride + sizeof(int4)) * (size_t)threads;
 }
+size_t raster_smem_bytes(int G) { return raster_smem(G, kRasterThreads); }
 // Long visits of a heavy part, behind that: their integer coefficients by group
 // (three int4) and one of (column | length, profile offset, scaled charge, depo).
 constexpr int kLongQuads = 4;
@@ -714,8 +716,8 @@ static size_t raster_heavy_smem_bytes(int G)
     return raster_smem_bytes(G) + sizeof(int4) * (size_t)kRasterThreads * kLongQuads;
 }
 
-// The first launch rasterises the light tiles, a block each, and lists the
-// heavy ones -- those with long patches (over kTprof ticks; a shower's run over
+// The first launch rasterises the light tiles, a block each, lists middling ones
+// for blocks of their own size and the heavy ones -- those with long patches (over kTprof ticks; a shower's run over
 // a hundred) or with more visits than kHeavyVisits -- for the second, whose
 // blocks take 256 visits of a tile each: the heaviest tile of an event (a
 // shower's core, a track along a wire) holds thousands of visits and ran on
@@ -735,14 +737,20 @@ constexpr int kWideAhead = 4;      // visits whose tick values are loaded togeth
 // (full APA, 520k track depos, fullest tile 3300: 478 us whole; 549 us with tiles
 // over 1024 in parts, 744 us over 512: a part pays for its grid again)
 constexpr int kHeavyVisits = 4096;
+// The other tiles: two blocks' warps of visits and no more stay with the first
+// launch (its 64-thread blocks: 11 an SM, a tile's chain of loads, staging and
+// barriers is what takes the time), the rest are listed for blocks of 256.
+// Whole, in 256-thread blocks -> so, us: plane 2k depos 55 -> 38, full APA on
+// tracks 20k 165 -> 114, 100k 216 -> 180, 200k 256 -> 254, shower 200k (without
+// the heavy parts) 180 -> 170, 16 batched events 594 -> 380.  Lines at 128, 256,
+// 512 visits: 20k 117, 107, 108; 100k 174, 191, 209; batch + 40, + 23, + 91.
+constexpr int kLightVisits = kLightThreads;
+// Mean visits a tile over which one launch of 256-thread blocks is the faster
+// form (full APA on tracks, 520k depos, 147 a tile: 418 against 442 us; 200k,
+// 56 a tile: 256 against 254).
+constexpr long long kDenseVisits = 96;
 static_assert(kRasterThreads == kHeavyPart, "a part is a block's chunk");
 
-// One raster work item: charge row `row` (wire start_ch + row) of plane P and
-// absolute tick tile ktile.  Visit keys are key_base + wire * ntiles_abs +
-// tile; at most vcap visits exist.  HEAVY: part `seg` of the nseg parts of a
-// heavy tile (slot: its entry of heavy.done); otherwise the whole tile, or its
-// listing under tile_id.  Called by all threads of the block; smem_i holds the
-// dynamic shared memory of raster_smem_bytes(P.G).
 // A tile without work in this launch: its G rows are zero. Of one without
 // visits in a sparse grid the transform reads only the 16-byte pieces that it
 // shares with a neighbour.
@@ -764,7 +772,13 @@ __device__ __forceinline__ void zero_tile(const GridPlane& P, int row, int qc0, 
     }
 }
 
-template <bool HEAVY>
+// One raster work item: charge row `row` (wire start_ch + row) of plane P and
+// absolute tick tile ktile.  Visit keys are key_base + wire * ntiles_abs +
+// tile; at most vcap visits exist.  HEAVY: part `seg` of the nseg parts of a
+// heavy tile (slot: its entry of heavy.done); otherwise the whole tile, or its
+// listing under tile_id.  Called by all threads of the block; smem_i holds the
+// dynamic shared memory of raster_smem_bytes(P.G).
+template <bool HEAVY, int T, bool LIST>
 __device__ __forceinline__ void raster_tile(const GridPlane& P, int row, int ktile, int key_base, int ntiles_abs,
                                             const PatchRec* __restrict__ rec, const float* __restrict__ tprof,
                                             const TprofPool& pool, const unsigned char* __restrict__ wide_key,
@@ -782,8 +796,8 @@ __device__ __forceinline__ void raster_tile(const GridPlane& P, int row, int kti
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     int* grid = smem_i;                                       // [G][kGridLd], column = tick - tick_lo
     float* stage = reinterpret_cast<float*>(smem_i + (size_t)G * kGridLd);
-    int4* stagei = reinterpret_cast<int4*>(stage + (size_t)kRasterThreads * kStageStride);
-    int4* longq = stagei + kRasterThreads;  // heavy parts only
+    int4* stagei = reinterpret_cast<int4*>(stage + (size_t)T * kStageStride);
+    int4* longq = stagei + T;  // heavy parts only
     int cnt = 0, held = 1;
     const Visit* list = nullptr;
     int key = -1;
@@ -796,7 +810,11 @@ __device__ __forceinline__ void raster_tile(const GridPlane& P, int row, int kti
     }
     const bool spread = cnt > 0 && wide_key[key];
     const bool longs = HEAVY && spread;  // the tile holds long patches
-    const bool listed = !HEAVY && (spread || cnt > kHeavyVisits);
+    if (LIST && !spread && cnt > kLightVisits && cnt <= kHeavyVisits && heavy.mid) {
+        if (tid == 0) heavy.mid[atomicAdd(heavy.count + 2, 1)] = tile_id;
+        return;
+    }
+    const bool listed = LIST && (spread || cnt > kHeavyVisits);
     if (listed) {
         const int parts = (cnt + kHeavyPart - 1) / kHeavyPart;
         if (tid == 0) {
@@ -820,7 +838,7 @@ __device__ __forceinline__ void raster_tile(const GridPlane& P, int row, int kti
         if (HEAVY && tid == 0) *s_unit = 0;
         int4* g4 = reinterpret_cast<int4*>(grid);
         const int n4 = G * kGridLd / 4;
-        for (int k = tid; k < n4; k += kRasterThreads) g4[k] = make_int4(0, 0, 0, 0);
+        for (int k = tid; k < n4; k += T) g4[k] = make_int4(0, 0, 0, 0);
         if (tid < kTileBlocks) {
             const float b = key >= 0 ? __ull2float_ru(key_bound[(size_t)key * kTileBlocks + tid]) * (1.0f / 65536.0f)
                                      : 0.f;
@@ -838,15 +856,15 @@ __device__ __forceinline__ void raster_tile(const GridPlane& P, int row, int kti
     float* my = stage + (size_t)tid * kStageStride;
     const int wbase = wid * 32;
     const float inv_pbs = 1.0f / pbs;
-    const int nchunks = (cnt + kRasterThreads - 1) / kRasterThreads;
+    const int nchunks = (cnt + T - 1) / T;
     for (int ch = 0; ch < nchunks; ++ch) {
         // visit of this thread: in blocks with long patches, lanes 2k, 2k+1
         // hold consecutive visits (a pair) and consecutive pairs go to
         // different warps (the lists hold one depo kind in runs: long patches
-        // would otherwise pile up on a few warps); elsewhere visits stay in
-        // list order (coalesced reads, alike neighbours along a track)
-        const int e = ch * kRasterThreads +
-                      (longs ? (lane >> 1) * (kRasterThreads / 16) + wid * 2 + (lane & 1) : tid);
+        // would otherwise pile up on a few warps); elsewhere a warp's visits are
+        // neighbours in the list (coalesced reads, alike along a track)
+        const int e = ch * T +
+                      (longs ? (lane >> 1) * (T / 16) + wid * 2 + (lane & 1) : tid);
         const bool valid = e < cnt;
         int4 si = make_int4(0, 0, 0, 0);  // d, l_lo, ng, (cb << 11) | nt  (cb = toff - tick_lo, ng = 0: none)
         if (valid) {
@@ -991,7 +1009,7 @@ __device__ __forceinline__ void raster_tile(const GridPlane& P, int row, int kti
                 int unit = 0;
                 if (lane == 0) unit = atomicAdd(s_unit, 1);
                 unit = __shfl_sync(0xffffffffu, unit, 0);
-                if (unit >= (kTile / 32) * (kRasterThreads / 32)) break;
+                if (unit >= (kTile / 32) * (T / 32)) break;
                 const int slab = unit & (kTile / 32 - 1), b0 = (unit / (kTile / 32)) * 32;
                 const int c = slab * 32 + lane;  // this lane's column
                 const float sc = scale[c / kScaleBlock];
@@ -1065,7 +1083,7 @@ __device__ __forceinline__ void raster_tile(const GridPlane& P, int row, int kti
         // this part into the tile's rows, as integers; the last part to arrive makes them charges
         const int qc0 = tick_lo - P.col0;
         int* const Qi = reinterpret_cast<int*>(Q) + P.qoff + (size_t)row * P.N;
-        for (int k = tid; k < G * kTile; k += kRasterThreads) {
+        for (int k = tid; k < G * kTile; k += T) {
             const int g = k / kTile, c = k - g * kTile, q = qc0 + c;
             const int v = grid[g * kGridLd + c];
             if (v && q >= 0 && q < min(P.N, P.ncols)) atomicAdd(Qi + (size_t)g * P.nin * P.N + q, v);
@@ -1077,7 +1095,7 @@ __device__ __forceinline__ void raster_tile(const GridPlane& P, int row, int kti
         __syncthreads();
         if (!s_last) return;
         __threadfence();
-        for (int k = tid; k < G * kTile; k += kRasterThreads) {
+        for (int k = tid; k < G * kTile; k += T) {
             const int g = k / kTile, c = k - g * kTile, q = qc0 + c;
             if (q < 0 || q >= min(P.N, P.ncols)) continue;
             int* const at = Qi + (size_t)g * P.nin * P.N + q;
@@ -1085,20 +1103,17 @@ __device__ __forceinline__ void raster_tile(const GridPlane& P, int row, int kti
         }
         return;
     }
-    // write the tile's G rows, four columns per thread: grid column c is plane
-    // column tick_lo + c - col0 (zero at or past the window's ncols)
-    const int qc0 = tick_lo - P.col0;
-    constexpr int kQuads = kTile / 4;
-    for (int k = tid; k < G * kQuads; k += kRasterThreads) {
-        const int g = k / kQuads, c = (k - g * kQuads) * 4;
-        const int4 cell = *reinterpret_cast<const int4*>(grid + g * kGridLd + c);
-        const float is = iscale[c / kScaleBlock];  // the four columns share one 64-tick block
-        float* dst = Q + P.qoff + ((size_t)g * P.nin + row) * P.N + qc0 + c;
-        const int q0 = qc0 + c;
-        const float v[4] = {(float)cell.x * is, (float)cell.y * is, (float)cell.z * is, (float)cell.w * is};
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-            if (q0 + u >= 0 && q0 + u < P.N) dst[u] = q0 + u < P.ncols ? v[u] : 0.f;
+    // write the tile's G rows, a column per thread (a warp's 128 bytes together: quads of
+    // columns per thread left as 4-byte pieces of 16 sectors): grid column c is plane column
+    // tick_lo + c - col0 (zero at or past the window's ncols)
+    const size_t gs = (size_t)P.nin * P.N;
+    for (int c = tid; c < kTile; c += T) {
+        const int q = tick_lo - P.col0 + c;
+        if (q < 0 || q >= P.N) continue;
+        const float is = q < P.ncols ? iscale[c / kScaleBlock] : 0.f;
+        float* dst = Q + P.qoff + (size_t)row * P.N + q;
+#pragma unroll 4
+        for (int g = 0; g < G; ++g, dst += gs) *dst = (float)grid[g * kGridLd + c] * is;
     }
 }
 
@@ -1114,7 +1129,8 @@ __device__ __forceinline__ int grid_tile(const GridSet& gs, int tile, int& row, 
     return ip;
 }
 
-__global__ void __launch_bounds__(kRasterThreads, 5)
+template <int T>
+__global__ void __launch_bounds__(T, T == kLightThreads ? kLightBlocks : kMidBlocks)
     k_raster_wires(const PatchRec* __restrict__ rec, const float* __restrict__ tprof,
                    const int* __restrict__ wire_cnt, const int* __restrict__ wire_off,
                    const Visit* __restrict__ visits, long long vcap, const unsigned long long* __restrict__ key_bound,
@@ -1125,8 +1141,36 @@ __global__ void __launch_bounds__(kRasterThreads, 5)
     __shared__ float scale[kTileBlocks], iscale[kTileBlocks];
     int row, ktile;
     const int ip = grid_tile(gs, blockIdx.x, row, ktile);
-    raster_tile<false>(gs.p[ip], row, ktile, 0, gs.ntiles_abs, rec, tprof, pool, wide_key, wire_cnt, wire_off, visits,
-                       vcap, key_bound, Q, row_flag, heavy, blockIdx.x, 0, 1, 0, smem_i, scale, iscale);
+    raster_tile<false, T, true>(gs.p[ip], row, ktile, 0, gs.ntiles_abs, rec, tprof, pool, wide_key, wire_cnt, wire_off,
+                                visits, vcap, key_bound, Q, row_flag, heavy, blockIdx.x, 0, 1, 0, smem_i, scale, iscale);
+}
+
+// The next of the listed middling tiles, -1 after the last (block-uniform).
+__device__ __forceinline__ int next_mid(const HeavyList& heavy)
+{
+    __shared__ int s_next;
+    __syncthreads();
+    if (threadIdx.x == 0) s_next = atomicAdd(heavy.count + 3, 1);
+    __syncthreads();
+    return s_next < heavy.count[2] ? heavy.mid[s_next] : -1;
+}
+
+__global__ void __launch_bounds__(kRasterThreads, kMidBlocks)
+    k_raster_mid(const PatchRec* __restrict__ rec, const float* __restrict__ tprof,
+                 const int* __restrict__ wire_cnt, const int* __restrict__ wire_off,
+                 const Visit* __restrict__ visits, long long vcap, const unsigned long long* __restrict__ key_bound,
+                 GridSet gs, float* __restrict__ Q, TprofPool pool, const unsigned char* __restrict__ wide_key,
+                 unsigned char* __restrict__ row_flag, HeavyList heavy)
+{
+    extern __shared__ int smem_i[];
+    __shared__ float scale[kTileBlocks], iscale[kTileBlocks];
+    for (int it = next_mid(heavy); it >= 0; it = next_mid(heavy)) {
+        int row, ktile;
+        const int ip = grid_tile(gs, it, row, ktile);
+        raster_tile<false, kRasterThreads, false>(gs.p[ip], row, ktile, 0, gs.ntiles_abs, rec, tprof, pool, wide_key,
+                                                  wire_cnt, wire_off, visits, vcap, key_bound, Q, row_flag, heavy, it,
+                                                  0, 1, 0, smem_i, scale, iscale);
+    }
 }
 
 __global__ void __launch_bounds__(kRasterThreads, kHeavyBlocks)
@@ -1143,7 +1187,7 @@ __global__ void __launch_bounds__(kRasterThreads, kHeavyBlocks)
         const int4 it = heavy.item[k];
         int row, ktile;
         const int ip = grid_tile(gs, it.x, row, ktile);
-        raster_tile<true>(gs.p[ip], row, ktile, 0, gs.ntiles_abs, rec, tprof, pool, wide_key, wire_cnt, wire_off,
+        raster_tile<true, kRasterThreads, false>(gs.p[ip], row, ktile, 0, gs.ntiles_abs, rec, tprof, pool, wide_key, wire_cnt, wire_off,
                           visits, vcap, key_bound, Q, row_flag, heavy, it.x, it.y, it.z, it.w, smem_i, scale, iscale);
     }
 }
@@ -1152,19 +1196,30 @@ void launch_raster_wires(const PatchRec* rec, const float* tprof, const TprofPoo
                          const int* wire_cnt,
                          const int* wire_off, const Visit* visits, long long vcap,
                          const unsigned long long* key_bound, const GridSet& gs, float* Q, unsigned char* row_flag,
-                         const HeavyList& heavy, int heavy_blocks, cudaStream_t s)
+                         const HeavyList& heavy, int nsm, cudaStream_t s)
 {
     if (gs.nrows_total <= 0) return;
-    size_t smem = 0;
-    for (int i = 0; i < gs.nplanes; ++i) smem = std::max(smem, raster_smem_bytes(gs.p[i].G));
-    cudaFuncSetAttribute((const void*)k_raster_wires, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k_raster_wires<<<gs.nrows_total, kRasterThreads, smem, s>>>(rec, tprof, wire_cnt, wire_off, visits, vcap,
-                                                                key_bound, gs, Q, pool, wide_key, row_flag, heavy);
-    if (heavy_blocks <= 0) return;  // no tile can be heavy
-    smem = 0;
-    for (int i = 0; i < gs.nplanes; ++i) smem = std::max(smem, raster_heavy_smem_bytes(gs.p[i].G));
+    int maxG = 0;
+    for (int i = 0; i < gs.nplanes; ++i) maxG = std::max(maxG, gs.p[i].G);
+    const bool dense = vcap > kDenseVisits * gs.nrows_total;
+    const int T = dense ? kRasterThreads : kLightThreads;
+    auto* light = dense ? k_raster_wires<kRasterThreads> : k_raster_wires<kLightThreads>;
+    HeavyList lists = heavy;
+    if (dense) lists.mid = nullptr;
+    size_t smem = raster_smem(maxG, T);
+    cudaFuncSetAttribute((const void*)light, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    light<<<gs.nrows_total, T, smem, s>>>(rec, tprof, wire_cnt, wire_off, visits, vcap, key_bound, gs, Q, pool,
+                                          wide_key, row_flag, lists);
+    if (nsm <= 0) return;  // no tile can be listed
+    if (!dense) {
+        smem = raster_smem_bytes(maxG);
+        cudaFuncSetAttribute((const void*)k_raster_mid, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        k_raster_mid<<<kMidBlocks * nsm, kRasterThreads, smem, s>>>(rec, tprof, wire_cnt, wire_off, visits, vcap,
+                                                                    key_bound, gs, Q, pool, wide_key, row_flag, heavy);
+    }
+    smem = raster_heavy_smem_bytes(maxG);
     cudaFuncSetAttribute((const void*)k_raster_heavy, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k_raster_heavy<<<heavy_blocks, kRasterThreads, smem, s>>>(rec, tprof, wire_cnt, wire_off, visits, vcap, key_bound,
+    k_raster_heavy<<<kHeavyBlocks * nsm, kRasterThreads, smem, s>>>(rec, tprof, wire_cnt, wire_off, visits, vcap, key_bound,
                                                               gs, Q, pool, wide_key, row_flag, heavy);
 }
 
@@ -2751,7 +2806,7 @@ __device__ __forceinline__ GridPlane batch_tile(const BatchPlan* __restrict__ pl
 }
 
 template <bool FLUC>
-__global__ void __launch_bounds__(kRasterThreads, FLUC ? 4 : 5)
+__global__ void __launch_bounds__(FLUC ? kRasterThreads : kLightThreads, FLUC ? 4 : kLightBlocks)
     k_raster_batch(const BatchPlan* __restrict__ plan, BatchStatic bs, PlaneSet ps, const PatchRec* __restrict__ rec,
                    long long recstride, const float* __restrict__ tprof, TprofPool pool,
                    const unsigned char* __restrict__ wide_key, const int* __restrict__ wire_cnt,
@@ -2774,8 +2829,31 @@ __global__ void __launch_bounds__(kRasterThreads, FLUC ? 4 : 5)
             raster_tile_fluc(P, ip, row, ktile, e * bs.nkeys, bs.ntiles, evt, fp, rec, fluc, draws, wire_cnt, wire_off,
                              visits, vcap, Q, flags, reinterpret_cast<long long*>(smem_i));
         else
-            raster_tile<false>(P, row, ktile, e * bs.nkeys, bs.ntiles, rec, tprof, pool, wide_key, wire_cnt, wire_off,
-                               visits, vcap, key_bound, Q, flags, heavy, item, 0, 1, 0, smem_i, scale, iscale);
+            raster_tile<false, kLightThreads, true>(P, row, ktile, e * bs.nkeys, bs.ntiles, rec, tprof, pool, wide_key,
+                                                    wire_cnt, wire_off, visits, vcap, key_bound, Q, flags, heavy, item,
+                                                    0, 1, 0, smem_i, scale, iscale);
+    }
+}
+
+__global__ void __launch_bounds__(kRasterThreads, kMidBlocks)
+    k_raster_mid_batch(const BatchPlan* __restrict__ plan, BatchStatic bs, PlaneSet ps,
+                       const PatchRec* __restrict__ rec, long long recstride, const float* __restrict__ tprof,
+                       TprofPool pool, const unsigned char* __restrict__ wide_key,
+                       const int* __restrict__ wire_cnt, const int* __restrict__ wire_off,
+                       const Visit* __restrict__ visits, long long vcap,
+                       const unsigned long long* __restrict__ key_bound, float* __restrict__ Q,
+                       unsigned char* __restrict__ row_flag, HeavyList heavy)
+{
+    extern __shared__ int smem_i[];
+    __shared__ float scale[kTileBlocks], iscale[kTileBlocks];
+    if (plan->status & kBatchSkip) return;
+    for (int it = next_mid(heavy); it >= 0; it = next_mid(heavy)) {
+        int e, ip, row, ktile;
+        const GridPlane P = batch_tile(plan, bs, ps, recstride, it, e, ip, row, ktile);
+        raster_tile<false, kRasterThreads, false>(P, row, ktile, e * bs.nkeys, bs.ntiles, rec, tprof, pool, wide_key,
+                                                  wire_cnt, wire_off, visits, vcap, key_bound, Q,
+                                                  row_flag + (size_t)e * bs.nwires_total, heavy, it, 0, 1, 0, smem_i,
+                                                  scale, iscale);
     }
 }
 
@@ -2796,7 +2874,7 @@ __global__ void __launch_bounds__(kRasterThreads, kHeavyBlocks)
         const int4 it = heavy.item[k];
         int e, ip, row, ktile;
         const GridPlane P = batch_tile(plan, bs, ps, recstride, it.x, e, ip, row, ktile);
-        raster_tile<true>(P, row, ktile, e * bs.nkeys, bs.ntiles, rec, tprof, pool, wide_key, wire_cnt, wire_off,
+        raster_tile<true, kRasterThreads, false>(P, row, ktile, e * bs.nkeys, bs.ntiles, rec, tprof, pool, wide_key, wire_cnt, wire_off,
                           visits, vcap, key_bound, Q, row_flag + (size_t)e * bs.nwires_total, heavy, it.x, it.y, it.z,
                           it.w, smem_i, scale, iscale);
     }
@@ -2807,22 +2885,24 @@ void launch_raster_batch(const BatchPlan* plan, const BatchStatic& bs, const Pla
                          const unsigned char* wide_key, const int* wire_cnt, const int* wire_off,
                          const Visit* visits, long long vcap, const unsigned long long* key_bound, float* Q,
                          int nblocks, int maxG, const EventTable& evt, const FlucParams& fp, const FlucRec* fluc,
-                         const int* draws, unsigned char* row_flag, const HeavyList& heavy, int heavy_blocks,
+                         const int* draws, unsigned char* row_flag, const HeavyList& heavy, int nsm,
                          cudaStream_t s)
 {
-    const size_t smem = std::max(raster_smem_bytes(maxG), raster_fluc_smem_bytes(maxG));
     if (fp.on_patch) {
-        k_raster_batch<true><<<nblocks, kRasterThreads, smem, s>>>(plan, bs, ps, rec, recstride, tprof, pool, wide_key,
-                                                                    wire_cnt, wire_off, visits, vcap, key_bound, Q,
-                                                                    evt, fp, fluc, draws, row_flag, heavy);
+        k_raster_batch<true><<<nblocks, kRasterThreads, raster_fluc_smem_bytes(maxG), s>>>(
+            plan, bs, ps, rec, recstride, tprof, pool, wide_key, wire_cnt, wire_off, visits, vcap, key_bound, Q, evt,
+            fp, fluc, draws, row_flag, heavy);
         return;
     }
-    k_raster_batch<false><<<nblocks, kRasterThreads, smem, s>>>(plan, bs, ps, rec, recstride, tprof, pool, wide_key,
-                                                                 wire_cnt, wire_off, visits, vcap, key_bound, Q, evt,
-                                                                 fp, fluc, draws, row_flag, heavy);
-    k_raster_heavy_batch<<<heavy_blocks, kRasterThreads, raster_heavy_smem_bytes(maxG), s>>>(plan, bs, ps, rec, recstride, tprof, pool,
-                                                                     wide_key, wire_cnt, wire_off, visits, vcap,
-                                                                     key_bound, Q, row_flag, heavy);
+    k_raster_batch<false><<<kLightBlocks * nsm, kLightThreads, raster_smem(maxG, kLightThreads), s>>>(
+        plan, bs, ps, rec, recstride, tprof, pool, wide_key, wire_cnt, wire_off, visits, vcap, key_bound, Q, evt, fp,
+        fluc, draws, row_flag, heavy);
+    k_raster_mid_batch<<<nblocks, kRasterThreads, raster_smem_bytes(maxG), s>>>(
+        plan, bs, ps, rec, recstride, tprof, pool, wide_key, wire_cnt, wire_off, visits, vcap, key_bound, Q, row_flag,
+        heavy);
+    k_raster_heavy_batch<<<kHeavyBlocks * nsm, kRasterThreads, raster_heavy_smem_bytes(maxG), s>>>(
+        plan, bs, ps, rec, recstride, tprof, pool, wide_key, wire_cnt, wire_off, visits, vcap, key_bound, Q, row_flag,
+        heavy);
 }
 
 // Time FFT of every charge-grid row of the pass, in place (rows of N reals
@@ -3025,6 +3105,7 @@ void batch_kernel_attributes(int maxG, int maxM)
     const int sf = (int)(2 * (size_t)maxM * sizeof(float2));
     cudaFuncSetAttribute((const void*)k_raster_batch<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, sr);
     cudaFuncSetAttribute((const void*)k_raster_batch<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sr);
+    cudaFuncSetAttribute((const void*)k_raster_mid_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, sr);
     cudaFuncSetAttribute((const void*)k_raster_heavy_batch, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)raster_heavy_smem_bytes(maxG));
     cudaFuncSetAttribute((const void*)k_rfft_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, sf);

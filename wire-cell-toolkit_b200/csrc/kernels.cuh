@@ -121,13 +121,16 @@ struct GridSet {
 // Tiles of the raster that are worked off in parts of kHeavyPart visits:
 // count[0] parts and count[1] tiles (zeroed by the caller), a part's (tile, part,
 // parts of the tile, tile's entry of done), and the parts done of each tile.
-// Room: heavy_items(visits, keys) parts, a tile per key.
+// Room: heavy_items(visits, keys) parts, a tile per key.  mid: the tiles with
+// over kLightVisits visits that are not heavy (count[2] listed, count[3] taken).
 constexpr int kHeavyPart = 256;
 constexpr int kHeavyBlocks = 3;  // resident blocks an SM of the kernels that take them
+constexpr int kMidBlocks = 5;
 struct HeavyList {
     int* count;
     int4* item;
     int* done;
+    int* mid;  // null: none are listed
 };
 inline size_t heavy_items(long long visits, long long keys) { return (size_t)(visits / kHeavyPart + keys + 1); }
 
@@ -289,9 +292,9 @@ void launch_raster_wires(const PatchRec* rec, const float* tprof, const TprofPoo
                          const int* wire_cnt,
                          const int* wire_off, const Visit* visits, long long vcap,
                          const unsigned long long* key_bound, const GridSet& gs, float* Q, unsigned char* row_flag,
-                         const HeavyList& heavy, int heavy_blocks, cudaStream_t s);
-// (row_flag[wire_base + wire] = 1 for every wire with a visit; heavy_blocks 0:
-// the event has neither patches over kTprof ticks nor enough visits for a heavy tile)
+                         const HeavyList& heavy, int nsm, cudaStream_t s);
+// (row_flag[wire_base + wire] = 1 for every wire with a visit; nsm 0: the event
+// has neither patches over kTprof ticks nor enough visits for a list of tiles)
 void launch_rfft_rows(const float* in, long in_ld, int in_len, float2* out, long out_ld, int nrows,
                       const FftDesc& d, cudaStream_t s, const TileMap& tiles = TileMap{});
 void launch_wire_conv(const float2* Qh, const float2* Rh, float2* Vh, int ngroups, int npad, int nrows_in,
@@ -415,7 +418,7 @@ void launch_raster_batch(const BatchPlan* plan, const BatchStatic& bs, const Pla
                          const unsigned char* wide_key, const int* wire_cnt, const int* wire_off,
                          const Visit* visits, long long vcap, const unsigned long long* key_bound, float* Q,
                          int nblocks, int maxG, const EventTable& evt, const FlucParams& fp, const FlucRec* fluc,
-                         const int* draws, unsigned char* row_flag, const HeavyList& heavy, int heavy_blocks, cudaStream_t s);  // row_flag: [event][wire]
+                         const int* draws, unsigned char* row_flag, const HeavyList& heavy, int nsm, cudaStream_t s);  // row_flag: [event][wire]
 void launch_rfft_batch(const BatchPlan* plan, const FftDesc* descs, float* Q, int nblocks, int nthreads, int maxM,
                        cudaStream_t s);
 // Wire convolution of planes [ip0, ip1) (all with the same pad and pairing) in one launch.
