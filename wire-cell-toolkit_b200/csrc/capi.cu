@@ -863,6 +863,7 @@ static int forward_device(Core& c, const double* d_depos, size_t ndepos, float* 
                 (long long)std::max(total_visits, 1), s);
     if (!ev.fp.on_patch && wide > 0)
         launch_tprof_pool(c.d_rec.as<PatchRec>(), ev.et, np, (float)ev.tb.bs, pool, nullptr, s);
+    int raster_launches = 1;
     if (ev.fp.on_patch) {
         // room for every cell's draw, as counted by the prep kernel, up to kMaxDrawCells
         const long long cells = (long long)std::min<unsigned long long>(c.h_win[0].ncells, kMaxDrawCells);
@@ -877,12 +878,13 @@ static int forward_device(Core& c, const double* d_depos, size_t ndepos, float* 
                            c.d_Q.as<float>(), row_flag, s);
     }
     else
-        launch_raster_wires(c.d_rec.as<PatchRec>(), c.d_tprof.as<float>(), pool, c.d_wide.as<unsigned char>(),
-                            c.d_wcnt.as<int>(),
-                            c.d_woff.as<int>(), c.d_wlist.as<Visit>(), (long long)std::max(total_visits, 1),
-                            c.d_kbound.as<unsigned long long>(), gset, c.d_Q.as<float>(), row_flag, heavy, nsm, s);
+        raster_launches =
+            launch_raster_wires(c.d_rec.as<PatchRec>(), c.d_tprof.as<float>(), pool, c.d_wide.as<unsigned char>(),
+                                c.d_wcnt.as<int>(), c.d_woff.as<int>(), c.d_wlist.as<Visit>(),
+                                (long long)std::max(total_visits, 1), c.d_kbound.as<unsigned long long>(), gset,
+                                c.d_Q.as<float>(), row_flag, heavy, nsm, s);
     t_r.close((n > 0 ? 1 : 0) + (ev.fp.on_patch && n > 0 ? 1 : 0) + (!ev.fp.on_patch && wide > 0 ? 1 : 0) +
-              (rows > 0 ? 1 : 0));
+              (rows > 0 ? raster_launches : 0));
     CUDA_TRY(cudaGetLastError());
 
     // the planes' chains: on streams of their own unless profiling or a long-range step needs s alone

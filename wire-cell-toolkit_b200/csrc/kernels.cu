@@ -5,17 +5,20 @@
 //                  patch sample ranges + event window reduction + per-wire
 //                  visit counts, all planes, one thread per depo
 //   k_scan/k_fill  per-wire visit lists (CSR)
-//   k_raster_wires erf-integrated patches with linear impact weights,
-//                  accumulated per wire row in shared memory, written as the
-//                  impact-group x tick charge grids       gen/src/BinnedDiffusion_transform.cxx:227-391
-//   k_rfft_rows    real FFT along time of each group row   gen/src/ImpactTransform.cxx:149-151,237
-//   k_wire_conv    wire-direction convolution with the     gen/src/ImpactTransform.cxx:153-212,242-300
-//                  per-group response spectra (direct taps)
-//   k_irfft_rows   inverse FFT along time, frame write     gen/src/ImpactTransform.cxx:303-347
+//   k_raster_*     erf-integrated patches with linear impact weights,
+//                  accumulated per (wire, 256 ticks) in shared memory, written
+//                  as the impact-group x tick charge grids: light, middling and
+//                  heavy tiles                            gen/src/BinnedDiffusion_transform.cxx:227-391
+//   k_rfft3        real FFT along time of each group row (fft3.cu; lengths
+//                  without a plan: k_rfft_rows)            gen/src/ImpactTransform.cxx:149-151,237
+//   k_wire_conv_fft  wire-direction convolution with the per-group response
+//                  spectra, overlap-save (wire_fft.cu; short pads and rows:
+//                  direct taps, k_wire_conv*)              gen/src/ImpactTransform.cxx:153-212,242-300
+//   k_irfft3       inverse FFT along time, frame write     gen/src/ImpactTransform.cxx:303-347
 //
-// The 2-D FFT convolution of the reference is replaced by an exactly
-// equivalent (no wrap-around) real FFT along time plus a direct
-// (2*npad+1)-tap convolution along wires in the frequency domain.
+// The 2-D FFT convolution of the reference is replaced by an equivalent (no
+// wrap-around) real FFT along time plus a convolution along wires in the
+// frequency domain.
 //
 // Index arithmetic that decides bins (drift, pitch distance, rejection,
 // sample_bin_range, window min/max) is written with explicit _rn intrinsics
@@ -849,10 +852,8 @@ __device__ __forceinline__ void raster_tile(const GridPlane& P, int row, int kti
     __syncthreads();
     const float pbs = P.pbs, tbs = P.tbs;
     const int wlo = w * nimp;
-    // pass 2: each lane stages the group coefficients of one visit, then the
-    // warp scatters its 32 staged visits, two at a time (half-warp per visit,
-    // lanes over ticks, loop over the covered groups; whole warp for a pair
-    // with a visit longer than 16 ticks).
+    // each lane stages the group coefficients and tick values of one visit, then
+    // the warp scatters its 32 staged visits, eight at a time
     float* my = stage + (size_t)tid * kStageStride;
     const int wbase = wid * 32;
     const float inv_pbs = 1.0f / pbs;
@@ -1192,13 +1193,13 @@ __global__ void __launch_bounds__(kRasterThreads, kHeavyBlocks)
     }
 }
 
-void launch_raster_wires(const PatchRec* rec, const float* tprof, const TprofPool& pool, const unsigned char* wide_key,
+int launch_raster_wires(const PatchRec* rec, const float* tprof, const TprofPool& pool, const unsigned char* wide_key,
                          const int* wire_cnt,
                          const int* wire_off, const Visit* visits, long long vcap,
                          const unsigned long long* key_bound, const GridSet& gs, float* Q, unsigned char* row_flag,
                          const HeavyList& heavy, int nsm, cudaStream_t s)
 {
-    if (gs.nrows_total <= 0) return;
+    if (gs.nrows_total <= 0) return 0;
     int maxG = 0;
     for (int i = 0; i < gs.nplanes; ++i) maxG = std::max(maxG, gs.p[i].G);
     const bool dense = vcap > kDenseVisits * gs.nrows_total;
@@ -1210,7 +1211,7 @@ void launch_raster_wires(const PatchRec* rec, const float* tprof, const TprofPoo
     cudaFuncSetAttribute((const void*)light, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     light<<<gs.nrows_total, T, smem, s>>>(rec, tprof, wire_cnt, wire_off, visits, vcap, key_bound, gs, Q, pool,
                                           wide_key, row_flag, lists);
-    if (nsm <= 0) return;  // no tile can be listed
+    if (nsm <= 0) return 1;  // no tile can be listed
     if (!dense) {
         smem = raster_smem_bytes(maxG);
         cudaFuncSetAttribute((const void*)k_raster_mid, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -1221,6 +1222,7 @@ void launch_raster_wires(const PatchRec* rec, const float* tprof, const TprofPoo
     cudaFuncSetAttribute((const void*)k_raster_heavy, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     k_raster_heavy<<<kHeavyBlocks * nsm, kRasterThreads, smem, s>>>(rec, tprof, wire_cnt, wire_off, visits, vcap, key_bound,
                                                               gs, Q, pool, wide_key, row_flag, heavy);
+    return dense ? 2 : 3;
 }
 
 // ---------------------------------------------------------------------------

@@ -288,13 +288,14 @@ void launch_tprof_pool(const PatchRec* rec, const EventTable& et, int nplanes, f
 void launch_fill(const PatchRec* rec, const EventTable& et, int nkeys, const PlaneSet& ps, int* wire_cur,
                  Visit* visits, long long cap, cudaStream_t s);
 size_t raster_smem_bytes(int G);
-void launch_raster_wires(const PatchRec* rec, const float* tprof, const TprofPool& pool, const unsigned char* wide_key,
+int launch_raster_wires(const PatchRec* rec, const float* tprof, const TprofPool& pool, const unsigned char* wide_key,
                          const int* wire_cnt,
                          const int* wire_off, const Visit* visits, long long vcap,
                          const unsigned long long* key_bound, const GridSet& gs, float* Q, unsigned char* row_flag,
                          const HeavyList& heavy, int nsm, cudaStream_t s);
 // (row_flag[wire_base + wire] = 1 for every wire with a visit; nsm 0: the event
-// has neither patches over kTprof ticks nor enough visits for a list of tiles)
+// has neither patches over kTprof ticks nor enough visits for a list of tiles;
+// returns the number of launches)
 void launch_rfft_rows(const float* in, long in_ld, int in_len, float2* out, long out_ld, int nrows,
                       const FftDesc& d, cudaStream_t s, const TileMap& tiles = TileMap{});
 void launch_wire_conv(const float2* Qh, const float2* Rh, float2* Vh, int ngroups, int npad, int nrows_in,
