@@ -166,8 +166,8 @@ def max_over_ranks(x, world, device="cuda"):
     return float(t.item())
 
 
-STAGE_KERNELS = {"raster": "k_fill + k_raster_wires", "time_fft": "k_rfft_rows x planes",
-                 "wire_conv": "k_wire_conv x planes", "inverse_fft+frame": "k_irfft_rows x planes",
+STAGE_KERNELS = {"raster": "k_fill + k_raster_*", "time_fft": "k_rfft3 x planes",
+                 "wire_conv": "k_wire_conv_fft x planes", "inverse_fft+frame": "k_irfft3 x planes",
                  "drift+prep": "k_prep_all + k_scan_*"}
 
 
@@ -358,7 +358,8 @@ def run_b200(args):
         },
         "stages_ms_per_step": {k: v[0] / args.steps for k, v in stages.items() if not k.startswith("adj_")},
         "stages_note": "stage times from the same steps run again with the stage timers on (planes one after "
-                       "another); the timed steps run each plane's FFT chain on its own stream",
+                       "another); the timed steps run each plane's FFT chain on its own stream; algorithmic "
+                       "bytes count every cell of the grids, also of tiles that hold no charge",
         "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": int(depos.nbytes),
                 "d2h_bytes_per_step": int(nsamples * 4 + nrows * 8),
                 "call": "wct_dt_forward_traces: host depos in, the trace list out (window blocks + trace edges)",
