@@ -756,7 +756,9 @@ static_assert(kRasterThreads == kHeavyPart, "a part is a block's chunk");
 
 // A tile without work in this launch: its G rows are zero. Of one without
 // visits in a sparse grid the transform reads only the 16-byte pieces that it
-// shares with a neighbour.
+// shares with a neighbour. (Half to two thirds of the tiles: their zeros took
+// the raster 24 of 81 us at 2k depos on a plane, 42 of 213 at 20k on a full APA,
+// 198 of 792 for 16 batched events.)
 __device__ __forceinline__ void zero_tile(const GridPlane& P, int row, int qc0, bool unread, float* __restrict__ Q)
 {
     if (unread) {
