@@ -379,64 +379,10 @@ void launch_digitize(const float* in, long ld_in, float* out, long ld_out, int n
 // group's (coherent, so every channel of a group gets the same waveform).
 // One row per block; N even, N/2 a supported FFT length.
 // ---------------------------------------------------------------------------
-// Box-Muller, sqrt(-2 log u1) cos(2 pi u2), in double precision to about 1e-11
-// and rounded to float.  The series are Taylor's, on the ranges that exact
-// reductions leave: the logarithm as e log 2 + 2 atanh((m - 1) / (m + 1)) with m
-// in [sqrt(1/2), sqrt(2)), sine and cosine within pi / 4 of a quarter turn; the
-// root starts from the single-precision one and takes one Newton step.
-// Integers become doubles by additions: conversions run at a quarter of their
-// rate.  (The library's log, sincospi and sqrt, to the last bit of a double, took
-// four times the operations: 248 us for the noise of a 2560 x 6000 frame, 15 M
-// normals, with the generic transform; now 194 us: half the FP64 chains, a quarter each Philox
-// and transform.)
 __device__ __forceinline__ float noise_normal(unsigned k0, unsigned k1, unsigned stream, unsigned model, int i)
 {
     const uint4 o = philox_block(k0, k1, stream, model, (unsigned)i, 0u);
-    const double u1 = uniform53(o.x, o.y), u2 = uniform53(o.z, o.w);
-    // u1 = m 2^e
-    long long bits = __double_as_longlong(u1);
-    int e = (int)(bits >> 52) - 1023;
-    double m = __longlong_as_double((bits & 0x000fffffffffffffll) | 0x3ff0000000000000ll);
-    if (m > 1.4142135623730951) {
-        m *= 0.5;
-        ++e;
-    }
-    // 1 / d on [1.7, 2.42]: a parabola good to 0.16 %, and two Newton steps
-    const double d = m + 1.0;
-    double r = fma(fma(0.1175, d, -0.7253), d, 1.4810);
-    r = r * fma(-d, r, 2.0);
-    r = r * fma(-d, r, 2.0);
-    const double s = (m - 1.0) * r, s2 = s * s;
-    double p = 1.0 / 13.0;
-    p = fma(p, s2, 1.0 / 11.0);
-    p = fma(p, s2, 1.0 / 9.0);
-    p = fma(p, s2, 1.0 / 7.0);
-    p = fma(p, s2, 1.0 / 5.0);
-    p = fma(p, s2, 1.0 / 3.0);
-    p = fma(p * s2, s, s);  // atanh s
-    const double ed = __hiloint2double(0x43300000, e ^ 0x80000000) - 4503601774854144.0;  // e + 2^31 + 2^52
-    const double x = -2.0 * fma(ed, 0.69314718055994531, 2.0 * p);
-    double y = (double)rsqrtf((float)x);
-    y = y * fma(-0.5 * x * y, y, 1.5);
-    // 4 u2 = q + f, f in [-1/2, 1/2]
-    const double v = 4.0 * u2, w = v + 6755399441055744.0;  // 1.5 2^52: rounds, the quarter in the low bits
-    const double f = (v - (w - 6755399441055744.0)) * 1.5707963267948966, f2 = f * f;
-    double c = 1.0 / 479001600.0, z = 1.0 / 6227020800.0;  // 12!, 13!
-    c = fma(c, f2, -1.0 / 3628800.0);
-    c = fma(c, f2, 1.0 / 40320.0);
-    c = fma(c, f2, -1.0 / 720.0);
-    c = fma(c, f2, 1.0 / 24.0);
-    c = fma(c, f2, -0.5);
-    c = fma(c, f2, 1.0);
-    z = fma(z, f2, -1.0 / 39916800.0);
-    z = fma(z, f2, 1.0 / 362880.0);
-    z = fma(z, f2, -1.0 / 5040.0);
-    z = fma(z, f2, 1.0 / 120.0);
-    z = fma(z, f2, -1.0 / 6.0);
-    z = fma(z * f2, f, f);
-    const int turn = __double2loint(w) & 3;
-    const double t = (turn & 1) ? z : c;
-    return (float)(x * y * (turn == 1 || turn == 2 ? -t : t));
+    return box_muller(uniform53(o.x, o.y), uniform53(o.z, o.w));
 }
 
 // Bin k of a row's packed noise spectrum: bin 0 = (|X_0|, |X_M|), then X_k (Sk = S[k]).
