@@ -1255,10 +1255,12 @@ static int batch_setup(Core& c)
     bs.tbs = (c.start_time + c.readout_time - c.start_time) / (int)(c.readout_time / c.tick);
     // ladder of time-FFT lengths from the shortest possible window up
     std::vector<int> cls;
-    // (each a length with a three-stage plan, while there is one)
+    // (each a length with a three-stage plan, where that is not over 15 % longer:
+    // rows of up to 12000 for windows just past the last plan before it cost the
+    // raster, the wire convolution and the arenas more than the plan gives)
     auto class_length = [](int n) {
-        const int M = fft3_next((n + 1) / 2);
-        return M ? 2 * M : gpu_fft_length(n);
+        const int N = 2 * fft3_next((n + 1) / 2);
+        return N && (n <= 512 || 20LL * N <= 23LL * n) ? N : gpu_fft_length(n);
     };
     const int nfirst = class_length(std::max(64, (int)fft_best_length((size_t)4 + std::max(minpad, 0), false)));
     for (double ratio = 1.1;; ratio *= 1.05) {
@@ -1267,7 +1269,8 @@ static int batch_setup(Core& c)
         for (;;) {
             cls.push_back(N);
             if ((size_t)N >= nneed) break;
-            N = class_length(std::max((int)std::ceil(N * ratio), N + 4));
+            // the last one as long as the longest window asks for
+            N = class_length(std::min(std::max((int)std::ceil(N * ratio), N + 4), (int)nneed));
         }
         if ((int)cls.size() <= kMaxClasses) break;
     }

@@ -34,17 +34,20 @@ namespace wctb200 {
 
 // The plans: radices of the forward order (the inverse runs them reversed).
 // The smallest is last, where the forward pairs two butterflies a thread.
-// Lengths: the halves of the time-FFT lengths that the reference's window
-// lengths lead to (gpu_fft_length), and the common transform sizes beside
-// them; other lengths take the transforms of fft.cuh.
+// Lengths: from 256 to 6000, the halves of the time-FFT lengths that the
+// reference's window lengths lead to (gpu_fft_length) as far as three of the
+// radices make them (not 2058, 2430, 4116, 4704 and 5376), and the halves of
+// round record lengths, which the noise and the 2-D transforms run at (1000,
+// 1120, 1200, 1500, 1536, 1920, 2000, 2400, 3072, 4000). Other lengths take the
+// transforms of fft.cuh.
 #define WCT_FFT3_PLANS(X)                                                                              \
-    X(8, 8, 4) X(8, 7, 5) X(8, 8, 5) X(10, 7, 5) X(8, 8, 6) X(10, 8, 5) X(8, 8, 7) X(8, 8, 8)           \
+    X(8, 8, 4) X(8, 7, 5) X(8, 8, 5) X(10, 7, 5) X(8, 8, 6) X(10, 8, 5) X(12, 6, 6) X(8, 8, 7) X(8, 8, 8) \
     X(10, 8, 7) X(10, 8, 8) X(12, 8, 7) X(14, 7, 7) X(10, 10, 7) X(12, 8, 8) X(10, 10, 8) X(14, 8, 8)   \
     X(10, 10, 10) X(16, 8, 8) X(14, 10, 8) X(12, 10, 10) X(16, 10, 8) X(14, 12, 8) X(14, 14, 7)         \
     X(15, 10, 10) X(16, 12, 8) X(16, 10, 10) X(16, 14, 8) X(16, 15, 8) X(20, 10, 10) X(16, 16, 8)       \
     X(16, 14, 10) X(16, 15, 10) X(16, 16, 10) X(16, 14, 12) X(20, 14, 10) X(16, 15, 12) X(20, 15, 10)   \
     X(16, 14, 14) X(15, 15, 14) X(16, 16, 12) X(16, 15, 14) X(16, 16, 14) X(20, 14, 14) X(20, 20, 10)   \
-    X(16, 16, 16) X(20, 20, 15)
+    X(16, 16, 16) X(20, 16, 14) X(20, 16, 16) X(20, 20, 15)
 
 template <int R1_, int R2_, int R3_>
 struct Fft3 {
