@@ -2669,7 +2669,7 @@ __global__ void __launch_bounds__(256) k_plan_batch(BatchPlan* __restrict__ plan
 {
     __shared__ int s_status;
     __shared__ int c_raster[kMaxBatch * kMaxPlanes], c_rows[kMaxBatch * kMaxPlanes],
-        c_orows[kMaxBatch * kMaxPlanes], c_conv[kMaxBatch * kMaxPlanes];
+        c_orows[kMaxBatch * kMaxPlanes], c_conv[kMaxBatch * kMaxPlanes], c_wire[kMaxBatch * kMaxPlanes];
     const int np = bs.np, ne = nev * np;
     if (threadIdx.x == 0) s_status = 0;
     __syncthreads();
@@ -2707,9 +2707,9 @@ __global__ void __launch_bounds__(256) k_plan_batch(BatchPlan* __restrict__ plan
         c_raster[k] = o.nin * o.ntile;
         c_rows[k] = bs.cls_fft3[cls] ? 0 : pl.G * o.nin;
         c_orows[k] = bs.cls_fft3[cls] ? 0 : o.nout;
-        c_conv[k] = !o.nin        ? 0
-                    : pl.wire_fft ? wire_fblocks(o.M) * wire_blocks(o.nout, pl.npad)
-                                  : ((o.M + 31) / 32) * ((o.nout + kConvRows - 1) / kConvRows);
+        const bool wire = (pl.wire_cls >> cls) & 1;
+        c_conv[k] = wire || !o.nin ? 0 : ((o.M + 31) / 32) * ((o.nout + kConvRows - 1) / kConvRows);
+        c_wire[k] = wire && o.nin ? wire_fblocks(o.M) * wire_blocks(o.nout, pl.npad) : 0;
         if (st) atomicOr(&s_status, st);
     }
     __syncthreads();
@@ -2727,12 +2727,15 @@ __global__ void __launch_bounds__(256) k_plan_batch(BatchPlan* __restrict__ plan
         plan->pre_rows[ne] = b;
         plan->pre_orows[ne] = c;
         for (int ip = 0; ip < np; ++ip) {
-            int t = 0;
+            int t = 0, u = 0;
             for (int e = 0; e < nev; ++e) {
                 plan->pre_conv[ip][e] = t;
+                plan->pre_wire[ip][e] = u;
                 t += c_conv[e * np + ip];
+                u += c_wire[e * np + ip];
             }
             plan->pre_conv[ip][nev] = t;
+            plan->pre_wire[ip][nev] = u;
         }
         unsigned long long tv = 0;  // visits of the pass, 64-bit (the list offsets are int)
         for (int e = 0; e < nev; ++e) tv += win[(size_t)e * np].nvisits;
@@ -2741,7 +2744,7 @@ __global__ void __launch_bounds__(256) k_plan_batch(BatchPlan* __restrict__ plan
         plan->np = np;
         plan->status = s_status | (tv > (unsigned long long)vcap ? kBatchVisitOverflow : 0) |
                        (tv >= 0x7fffffffull ? kBatchTooBig : 0);
-        for (int k = 0; k < 3 + kMaxPlanes; ++k) plan->next[k] = 0;
+        for (int k = 0; k < 4 + kMaxPlanes; ++k) plan->next[k] = 0;
     }
 }
 
@@ -2985,7 +2988,7 @@ __global__ void __launch_bounds__(32 * kConvRG) k_conv_batch(const BatchPlan* __
     const int nev = plan->nev, np = plan->np;
     int total = 0;
     for (int ip = ip0; ip < ip1; ++ip) total += plan->pre_conv[ip][nev];
-    int* ctr = const_cast<int*>(&plan->next[3 + ip0]);
+    int* ctr = const_cast<int*>(&plan->next[4 + ip0]);
     for (int item = next_item(ctr, &s_item); item < total; item = next_item(ctr, &s_item)) {
         int ip = ip0, rel = item;
         while (rel >= plan->pre_conv[ip][nev]) {
@@ -3007,10 +3010,8 @@ __global__ void __launch_bounds__(32 * kConvRG) k_conv_batch(const BatchPlan* __
     }
 }
 
-// The same by overlap-save (wire_fft.cuh): items of planes ip0 .. ip1-1, all
-// with wire_fft set.
+// The same by overlap-save (wire_fft.cuh): the items of every plane.
 __global__ void __launch_bounds__(kWThreads, 2) k_conv_fft_batch(const BatchPlan* __restrict__ plan, BatchStatic bs,
-                                                                 int ip0, int ip1,
                                                                  const float2* const* __restrict__ wspec,
                                                                  const float* __restrict__ Q, float2* __restrict__ V)
 {
@@ -3020,15 +3021,15 @@ __global__ void __launch_bounds__(kWThreads, 2) k_conv_fft_batch(const BatchPlan
     wfft::load_twiddles(wsm + 2 * kWEx, threadIdx.x);
     const int nev = plan->nev, np = plan->np;
     int total = 0;
-    for (int ip = ip0; ip < ip1; ++ip) total += plan->pre_conv[ip][nev];
-    int* ctr = const_cast<int*>(&plan->next[3 + ip0]);
+    for (int ip = 0; ip < np; ++ip) total += plan->pre_wire[ip][nev];
+    int* ctr = const_cast<int*>(&plan->next[3]);
     for (int item = next_item(ctr, &s_item); item < total; item = next_item(ctr, &s_item)) {
-        int ip = ip0, rel = item;
-        while (rel >= plan->pre_conv[ip][nev]) {
-            rel -= plan->pre_conv[ip][nev];
+        int ip = 0, rel = item;
+        while (rel >= plan->pre_wire[ip][nev]) {
+            rel -= plan->pre_wire[ip][nev];
             ++ip;
         }
-        const int* pre = plan->pre_conv[ip];
+        const int* pre = plan->pre_wire[ip];
         const int e = find_entry(pre, nev, rel);
         const EvPlane& E = plan->ep[e * np + ip];
         rel -= pre[e];
@@ -3039,10 +3040,10 @@ __global__ void __launch_bounds__(kWThreads, 2) k_conv_fft_batch(const BatchPlan
     }
 }
 
-void launch_conv_fft_batch(const BatchPlan* plan, const BatchStatic& bs, int ip0, int ip1,
-                           const float2* const* wspec, const float* Q, float2* V, int nblocks, cudaStream_t s)
+void launch_conv_fft_batch(const BatchPlan* plan, const BatchStatic& bs, const float2* const* wspec, const float* Q,
+                           float2* V, int nblocks, cudaStream_t s)
 {
-    k_conv_fft_batch<<<nblocks, kWThreads, kWConvSmem, s>>>(plan, bs, ip0, ip1, wspec, Q, V);
+    k_conv_fft_batch<<<nblocks, kWThreads, kWConvSmem, s>>>(plan, bs, wspec, Q, V);
 }
 
 size_t conv_smem_bytes(int npad, bool pair)

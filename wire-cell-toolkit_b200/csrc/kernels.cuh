@@ -166,7 +166,7 @@ constexpr int kMaxClasses = 48;  // time-FFT length classes of the batched path
 struct BatchPlaneStatic {
     int G, npad, waveform_pad, nwires, imp_nbins, row0, nin_max;
     int wire_base;    // first entry of the plane's wires in the event's wire flags
-    int wire_fft;     // overlap-save wire convolution (wire_fft.cuh) at every length class
+    unsigned long long wire_cls;  // length classes with wire spectra (bit per class): overlap-save form
     double imp_min, imp_bs;
     long long qslot;  // offset of the plane's grid within an event slot (floats)
     long long vslot;  // offset of the plane's V rows within an event slot (complex values)
@@ -205,8 +205,9 @@ struct BatchPlan {
     int pre_raster[kMaxBatch * kMaxPlanes + 1];
     int pre_rows[kMaxBatch * kMaxPlanes + 1];   // time-FFT rows: G * nin
     int pre_orows[kMaxBatch * kMaxPlanes + 1];  // inverse-FFT rows: nout
-    int pre_conv[kMaxPlanes][kMaxBatch + 1];    // wire-convolution tiles of plane ip over events
-    int next[3 + kMaxPlanes];                   // work-stealing counters: raster, rfft, irfft, conv from plane ip0
+    int pre_conv[kMaxPlanes][kMaxBatch + 1];    // direct wire-convolution tiles of plane ip over events
+    int pre_wire[kMaxPlanes][kMaxBatch + 1];    // the same of the overlap-save form
+    int next[4 + kMaxPlanes];  // work-stealing counters: raster, rfft, irfft, overlap-save, direct from plane ip0
     EvPlane ep[kMaxBatch * kMaxPlanes];
 };
 constexpr int kBatchVisitOverflow = 1;
@@ -428,8 +429,8 @@ void launch_conv_batch(const BatchPlan* plan, const BatchStatic& bs, int ip0, in
 void launch_irfft_batch(const BatchPlan* plan, const BatchStatic& bs, const FftDesc* descs, const float2* V,
                         float* frames, long long frame_stride, int nblocks, int nthreads, int maxM,
                         const unsigned char* row_flag, cudaStream_t s);
-void launch_conv_fft_batch(const BatchPlan* plan, const BatchStatic& bs, int ip0, int ip1,
-                           const float2* const* wspec, const float* Q, float2* V, int nblocks, cudaStream_t s);
+void launch_conv_fft_batch(const BatchPlan* plan, const BatchStatic& bs, const float2* const* wspec, const float* Q,
+                           float2* V, int nblocks, cudaStream_t s);
 size_t conv_smem_bytes(int npad, bool pair);
 void batch_kernel_attributes(int maxG, int maxM);
 
