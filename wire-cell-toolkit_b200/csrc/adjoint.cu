@@ -20,6 +20,7 @@
 
 #include "gauss.cuh"
 #include "kernels.cuh"
+#include "wire_fft.cuh"
 
 namespace wctb200 {
 
@@ -61,21 +62,21 @@ constexpr int kAdjRB = 8;
 constexpr int kAdjRG = 8;
 constexpr int kAdjRows = kAdjRB * kAdjRG;
 
-__global__ void __launch_bounds__(32 * kAdjRG) k_wire_conv_adj(const float2* __restrict__ Gh,
-                                                                const float2* __restrict__ Rh,
-                                                                float2* __restrict__ dQh, int G, int PAD, int nin,
-                                                                int nout, int M)
+// Rows at 32 frequencies: a warp's RB rows from i0 + rb0 on (rb0 < 0: none) of
+// every group, of which mask are written; the block's rows lie within span (at
+// most kAdjRows) of i0.  Called by all threads of a (32, kAdjRG) block.
+template <int RB>
+__device__ __forceinline__ void adj_unit(const float2* __restrict__ Gh, const float2* __restrict__ Rh,
+                                         float2* __restrict__ dQh, int G, int PAD, int nin, int nout, int M, int f0,
+                                         int i0, int span, int rb0, unsigned mask, float2* adj_smem)
 {
-    extern __shared__ __align__(16) float2 adj_smem[];
-    const int SROWS = kAdjRows + 2 * PAD;
+    const int SROWS = span + 2 * PAD;
     const int NT = 2 * PAD + 1;
     float2(*Gs)[32] = reinterpret_cast<float2(*)[32]>(adj_smem);
-    float2* Rbuf = adj_smem + (size_t)SROWS * 32;  // two tap buffers of NT x 32
+    float2* Rbuf = adj_smem + (size_t)(kAdjRows + 2 * PAD) * 32;  // two tap buffers of NT x 32
     const int lane = threadIdx.x, rg = threadIdx.y;
     const int tid = rg * 32 + lane;
-    const int f0 = blockIdx.x * 32;
     const int f = f0 + lane;
-    const int i0 = blockIdx.y * kAdjRows;
     const bool fok = f < M;
     const bool dc = f == 0;
     // taps of group g into buffer st: 16 pieces of 16 bytes per 32-frequency row (M even)
@@ -95,7 +96,6 @@ __global__ void __launch_bounds__(32 * kAdjRG) k_wire_conv_adj(const float2* __r
         const int o = i0 + s;
         Gs[s][lane] = (fok && o < nout) ? Gh[(size_t)o * M + f] : make_float2(0.f, 0.f);
     }
-    const int rb0 = rg * kAdjRB;
     for (int g = 0; g < G; ++g) {
         if (g + 1 < G) {
             issue(g + 1, (g + 1) & 1);
@@ -105,10 +105,10 @@ __global__ void __launch_bounds__(32 * kAdjRG) k_wire_conv_adj(const float2* __r
             cp_async_wait<0>();
         __syncthreads();  // group g's taps (and, at g = 0, the G rows) visible to every thread
         const float2* Rs = Rbuf + (size_t)(g & 1) * NT * 32;
-        if (fok) {
-            float2 acc[kAdjRB], win[kAdjRB];
+        if (fok && rb0 >= 0) {
+            float2 acc[RB], win[RB];
 #pragma unroll
-            for (int r = 0; r < kAdjRB; ++r) {
+            for (int r = 0; r < RB; ++r) {
                 acc[r] = make_float2(0.f, 0.f);
                 win[r] = Gs[rb0 + r][lane];
             }
@@ -118,23 +118,75 @@ __global__ void __launch_bounds__(32 * kAdjRG) k_wire_conv_adj(const float2* __r
                 const float rc = dc ? 0.f : rr.y;
                 const float ry = dc ? rr.y : rr.x;
 #pragma unroll
-                for (int r = 0; r < kAdjRB; ++r) {
+                for (int r = 0; r < RB; ++r) {
                     const float2 q = win[r];  // G row rb0 + r + jj
                     acc[r].x = fmaf(rr.x, q.x, fmaf(rc, q.y, acc[r].x));
                     acc[r].y = fmaf(ry, q.y, fmaf(-rc, q.x, acc[r].y));
                 }
 #pragma unroll
-                for (int r = 0; r < kAdjRB - 1; ++r) win[r] = win[r + 1];
-                win[kAdjRB - 1] = Gs[min(rb0 + kAdjRB + jj, SROWS - 1)][lane];
+                for (int r = 0; r < RB - 1; ++r) win[r] = win[r + 1];
+                win[RB - 1] = Gs[min(rb0 + RB + jj, SROWS - 1)][lane];
             }
 #pragma unroll
-            for (int r = 0; r < kAdjRB; ++r) {
-                const int i = i0 + rb0 + r;
-                if (i < nin) dQh[((size_t)g * nin + i) * M + f] = acc[r];
-            }
+            for (int r = 0; r < RB; ++r)
+                if (mask >> r & 1) dQh[((size_t)g * nin + i0 + rb0 + r) * M + f] = acc[r];
         }
         __syncthreads();  // buffer g & 1 is refilled with group g + 2 next
     }
+}
+
+__global__ void __launch_bounds__(32 * kAdjRG) k_wire_conv_adj(const float2* __restrict__ Gh,
+                                                                const float2* __restrict__ Rh,
+                                                                float2* __restrict__ dQh, int G, int PAD, int nin,
+                                                                int nout, int M)
+{
+    extern __shared__ __align__(16) float2 adj_smem[];
+    const int i0 = blockIdx.y * kAdjRows, rb0 = threadIdx.y * kAdjRB, left = nin - (i0 + rb0);
+    adj_unit<kAdjRB>(Gh, Rh, dQh, G, PAD, nin, nout, M, blockIdx.x * 32, i0, kAdjRows, rb0,
+             left >= kAdjRB ? 0xffu : (1u << max(left, 0)) - 1u, adj_smem);
+}
+
+// The chunks of a list (wire_fft.cuh), WAYS warps a group of rows.
+static_assert(kAdjGroups == kAdjRG, "a chunk is a block's rows");
+template <int WAYS>
+__device__ __forceinline__ void adj_ways(const float2* __restrict__ Gh, const float2* __restrict__ Rh,
+                                         float2* __restrict__ dQh, int G, int PAD, int nin, int nout, int M, int f0,
+                                         const RowList& list, const int4& c, float2* adj_smem)
+{
+    constexpr int RB = kAdjRB / WAYS;
+    const int mine = threadIdx.y / WAYS, first = RB * (threadIdx.y & (WAYS - 1));
+    const int i0 = list.item[c.x].x;
+    const int2 it = mine < c.y ? list.item[c.x + mine] : make_int2(0, 0);
+    adj_unit<RB>(Gh, Rh, dQh, G, PAD, nin, nout, M, f0, i0, c.w, mine < c.y ? it.x - i0 + first : -1,
+                 (unsigned)it.y >> first & ((1u << RB) - 1u), adj_smem);
+}
+__global__ void __launch_bounds__(32 * kAdjRG) k_wire_rows_adj(const float2* __restrict__ Gh,
+                                                               const float2* __restrict__ Rh,
+                                                               float2* __restrict__ dQh, int G, int PAD, int nin,
+                                                               int nout, int M, RowList list)
+{
+    extern __shared__ __align__(16) float2 adj_smem[];
+    const int nf = (M + 31) / 32, total = list.count[1] * nf;
+    for (int u = blockIdx.x; u < total; u += gridDim.x) {
+        const int4 c = list.chunk[u / nf];
+        const int f0 = u % nf * 32;
+        if (c.y <= kAdjRG / 4) adj_ways<4>(Gh, Rh, dQh, G, PAD, nin, nout, M, f0, list, c, adj_smem);
+        else if (c.y <= kAdjRG / 2) adj_ways<2>(Gh, Rh, dQh, G, PAD, nin, nout, M, f0, list, c, adj_smem);
+        else adj_ways<1>(Gh, Rh, dQh, G, PAD, nin, nout, M, f0, list, c, adj_smem);
+    }
+}
+
+static size_t adj_smem_bytes(int npad)
+{
+    return sizeof(float2) * 32 * ((size_t)(kAdjRows + 2 * npad) + 2 * (size_t)(2 * npad + 1));
+}
+
+void launch_wire_rows_adj(const float2* Gh, const float2* taps, float2* dQh, int G, int npad, int nin, int nout, int M,
+                          const RowList& list, cudaStream_t s)
+{
+    const size_t smem = adj_smem_bytes(npad);
+    cudaFuncSetAttribute((const void*)k_wire_rows_adj, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    k_wire_rows_adj<<<148 * 4, dim3(32, kAdjRG), smem, s>>>(Gh, taps, dQh, G, npad, nin, nout, M, list);
 }
 
 void launch_wire_conv_adj(const float2* Gh, const float2* Rh, float2* dQh, int G, int npad, int nin, int nout, int M,
@@ -143,7 +195,7 @@ void launch_wire_conv_adj(const float2* Gh, const float2* Rh, float2* dQh, int G
     if (nin <= 0) return;
     dim3 grid((M + 31) / 32, (nin + kAdjRows - 1) / kAdjRows);
     dim3 block(32, kAdjRG);
-    const size_t smem = sizeof(float2) * 32 * ((size_t)(kAdjRows + 2 * npad) + 2 * (size_t)(2 * npad + 1));
+    const size_t smem = adj_smem_bytes(npad);
     cudaFuncSetAttribute((const void*)k_wire_conv_adj, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     k_wire_conv_adj<<<grid, block, smem, s>>>(Gh, Rh, dQh, G, npad, nin, nout, M);
 }

@@ -288,6 +288,7 @@ struct Core {
     DevBuf d_fq, d_fluc;               // fluctuation: drifted charges, per (plane, depo) draw sums
     DevBuf d_draws, d_draws_used;            // fluctuation: the cells' draws
     DevBuf d_heavy;                          // the raster's heavy tiles
+    DevBuf d_energy, d_rows;                 // row energies of the wire convolution, its faint rows
     DevBuf d_pool, d_pool_off, d_pool_used;  // time profiles of long patches
     DevBuf d_wide;                           // per visit key: holds a long patch
     // modify_depo charge scale ([depo][plane], wct_dt_set_charge_scale); used
@@ -576,9 +577,14 @@ static FlucParams fluc_params(const Core& c, bool fluct, int ident0, const int* 
     return fp;
 }
 
-// The d_wide buffer: a byte per key, one per wire, then two counters.
+// The d_wide buffer: a byte per key, one per wire, then counters: the heavy tiles'
+// four, the faint rows' two of each plane (batch: of all planes).
+constexpr int kRowCounter = 4;
 static size_t wide_counters(size_t nkeys, size_t nwires) { return (nkeys + nwires + 15) & ~(size_t)15; }
-static size_t wide_bytes(size_t nkeys, size_t nwires) { return wide_counters(nkeys, nwires) + 4 * sizeof(int); }
+static size_t wide_bytes(size_t nkeys, size_t nwires)
+{
+    return wide_counters(nkeys, nwires) + (kRowCounter + 2 * kMaxPlanes) * sizeof(int);
+}
 
 // h_depos (optional): the depos in host memory, uploaded into d_depos here
 // in chunks on the copy stream, each chunk's prep blocks launched as soon as
@@ -753,6 +759,37 @@ static int prepare_event(Core& c, const double* d_depos, size_t ndepos, cudaStre
     return WCT_OK;
 }
 
+// The overlap-save wire convolution's energies and list of faint rows of every plane.
+struct WireFix {
+    size_t energy[kMaxPlanes], item[kMaxPlanes], chunk[kMaxPlanes], items;
+};
+static int wire_fix(Core& c, const EventPlan& ev, bool adjoint, WireFix& f)
+{
+    size_t ne = 0, ni = 0, nc = 0;
+    for (int ip = 0; ip < ev.np; ++ip) {
+        const PlaneState& ps = *c.planes[ip];
+        const GridPlane& g = ev.gset.p[ip];
+        f.energy[ip] = ne;
+        f.item[ip] = ni;
+        f.chunk[ip] = nc;
+        if (!g.nin || !ps.have_wspec) continue;
+        const int n = adjoint ? g.nin : g.nin + 2 * ps.npad;
+        ne += wire_energy_count(n, ps.npad, g.N / 2);
+        ni += wire_list_count(n, ps.npad);
+        nc += wire_chunk_count(n, ps.npad);
+    }
+    f.items = (ni + 1) & ~(size_t)1;
+    CUDA_TRY(c.d_energy.ensure(sizeof(double) * std::max<size_t>(ne, 1)));
+    CUDA_TRY(c.d_rows.ensure(sizeof(int2) * f.items + sizeof(int4) * nc));
+    return WCT_OK;
+}
+static RowList row_list(Core& c, const EventPlan& ev, const WireFix& f, int ip)
+{
+    int* counters = reinterpret_cast<int*>(c.d_wide.as<char>() + wide_counters(ev.nkeys, ev.pset.nwires_total));
+    return RowList{counters + kRowCounter + 2 * ip, c.d_rows.as<int2>() + f.item[ip],
+                   reinterpret_cast<int4*>(c.d_rows.as<int2>() + f.items) + f.chunk[ip]};
+}
+
 static int dft_rows(const float2* in, long ld_in, float2* out, long ld_out, int nrows, int n, int sign,
                     cudaStream_t s);
 
@@ -887,6 +924,9 @@ static int forward_device(Core& c, const double* d_depos, size_t ndepos, float* 
               (rows > 0 ? raster_launches : 0));
     CUDA_TRY(cudaGetLastError());
 
+    WireFix fix;
+    int frc = wire_fix(c, ev, false, fix);
+    if (frc) return frc;
     // the planes' chains: on streams of their own unless profiling or a long-range step needs s alone
     bool fork = fork_planes && !c.profiling && np > 1;
     for (int ip = 0; ip < np; ++ip)
@@ -946,19 +986,23 @@ static int forward_device(Core& c, const double* d_depos, size_t ndepos, float* 
                                                     g.ntile}
                                           : TileMap{});
                 t_f.close(1);
+                const int wlo = std::max(0, w.m_start_ch), whi = std::min(ps.desc.nwires, w.m_end_ch);
+                const unsigned char* flags = row_flag + pset.p[ip].wire_base;
                 Core::StageTimer t_c(&c, 3, ps_s);
-                if (ps.have_wspec && wire_fft_pays(ps.npad, nout))
-                    launch_wire_conv_fft(reinterpret_cast<const float2*>(Q), ps.d_wspec.as<float2>(), V, ps.G,
-                                         ps.npad, nin, nout, M, ps_s);
+                const bool wire = ps.have_wspec && wire_fft_pays(ps.npad, nout);
+                if (wire)
+                    launch_wire_conv_fft(reinterpret_cast<const float2*>(Q), ps.d_wspec.as<float2>(),
+                                         ps.d_spec.as<float2>(), V, ps.G, ps.npad, nin, nout, M, ps.mirror,
+                                         c.d_energy.as<double>() + fix.energy[ip],
+                                         WantRows{w.start_ch - ps.npad, wlo, whi, ps.desc.nwires, flags, nullptr, 0},
+                                         row_list(c, ev, fix, ip), ps_s);
                 else
                     launch_wire_conv(reinterpret_cast<const float2*>(Q), ps.d_spec.as<float2>(), V, ps.G, ps.npad,
                                      nin, nout, M, ps.mirror, ps_s);
-                t_c.close(1);
-                const int wlo = std::max(0, w.m_start_ch), whi = std::min(ps.desc.nwires, w.m_end_ch);
+                t_c.close(wire ? 3 : 1);
                 Core::StageTimer t_i(&c, 4, ps_s);
                 launch_irfft_rows(V, nout, d, w.start_ch - ps.npad, wlo, whi, w.start_tick, std::min(N, w.nt_ref),
-                                  nticks, d_frame + (size_t)ps.row0 * nticks, ps_s, row_flag + pset.p[ip].wire_base,
-                                  ps.desc.nwires, ps.npad);
+                                  nticks, d_frame + (size_t)ps.row0 * nticks, ps_s, flags, ps.desc.nwires, ps.npad);
                 if (!ps.long_wf.empty() && whi > wlo) {
                     rc = long_conv_rows(c, ps, d_frame + ((size_t)ps.row0 + wlo) * nticks, nticks, whi - wlo, nticks,
                                         false, ps_s);
@@ -1019,6 +1063,9 @@ static int adjoint_device(Core& c, const double* d_depos, size_t ndepos, const f
     CUDA_TRY(c.d_gglob.ensure(sizeof(double) * 3));
     double* gg = d_gglob ? d_gglob : c.d_gglob.as<double>();
     if (!d_gglob) CUDA_TRY(cudaMemsetAsync(gg, 0, sizeof(double) * 3, s));
+    WireFix fix;
+    prc = wire_fix(c, ev, true, fix);
+    if (prc) return prc;
     AdjSet as{};
     as.nplanes = np;
     for (int ip = 0; ip < np; ++ip) {
@@ -1062,13 +1109,19 @@ static int adjoint_device(Core& c, const double* d_depos, size_t ndepos, const f
         t_f.close(2);
         float* dQ = c.d_Q.as<float>() + g.qoff;
         Core::StageTimer t_c(&c, 7, s);
-        if (ps.have_wspec && wire_adj_fft_pays(ps.npad))
-            launch_wire_adj_fft(reinterpret_cast<const float2*>(Gr), ps.d_wspec.as<float2>(),
-                                reinterpret_cast<float2*>(dQ), ps.G, ps.npad, nin, nout, M, s);
+        const bool wire = ps.have_wspec && wire_adj_fft_pays(ps.npad);
+        if (wire)
+            launch_wire_adj_fft(reinterpret_cast<const float2*>(Gr), ps.d_wspec.as<float2>(), ps.d_spec.as<float2>(),
+                                reinterpret_cast<float2*>(dQ), ps.G, ps.npad, nin, nout, M,
+                                c.d_energy.as<double>() + fix.energy[ip],
+                                WantRows{w.start_ch, 0, ps.desc.nwires, ps.desc.nwires, nullptr,
+                                         c.d_wcnt.as<int>() + (size_t)g.wire_base * ev.gset.ntiles_abs,
+                                         ev.gset.ntiles_abs},
+                                row_list(c, ev, fix, ip), s);
         else
             launch_wire_conv_adj(reinterpret_cast<const float2*>(Gr), ps.d_spec.as<float2>(),
                                  reinterpret_cast<float2*>(dQ), ps.G, ps.npad, nin, nout, M, s);
-        t_c.close(1);
+        t_c.close(wire ? 3 : 1);
         Core::StageTimer t_i(&c, 8, s);
         launch_irfft_rows(reinterpret_cast<const float2*>(dQ), ps.G * nin, d, 0, 0, ps.G * nin, 0, N, N, dQ, s);
         t_i.close(1);
@@ -1190,6 +1243,8 @@ struct BatchState {
     DevBuf d_pool, d_pool_off, d_pool_used;  // time profiles of long patches
     DevBuf d_draws, d_draws_used;            // fluctuation: the cells' draws
     DevBuf d_heavy;                          // the raster's heavy tiles
+    DevBuf d_energy, d_rows;                 // row energies of the wire convolution, its faint rows
+    int maxblocks{0};                        // wire row blocks of a plane at most
     long long draws_cap{0};
     DevBuf d_wide;                           // per key: holds a long patch
     long long pool_cap{0};
@@ -1294,9 +1349,9 @@ static int batch_setup(Core& c)
     CUDA_TRY(b.d_descs.ensure(sizeof(FftDesc) * descs.size()));
     CUDA_TRY(cudaMemcpy(b.d_descs.p, descs.data(), sizeof(FftDesc) * descs.size(), cudaMemcpyHostToDevice));
     bs.nwires_total = nwt;
-    long long q = 0, v = 0;
+    long long q = 0, v = 0, en = 0;
     int wbase = 0;
-    b.maxG = 0;
+    b.maxG = b.maxblocks = 0;
     std::vector<const float2*> tab(2 * (size_t)np * bs.ncls);  // taps, then wire spectra
     for (int ip = 0; ip < np; ++ip) {
         PlaneState& ps = *c.planes[ip];
@@ -1323,9 +1378,17 @@ static int batch_setup(Core& c)
     for (int k = 0; k < bs.ncls; ++k)
         for (int ip = 0; ip < np; ++ip)
             if (wire_fft_fits(c.planes[ip]->G, c.planes[ip]->npad, cls[k] / 2)) bs.pl[ip].wire_cls |= 1ull << k;
-    // every plane's response spectra at every length, in one allocation: the wire
-    // spectra where the overlap-save form applies (their taps are scratch), else the taps
-    size_t total = 0, scratch = 0;
+    for (int ip = 0; ip < np; ++ip) {
+        BatchPlaneStatic& pl = bs.pl[ip];
+        pl.eslot = en;
+        if (!pl.wire_cls) continue;
+        en += (long long)wire_energy_count(pl.nin_max + 2 * pl.npad, pl.npad, b.maxM);
+        b.maxblocks = std::max(b.maxblocks, wire_row_blocks(pl.nin_max + 2 * pl.npad, pl.npad));
+    }
+    bs.eslot_total = en;
+    // every plane's response spectra at every length, in one allocation: the taps, and
+    // the wire spectra where the overlap-save form applies
+    size_t total = 0;
     auto taps_count = [&](int ip, int k) {
         return (size_t)c.planes[ip]->G * (2 * c.planes[ip]->npad + 1) * (cls[k] / 2);
     };
@@ -1333,26 +1396,19 @@ static int batch_setup(Core& c)
     auto room = [](size_t n) { return (n + 15) & ~(size_t)15; };
     for (int ip = 0; ip < np; ++ip)
         for (int k = 0; k < bs.ncls; ++k) {
-            if (has_wire(ip, k)) {
-                total += room(wire_spec_count(c.planes[ip]->G, cls[k] / 2));
-                scratch = std::max(scratch, taps_count(ip, k));
-            }
-            else total += room(taps_count(ip, k));
+            total += room(taps_count(ip, k));
+            if (has_wire(ip, k)) total += room(wire_spec_count(c.planes[ip]->G, cls[k] / 2));
         }
-    DevBuf taps_scratch;
     CUDA_TRY(b.d_spec.ensure(sizeof(float2) * std::max<size_t>(total, 1)));
-    CUDA_TRY(taps_scratch.ensure(sizeof(float2) * std::max<size_t>(scratch, 1)));
     float2* at = b.d_spec.as<float2>();
     for (int ip = 0; ip < np; ++ip) {
         PlaneState& ps = *c.planes[ip];
         const int rows = ps.G * (2 * ps.npad + 1);
         for (int k = 0; k < bs.ncls; ++k) {
             const int N = cls[k];
-            float2* taps = taps_scratch.as<float2>();
-            if (!has_wire(ip, k)) {
-                tab[(size_t)ip * bs.ncls + k] = taps = at;
-                at += room(taps_count(ip, k));
-            }
+            float2* taps = at;
+            tab[(size_t)ip * bs.ncls + k] = taps;
+            at += room(taps_count(ip, k));
             launch_rfft_rows(ps.d_table.as<float>(), ps.ldr, std::min(ps.nresp, N), taps, N / 2, rows,
                              b.cls_plans[k]->desc, c.own_stream);
             if (has_wire(ip, k)) {
@@ -1466,7 +1522,7 @@ static int forward_batch_device(Core& c, const double* d_depos, const long long*
         std::vector<void*> before = {b.d_Q.p, b.d_V.p, b.d_rec.p, b.d_tprof.p, b.d_win.p, b.d_wcnt.p, b.d_woff.p,
                                      b.d_wcur.p, b.d_kbound.p, b.d_wlist.p, b.d_plans.p, b.d_fq.p, b.d_fluc.p,
                                      b.d_ident.p, b.d_pool.p, b.d_pool_off.p, b.d_pool_used.p, b.d_wide.p, b.d_draws.p,
-                                     b.d_draws_used.p, b.d_heavy.p,
+                                     b.d_draws_used.p, b.d_heavy.p, b.d_energy.p, b.d_rows.p,
                                      const_cast<double*>(c.qscale())};
         CUDA_TRY(b.d_Q.ensure(sizeof(float) * (size_t)bs.qslot_total * K));
         CUDA_TRY(b.d_V.ensure(sizeof(float2) * (size_t)bs.vslot_total * K));
@@ -1480,6 +1536,16 @@ static int forward_batch_device(Core& c, const double* d_depos, const long long*
         CUDA_TRY(b.d_wide.ensure(wide_bytes((size_t)nkeysK, (size_t)K * bs.nwires_total)));
         const size_t parts = heavy_items(b.vcap, nkeysK);
         CUDA_TRY(b.d_heavy.ensure(sizeof(int4) * parts + 2 * sizeof(int) * (size_t)nkeysK));
+        size_t row_items = 0, row_chunks = 0;
+        for (int ip = 0; ip < np; ++ip)
+            if (bs.pl[ip].wire_cls) {
+                const int n = bs.pl[ip].nin_max + 2 * bs.pl[ip].npad;
+                row_items += wire_list_count(n, bs.pl[ip].npad) * K;
+                row_chunks += wire_chunk_count(n, bs.pl[ip].npad) * K;
+            }
+        row_items = (row_items + 1) & ~(size_t)1;
+        CUDA_TRY(b.d_energy.ensure(sizeof(double) * std::max<size_t>((size_t)bs.eslot_total * K, 1)));
+        CUDA_TRY(b.d_rows.ensure(sizeof(int2) * row_items + sizeof(int4) * row_chunks));
         CUDA_TRY(b.d_wlist.ensure(sizeof(Visit) * (size_t)b.vcap));
         CUDA_TRY(b.d_plans.ensure(sizeof(BatchPlan) * (size_t)nch));
         CUDA_TRY(b.d_ident.ensure(sizeof(int)));
@@ -1500,7 +1566,7 @@ static int forward_batch_device(Core& c, const double* d_depos, const long long*
         std::vector<void*> after = {b.d_Q.p, b.d_V.p, b.d_rec.p, b.d_tprof.p, b.d_win.p, b.d_wcnt.p, b.d_woff.p,
                                     b.d_wcur.p, b.d_kbound.p, b.d_wlist.p, b.d_plans.p, b.d_fq.p, b.d_fluc.p,
                                     b.d_ident.p, b.d_pool.p, b.d_pool_off.p, b.d_pool_used.p, b.d_wide.p, b.d_draws.p,
-                                     b.d_draws_used.p, b.d_heavy.p,
+                                     b.d_draws_used.p, b.d_heavy.p, b.d_energy.p, b.d_rows.p,
                                     const_cast<double*>(c.qscale())};
         if (b.h_plans_n < (size_t)nch) {
             if (b.h_plans) cudaFreeHost(b.h_plans);
@@ -1587,22 +1653,31 @@ static int forward_batch_device(Core& c, const double* d_depos, const long long*
                 // by overlap-save: every plane at once
                 unsigned long long any_wire = 0;
                 for (int ip = 0; ip < np; ++ip) any_wire |= bs.pl[ip].wire_cls;
+                const RowList faint{heavy.count + kRowCounter, b.d_rows.as<int2>(),
+                                    reinterpret_cast<int4*>(b.d_rows.as<int2>() + row_items)};
                 if (any_wire)
-                    launch_conv_fft_batch(plans + ch, bs, b.d_spec_tab.as<const float2*>() + (size_t)np * bs.ncls,
-                                          b.d_Q.as<float>(), b.d_V.as<float2>(), b.nsm * 2, s);
-                // directly: one launch per run of planes that share the pad and the group pairing
+                    launch_conv_fft_batch(plans + ch, bs, ne, b.maxblocks,
+                                          b.d_spec_tab.as<const float2*>() + (size_t)np * bs.ncls, b.d_Q.as<float>(),
+                                          b.d_V.as<float2>(), b.d_energy.as<double>(), row_flag, faint, b.nsm * 2, s);
+                // directly: the faint rows of those and the other classes, one launch each per run
+                // of planes that share the pad and the group pairing
                 const unsigned long long every = ~0ull >> (64 - bs.ncls);
                 for (int ip0 = 0; ip0 < np;) {
-                    int ip1 = ip0 + 1;
-                    if (bs.pl[ip0].wire_cls == every) {
-                        ip0 = ip1;
-                        continue;
-                    }
+                    int ip1 = ip0;
+                    unsigned long long some = 0, all = every;  // classes by overlap-save in one of the planes, in all
                     while (ip1 < np && c.planes[ip1]->npad == c.planes[ip0]->npad &&
-                           c.planes[ip1]->mirror == c.planes[ip0]->mirror)
-                        ++ip1;
-                    launch_conv_batch(plans + ch, bs, ip0, ip1, c.planes[ip0]->mirror,
-                                      b.d_spec_tab.as<const float2*>(), b.d_Q.as<float>(), b.d_V.as<float2>(), nb_c, s);
+                           c.planes[ip1]->mirror == c.planes[ip0]->mirror) {
+                        some |= bs.pl[ip1].wire_cls;
+                        all &= bs.pl[ip1++].wire_cls;
+                    }
+                    if (some)
+                        launch_rows_batch(plans + ch, bs, ip0, ip1, c.planes[ip0]->mirror, b.maxM,
+                                          b.d_spec_tab.as<const float2*>(), b.d_Q.as<float>(), b.d_V.as<float2>(),
+                                          faint, b.nsm * 2, s);
+                    if (all != every)
+                        launch_conv_batch(plans + ch, bs, ip0, ip1, c.planes[ip0]->mirror,
+                                          b.d_spec_tab.as<const float2*>(), b.d_Q.as<float>(), b.d_V.as<float2>(),
+                                          nb_c, s);
                     ip0 = ip1;
                 }
                 for (int k = 0; k < bs.ncls; ++k)

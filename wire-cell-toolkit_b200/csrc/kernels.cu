@@ -33,6 +33,7 @@
 #include <algorithm>
 #include <cfloat>
 #include <climits>
+#include <type_traits>
 
 namespace wctb200 {
 
@@ -2225,16 +2226,12 @@ __global__ void __launch_bounds__(32 * kConvRG) k_wire_conv(const float2* __rest
     wire_conv_tile<PAD, PAIR>(Qh, Rh, Vh, G, nin, nout, M, blockIdx.x, blockIdx.y, conv_smem);
 }
 
-// Same convolution with a run-time pad (any response width).
-__global__ void __launch_bounds__(32 * kConvRG) k_wire_conv_any(const float2* __restrict__ Qh,
-                                                                 const float2* __restrict__ Rh,
-                                                                 float2* __restrict__ Vh, int G, int PAD, int nin,
-                                                                 int nout, int M)
+// One frequency (per lane) of the eight output rows o0 .. with a run-time pad; mask
+// are written.
+__device__ __forceinline__ void conv_rows_any(const float2* __restrict__ Qh, const float2* __restrict__ Rh,
+                                              float2* __restrict__ Vh, int G, int PAD, int nin, int M, int f, int o0,
+                                              unsigned mask)
 {
-    const int lane = threadIdx.x, rg = threadIdx.y;
-    const int f = blockIdx.x * 32 + lane;
-    const int o0 = blockIdx.y * kConvRows;
-    if (f >= M) return;
     float2 acc[kConvRB];
 #pragma unroll
     for (int r = 0; r < kConvRB; ++r) acc[r] = make_float2(0.f, 0.f);
@@ -2247,7 +2244,7 @@ __global__ void __launch_bounds__(32 * kConvRG) k_wire_conv_any(const float2* __
             const int j = jj - PAD;
 #pragma unroll
             for (int r = 0; r < kConvRB; ++r) {
-                const int i = o0 + rg * kConvRB + r - PAD - j;
+                const int i = o0 + r - PAD - j;
                 if (i < 0 || i >= nin) continue;
                 const float2 q = Qh[((size_t)g * nin + i) * M + f];
                 acc[r].x = fmaf(rr.x, q.x, fmaf(-rc, q.y, acc[r].x));
@@ -2256,9 +2253,32 @@ __global__ void __launch_bounds__(32 * kConvRG) k_wire_conv_any(const float2* __
         }
     }
 #pragma unroll
-    for (int r = 0; r < kConvRB; ++r) {
-        const int o = o0 + rg * kConvRB + r;
-        if (o < nout) Vh[(size_t)o * M + f] = acc[r];
+    for (int r = 0; r < kConvRB; ++r)
+        if (mask >> r & 1) Vh[(size_t)(o0 + r) * M + f] = acc[r];
+}
+
+// Same convolution with a run-time pad (any response width).
+__global__ void __launch_bounds__(32 * kConvRG) k_wire_conv_any(const float2* __restrict__ Qh,
+                                                                 const float2* __restrict__ Rh,
+                                                                 float2* __restrict__ Vh, int G, int PAD, int nin,
+                                                                 int nout, int M)
+{
+    const int f = blockIdx.x * 32 + threadIdx.x, o0 = blockIdx.y * kConvRows + threadIdx.y * kConvRB;
+    if (f >= M) return;
+    conv_rows_any(Qh, Rh, Vh, G, PAD, nin, M, f, o0, o0 + kConvRB <= nout ? 0xffu : (1u << max(nout - o0, 0)) - 1u);
+}
+
+// The rows of a list, a warp a group of eight at 32 frequencies.
+__global__ void __launch_bounds__(32 * kConvRG) k_wire_rows_any(const float2* __restrict__ Qh,
+                                                                const float2* __restrict__ Rh,
+                                                                float2* __restrict__ Vh, int G, int PAD, int nin, int M,
+                                                                RowList list)
+{
+    const int nf = (M + 31) / 32, total = list.count[0] * nf;
+    for (int u = blockIdx.x * kConvRG + threadIdx.y; u < total; u += gridDim.x * kConvRG) {
+        const int2 it = list.item[u / nf];
+        const int f = u % nf * 32 + threadIdx.x;
+        if (f < M) conv_rows_any(Qh, Rh, Vh, G, PAD, nin, M, f, it.x, it.y);
     }
 }
 
@@ -2273,30 +2293,28 @@ __global__ void __launch_bounds__(32 * kConvRG) k_wire_conv_any(const float2* __
 constexpr int kConv2F = 16;  // frequencies per block
 constexpr int kConv2RG = 16; // row groups per block (kConvRB output rows each)
 constexpr int kConv2Rows = kConv2RG * kConvRB;
+constexpr int kRowsBlocks = 148 * 2;  // resident blocks that take a list's rows
 
 
-template <int PAD, bool PAIR>
+template <int PAD, bool PAIR, int RG>
 constexpr size_t conv2_stage_f2()  // float2 values per pipeline stage
 {
-    return (size_t)kConv2F * ((PAIR ? 2 : 1) * (kConv2Rows + 2 * PAD) + (2 * PAD + 1));
+    return (size_t)kConv2F * ((PAIR ? 2 : 1) * (RG * kConvRB + 2 * PAD) + (2 * PAD + 1));
 }
 
-template <int PAD, bool PAIR>
-__global__ void __launch_bounds__(kConv2F * kConv2RG) k_wire_conv2(const float2* __restrict__ Qh,
-                                                                  const float2* __restrict__ Rh,
-                                                                  float2* __restrict__ Vh, int G, int nin, int nout,
-                                                                  int M)
+// Output rows at 16 frequencies: a thread's RB rows from o0 + rb0 on (rb0 < 0:
+// none), of which mask are written; the block's rows lie within span (at most
+// 8 RG) of o0.  Called by all 16 RG threads of the block.
+template <int PAD, bool PAIR, int RB, int RG>
+__device__ __forceinline__ void conv2_unit(const float2* __restrict__ Qh, const float2* __restrict__ Rh,
+                                           float2* __restrict__ Vh, int G, int nin, int M, int f0, int o0, int span,
+                                           int rb0, unsigned mask, float2* conv2_smem)
 {
-    constexpr int SROWS = kConv2Rows + 2 * PAD;
+    constexpr int SROWS = RG * kConvRB + 2 * PAD;
     constexpr int NT = 2 * PAD + 1;
-    constexpr size_t STAGE = conv2_stage_f2<PAD, PAIR>();
-    extern __shared__ __align__(16) float2 conv2_smem[];
-    const int lane = threadIdx.x, rg = threadIdx.y;
-    const int tid = rg * kConv2F + lane;
-    const int f0 = blockIdx.x * kConv2F;
+    constexpr size_t STAGE = conv2_stage_f2<PAD, PAIR, RG>();
+    const int tid = threadIdx.x, lane = tid & (kConv2F - 1);
     const int f = f0 + lane;
-    const int o0 = blockIdx.y * kConv2Rows;
-    const bool fok = f < M;
     const bool dc = f == 0;
     const int ng = PAIR ? (G + 1) / 2 : G;
     // copy of group gi into stage buffer st: 8 16-byte pieces per row of 16 frequencies
@@ -2310,8 +2328,8 @@ __global__ void __launch_bounds__(kConv2F * kConv2RG) k_wire_conv2(const float2*
         const int fp = f0 + 2 * (tid & 7);           // first frequency of this thread's piece
         const int fbytes = fp < M ? 16 : 0;          // M even: both or neither of fp, fp + 1
         constexpr int kPieces = kConv2F / 2;
-        constexpr int nthr = kConv2F * kConv2RG;
-        for (int e = tid; e < SROWS * kPieces; e += nthr) {
+        constexpr int nthr = kConv2F * RG;
+        for (int e = tid; e < (span + 2 * PAD) * kPieces; e += nthr) {
             const int srow = e / kPieces;
             const int i = o0 - 2 * PAD + srow;
             const bool ok = i >= 0 && i < nin && fbytes;
@@ -2330,10 +2348,9 @@ __global__ void __launch_bounds__(kConv2F * kConv2RG) k_wire_conv2(const float2*
         }
         cp_async_commit();
     };
-    float2 acc[kConvRB];
+    float2 acc[RB];
 #pragma unroll
-    for (int r = 0; r < kConvRB; ++r) acc[r] = make_float2(0.f, 0.f);
-    const int rb0 = rg * kConvRB;
+    for (int r = 0; r < RB; ++r) acc[r] = make_float2(0.f, 0.f);
     issue(0, 0);
     for (int gi = 0; gi < ng; ++gi) {
         if (gi + 1 < ng) {
@@ -2343,49 +2360,98 @@ __global__ void __launch_bounds__(kConv2F * kConv2RG) k_wire_conv2(const float2*
         else
             cp_async_wait<0>();
         __syncthreads();
-        const float2* base = conv2_smem + (size_t)(gi & 1) * STAGE;
-        const float2* Qs = base;
-        const float2* Qs2 = base + SROWS * kConv2F;
-        const float2* Rs = base + (PAIR ? 2 : 1) * SROWS * kConv2F;
-        float2 win[kConvRB], win2[kConvRB];
+        if (rb0 >= 0) {
+            const float2* base = conv2_smem + (size_t)(gi & 1) * STAGE;
+            const float2* Qs = base;
+            const float2* Qs2 = base + SROWS * kConv2F;
+            const float2* Rs = base + (PAIR ? 2 : 1) * SROWS * kConv2F;
+            float2 win[RB], win2[RB];
 #pragma unroll
-        for (int r = 0; r < kConvRB; ++r) {
-            win[r] = Qs[(rb0 + r + 2 * PAD) * kConv2F + lane];  // input row o - PAD - j at j = -PAD
-            if (PAIR) win2[r] = Qs2[(rb0 + r) * kConv2F + lane];  // input row o - PAD + j at j = -PAD
-        }
-#pragma unroll
-        for (int jj = 0; jj < NT; ++jj) {
-            const float2 rr = Rs[jj * kConv2F + lane];
-            // bin 0 packs two real spectra (DC, Nyquist): multiply component-wise there
-            const float rc = dc ? 0.f : rr.y;
-            const float ry = dc ? rr.y : rr.x;
-#pragma unroll
-            for (int r = 0; r < kConvRB; ++r) {
-                float2 q = win[r];
-                if (PAIR) q = make_float2(q.x + win2[r].x, q.y + win2[r].y);
-                acc[r].x = fmaf(rr.x, q.x, fmaf(-rc, q.y, acc[r].x));
-                acc[r].y = fmaf(ry, q.y, fmaf(rc, q.x, acc[r].y));
+            for (int r = 0; r < RB; ++r) {
+                win[r] = Qs[(rb0 + r + 2 * PAD) * kConv2F + lane];  // input row o - PAD - j at j = -PAD
+                if (PAIR) win2[r] = Qs2[(rb0 + r) * kConv2F + lane];  // input row o - PAD + j at j = -PAD
             }
-            if (jj < NT - 1) {
 #pragma unroll
-                for (int r = kConvRB - 1; r > 0; --r) win[r] = win[r - 1];
-                win[0] = Qs[(rb0 + 2 * PAD - jj - 1) * kConv2F + lane];
-                if (PAIR) {
+            for (int jj = 0; jj < NT; ++jj) {
+                const float2 rr = Rs[jj * kConv2F + lane];
+                // bin 0 packs two real spectra (DC, Nyquist): multiply component-wise there
+                const float rc = dc ? 0.f : rr.y;
+                const float ry = dc ? rr.y : rr.x;
 #pragma unroll
-                    for (int r = 0; r < kConvRB - 1; ++r) win2[r] = win2[r + 1];
-                    win2[kConvRB - 1] = Qs2[(rb0 + kConvRB + jj) * kConv2F + lane];
+                for (int r = 0; r < RB; ++r) {
+                    float2 q = win[r];
+                    if (PAIR) q = make_float2(q.x + win2[r].x, q.y + win2[r].y);
+                    acc[r].x = fmaf(rr.x, q.x, fmaf(-rc, q.y, acc[r].x));
+                    acc[r].y = fmaf(ry, q.y, fmaf(rc, q.x, acc[r].y));
+                }
+                if (jj < NT - 1) {
+#pragma unroll
+                    for (int r = RB - 1; r > 0; --r) win[r] = win[r - 1];
+                    win[0] = Qs[(rb0 + 2 * PAD - jj - 1) * kConv2F + lane];
+                    if (PAIR) {
+#pragma unroll
+                        for (int r = 0; r < RB - 1; ++r) win2[r] = win2[r + 1];
+                        win2[RB - 1] = Qs2[(rb0 + RB + jj) * kConv2F + lane];
+                    }
                 }
             }
         }
         __syncthreads();  // buffer gi & 1 is refilled with group gi + 2 next
     }
-    if (fok) {
+    if (f < M && rb0 >= 0) {
 #pragma unroll
-        for (int r = 0; r < kConvRB; ++r) {
-            const int o = o0 + rb0 + r;
-            if (o < nout) Vh[(size_t)o * M + f] = acc[r];
-        }
+        for (int r = 0; r < RB; ++r)
+            if (mask >> r & 1) Vh[(size_t)(o0 + rb0 + r) * M + f] = acc[r];
     }
+}
+
+template <int PAD, bool PAIR>
+__global__ void __launch_bounds__(kConv2F * kConv2RG) k_wire_conv2(const float2* __restrict__ Qh,
+                                                                  const float2* __restrict__ Rh,
+                                                                  float2* __restrict__ Vh, int G, int nin, int nout,
+                                                                  int M)
+{
+    extern __shared__ __align__(16) float2 conv2_smem[];
+    const int o0 = blockIdx.y * kConv2Rows, rb0 = threadIdx.x / kConv2F * kConvRB, left = nout - (o0 + rb0);
+    conv2_unit<PAD, PAIR, kConvRB, kConv2RG>(Qh, Rh, Vh, G, nin, M, blockIdx.x * kConv2F, o0, kConv2Rows, rb0,
+                          left >= kConvRB ? 0xffu : (1u << max(left, 0)) - 1u, conv2_smem);
+}
+
+// A list's chunk at 16 frequencies: a group of rows per 16 threads, where that
+// leaves half of the block without one two or four 16 a group (a chunk is a chain
+// of copies and sums: few rows take as long as many).
+template <int PAD, bool PAIR, int WAYS>
+__device__ __forceinline__ void conv2_ways(const float2* __restrict__ Qh, const float2* __restrict__ Rh,
+                                           float2* __restrict__ Vh, int G, int nin, int M, int f0,
+                                           const RowList& list, const int4& c, float2* conv2_smem)
+{
+    constexpr int RB = kConvRB / WAYS;
+    const int rg = threadIdx.x / kConv2F, mine = rg / WAYS, first = RB * (rg & (WAYS - 1));
+    const int o0 = list.item[c.x].x;
+    const int2 it = mine < c.y ? list.item[c.x + mine] : make_int2(0, 0);
+    conv2_unit<PAD, PAIR, RB, kConvGroups>(Qh, Rh, Vh, G, nin, M, f0, o0, c.w, mine < c.y ? it.x - o0 + first : -1,
+                              (unsigned)it.y >> first & ((1u << RB) - 1u), conv2_smem);
+}
+template <int PAD, bool PAIR>
+__device__ __forceinline__ void conv2_chunk(const float2* __restrict__ Qh, const float2* __restrict__ Rh,
+                                            float2* __restrict__ Vh, int G, int nin, int M, int f0,
+                                            const RowList& list, const int4& c, float2* conv2_smem)
+{
+    if (c.y <= kConvGroups / 4) conv2_ways<PAD, PAIR, 4>(Qh, Rh, Vh, G, nin, M, f0, list, c, conv2_smem);
+    else if (c.y <= kConvGroups / 2) conv2_ways<PAD, PAIR, 2>(Qh, Rh, Vh, G, nin, M, f0, list, c, conv2_smem);
+    else conv2_ways<PAD, PAIR, 1>(Qh, Rh, Vh, G, nin, M, f0, list, c, conv2_smem);
+}
+
+template <int PAD, bool PAIR>
+__global__ void __launch_bounds__(kConv2F * kConvGroups) k_wire_rows2(const float2* __restrict__ Qh,
+                                                                  const float2* __restrict__ Rh,
+                                                                  float2* __restrict__ Vh, int G, int nin, int M,
+                                                                  RowList list)
+{
+    extern __shared__ __align__(16) float2 conv2_smem[];
+    const int nf = (M + kConv2F - 1) / kConv2F, total = list.count[1] * nf;
+    for (int u = blockIdx.x; u < total; u += gridDim.x)
+        conv2_chunk<PAD, PAIR>(Qh, Rh, Vh, G, nin, M, u % nf * kConv2F, list, list.chunk[u / nf], conv2_smem);
 }
 
 void launch_wire_conv(const float2* Qh, const float2* Rh, float2* Vh, int ngroups, int npad, int nrows_in,
@@ -2395,10 +2461,10 @@ void launch_wire_conv(const float2* Qh, const float2* Rh, float2* Vh, int ngroup
     const bool al16 = ((reinterpret_cast<uintptr_t>(Qh) | reinterpret_cast<uintptr_t>(Rh)) & 15) == 0 && M % 2 == 0;
     if (al16 && (npad == 21 || npad == 10)) {
         dim3 grid2((M + kConv2F - 1) / kConv2F, (nrows_out + kConv2Rows - 1) / kConv2Rows);
-        dim3 block2(kConv2F, kConv2RG);
+        const int block2 = kConv2F * kConv2RG;
 #define WCT_CONV2(P, B)                                                                                       \
     do {                                                                                                      \
-        const size_t sm = 2 * conv2_stage_f2<P, B>() * sizeof(float2);                                       \
+        const size_t sm = 2 * conv2_stage_f2<P, B, kConv2RG>() * sizeof(float2);                                       \
         cudaFuncSetAttribute((const void*)k_wire_conv2<P, B>, cudaFuncAttributeMaxDynamicSharedMemorySize,   \
                              (int)sm);                                                                        \
         k_wire_conv2<P, B><<<grid2, block2, sm, s>>>(Qh, Rh, Vh, ngroups, nrows_in, nrows_out, M);            \
@@ -2939,42 +3005,6 @@ void launch_rfft_batch(const BatchPlan* plan, const FftDesc* descs, float* Q, in
     k_rfft_batch<<<nblocks, nthreads, smem, s>>>(plan, descs, Q);
 }
 
-// Wire convolution with a run-time pad, one tile (generic response widths).
-__device__ __forceinline__ void wire_conv_tile_any(const float2* __restrict__ Qh, const float2* __restrict__ Rh,
-                                                   float2* __restrict__ Vh, int G, int PAD, int nin, int nout, int M,
-                                                   int fblk, int oblk)
-{
-    const int lane = threadIdx.x, rg = threadIdx.y;
-    const int f = fblk * 32 + lane;
-    const int o0 = oblk * kConvRows;
-    if (f >= M) return;
-    float2 acc[kConvRB];
-#pragma unroll
-    for (int r = 0; r < kConvRB; ++r) acc[r] = make_float2(0.f, 0.f);
-    for (int g = 0; g < G; ++g) {
-        const float2* Rg = Rh + (size_t)g * (2 * PAD + 1) * M + f;
-        for (int jj = 0; jj <= 2 * PAD; ++jj) {
-            const float2 rr = Rg[(size_t)jj * M];
-            const float rc = f == 0 ? 0.f : rr.y;
-            const float ry = f == 0 ? rr.y : rr.x;
-            const int j = jj - PAD;
-#pragma unroll
-            for (int r = 0; r < kConvRB; ++r) {
-                const int i = o0 + rg * kConvRB + r - PAD - j;
-                if (i < 0 || i >= nin) continue;
-                const float2 q = Qh[((size_t)g * nin + i) * M + f];
-                acc[r].x = fmaf(rr.x, q.x, fmaf(-rc, q.y, acc[r].x));
-                acc[r].y = fmaf(ry, q.y, fmaf(rc, q.x, acc[r].y));
-            }
-        }
-    }
-#pragma unroll
-    for (int r = 0; r < kConvRB; ++r) {
-        const int o = o0 + rg * kConvRB + r;
-        if (o < nout) Vh[(size_t)o * M + f] = acc[r];
-    }
-}
-
 // PAD < 0: run-time pad (bs.pl[ip].npad) without shared-memory staging.
 // Items of planes ip0 .. ip1-1 in order; within a plane, events in order.
 template <int PAD, bool PAIR>
@@ -3005,15 +3035,20 @@ __global__ void __launch_bounds__(32 * kConvRG) k_conv_batch(const BatchPlan* __
         const float2* R = spec[(size_t)ip * bs.ncls + E.cls];
         if constexpr (PAD >= 0)
             wire_conv_tile<PAD, PAIR>(Qh, R, V + E.voff, bs.pl[ip].G, E.nin, E.nout, E.M, fblk, oblk, conv_smem);
-        else
-            wire_conv_tile_any(Qh, R, V + E.voff, bs.pl[ip].G, bs.pl[ip].npad, E.nin, E.nout, E.M, fblk, oblk);
+        else {
+            const int f = fblk * 32 + threadIdx.x, o0 = oblk * kConvRows + threadIdx.y * kConvRB;
+            if (f < E.M)
+                conv_rows_any(Qh, R, V + E.voff, bs.pl[ip].G, bs.pl[ip].npad, E.nin, E.M, f, o0,
+                              o0 + kConvRB <= E.nout ? 0xffu : (1u << max(E.nout - o0, 0)) - 1u);
+        }
     }
 }
 
 // The same by overlap-save (wire_fft.cuh): the items of every plane.
 __global__ void __launch_bounds__(kWThreads, 2) k_conv_fft_batch(const BatchPlan* __restrict__ plan, BatchStatic bs,
                                                                  const float2* const* __restrict__ wspec,
-                                                                 const float* __restrict__ Q, float2* __restrict__ V)
+                                                                 const float* __restrict__ Q, float2* __restrict__ V,
+                                                                 double* __restrict__ energy)
 {
     extern __shared__ float2 wsm[];
     __shared__ int s_item;
@@ -3036,14 +3071,103 @@ __global__ void __launch_bounds__(kWThreads, 2) k_conv_fft_batch(const BatchPlan
         const int nfb = wire_fblocks(E.M);
         const int oblk = rel / nfb, fblk = rel - oblk * nfb;
         wfft::conv_tile(reinterpret_cast<const float2*>(Q + E.qoff), wspec[(size_t)ip * bs.ncls + E.cls], V + E.voff,
-                        bs.pl[ip].G, bs.pl[ip].npad, E.nin, E.nout, E.M, fblk, oblk, wsm);
+                        bs.pl[ip].G, bs.pl[ip].npad, E.nin, E.nout, E.M, fblk, oblk,
+                        energy + e * bs.eslot_total + bs.pl[ip].eslot + (size_t)rel * kWL, wsm);
     }
 }
 
-void launch_conv_fft_batch(const BatchPlan* plan, const BatchStatic& bs, const float2* const* wspec, const float* Q,
-                           float2* V, int nblocks, cudaStream_t s)
+// Their faint rows: block x of a wire row block, y of an entry of the pass.
+__global__ void __launch_bounds__(kPickThreads) k_pick_batch(const BatchPlan* __restrict__ plan, BatchStatic bs,
+                                                             const double* __restrict__ energy,
+                                                             const unsigned char* __restrict__ row_flag, RowList list)
 {
-    k_conv_fft_batch<<<nblocks, kWThreads, kWConvSmem, s>>>(plan, bs, wspec, Q, V);
+    if (plan->status & kBatchSkip) return;
+    const int k = blockIdx.y, e = k / bs.np, ip = k - e * bs.np;
+    const EvPlane& E = plan->ep[k];
+    const BatchPlaneStatic& pl = bs.pl[ip];
+    if (!E.nin || !((pl.wire_cls >> E.cls) & 1) || (int)blockIdx.x >= wire_blocks(E.nout, pl.npad)) return;
+    const int nfb = wire_fblocks(E.M);
+    const WantRows want{E.start_ch - pl.npad, max(0, E.m_start_ch), min(pl.nwires, E.m_end_ch), pl.nwires,
+                        row_flag + (size_t)e * bs.nwires_total + pl.wire_base, nullptr, 0};
+    wfft::pick_tile<false>(energy + e * bs.eslot_total + pl.eslot + (size_t)blockIdx.x * nfb * kWL, nfb, pl.npad,
+                           blockIdx.x, E.nout, want, k, list);
+}
+
+// The listed rows of planes ip0 .. ip1-1 (PAD < 0: run-time pad).
+template <int PAD, bool PAIR>
+__global__ void __launch_bounds__(kConv2F * kConvGroups) k_rows_batch(const BatchPlan* __restrict__ plan, BatchStatic bs,
+                                                                  int ip0, int ip1, int nf,
+                                                                  const float2* const* __restrict__ spec,
+                                                                  const float* __restrict__ Q, float2* V, RowList list)
+{
+    extern __shared__ __align__(16) float2 conv2_smem[];
+    if (plan->status & kBatchSkip) return;
+    const long long total = (long long)list.count[1] * nf;
+    for (long long u = blockIdx.x; u < total; u += gridDim.x) {
+        const int i = (int)(u / nf), f0 = (int)(u - (long long)i * nf) * kConv2F;
+        const int4 c = list.chunk[i];
+        const int e = c.z / bs.np, ip = c.z - e * bs.np;
+        const EvPlane& E = plan->ep[c.z];
+        if (ip < ip0 || ip >= ip1 || f0 >= E.M) continue;
+        const float2* Qh = reinterpret_cast<const float2*>(Q + E.qoff);
+        const float2* R = spec[(size_t)ip * bs.ncls + E.cls];
+        if constexpr (PAD >= 0)
+            conv2_chunk<PAD, PAIR>(Qh, R, V + E.voff, bs.pl[ip].G, E.nin, E.M, f0, list, c, conv2_smem);
+        else {
+            const int rg = threadIdx.x / kConv2F, f = f0 + (threadIdx.x & (kConv2F - 1));
+            if (rg >= c.y || f >= E.M) continue;
+            const int2 it = list.item[c.x + rg];
+            conv_rows_any(Qh, R, V + E.voff, bs.pl[ip].G, bs.pl[ip].npad, E.nin, E.M, f, it.x, it.y);
+        }
+    }
+}
+
+void launch_conv_fft_batch(const BatchPlan* plan, const BatchStatic& bs, int nev, int maxblocks,
+                           const float2* const* wspec, const float* Q, float2* V, double* energy,
+                           const unsigned char* row_flag, const RowList& list, int nblocks, cudaStream_t s)
+{
+    k_conv_fft_batch<<<nblocks, kWThreads, kWConvSmem, s>>>(plan, bs, wspec, Q, V, energy);
+    k_pick_batch<<<dim3(maxblocks, nev * bs.np), kPickThreads, 0, s>>>(plan, bs, energy, row_flag, list);
+}
+
+// f(std::integral_constant pad, bool_constant pair) for the pads with kernels of
+// their own; false for others.
+template <class F>
+static bool with_pad(int npad, bool pair, F f)
+{
+    using std::integral_constant;
+    if (npad == 10 && pair) f(integral_constant<int, 10>{}, std::true_type{});
+    else if (npad == 10) f(integral_constant<int, 10>{}, std::false_type{});
+    else if (npad == 21 && pair) f(integral_constant<int, 21>{}, std::true_type{});
+    else if (npad == 21) f(integral_constant<int, 21>{}, std::false_type{});
+    else return false;
+    return true;
+}
+
+void launch_rows_batch(const BatchPlan* plan, const BatchStatic& bs, int ip0, int ip1, bool pair, int maxM,
+                       const float2* const* spec, const float* Q, float2* V, const RowList& list, int nblocks,
+                       cudaStream_t s)
+{
+    const int nf = (maxM + kConv2F - 1) / kConv2F, nth = kConv2F * kConvGroups;
+    if (with_pad(bs.pl[ip0].npad, pair, [&](auto pad, auto pr) {
+            const size_t sm = 2 * conv2_stage_f2<pad.value, pr.value, kConvGroups>() * sizeof(float2);
+            k_rows_batch<pad.value, pr.value><<<nblocks, nth, sm, s>>>(plan, bs, ip0, ip1, nf, spec, Q, V, list);
+        }))
+        return;
+    k_rows_batch<-1, false><<<nblocks, nth, 0, s>>>(plan, bs, ip0, ip1, nf, spec, Q, V, list);
+}
+
+void launch_wire_rows(const float2* Qh, const float2* taps, float2* Vh, int G, int npad, int nin, int nout, int M,
+                      bool pair, const RowList& list, cudaStream_t s)
+{
+    const int nblocks = kRowsBlocks;
+    if (with_pad(npad, pair, [&](auto pad, auto pr) {
+            const size_t sm = 2 * conv2_stage_f2<pad.value, pr.value, kConvGroups>() * sizeof(float2);
+            allow_smem((const void*)k_wire_rows2<pad.value, pr.value>, sm);
+            k_wire_rows2<pad.value, pr.value><<<nblocks, kConv2F * kConvGroups, sm, s>>>(Qh, taps, Vh, G, nin, M, list);
+        }))
+        return;
+    k_wire_rows_any<<<2 * nblocks, dim3(32, kConvRG), 0, s>>>(Qh, taps, Vh, G, npad, nin, M, list);
 }
 
 size_t conv_smem_bytes(int npad, bool pair)
@@ -3116,6 +3240,13 @@ void batch_kernel_attributes(int maxG, int maxM)
     cudaFuncSetAttribute((const void*)k_rfft_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, sf);
     cudaFuncSetAttribute((const void*)k_irfft_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, sf);
     cudaFuncSetAttribute((const void*)k_conv_fft_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWConvSmem);
+    for (int npad : {10, 21})
+        for (bool pair : {false, true})
+            with_pad(npad, pair, [](auto pad, auto pr) {
+                cudaFuncSetAttribute((const void*)k_rows_batch<pad.value, pr.value>,
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)(2 * conv2_stage_f2<pad.value, pr.value, kConvGroups>() * sizeof(float2)));
+            });
     cudaFuncSetAttribute((const void*)k_conv_batch<10, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)conv_smem_bytes(10, true));
     cudaFuncSetAttribute((const void*)k_conv_batch<10, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,

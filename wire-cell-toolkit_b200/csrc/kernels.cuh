@@ -134,6 +134,24 @@ struct HeavyList {
 };
 inline size_t heavy_items(long long visits, long long keys) { return (size_t)(visits / kHeavyPart + keys + 1); }
 
+// Output rows of the overlap-save wire convolution that are worth convolving
+// again: row i is wire wire0 + i, in [wlo, whi); forward: within pad wires of a
+// flagged charge wire, adjoint: a wire with visits (cnt [wire][ntiles]).
+struct WantRows {
+    int wire0, wlo, whi, nwires;
+    const unsigned char* flag;
+    const int* cnt;
+    int ntiles;
+};
+// Their list (wire_fft.cuh): count[0] groups of eight rows (first row, mask of
+// rows) and count[1] chunks of neighbouring groups (first group, groups, entry of
+// the pass, rows from the first to the last); the counts zeroed by the caller.
+struct RowList {
+    int* count;
+    int2* item;
+    int4* chunk;
+};
+
 // Per-plane parameters of the adjoint's gather (adjoint.cu).
 struct AdjPlane {
     int nimp, nin, N, start_ch, col0;
@@ -170,6 +188,7 @@ struct BatchPlaneStatic {
     double imp_min, imp_bs;
     long long qslot;  // offset of the plane's grid within an event slot (floats)
     long long vslot;  // offset of the plane's V rows within an event slot (complex values)
+    long long eslot;  // offset of the plane's row energies within an event slot (doubles)
 };
 
 struct BatchStatic {
@@ -178,7 +197,7 @@ struct BatchStatic {
     int ncls;
     int cls_N[kMaxClasses];   // ascending time-FFT lengths
     unsigned char cls_fft3[kMaxClasses];  // the class has a three-stage plan (launches of its own)
-    long long qslot_total, vslot_total;
+    long long qslot_total, vslot_total, eslot_total;
     BatchPlaneStatic pl[kMaxPlanes];
 };
 
@@ -326,16 +345,29 @@ void launch_irfft3_batch(const BatchPlan* plan, const BatchStatic& bs, int cls, 
                          cudaStream_t s);
 // Overlap-save forms (wire_fft.cu): Rw holds wire_spec_count(G, M) values made
 // from the taps by launch_wire_spec; wire_fft_fits says whether they apply,
-// wire_fft_pays and wire_adj_fft_pays where they are the faster form.
+// wire_fft_pays and wire_adj_fft_pays where they are the faster form.  Faint rows
+// are convolved from the taps: energy holds wire_energy_count(n, ...) values,
+// list.item wire_list_count(n, ...) and list.chunk wire_chunk_count(n, ...)
+// entries for n output rows (adjoint: nin).
+size_t wire_energy_count(int n, int npad, int M);
+size_t wire_list_count(int n, int npad);
+size_t wire_chunk_count(int n, int npad);
+int wire_row_blocks(int n, int npad);
 size_t wire_spec_count(int G, int M);
 bool wire_fft_fits(int G, int npad, int M);
 bool wire_fft_pays(int npad, int nout);
 bool wire_adj_fft_pays(int npad);
 void launch_wire_spec(const float2* taps, float2* Rw, int G, int npad, int M, cudaStream_t s);
-void launch_wire_conv_fft(const float2* Qh, const float2* Rw, float2* Vh, int G, int npad, int nin, int nout, int M,
+void launch_wire_conv_fft(const float2* Qh, const float2* Rw, const float2* taps, float2* Vh, int G, int npad, int nin,
+                          int nout, int M, bool pair, double* energy, const WantRows& want, const RowList& list,
                           cudaStream_t s);
-void launch_wire_adj_fft(const float2* Gh, const float2* Rw, float2* dQh, int G, int npad, int nin, int nout, int M,
-                         cudaStream_t s);
+// The rows of a list by the direct sums (kernels.cu, adjoint.cu).
+void launch_wire_rows(const float2* Qh, const float2* taps, float2* Vh, int G, int npad, int nin, int nout, int M,
+                      bool pair, const RowList& list, cudaStream_t s);
+void launch_wire_rows_adj(const float2* Gh, const float2* taps, float2* dQh, int G, int npad, int nin, int nout, int M,
+                          const RowList& list, cudaStream_t s);
+void launch_wire_adj_fft(const float2* Gh, const float2* Rw, const float2* taps, float2* dQh, int G, int npad, int nin,
+                         int nout, int M, double* energy, const WantRows& want, const RowList& list, cudaStream_t s);
 // the single-buffered 32-frequency tiles (any alignment; the fallback of launch_wire_conv)
 void launch_wire_conv_tiles(const float2* Qh, const float2* Rh, float2* Vh, int ngroups, int npad, int nrows_in,
                             int nrows_out, int M, bool pair, cudaStream_t s);
@@ -429,8 +461,15 @@ void launch_conv_batch(const BatchPlan* plan, const BatchStatic& bs, int ip0, in
 void launch_irfft_batch(const BatchPlan* plan, const BatchStatic& bs, const FftDesc* descs, const float2* V,
                         float* frames, long long frame_stride, int nblocks, int nthreads, int maxM,
                         const unsigned char* row_flag, cudaStream_t s);
-void launch_conv_fft_batch(const BatchPlan* plan, const BatchStatic& bs, const float2* const* wspec, const float* Q,
-                           float2* V, int nblocks, cudaStream_t s);
+// The overlap-save items of every plane and the list of their faint rows; wspec:
+// wire spectra.  launch_rows_batch: the listed rows of planes [ip0, ip1), all
+// with the same pad and pairing.
+void launch_conv_fft_batch(const BatchPlan* plan, const BatchStatic& bs, int nev, int maxblocks,
+                           const float2* const* wspec, const float* Q, float2* V, double* energy,
+                           const unsigned char* row_flag, const RowList& list, int nblocks, cudaStream_t s);
+void launch_rows_batch(const BatchPlan* plan, const BatchStatic& bs, int ip0, int ip1, bool pair, int maxM,
+                       const float2* const* spec, const float* Q, float2* V, const RowList& list, int nblocks,
+                       cudaStream_t s);
 size_t conv_smem_bytes(int npad, bool pair);
 void batch_kernel_attributes(int maxG, int maxM);
 

@@ -7,23 +7,32 @@ namespace wctb200 {
 __global__ void __launch_bounds__(kWThreads, 2) k_wire_conv_fft(const float2* __restrict__ Qh,
                                                                 const float2* __restrict__ Rw,
                                                                 float2* __restrict__ Vh, int G, int P, int nin,
-                                                                int nout, int M)
+                                                                int nout, int M, double* __restrict__ energy)
 {
     extern __shared__ float2 wsm[];
     wfft::load_twiddles(wsm + 2 * kWEx, threadIdx.x);
     __syncthreads();
-    wfft::conv_tile(Qh, Rw, Vh, G, P, nin, nout, M, blockIdx.x, blockIdx.y, wsm);
+    wfft::conv_tile(Qh, Rw, Vh, G, P, nin, nout, M, blockIdx.x, blockIdx.y,
+                    energy + ((size_t)blockIdx.y * gridDim.x + blockIdx.x) * kWL, wsm);
 }
 
 __global__ void __launch_bounds__(kWThreads, 2) k_wire_adj_fft(const float2* __restrict__ Gh,
                                                                const float2* __restrict__ Rw,
                                                                float2* __restrict__ dQh, int G, int P, int nin,
-                                                               int nout, int M)
+                                                               int nout, int M, double* __restrict__ energy)
 {
     extern __shared__ float2 wsm[];
     wfft::load_twiddles(wsm + kWEx, threadIdx.x);
     __syncthreads();
-    wfft::adj_tile(Gh, Rw, dQh, G, P, nin, nout, M, blockIdx.x, blockIdx.y, wsm);
+    wfft::adj_tile(Gh, Rw, dQh, G, P, nin, nout, M, blockIdx.x, blockIdx.y,
+                   energy + ((size_t)blockIdx.y * gridDim.x + blockIdx.x) * kWL, wsm);
+}
+
+template <bool ADJ>
+__global__ void __launch_bounds__(kPickThreads) k_wire_pick(const double* __restrict__ energy, int nfb, int P, int n,
+                                                            WantRows want, RowList list)
+{
+    wfft::pick_tile<ADJ>(energy + (size_t)blockIdx.x * nfb * kWL, nfb, P, blockIdx.x, n, want, 0, list);
 }
 
 __global__ void __launch_bounds__(kWThreads) k_wire_spec(const float2* __restrict__ taps, float2* __restrict__ Rw,
@@ -62,22 +71,32 @@ void launch_wire_spec(const float2* taps, float2* Rw, int G, int npad, int M, cu
     k_wire_spec<<<dim3(wire_fblocks(M), G), kWThreads, kWAdjSmem, s>>>(taps, Rw, npad, M);
 }
 
-void launch_wire_conv_fft(const float2* Qh, const float2* Rw, float2* Vh, int G, int npad, int nin, int nout, int M,
+size_t wire_energy_count(int n, int npad, int M) { return (size_t)wire_blocks(n, npad) * wire_fblocks(M) * kWL; }
+size_t wire_list_count(int n, int npad) { return (size_t)wire_blocks(n, npad) * ((wire_valid(npad) + 7) / 8); }
+size_t wire_chunk_count(int n, int npad) { return (size_t)wire_blocks(n, npad) * 4; }
+int wire_row_blocks(int n, int npad) { return wire_blocks(n, npad); }
+
+void launch_wire_conv_fft(const float2* Qh, const float2* Rw, const float2* taps, float2* Vh, int G, int npad, int nin,
+                          int nout, int M, bool pair, double* energy, const WantRows& want, const RowList& list,
                           cudaStream_t s)
 {
     if (nout <= 0) return;
     cudaFuncSetAttribute((const void*)k_wire_conv_fft, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWConvSmem);
     k_wire_conv_fft<<<dim3(wire_fblocks(M), wire_blocks(nout, npad)), kWThreads, kWConvSmem, s>>>(
-        Qh, Rw, Vh, G, npad, nin, nout, M);
+        Qh, Rw, Vh, G, npad, nin, nout, M, energy);
+    k_wire_pick<false><<<wire_blocks(nout, npad), kPickThreads, 0, s>>>(energy, wire_fblocks(M), npad, nout, want, list);
+    launch_wire_rows(Qh, taps, Vh, G, npad, nin, nout, M, pair, list, s);
 }
 
-void launch_wire_adj_fft(const float2* Gh, const float2* Rw, float2* dQh, int G, int npad, int nin, int nout, int M,
-                         cudaStream_t s)
+void launch_wire_adj_fft(const float2* Gh, const float2* Rw, const float2* taps, float2* dQh, int G, int npad, int nin,
+                         int nout, int M, double* energy, const WantRows& want, const RowList& list, cudaStream_t s)
 {
     if (nin <= 0) return;
     cudaFuncSetAttribute((const void*)k_wire_adj_fft, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWAdjSmem);
-    k_wire_adj_fft<<<dim3(wire_fblocks(M), wire_blocks(nin, npad)), kWThreads, kWAdjSmem, s>>>(Gh, Rw, dQh, G, npad,
-                                                                                               nin, nout, M);
+    k_wire_adj_fft<<<dim3(wire_fblocks(M), wire_blocks(nin, npad)), kWThreads, kWAdjSmem, s>>>(
+        Gh, Rw, dQh, G, npad, nin, nout, M, energy);
+    k_wire_pick<true><<<wire_blocks(nin, npad), kPickThreads, 0, s>>>(energy, wire_fblocks(M), npad, nin, want, list);
+    launch_wire_rows_adj(Gh, taps, dQh, G, npad, nin, nout, M, list, s);
 }
 
 }  // namespace wctb200

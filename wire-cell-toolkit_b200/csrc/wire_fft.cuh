@@ -19,12 +19,22 @@
 // 960 wires, 11 groups of 43 taps, M = 1600: 148 -> 71 us (direct, cp.async
 // double buffered -> this); the adjoint 195 -> 113 us.
 //
+// Rounding: a transform spreads the rounding of a block's strong rows evenly over
+// all 256, about 1e-7 of the block's rms a row, where the direct sum's stays with
+// the wires within P.  So each tile also leaves the energy of its 256 rows, and
+// rows with under a ninth of the block's mean energy (or where that is not
+// finite) are convolved again directly (pick_tile below): wires beside a
+// bright one keep their own precision, and a NaN stays within P wires.
+//
 // Bin 0 of a packed row holds two real spectra (DC and Nyquist).  The DC
 // value is column 0 here and the Nyquist value column M, each real with
 // its own (real-tap) wire spectrum, so no bin needs a special product.
 #pragma once
 
+#include <cmath>
+
 #include "fft.cuh"
+#include "kernels.cuh"
 
 namespace wctb200 {
 
@@ -35,6 +45,9 @@ constexpr int kWEx = kWL * kWF;   // complex values of one exchange buffer
 // shared memory: the exchange buffer (and the tile of grid rows), the twiddles
 constexpr size_t kWConvSmem = sizeof(float2) * (2 * kWEx + kWL);
 constexpr size_t kWAdjSmem = sizeof(float2) * (kWEx + kWL);
+constexpr int kPickThreads = 4 * kWL;
+constexpr int kConvGroups = 16;  // groups of eight rows in a chunk's window: forward, adjoint
+constexpr int kAdjGroups = 8;
 constexpr int kWMaxPad = 64;      // at least half of every block's rows are outputs
 constexpr size_t kWMaxSpec = (size_t)1 << 24;  // wire-spectrum values of a plane (128 MB)
 
@@ -104,14 +117,34 @@ __device__ __forceinline__ const float4* spec_at(const float2* Rw, int M, int g,
     return reinterpret_cast<const float4*>(Rw) + ((size_t)g * wire_fblocks(M) + fblk) * (kWEx / 2) + threadIdx.x;
 }
 
+// Energies of a tile's rows are kept as [thread]: thread ty * 16 + fl holds point ty + 16 fl.
+__device__ __forceinline__ int energy_point(int t) { return t / kWF + 16 * (t & (kWF - 1)); }
+
+// Sums over the 16 lanes of a half warp that hold a row's columns: lane fl
+// returns the sum of e[fl] (the other half of the values goes to the lane across).
+template <typename T>
+__device__ __forceinline__ T row_sums(T* e, int fl)
+{
+#pragma unroll
+    for (int h = 8; h; h >>= 1) {
+        const bool up = fl & h;
+#pragma unroll
+        for (int j = 0; j < h; ++j) {
+            const T keep = up ? e[j + h] : e[j], give = up ? e[j] : e[j + h];
+            e[j] = keep + __shfl_xor_sync(0xffffffffu, give, h);
+        }
+    }
+    return e[0];
+}
+
 // One forward tile: columns fblk * 16 .. +15, outputs oblk * (256 - 2P) ...
 // All kWThreads threads call it; sm holds kWConvSmem bytes, its twiddles
 // loaded.  The rows of group g + 1 are copied into shared memory (16 bytes a
 // copy) while group g is transformed; its wire spectra go straight to
-// registers, asked for before the exchange.
+// registers, asked for before the exchange.  energy: of the tile's 256 rows.
 __device__ __forceinline__ void conv_tile(const float2* __restrict__ Qh, const float2* __restrict__ Rw,
                                           float2* __restrict__ Vh, int G, int P, int nin, int nout, int M, int fblk,
-                                          int oblk, float2* sm)
+                                          int oblk, double* __restrict__ energy, float2* sm)
 {
     const int tid = threadIdx.x;
     float2* ex = sm;
@@ -183,13 +216,18 @@ __device__ __forceinline__ void conv_tile(const float2* __restrict__ Qh, const f
             if (ty + 16 * n >= 2 * P && o < nout) store_col(Vh + (size_t)o * M, F, M, acc[n]);
         }
     }
+    double e[16];  // (columns past M are zero)
+#pragma unroll
+    for (int n = 0; n < 16; ++n) e[n] = (double)acc[n].x * (double)acc[n].x + (double)acc[n].y * (double)acc[n].y;
+    energy[tid] = row_sums(e, fl);
 }
 
 // One adjoint tile: rows i = iblk * (256 - 2P) ... of dQ for every group, from
-// nout rows of G: one transform forward, one back per group.  sm: kWAdjSmem.
+// nout rows of G: one transform forward, one back per group.  energy: of the
+// tile's 256 rows, over the groups.  sm: kWAdjSmem.
 __device__ __forceinline__ void adj_tile(const float2* __restrict__ Gh, const float2* __restrict__ Rw,
                                          float2* __restrict__ dQh, int G, int P, int nin, int nout, int M, int fblk,
-                                         int iblk, float2* sm)
+                                         int iblk, double* __restrict__ energy, float2* sm)
 {
     const int tid = threadIdx.x;
     float2* ex = sm;
@@ -205,8 +243,21 @@ __device__ __forceinline__ void adj_tile(const float2* __restrict__ Gh, const fl
     }
 #pragma unroll
     for (int r = 0; r < 16; ++r) x[r] = col_value(x[r], F, M);
+    // a power of two that brings the tile's gradients near 2^40, so that squares of their
+    // products with the responses neither vanish nor overflow
+    __shared__ unsigned s_top[kWThreads / 32];
+    unsigned top = 0;
+#pragma unroll
+    for (int r = 0; r < 16; ++r) top = max(top, max(__float_as_uint(fabsf(x[r].x)), __float_as_uint(fabsf(x[r].y))));
+    top = __reduce_max_sync(0xffffffffu, top);
+    if ((tid & 31) == 0) s_top[tid >> 5] = top;
     fft256_a<-1>(x, tw, ty);
-    fft256_b<-1>(x, ex, fl, ty);
+    fft256_b<-1>(x, ex, fl, ty);  // (its barriers stand between s_top's writes and reads)
+#pragma unroll
+    for (int k = 0; k < kWThreads / 32; ++k) top = max(top, s_top[k]);
+    const int expo = min(max((int)(top >> 23), 42), 253);
+    const float sc = __uint_as_float((unsigned)(254 + 40 - expo) << 23);  // 2^(40 + 127 - expo), at most 2^125
+    float es = 0.f;
     for (int g = 0; g < G; ++g) {
         const float4* rp = spec_at(Rw, M, g, fblk);
         float2 v[16];
@@ -226,7 +277,16 @@ __device__ __forceinline__ void adj_tile(const float2* __restrict__ Gh, const fl
                     store_col(dq + (size_t)(16 * n) * M, F, M, v[n]);
             }
         }
+        float e[16];
+#pragma unroll
+        for (int n = 0; n < 16; ++n) {
+            const float a = v[n].x * sc, b = v[n].y * sc;
+            e[n] = a * a + b * b;
+        }
+        es += row_sums(e, fl);
     }
+    const double back = 1.0 / (double)sc;
+    energy[tid] = (double)es * back * back;
 }
 
 // One table tile: the wire spectrum of group g's taps [2P + 1][M] (packed
@@ -252,6 +312,121 @@ __device__ __forceinline__ void spec_tile(const float2* __restrict__ taps, float
 #pragma unroll
     for (int j = 0; j < 8; ++j)
         w[j * kWThreads] = make_float4(v[2 * j].x * sc, v[2 * j].y * sc, v[2 * j + 1].x * sc, v[2 * j + 1].y * sc);
+}
+
+// ---------------------------------------------------------------------------
+// Rows whose energy is under a ninth of their block's mean: picked here, convolved
+// directly by conv2_chunk (kernels.cu) and adj_ways (adjoint.cu).
+//
+// kFaintEnergy: a row's rms at a third of its block's. The rounding that reaches a
+// row, in 1e-7 of the row itself against 64 bits (full APA, 20k track depos; by
+// rms around the row / rms of the row): 1 to 2: 2.2, worst 3.0 in overlap-save
+// blocks; 2 to 4: 2.9, worst 8.1; 4 to 8: 9; 8 to 16: 19; over 64: 4500.  The
+// direct sum: 3.8 throughout, worst 5.1, with the row transforms of then, 3.4 now.
+//
+// What it costs, and why this form: a launch that adds up the energies (9 us, a
+// block per 256 wires) and one that takes the list.  Rows are few on tracks (3 %
+// of a full APA's) and up to two thirds of a plane's around showers, where the
+// direct kernel's time a row decides, so the list keeps the shape of its blocks:
+// windows of sixteen groups of eight rows, staged once (one warp a group from L2:
+// 348 us against 146 for the three planes of 200k shower depos).  Events without
+// -> with this, us: plane 2k 267 -> 282, full APA on tracks 20k 523 -> 561, 520k
+// 1034 -> 1062, shower 200k 1665 -> 1744, fit step 20k 1443 -> 1518; 16 batched
+// events, kernels 4761 -> 5900.
+// ---------------------------------------------------------------------------
+constexpr double kFaintEnergy = 9.0;
+
+// Block blk's rows that are faint and wanted into the list, as groups of eight,
+// those of a window of neighbouring groups a chunk (the kernels that take them
+// stage the window's input rows).  energy: [nfb][256] of the block, an eighth of
+// the columns per 128 threads, added in a fixed order.
+template <bool ADJ>
+__device__ __forceinline__ void pick_tile(const double* __restrict__ energy, int nfb, int P, int blk, int n,
+                                          const WantRows& want, int entry, const RowList& list)
+{
+    __shared__ double2 s_e[8][kWL / 2];
+    __shared__ double s_w[kWL / 32];
+    __shared__ unsigned char s_f[kWL], s_want[4][kWL + 2 * kWMaxPad];
+    const int t = threadIdx.x & (kWL - 1), q = threadIdx.x / kWL;
+    const int base = blk * wire_valid(P), p0 = ADJ ? 0 : 2 * P;  // first row, its point
+    // forward: the flags of wires base .. of the block's rows and P on either side; adjoint: a
+    // quarter of the tiles of each row's wire
+    if (ADJ) {
+        const int W = want.wire0 + base + t;
+        int any = 0;
+        if (W >= 0 && W < want.nwires)
+            for (int k = q; k < want.ntiles; k += 4) any |= want.cnt[(size_t)W * want.ntiles + k];
+        s_want[q][t] = any != 0;
+    }
+    else if (threadIdx.x < wire_valid(P) + 2 * P) {
+        const int W = want.wire0 + base - P + (int)threadIdx.x;
+        s_want[0][threadIdx.x] = W >= 0 && W < want.nwires ? want.flag[W] : 0;
+    }
+    double e = 0.0;
+    {
+        const int h = threadIdx.x & (kWL / 2 - 1), part = threadIdx.x / (kWL / 2);
+        const double2* at = reinterpret_cast<const double2*>(energy) + h;
+        const int f1 = nfb * (part + 1) / 8;
+        double2 v = make_double2(0.0, 0.0);
+        for (int f = nfb * part / 8; f < f1; f += 8) {
+            double2 x[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k)
+                x[k] = f + k < f1 ? at[(size_t)(f + k) * (kWL / 2)] : make_double2(0.0, 0.0);
+#pragma unroll
+            for (int k = 0; k < 8; ++k) v = make_double2(v.x + x[k].x, v.y + x[k].y);
+        }
+        s_e[part][h] = v;
+    }
+    __syncthreads();
+    if (q == 0) {
+        const double* s = reinterpret_cast<const double*>(s_e) + t;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) e += s[k * kWL];
+        double m = e;
+#pragma unroll
+        for (int o = 16; o; o >>= 1) m += __shfl_xor_sync(0xffffffffu, m, o);
+        if ((t & 31) == 0) s_w[t >> 5] = m;
+    }
+    __syncthreads();
+    if (q == 0) {
+        double mean = 0.0;
+#pragma unroll
+        for (int k = 0; k < kWL / 32; ++k) mean += s_w[k];
+        mean *= 1.0 / kWL;
+        const int p = energy_point(t), r = p - p0, W = want.wire0 + base + r;
+        // (a NaN in either, or an infinite mean: faint)
+        bool faint = r >= 0 && r < wire_valid(P) && base + r < n && W >= want.wlo && W < want.whi &&
+                     !(kFaintEnergy * e >= mean && mean < INFINITY);
+        if (faint) {
+            int any = 0;
+            if (ADJ) any = s_want[0][r] | s_want[1][r] | s_want[2][r] | s_want[3][r];
+            else {
+#pragma unroll 1
+                for (int k = 0; k <= 2 * P; ++k) any |= s_want[0][r + k];
+            }
+            faint = any;
+        }
+        s_f[p] = faint;
+    }
+    __syncthreads();
+    if (threadIdx.x < 32) {  // at most 32 groups
+        const int g = threadIdx.x;
+        int mask = 0;
+#pragma unroll 1
+        for (int r = 0; r < 8 && 8 * g + r < wire_valid(P); ++r) mask |= s_f[p0 + 8 * g + r] << r;
+        const unsigned on = __ballot_sync(0xffffffffu, mask != 0);
+        int at = 0;
+        if (g == 0 && on) at = atomicAdd(list.count, __popc(on));
+        at = __shfl_sync(0xffffffffu, at, 0);
+        if (mask) list.item[at + __popc(on & ((1u << g) - 1))] = make_int2(base + 8 * g, mask);
+        constexpr int kWindow = ADJ ? kAdjGroups : kConvGroups;
+        const unsigned here = g * kWindow < 32 ? on >> (g * kWindow) & ((1u << kWindow) - 1) : 0u;
+        if (here)
+            list.chunk[atomicAdd(list.count + 1, 1)] =
+                make_int4(at + __popc(on & ((1u << (g * kWindow)) - 1)), __popc(here), entry,
+                          8 * (32 - __clz(here) - (__ffs(here) - 1)));
+    }
 }
 
 }  // namespace wfft
