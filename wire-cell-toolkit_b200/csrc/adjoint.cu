@@ -427,15 +427,13 @@ __global__ void __launch_bounds__(kGatherWarps * 32, 5) k_adj_gather(int n, Plan
                         add_carried(Vc, Vce, vc[0] + vc[1]);
                         add_carried(Vs, Vse, vs[0] + vs[1]);
                     }
-                    U += Ue;
-                    Vc += Vce;
-                    Vs += Vse;
+                    const double dU = (double)U + (double)Ue;
                     const float4 tq = s_t[wib][tau];
-                    acc_qn = fma((double)tq.x, (double)U, acc_qn);
-                    acc_cp = fma((double)tq.x, (double)Vc, acc_cp);
-                    acc_sp = fma((double)tq.x, (double)Vs, acc_sp);
-                    acc_ct = fma((double)tq.y, (double)U, acc_ct);
-                    acc_st = fma((double)tq.z, (double)U, acc_st);
+                    acc_qn = fma((double)tq.x, dU, acc_qn);
+                    acc_cp = fma((double)tq.x, (double)Vc + (double)Vce, acc_cp);
+                    acc_sp = fma((double)tq.x, (double)Vs + (double)Vse, acc_sp);
+                    acc_ct = fma((double)tq.y, dU, acc_ct);
+                    acc_st = fma((double)tq.z, dU, acc_st);
                 }
             }
         }
