@@ -2268,20 +2268,6 @@ __global__ void __launch_bounds__(32 * kConvRG) k_wire_conv_any(const float2* __
     conv_rows_any(Qh, Rh, Vh, G, PAD, nin, M, f, o0, o0 + kConvRB <= nout ? 0xffu : (1u << max(nout - o0, 0)) - 1u);
 }
 
-// The rows of a list, a warp a group of eight at 32 frequencies.
-__global__ void __launch_bounds__(32 * kConvRG) k_wire_rows_any(const float2* __restrict__ Qh,
-                                                                const float2* __restrict__ Rh,
-                                                                float2* __restrict__ Vh, int G, int PAD, int nin, int M,
-                                                                RowList list)
-{
-    const int nf = (M + 31) / 32, total = list.count[0] * nf;
-    for (int u = blockIdx.x * kConvRG + threadIdx.y; u < total; u += gridDim.x * kConvRG) {
-        const int2 it = list.item[u / nf];
-        const int f = u % nf * 32 + threadIdx.x;
-        if (f < M) conv_rows_any(Qh, Rh, Vh, G, PAD, nin, M, f, it.x, it.y);
-    }
-}
-
 // ---------------------------------------------------------------------------
 // The same convolution with the staging of the next group (pair) overlapped
 // with the arithmetic of the current one: 16 frequencies x 16 row groups per
@@ -2296,23 +2282,24 @@ constexpr int kConv2Rows = kConv2RG * kConvRB;
 constexpr int kRowsBlocks = 148 * 2;  // resident blocks that take a list's rows
 
 
-template <int PAD, bool PAIR, int RG>
-constexpr size_t conv2_stage_f2()  // float2 values per pipeline stage
+template <bool PAIR, int RG>
+constexpr size_t conv2_stage_f2(int pad)  // float2 values per pipeline stage
 {
-    return (size_t)kConv2F * ((PAIR ? 2 : 1) * (RG * kConvRB + 2 * PAD) + (2 * PAD + 1));
+    return (size_t)kConv2F * ((PAIR ? 2 : 1) * (RG * kConvRB + 2 * pad) + (2 * pad + 1));
 }
 
 // Output rows at 16 frequencies: a thread's RB rows from o0 + rb0 on (rb0 < 0:
 // none), of which mask are written; the block's rows lie within span (at most
-// 8 RG) of o0.  Called by all 16 RG threads of the block.
+// 8 RG) of o0.  PAD 0: run-time pad, the taps rolled by four.  Called by all 16 RG
+// threads of the block.
 template <int PAD, bool PAIR, int RB, int RG>
 __device__ __forceinline__ void conv2_unit(const float2* __restrict__ Qh, const float2* __restrict__ Rh,
-                                           float2* __restrict__ Vh, int G, int nin, int M, int f0, int o0, int span,
-                                           int rb0, unsigned mask, float2* conv2_smem)
+                                           float2* __restrict__ Vh, int G, int pad, int nin, int M, int f0, int o0,
+                                           int span, int rb0, unsigned mask, float2* conv2_smem)
 {
-    constexpr int SROWS = RG * kConvRB + 2 * PAD;
-    constexpr int NT = 2 * PAD + 1;
-    constexpr size_t STAGE = conv2_stage_f2<PAD, PAIR, RG>();
+    const int P = PAD ? PAD : pad;
+    const int SROWS = RG * kConvRB + 2 * P, NT = 2 * P + 1;
+    const size_t STAGE = conv2_stage_f2<PAIR, RG>(P);
     const int tid = threadIdx.x, lane = tid & (kConv2F - 1);
     const int f = f0 + lane;
     const bool dc = f == 0;
@@ -2329,9 +2316,9 @@ __device__ __forceinline__ void conv2_unit(const float2* __restrict__ Qh, const 
         const int fbytes = fp < M ? 16 : 0;          // M even: both or neither of fp, fp + 1
         constexpr int kPieces = kConv2F / 2;
         constexpr int nthr = kConv2F * RG;
-        for (int e = tid; e < (span + 2 * PAD) * kPieces; e += nthr) {
+        for (int e = tid; e < (span + 2 * P) * kPieces; e += nthr) {
             const int srow = e / kPieces;
-            const int i = o0 - 2 * PAD + srow;
+            const int i = o0 - 2 * P + srow;
             const bool ok = i >= 0 && i < nin && fbytes;
             const float2* src = ok ? Qh + ((size_t)g * nin + i) * M + fp : Qh;
             cp_async16(Qs + srow * kConv2F + 2 * (e % kPieces), src, ok ? 16 : 0);
@@ -2365,33 +2352,70 @@ __device__ __forceinline__ void conv2_unit(const float2* __restrict__ Qh, const 
             const float2* Qs = base;
             const float2* Qs2 = base + SROWS * kConv2F;
             const float2* Rs = base + (PAIR ? 2 : 1) * SROWS * kConv2F;
-            float2 win[RB], win2[RB];
-#pragma unroll
-            for (int r = 0; r < RB; ++r) {
-                win[r] = Qs[(rb0 + r + 2 * PAD) * kConv2F + lane];  // input row o - PAD - j at j = -PAD
-                if (PAIR) win2[r] = Qs2[(rb0 + r) * kConv2F + lane];  // input row o - PAD + j at j = -PAD
-            }
-#pragma unroll
-            for (int jj = 0; jj < NT; ++jj) {
-                const float2 rr = Rs[jj * kConv2F + lane];
-                // bin 0 packs two real spectra (DC, Nyquist): multiply component-wise there
-                const float rc = dc ? 0.f : rr.y;
-                const float ry = dc ? rr.y : rr.x;
+            if constexpr (PAD > 0) {
+                float2 win[RB], win2[RB];
 #pragma unroll
                 for (int r = 0; r < RB; ++r) {
-                    float2 q = win[r];
-                    if (PAIR) q = make_float2(q.x + win2[r].x, q.y + win2[r].y);
-                    acc[r].x = fmaf(rr.x, q.x, fmaf(-rc, q.y, acc[r].x));
-                    acc[r].y = fmaf(ry, q.y, fmaf(rc, q.x, acc[r].y));
+                    win[r] = Qs[(rb0 + r + 2 * PAD) * kConv2F + lane];  // input row o - PAD - j at j = -PAD
+                    if (PAIR) win2[r] = Qs2[(rb0 + r) * kConv2F + lane];  // input row o - PAD + j at j = -PAD
                 }
-                if (jj < NT - 1) {
 #pragma unroll
-                    for (int r = RB - 1; r > 0; --r) win[r] = win[r - 1];
-                    win[0] = Qs[(rb0 + 2 * PAD - jj - 1) * kConv2F + lane];
-                    if (PAIR) {
+                for (int jj = 0; jj <= 2 * PAD; ++jj) {
+                    const float2 rr = Rs[jj * kConv2F + lane];
+                    // bin 0 packs two real spectra (DC, Nyquist): multiply component-wise there
+                    const float rc = dc ? 0.f : rr.y;
+                    const float ry = dc ? rr.y : rr.x;
 #pragma unroll
-                        for (int r = 0; r < RB - 1; ++r) win2[r] = win2[r + 1];
-                        win2[RB - 1] = Qs2[(rb0 + RB + jj) * kConv2F + lane];
+                    for (int r = 0; r < RB; ++r) {
+                        float2 q = win[r];
+                        if (PAIR) q = make_float2(q.x + win2[r].x, q.y + win2[r].y);
+                        acc[r].x = fmaf(rr.x, q.x, fmaf(-rc, q.y, acc[r].x));
+                        acc[r].y = fmaf(ry, q.y, fmaf(rc, q.x, acc[r].y));
+                    }
+                    if (jj < 2 * PAD) {
+#pragma unroll
+                        for (int r = RB - 1; r > 0; --r) win[r] = win[r - 1];
+                        win[0] = Qs[(rb0 + 2 * PAD - jj - 1) * kConv2F + lane];
+                        if (PAIR) {
+#pragma unroll
+                            for (int r = 0; r < RB - 1; ++r) win2[r] = win2[r + 1];
+                            win2[RB - 1] = Qs2[(rb0 + RB + jj) * kConv2F + lane];
+                        }
+                    }
+                }
+            }
+            else {
+                float2 w[RB + 4], v[RB + 4];  // rows o - jj and o - 2P + jj of the next four taps
+#pragma unroll
+                for (int r = 0; r < RB; ++r) {
+                    w[4 + r] = Qs[(rb0 + r + 2 * P) * kConv2F + lane];
+                    if (PAIR) v[r] = Qs2[(rb0 + r) * kConv2F + lane];
+                }
+                for (int j0 = 0; j0 < NT; j0 += 4) {
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        w[3 - k] = Qs[max(rb0 + 2 * P - j0 - 1 - k, 0) * kConv2F + lane];
+                        if (PAIR) v[RB + k] = Qs2[min(rb0 + RB + j0 + k, SROWS - 1) * kConv2F + lane];
+                    }
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        if (j0 + k < NT) {
+                            const float2 rr = Rs[(j0 + k) * kConv2F + lane];
+                            const float rc = dc ? 0.f : rr.y;
+                            const float ry = dc ? rr.y : rr.x;
+#pragma unroll
+                            for (int r = 0; r < RB; ++r) {
+                                float2 q = w[4 + r - k];
+                                if (PAIR) q = make_float2(q.x + v[r + k].x, q.y + v[r + k].y);
+                                acc[r].x = fmaf(rr.x, q.x, fmaf(-rc, q.y, acc[r].x));
+                                acc[r].y = fmaf(ry, q.y, fmaf(rc, q.x, acc[r].y));
+                            }
+                        }
+                    }
+#pragma unroll
+                    for (int r = 0; r < RB; ++r) {
+                        w[3 + RB - r] = w[RB - 1 - r];
+                        if (PAIR) v[r] = v[r + 4];
                     }
                 }
             }
@@ -2413,7 +2437,7 @@ __global__ void __launch_bounds__(kConv2F * kConv2RG) k_wire_conv2(const float2*
 {
     extern __shared__ __align__(16) float2 conv2_smem[];
     const int o0 = blockIdx.y * kConv2Rows, rb0 = threadIdx.x / kConv2F * kConvRB, left = nout - (o0 + rb0);
-    conv2_unit<PAD, PAIR, kConvRB, kConv2RG>(Qh, Rh, Vh, G, nin, M, blockIdx.x * kConv2F, o0, kConv2Rows, rb0,
+    conv2_unit<PAD, PAIR, kConvRB, kConv2RG>(Qh, Rh, Vh, G, PAD, nin, M, blockIdx.x * kConv2F, o0, kConv2Rows, rb0,
                           left >= kConvRB ? 0xffu : (1u << max(left, 0)) - 1u, conv2_smem);
 }
 
@@ -2422,36 +2446,36 @@ __global__ void __launch_bounds__(kConv2F * kConv2RG) k_wire_conv2(const float2*
 // of copies and sums: few rows take as long as many).
 template <int PAD, bool PAIR, int WAYS>
 __device__ __forceinline__ void conv2_ways(const float2* __restrict__ Qh, const float2* __restrict__ Rh,
-                                           float2* __restrict__ Vh, int G, int nin, int M, int f0,
+                                           float2* __restrict__ Vh, int G, int pad, int nin, int M, int f0,
                                            const RowList& list, const int4& c, float2* conv2_smem)
 {
     constexpr int RB = kConvRB / WAYS;
     const int rg = threadIdx.x / kConv2F, mine = rg / WAYS, first = RB * (rg & (WAYS - 1));
     const int o0 = list.item[c.x].x;
     const int2 it = mine < c.y ? list.item[c.x + mine] : make_int2(0, 0);
-    conv2_unit<PAD, PAIR, RB, kConvGroups>(Qh, Rh, Vh, G, nin, M, f0, o0, c.w, mine < c.y ? it.x - o0 + first : -1,
+    conv2_unit<PAD, PAIR, RB, kConvGroups>(Qh, Rh, Vh, G, pad, nin, M, f0, o0, c.w, mine < c.y ? it.x - o0 + first : -1,
                               (unsigned)it.y >> first & ((1u << RB) - 1u), conv2_smem);
 }
 template <int PAD, bool PAIR>
 __device__ __forceinline__ void conv2_chunk(const float2* __restrict__ Qh, const float2* __restrict__ Rh,
-                                            float2* __restrict__ Vh, int G, int nin, int M, int f0,
+                                            float2* __restrict__ Vh, int G, int pad, int nin, int M, int f0,
                                             const RowList& list, const int4& c, float2* conv2_smem)
 {
-    if (c.y <= kConvGroups / 4) conv2_ways<PAD, PAIR, 4>(Qh, Rh, Vh, G, nin, M, f0, list, c, conv2_smem);
-    else if (c.y <= kConvGroups / 2) conv2_ways<PAD, PAIR, 2>(Qh, Rh, Vh, G, nin, M, f0, list, c, conv2_smem);
-    else conv2_ways<PAD, PAIR, 1>(Qh, Rh, Vh, G, nin, M, f0, list, c, conv2_smem);
+    if (c.y <= kConvGroups / 4) conv2_ways<PAD, PAIR, 4>(Qh, Rh, Vh, G, pad, nin, M, f0, list, c, conv2_smem);
+    else if (c.y <= kConvGroups / 2) conv2_ways<PAD, PAIR, 2>(Qh, Rh, Vh, G, pad, nin, M, f0, list, c, conv2_smem);
+    else conv2_ways<PAD, PAIR, 1>(Qh, Rh, Vh, G, pad, nin, M, f0, list, c, conv2_smem);
 }
 
 template <int PAD, bool PAIR>
 __global__ void __launch_bounds__(kConv2F * kConvGroups) k_wire_rows2(const float2* __restrict__ Qh,
                                                                   const float2* __restrict__ Rh,
-                                                                  float2* __restrict__ Vh, int G, int nin, int M,
-                                                                  RowList list)
+                                                                  float2* __restrict__ Vh, int G, int pad, int nin,
+                                                                  int M, RowList list)
 {
     extern __shared__ __align__(16) float2 conv2_smem[];
     const int nf = (M + kConv2F - 1) / kConv2F, total = list.count[1] * nf;
     for (int u = blockIdx.x; u < total; u += gridDim.x)
-        conv2_chunk<PAD, PAIR>(Qh, Rh, Vh, G, nin, M, u % nf * kConv2F, list, list.chunk[u / nf], conv2_smem);
+        conv2_chunk<PAD, PAIR>(Qh, Rh, Vh, G, pad, nin, M, u % nf * kConv2F, list, list.chunk[u / nf], conv2_smem);
 }
 
 void launch_wire_conv(const float2* Qh, const float2* Rh, float2* Vh, int ngroups, int npad, int nrows_in,
@@ -2464,7 +2488,7 @@ void launch_wire_conv(const float2* Qh, const float2* Rh, float2* Vh, int ngroup
         const int block2 = kConv2F * kConv2RG;
 #define WCT_CONV2(P, B)                                                                                       \
     do {                                                                                                      \
-        const size_t sm = 2 * conv2_stage_f2<P, B, kConv2RG>() * sizeof(float2);                                       \
+        const size_t sm = 2 * conv2_stage_f2<B, kConv2RG>(P) * sizeof(float2);                                       \
         cudaFuncSetAttribute((const void*)k_wire_conv2<P, B>, cudaFuncAttributeMaxDynamicSharedMemorySize,   \
                              (int)sm);                                                                        \
         k_wire_conv2<P, B><<<grid2, block2, sm, s>>>(Qh, Rh, Vh, ngroups, nrows_in, nrows_out, M);            \
@@ -3093,7 +3117,7 @@ __global__ void __launch_bounds__(kPickThreads) k_pick_batch(const BatchPlan* __
                            blockIdx.x, E.nout, want, k, list);
 }
 
-// The listed rows of planes ip0 .. ip1-1 (PAD < 0: run-time pad).
+// The listed rows of planes ip0 .. ip1-1, all of one pad and pairing (PAD 0: run-time pad).
 template <int PAD, bool PAIR>
 __global__ void __launch_bounds__(kConv2F * kConvGroups) k_rows_batch(const BatchPlan* __restrict__ plan, BatchStatic bs,
                                                                   int ip0, int ip1, int nf,
@@ -3111,14 +3135,7 @@ __global__ void __launch_bounds__(kConv2F * kConvGroups) k_rows_batch(const Batc
         if (ip < ip0 || ip >= ip1 || f0 >= E.M) continue;
         const float2* Qh = reinterpret_cast<const float2*>(Q + E.qoff);
         const float2* R = spec[(size_t)ip * bs.ncls + E.cls];
-        if constexpr (PAD >= 0)
-            conv2_chunk<PAD, PAIR>(Qh, R, V + E.voff, bs.pl[ip].G, E.nin, E.M, f0, list, c, conv2_smem);
-        else {
-            const int rg = threadIdx.x / kConv2F, f = f0 + (threadIdx.x & (kConv2F - 1));
-            if (rg >= c.y || f >= E.M) continue;
-            const int2 it = list.item[c.x + rg];
-            conv_rows_any(Qh, R, V + E.voff, bs.pl[ip].G, bs.pl[ip].npad, E.nin, E.M, f, it.x, it.y);
-        }
+        conv2_chunk<PAD, PAIR>(Qh, R, V + E.voff, bs.pl[ip].G, bs.pl[ip].npad, E.nin, E.M, f0, list, c, conv2_smem);
     }
 }
 
@@ -3130,44 +3147,41 @@ void launch_conv_fft_batch(const BatchPlan* plan, const BatchStatic& bs, int nev
     k_pick_batch<<<dim3(maxblocks, nev * bs.np), kPickThreads, 0, s>>>(plan, bs, energy, row_flag, list);
 }
 
-// f(std::integral_constant pad, bool_constant pair) for the pads with kernels of
-// their own; false for others.
+// f(std::integral_constant PAD, bool_constant PAIR): the pads with taps unrolled,
+// 0 (run-time pad) for others.
 template <class F>
-static bool with_pad(int npad, bool pair, F f)
+static void with_pad(int npad, bool pair, F f)
 {
-    using std::integral_constant;
-    if (npad == 10 && pair) f(integral_constant<int, 10>{}, std::true_type{});
-    else if (npad == 10) f(integral_constant<int, 10>{}, std::false_type{});
-    else if (npad == 21 && pair) f(integral_constant<int, 21>{}, std::true_type{});
-    else if (npad == 21) f(integral_constant<int, 21>{}, std::false_type{});
-    else return false;
-    return true;
+    auto go = [&](auto pad) {
+        if (pair) f(pad, std::true_type{});
+        else f(pad, std::false_type{});
+    };
+    if (npad == 10) go(std::integral_constant<int, 10>{});
+    else if (npad == 21) go(std::integral_constant<int, 21>{});
+    else go(std::integral_constant<int, 0>{});
 }
 
 void launch_rows_batch(const BatchPlan* plan, const BatchStatic& bs, int ip0, int ip1, bool pair, int maxM,
                        const float2* const* spec, const float* Q, float2* V, const RowList& list, int nblocks,
                        cudaStream_t s)
 {
-    const int nf = (maxM + kConv2F - 1) / kConv2F, nth = kConv2F * kConvGroups;
-    if (with_pad(bs.pl[ip0].npad, pair, [&](auto pad, auto pr) {
-            const size_t sm = 2 * conv2_stage_f2<pad.value, pr.value, kConvGroups>() * sizeof(float2);
-            k_rows_batch<pad.value, pr.value><<<nblocks, nth, sm, s>>>(plan, bs, ip0, ip1, nf, spec, Q, V, list);
-        }))
-        return;
-    k_rows_batch<-1, false><<<nblocks, nth, 0, s>>>(plan, bs, ip0, ip1, nf, spec, Q, V, list);
+    const int nf = (maxM + kConv2F - 1) / kConv2F, npad = bs.pl[ip0].npad;
+    with_pad(npad, pair, [&](auto PAD, auto PAIR) {
+        const size_t sm = 2 * conv2_stage_f2<PAIR.value, kConvGroups>(npad) * sizeof(float2);
+        k_rows_batch<PAD.value, PAIR.value>
+            <<<nblocks, kConv2F * kConvGroups, sm, s>>>(plan, bs, ip0, ip1, nf, spec, Q, V, list);
+    });
 }
 
 void launch_wire_rows(const float2* Qh, const float2* taps, float2* Vh, int G, int npad, int nin, int nout, int M,
                       bool pair, const RowList& list, cudaStream_t s)
 {
-    const int nblocks = kRowsBlocks;
-    if (with_pad(npad, pair, [&](auto pad, auto pr) {
-            const size_t sm = 2 * conv2_stage_f2<pad.value, pr.value, kConvGroups>() * sizeof(float2);
-            allow_smem((const void*)k_wire_rows2<pad.value, pr.value>, sm);
-            k_wire_rows2<pad.value, pr.value><<<nblocks, kConv2F * kConvGroups, sm, s>>>(Qh, taps, Vh, G, nin, M, list);
-        }))
-        return;
-    k_wire_rows_any<<<2 * nblocks, dim3(32, kConvRG), 0, s>>>(Qh, taps, Vh, G, npad, nin, M, list);
+    with_pad(npad, pair, [&](auto PAD, auto PAIR) {
+        const size_t sm = 2 * conv2_stage_f2<PAIR.value, kConvGroups>(npad) * sizeof(float2);
+        allow_smem((const void*)k_wire_rows2<PAD.value, PAIR.value>, sm);
+        k_wire_rows2<PAD.value, PAIR.value>
+            <<<kRowsBlocks, kConv2F * kConvGroups, sm, s>>>(Qh, taps, Vh, G, npad, nin, M, list);
+    });
 }
 
 size_t conv_smem_bytes(int npad, bool pair)
@@ -3240,12 +3254,12 @@ void batch_kernel_attributes(int maxG, int maxM)
     cudaFuncSetAttribute((const void*)k_rfft_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, sf);
     cudaFuncSetAttribute((const void*)k_irfft_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, sf);
     cudaFuncSetAttribute((const void*)k_conv_fft_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWConvSmem);
-    for (int npad : {10, 21})
+    for (int npad : {10, 21, kWMaxPad})
         for (bool pair : {false, true})
-            with_pad(npad, pair, [](auto pad, auto pr) {
-                cudaFuncSetAttribute((const void*)k_rows_batch<pad.value, pr.value>,
+            with_pad(npad, pair, [&](auto PAD, auto PAIR) {
+                cudaFuncSetAttribute((const void*)k_rows_batch<PAD.value, PAIR.value>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)(2 * conv2_stage_f2<pad.value, pr.value, kConvGroups>() * sizeof(float2)));
+                                     (int)(2 * conv2_stage_f2<PAIR.value, kConvGroups>(npad) * sizeof(float2)));
             });
     cudaFuncSetAttribute((const void*)k_conv_batch<10, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)conv_smem_bytes(10, true));
