@@ -8,6 +8,7 @@
 
 #include <algorithm>
 #include <charconv>
+#include <climits>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -525,7 +526,7 @@ static int ensure_spectra(Core& c, PlaneState& ps, int N)
     CUDA_TRY(ps.d_spec.ensure(sizeof(float2) * (size_t)rows * (N / 2)));
     launch_rfft_rows(ps.d_table.as<float>(), ps.ldr, std::min(ps.nresp, N), ps.d_spec.as<float2>(), N / 2, rows, d,
                      c.own_stream);
-    ps.have_wspec = wire_fft_fits(ps.G, ps.npad, N / 2);
+    ps.have_wspec = wire_fft_pays(ps.npad, INT_MAX) && wire_fft_fits(ps.G, ps.npad, N / 2);
     if (ps.have_wspec) {
         CUDA_TRY(ps.d_wspec.ensure(sizeof(float2) * wire_spec_count(ps.G, N / 2)));
         launch_wire_spec(ps.d_spec.as<float2>(), ps.d_wspec.as<float2>(), ps.G, ps.npad, N / 2, c.own_stream);
@@ -1109,7 +1110,7 @@ static int adjoint_device(Core& c, const double* d_depos, size_t ndepos, const f
         t_f.close(2);
         float* dQ = c.d_Q.as<float>() + g.qoff;
         Core::StageTimer t_c(&c, 7, s);
-        const bool wire = ps.have_wspec && wire_adj_fft_pays(ps.npad);
+        const bool wire = ps.have_wspec && wire_adj_fft_pays(ps.npad, nin);
         if (wire)
             launch_wire_adj_fft(reinterpret_cast<const float2*>(Gr), ps.d_wspec.as<float2>(), ps.d_spec.as<float2>(),
                                 reinterpret_cast<float2*>(dQ), ps.G, ps.npad, nin, nout, M,
@@ -1373,11 +1374,15 @@ static int batch_setup(Core& c)
         v += (long long)(pl.nin_max + 2 * ps.npad) * b.maxM;
         b.maxG = std::max(b.maxG, ps.G);
     }
-    // the wire form by length class (overlap-save wherever its spectra fit: at a pad of
-    // 10 too, 32 events in one block of wires 1.80 ms a call, 1.97 directly)
+    // the wire form by length class: overlap-save where its spectra fit, from a pad of 2 on
+    // (32 events, direct / overlap-save, ms a call: pad 1 1.65 / 2.05 on 150 wires, 6.0 / 6.7
+    // on 900, pad 2 equal at 1.9 and 6.5, pad 10 1.97 / 1.91 and 7.8 / 6.3: the batch's direct
+    // kernel stages one group at a time)
     for (int k = 0; k < bs.ncls; ++k)
-        for (int ip = 0; ip < np; ++ip)
-            if (wire_fft_fits(c.planes[ip]->G, c.planes[ip]->npad, cls[k] / 2)) bs.pl[ip].wire_cls |= 1ull << k;
+        for (int ip = 0; ip < np; ++ip) {
+            const PlaneState& ps = *c.planes[ip];
+            if (ps.npad >= 2 && wire_fft_fits(ps.G, ps.npad, cls[k] / 2)) bs.pl[ip].wire_cls |= 1ull << k;
+        }
     for (int ip = 0; ip < np; ++ip) {
         BatchPlaneStatic& pl = bs.pl[ip];
         pl.eslot = en;

@@ -356,7 +356,7 @@ int wire_row_blocks(int n, int npad);
 size_t wire_spec_count(int G, int M);
 bool wire_fft_fits(int G, int npad, int M);
 bool wire_fft_pays(int npad, int nout);
-bool wire_adj_fft_pays(int npad);
+bool wire_adj_fft_pays(int npad, int nin);
 void launch_wire_spec(const float2* taps, float2* Rw, int G, int npad, int M, cudaStream_t s);
 void launch_wire_conv_fft(const float2* Qh, const float2* Rw, const float2* taps, float2* Vh, int G, int npad, int nin,
                           int nout, int M, bool pair, double* energy, const WantRows& want, const RowList& list,

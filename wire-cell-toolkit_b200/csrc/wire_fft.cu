@@ -51,19 +51,25 @@ bool wire_fft_fits(int G, int npad, int M)
     return npad <= kWMaxPad && M % 2 == 0 && wire_spec_count(G, M) <= kWMaxSpec;
 }
 
-// Where the overlap-save form is the faster one (11 groups, M = 1600, times in
-// us, inputs not in L2).  Its time goes by blocks of 256 - 2P rows, the direct
-// forms' by G (2P + 1) a row.  P = 21: ahead at every size (nin = 2: 27 against
-// 31, 300: 37 / 78, 960: 71 / 148; adjoint 31 / 43, 59 / 74, 113 / 195).
-// P = 10: behind while one block holds all the rows (nin = 80: 29 / 21), ahead
-// from two blocks on (300: 37 / 47, 960: 72 / 86); the adjoint, with a
-// transform back per group, stays behind (960: 119 / 113).  Other pads have no
-// direct kernel of their own in the forward (P = 5, nin = 80: 29 / 87).
+// Where the overlap-save form, with its faint rows, is the faster one for an event
+// (11 groups, M = 1600, direct / overlap-save in us, inputs not in L2, a few faint
+// rows at the edges).  Its time goes by blocks of 256 - 2P rows, the direct
+// forms' by G (2P + 1) a row in tiles of 64 or 128 rows.
+//   P = 21: one tile 31 / 39, 170 charge wires 54 / 56, 240 78 / 61, 960 150 / 99
+//           (M = 3200: 54 / 52, 80 / 75, 125 / 104, 269 / 172);
+//   P = 10: 23 / 40, 47 / 54 (240), 86 / 91 (960; M = 3200: 150 / 158);
+//   others have no direct kernel of their own: P = 16 269 / 40, 539 / 102;
+//           P = 2 50 / 39, 56 / 45, 99 / 85; P = 1 39 / 39, 43 / 46, 64 / 86;
+//           P = 0 31 / 39, 45 / 85.
 bool wire_fft_pays(int npad, int nout)
 {
-    return npad >= 16 || npad != 10 || nout > wire_valid(npad);
+    if (npad == 21) return nout > 128;
+    return npad >= 2 && npad != 10;
 }
-bool wire_adj_fft_pays(int npad) { return npad >= 16; }
+// The adjoint, a transform back per group: P = 21: two tiles of 64 46 / 48, 170
+// wires 74 / 52, 960 197 / 101; P = 16: 37 / 48, 60 / 52, 160 / 103; P = 10: 46 /
+// 52 (170), 78 / 86 (600), 113 / 102 (960); P = 30, 40 wires: 54 / 46.
+bool wire_adj_fft_pays(int npad, int nin) { return npad > 21 || (npad >= 16 && nin > 128); }
 
 void launch_wire_spec(const float2* taps, float2* Rw, int G, int npad, int M, cudaStream_t s)
 {
