@@ -466,6 +466,11 @@ int wct_dt_set_drift_params(wct_depotransform* dt, double DL, double DT, double 
 int wct_dt_get_drift_params(const wct_depotransform* dt, double* DL, double* DT, double* lifetime);
 int wct_dt_destroy(wct_depotransform* dt);
 
+/* Gives the current device's memory that the library keeps for later calls (at
+ * most 1 GiB of what components and calls have freed) back to the device.
+ * Memory in use, and scratch of calls still running on a stream, stays. */
+int wct_release_memory(void);
+
 #ifdef __cplusplus
 }
 #endif

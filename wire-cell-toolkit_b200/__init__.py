@@ -156,6 +156,7 @@ SIGNATURES = {
     "wct_random_binomial_device": (C.c_int, [C.c_ulonglong, C.c_int, C.c_int, C.c_double, C.c_long, C.c_void_p,
                                              C.c_void_p]),
     "wct_dt_destroy": (C.c_int, [C.c_void_p]),
+    "wct_release_memory": (C.c_int, []),
 }
 
 STAGES = ("drift+prep", "raster", "time_fft", "wire_conv", "inverse_fft+frame", "other",
@@ -710,6 +711,11 @@ def binomial_device(seed, ident, n, p, count, d_out_ptr, stream=None):
     """``count`` Binomial(n, p) draws of the stream (seed, ident) into device memory."""
     _check(lib().wct_random_binomial_device(int(seed), int(ident), int(n), float(p), int(count),
                                             C.c_void_p(d_out_ptr), C.c_void_p(stream) if stream else None))
+
+
+def release_memory():
+    """Gives the device memory that the library keeps for later calls (at most 1 GiB) back to the current device."""
+    _check(lib().wct_release_memory())
 
 
 def drifter_json(dr):

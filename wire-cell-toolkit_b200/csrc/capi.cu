@@ -45,8 +45,8 @@ static int fail(int code, const std::string& msg) { return fail(code, msg.c_str(
 
 // ---------------------------------------------------------------------------
 // Device memory comes from a pool of the library's own, one per device.  What is
-// freed stays mapped up to kPoolKeep bytes and goes back to the device beyond
-// that: mapping and unmapping was most of a call that takes scratch and waits (a
+// freed stays mapped up to kPoolKeep bytes (until wct_release_memory) and goes
+// back to the device beyond that: mapping and unmapping was most of a call that takes scratch and waits (a
 // 2560 x 6000 2-D transform by itself: 1.9 ms, 0.2 ms of it kernels; the default
 // pool gives everything back at each synchronisation) and of a new component's
 // first event.  The pool may be used from several threads and streams; calls
@@ -2379,6 +2379,15 @@ int wct_pir_waveform(const wct_pir* p, int path, float* out)
 int wct_pir_destroy(wct_pir* p)
 {
     delete p;
+    return WCT_OK;
+}
+
+int wct_release_memory(void)
+{
+    int dev = 0;
+    CUDA_TRY(cudaGetDevice(&dev));
+    std::lock_guard<std::mutex> lk(g_pool_mtx);
+    if (dev >= 0 && dev < kPoolDevices && g_pools[dev]) CUDA_TRY(cudaMemPoolTrimTo(g_pools[dev], 0));
     return WCT_OK;
 }
 
