@@ -1286,6 +1286,10 @@ Core::~Core()
     destroy();
 }
 
+// Wire spectra of a batched component over its planes and length classes, 4 GB (a
+// full APA of 6000 ticks holds 1.6 GB of them, its taps 0.3 GB).
+constexpr size_t kMaxBatchSpec = (size_t)1 << 29;
+
 static int batch_setup(Core& c)
 {
     if (!c.batch) c.batch = std::make_unique<BatchState>();
@@ -1378,10 +1382,15 @@ static int batch_setup(Core& c)
     // (32 events, direct / overlap-save, ms a call: pad 1 1.65 / 2.05 on 150 wires, 6.0 / 6.7
     // on 900, pad 2 equal at 1.9 and 6.5, pad 10 1.97 / 1.91 and 7.8 / 6.3: the batch's direct
     // kernel stages one group at a time)
-    for (int k = 0; k < bs.ncls; ++k)
+    // -- the longest classes first, all planes' within kMaxBatchSpec values
+    size_t wire_total = 0;
+    for (int k = bs.ncls - 1; k >= 0; --k)
         for (int ip = 0; ip < np; ++ip) {
             const PlaneState& ps = *c.planes[ip];
-            if (ps.npad >= 2 && wire_fft_fits(ps.G, ps.npad, cls[k] / 2)) bs.pl[ip].wire_cls |= 1ull << k;
+            const size_t n = wire_spec_count(ps.G, cls[k] / 2);
+            if (ps.npad < 2 || !wire_fft_fits(ps.G, ps.npad, cls[k] / 2) || wire_total + n > kMaxBatchSpec) continue;
+            wire_total += n;
+            bs.pl[ip].wire_cls |= 1ull << k;
         }
     for (int ip = 0; ip < np; ++ip) {
         BatchPlaneStatic& pl = bs.pl[ip];
