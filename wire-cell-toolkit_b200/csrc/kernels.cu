@@ -1234,10 +1234,11 @@ int launch_raster_wires(const PatchRec* rec, const float* tprof, const TprofPool
 // redrawn as N ~ Binomial((int)|Q|, p_k t_tau / (sum p * sum t)) and the
 // patch is rescaled by Q / sum N; a patch whose draws are all zero adds
 // nothing.  The draws are counter-based: k_fluc_sums draws every cell to get
-// sum N, and the fluctuated raster draws the same cells again.  The unit bin
-// integrals that set each cell's probability come from one non-inlined
-// function with explicitly rounded operations, so both passes see the same
-// probabilities bit for bit and therefore the same draws.
+// sum N and keeps the draws for the fluctuated raster; cells past the room for
+// them are drawn again there.  The unit bin integrals that set each cell's
+// probability come from one non-inlined function with explicitly rounded
+// operations, so both see the same probabilities bit for bit and therefore the
+// same draws.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ int event_of_depo(const EventTable& et, int i)
 {

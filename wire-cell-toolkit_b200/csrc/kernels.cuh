@@ -70,7 +70,7 @@ struct WindowDev {
     // (plane 0 entry of an event only) 64-bit totals of the event: ticks of
     // its patches longer than kTprof, and raster visits of all its patches
     unsigned long long wide_ticks, nvisits;
-    unsigned long long ncells;  // (plane 0 entry) patch cells of the event, counted when patches fluctuate
+    unsigned long long ncells;  // (plane 0 entry) patch cells of the event
     int nadded, out_time, out_pitch, oversize;
     int bigcharge;  // patches whose raster bound exceeds kMaxVisitBound
 };
