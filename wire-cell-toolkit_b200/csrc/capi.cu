@@ -8,7 +8,6 @@
 
 #include <algorithm>
 #include <charconv>
-#include <climits>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -526,7 +525,7 @@ static int ensure_spectra(Core& c, PlaneState& ps, int N)
     CUDA_TRY(ps.d_spec.ensure(sizeof(float2) * (size_t)rows * (N / 2)));
     launch_rfft_rows(ps.d_table.as<float>(), ps.ldr, std::min(ps.nresp, N), ps.d_spec.as<float2>(), N / 2, rows, d,
                      c.own_stream);
-    ps.have_wspec = wire_fft_pays(ps.npad, INT_MAX) && wire_fft_fits(ps.G, ps.npad, N / 2);
+    ps.have_wspec = wire_blocks_pay(ps.npad) && wire_fft_fits(ps.G, ps.npad, N / 2);
     if (ps.have_wspec) {
         CUDA_TRY(ps.d_wspec.ensure(sizeof(float2) * wire_spec_count(ps.G, N / 2)));
         launch_wire_spec(ps.d_spec.as<float2>(), ps.d_wspec.as<float2>(), ps.G, ps.npad, N / 2, c.own_stream);
@@ -773,7 +772,7 @@ static int wire_fix(Core& c, const EventPlan& ev, bool adjoint, WireFix& f)
         f.energy[ip] = ne;
         f.item[ip] = ni;
         f.chunk[ip] = nc;
-        if (!g.nin || !ps.have_wspec) continue;
+        if (!g.nin || !wire_lists(ps.npad)) continue;
         const int n = adjoint ? g.nin : g.nin + 2 * ps.npad;
         ne += wire_energy_count(n, ps.npad, g.N / 2);
         ni += wire_list_count(n, ps.npad);
@@ -925,6 +924,8 @@ static int forward_device(Core& c, const double* d_depos, size_t ndepos, float* 
               (rows > 0 ? raster_launches : 0));
     CUDA_TRY(cudaGetLastError());
 
+    long long charge_rows = 0;
+    for (int ip = 0; ip < np; ++ip) charge_rows += gset.p[ip].nin;
     WireFix fix;
     int frc = wire_fix(c, ev, false, fix);
     if (frc) return frc;
@@ -990,17 +991,17 @@ static int forward_device(Core& c, const double* d_depos, size_t ndepos, float* 
                 const int wlo = std::max(0, w.m_start_ch), whi = std::min(ps.desc.nwires, w.m_end_ch);
                 const unsigned char* flags = row_flag + pset.p[ip].wire_base;
                 Core::StageTimer t_c(&c, 3, ps_s);
-                const bool wire = ps.have_wspec && wire_fft_pays(ps.npad, nout);
-                if (wire)
+                const WireForm form = wire_form(ps.npad, nout, M, total_visits, charge_rows, ps.have_wspec);
+                if (form != WireForm::Direct)
                     launch_wire_conv_fft(reinterpret_cast<const float2*>(Q), ps.d_wspec.as<float2>(),
                                          ps.d_spec.as<float2>(), V, ps.G, ps.npad, nin, nout, M, ps.mirror,
-                                         c.d_energy.as<double>() + fix.energy[ip],
+                                         form == WireForm::Blocks ? c.d_energy.as<double>() + fix.energy[ip] : nullptr,
                                          WantRows{w.start_ch - ps.npad, wlo, whi, ps.desc.nwires, flags, nullptr, 0},
                                          row_list(c, ev, fix, ip), ps_s);
                 else
                     launch_wire_conv(reinterpret_cast<const float2*>(Q), ps.d_spec.as<float2>(), V, ps.G, ps.npad,
                                      nin, nout, M, ps.mirror, ps_s);
-                t_c.close(wire ? 3 : 1);
+                t_c.close(form == WireForm::Blocks ? 3 : (form == WireForm::Listed ? 2 : 1));
                 Core::StageTimer t_i(&c, 4, ps_s);
                 launch_irfft_rows(V, nout, d, w.start_ch - ps.npad, wlo, whi, w.start_tick, std::min(N, w.nt_ref),
                                   nticks, d_frame + (size_t)ps.row0 * nticks, ps_s, flags, ps.desc.nwires, ps.npad);

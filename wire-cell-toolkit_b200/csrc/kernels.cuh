@@ -345,17 +345,22 @@ void launch_irfft3_batch(const BatchPlan* plan, const BatchStatic& bs, int cls, 
                          cudaStream_t s);
 // Overlap-save forms (wire_fft.cu): Rw holds wire_spec_count(G, M) values made
 // from the taps by launch_wire_spec; wire_fft_fits says whether they apply,
-// wire_fft_pays and wire_adj_fft_pays where they are the faster form.  Faint rows
-// are convolved from the taps: energy holds wire_energy_count(n, ...) values,
-// list.item wire_list_count(n, ...) and list.chunk wire_chunk_count(n, ...)
-// entries for n output rows (adjoint: nin).
+// wire_blocks_pay for which pads they are made, wire_form and wire_adj_fft_pays
+// where they are used.  Faint rows are convolved from the taps: energy holds
+// wire_energy_count(n, ...) values, list.item wire_list_count(n, ...) and
+// list.chunk wire_chunk_count(n, ...) entries for n output rows (adjoint: nin), at
+// pads that wire_lists names.  launch_wire_conv_fft with a null energy lists every
+// wanted row and runs no block.
 size_t wire_energy_count(int n, int npad, int M);
 size_t wire_list_count(int n, int npad);
 size_t wire_chunk_count(int n, int npad);
 int wire_row_blocks(int n, int npad);
 size_t wire_spec_count(int G, int M);
 bool wire_fft_fits(int G, int npad, int M);
-bool wire_fft_pays(int npad, int nout);
+enum class WireForm { Direct, Listed, Blocks };  // direct kernels; every wanted row listed; blocks, faint rows listed
+bool wire_lists(int npad);
+bool wire_blocks_pay(int npad);
+WireForm wire_form(int npad, int nout, int M, long long visits, long long rows, bool have_spectra);
 bool wire_adj_fft_pays(int npad, int nin);
 void launch_wire_spec(const float2* taps, float2* Rw, int G, int npad, int M, cudaStream_t s);
 void launch_wire_conv_fft(const float2* Qh, const float2* Rw, const float2* taps, float2* Vh, int G, int npad, int nin,

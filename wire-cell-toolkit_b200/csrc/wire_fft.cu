@@ -32,7 +32,7 @@ template <bool ADJ>
 __global__ void __launch_bounds__(kPickThreads) k_wire_pick(const double* __restrict__ energy, int nfb, int P, int n,
                                                             WantRows want, RowList list)
 {
-    wfft::pick_tile<ADJ>(energy + (size_t)blockIdx.x * nfb * kWL, nfb, P, blockIdx.x, n, want, 0, list);
+    wfft::pick_tile<ADJ>(energy ? energy + (size_t)blockIdx.x * nfb * kWL : nullptr, nfb, P, blockIdx.x, n, want, 0, list);
 }
 
 __global__ void __launch_bounds__(kWThreads) k_wire_spec(const float2* __restrict__ taps, float2* __restrict__ Rw,
@@ -51,20 +51,37 @@ bool wire_fft_fits(int G, int npad, int M)
     return npad <= kWMaxPad && M % 2 == 0 && wire_spec_count(G, M) <= kWMaxSpec;
 }
 
-// Where the overlap-save form, with its faint rows, is the faster one for an event
-// (11 groups, M = 1600, direct / overlap-save in us, inputs not in L2, a few faint
-// rows at the edges).  Its time goes by blocks of 256 - 2P rows, the direct
-// forms' by G (2P + 1) a row in tiles of 64 or 128 rows.
-//   P = 21: one tile 31 / 39, 170 charge wires 54 / 56, 240 78 / 61, 960 150 / 99
-//           (M = 3200: 54 / 52, 80 / 75, 125 / 104, 269 / 172);
+// The forms of an event's wire convolution.  The blocks' time goes by 256 - 2P rows,
+// that of the direct kernels and of the listed rows by G (2P + 1) a row.  Kernels
+// alone, direct / blocks with a few faint rows, us (11 groups, M = 1600, inputs not
+// in L2):
+//   P = 21: one tile of 128 rows 31 / 39, 170 charge wires 54 / 56, 240 78 / 61,
+//           960 150 / 99 (M = 3200: 54 / 52, 80 / 75, 125 / 104, 269 / 172);
 //   P = 10: 23 / 40, 47 / 54 (240), 86 / 91 (960; M = 3200: 150 / 158);
-//   others have no direct kernel of their own: P = 16 269 / 40, 539 / 102;
-//           P = 2 50 / 39, 56 / 45, 99 / 85; P = 1 39 / 39, 43 / 46, 64 / 86;
-//           P = 0 31 / 39, 45 / 85.
-bool wire_fft_pays(int npad, int nout)
+//   P = 1 39 / 39, 43 / 46, 64 / 86; P = 0 31 / 39, 45 / 85; other pads have no
+//           direct kernel of their own: P = 16 269 / 40, 539 / 102.
+bool wire_lists(int npad) { return npad >= 2 && npad != 10 && npad <= kWMaxPad; }
+bool wire_blocks_pay(int npad) { return wire_lists(npad) && npad > 5; }
+// Where few rows or little charge make the blocks, they leave most rows faint and
+// both forms are paid: events in us, rows listed at once / blocks (5000 point depos
+// on W wires unless given; M = 950 at 2000 ticks, 1792 at 6000):
+//   few visits a row, 960 wires: 0.3 366 / 426, 0.8 382 / 376, 2 386 / 323 (P = 16);
+//   few rows (the blocks pad them to 256): P = 16 W = 100 151 / 165 and 178 / 180, 230
+//     179 / 187 and 210 / 207, 500 223 / 209 and 277 / 267; P = 64 W = 40 246 / 299,
+//     230 307 / 295;
+//   few taps: P = 5 W = 100 150 / 172, 500 224 / 254, 940 305 / 313; P = 2 W = 300
+//     179 / 204, 940 283 / 315.
+// P = 21 has a direct kernel, 16 columns x 128 rows a block, which is the faster one
+// while all its blocks are resident at once: direct / blocks W = 190 169 / 182 and 188 /
+// 201, 300 181 / 193 and (two waves) 227 / 225, 400 211 / 199 and 263 / 257; full APA,
+// 1500 depos in showers on 200 wires a plane 279 / 324; visits a row 0.3 346 / 441, 0.8
+// 364 / 382, 2 370 / 315.
+WireForm wire_form(int npad, int nout, int M, long long visits, long long rows, bool have_spectra)
 {
-    if (npad == 21) return nout > 128;
-    return npad >= 2 && npad != 10;
+    if (!wire_lists(npad)) return WireForm::Direct;
+    const bool few = !have_spectra || visits < rows;
+    if (npad == 21) return few || ((M + 15) / 16) * ((nout + 127) / 128) <= 2 * 148 ? WireForm::Direct : WireForm::Blocks;
+    return few || nout <= kWL ? WireForm::Listed : WireForm::Blocks;
 }
 // The adjoint, a transform back per group: P = 21: two tiles of 64 46 / 48, 170
 // wires 74 / 52, 960 197 / 101; P = 16: 37 / 48, 60 / 52, 160 / 103; P = 10: 46 /
@@ -87,9 +104,12 @@ void launch_wire_conv_fft(const float2* Qh, const float2* Rw, const float2* taps
                           cudaStream_t s)
 {
     if (nout <= 0) return;
-    cudaFuncSetAttribute((const void*)k_wire_conv_fft, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWConvSmem);
-    k_wire_conv_fft<<<dim3(wire_fblocks(M), wire_blocks(nout, npad)), kWThreads, kWConvSmem, s>>>(
-        Qh, Rw, Vh, G, npad, nin, nout, M, energy);
+    if (energy) {
+        cudaFuncSetAttribute((const void*)k_wire_conv_fft, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)kWConvSmem);
+        k_wire_conv_fft<<<dim3(wire_fblocks(M), wire_blocks(nout, npad)), kWThreads, kWConvSmem, s>>>(
+            Qh, Rw, Vh, G, npad, nin, nout, M, energy);
+    }
     k_wire_pick<false><<<wire_blocks(nout, npad), kPickThreads, 0, s>>>(energy, wire_fblocks(M), npad, nout, want, list);
     launch_wire_rows(Qh, taps, Vh, G, npad, nin, nout, M, pair, list, s);
 }

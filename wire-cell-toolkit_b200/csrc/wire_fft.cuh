@@ -339,7 +339,7 @@ constexpr double kFaintEnergy = 9.0;
 // Block blk's rows that are faint and wanted into the list, as groups of eight,
 // those of a window of neighbouring groups a chunk (the kernels that take them
 // stage the window's input rows).  energy: [nfb][256] of the block, an eighth of
-// the columns per 128 threads, added in a fixed order.
+// the columns per 128 threads, added in a fixed order; null: every wanted row.
 template <bool ADJ>
 __device__ __forceinline__ void pick_tile(const double* __restrict__ energy, int nfb, int P, int blk, int n,
                                           const WantRows& want, int entry, const RowList& list)
@@ -362,8 +362,9 @@ __device__ __forceinline__ void pick_tile(const double* __restrict__ energy, int
         const int W = want.wire0 + base - P + (int)threadIdx.x;
         s_want[0][threadIdx.x] = W >= 0 && W < want.nwires ? want.flag[W] : 0;
     }
+    const bool every = energy == nullptr;  // no blocks: all wanted rows
     double e = 0.0;
-    {
+    if (!every) {
         const int h = threadIdx.x & (kWL / 2 - 1), part = threadIdx.x / (kWL / 2);
         const double2* at = reinterpret_cast<const double2*>(energy) + h;
         const int f1 = nfb * (part + 1) / 8;
@@ -379,7 +380,7 @@ __device__ __forceinline__ void pick_tile(const double* __restrict__ energy, int
         s_e[part][h] = v;
     }
     __syncthreads();
-    if (q == 0) {
+    if (q == 0 && !every) {
         const double* s = reinterpret_cast<const double*>(s_e) + t;
 #pragma unroll
         for (int k = 0; k < 8; ++k) e += s[k * kWL];
@@ -390,10 +391,13 @@ __device__ __forceinline__ void pick_tile(const double* __restrict__ energy, int
     }
     __syncthreads();
     if (q == 0) {
-        double mean = 0.0;
+        double mean = INFINITY;
+        if (!every) {
+            mean = 0.0;
 #pragma unroll
-        for (int k = 0; k < kWL / 32; ++k) mean += s_w[k];
-        mean *= 1.0 / kWL;
+            for (int k = 0; k < kWL / 32; ++k) mean += s_w[k];
+            mean *= 1.0 / kWL;
+        }
         const int p = energy_point(t), r = p - p0, W = want.wire0 + base + r;
         // (a NaN in either, or an infinite mean: faint)
         bool faint = r >= 0 && r < wire_valid(P) && base + r < n && W >= want.wlo && W < want.whi &&
