@@ -2136,6 +2136,17 @@ constexpr int kConvRB = 8;
 constexpr int kConvRG = 8;
 constexpr int kConvRows = kConvRB * kConvRG;
 
+// A group's taps are summed apart and then added to the groups before: one sum
+// over all of 473 taps (258 mirrored) rounds at its full size from the first
+// centre tap on, 3.4e-7 of a frame in all against 1.5 to 2.2e-7 so (full APA and
+// planes, tracks and showers; the row transforms' share 1.5e-7).
+template <int N>
+__device__ __forceinline__ void add_sums(float2* sum, const float2* acc)
+{
+#pragma unroll
+    for (int r = 0; r < N; ++r) sum[r] = make_float2(sum[r].x + acc[r].x, sum[r].y + acc[r].y);
+}
+
 // One tile of the wire convolution: frequencies fblk*32 .. +31, output rows
 // oblk*64 .. +63.  Called by all threads of a (32, kConvRG) block.
 // PAIR: groups g and G-1-g share one response up to a mirror in wire
@@ -2157,9 +2168,9 @@ __device__ __forceinline__ void wire_conv_tile(const float2* __restrict__ Qh, co
     const int o0 = oblk * kConvRows;
     const bool fok = f < M;
     const bool dc = f == 0;
-    float2 acc[kConvRB];
+    float2 sum[kConvRB];
 #pragma unroll
-    for (int r = 0; r < kConvRB; ++r) acc[r] = make_float2(0.f, 0.f);
+    for (int r = 0; r < kConvRB; ++r) sum[r] = make_float2(0.f, 0.f);
     const int rb0 = rg * kConvRB;
     const int ng = PAIR ? (G + 1) / 2 : G;
     for (int gi = 0; gi < ng; ++gi) {
@@ -2177,9 +2188,10 @@ __device__ __forceinline__ void wire_conv_tile(const float2* __restrict__ Qh, co
             Rs[jj][lane] = fok ? Rh[((size_t)g * NT + jj) * M + f] : make_float2(0.f, 0.f);
         __syncthreads();
         if (fok) {
-            float2 win[kConvRB], win2[kConvRB];
+            float2 acc[kConvRB], win[kConvRB], win2[kConvRB];  // acc: the group's sums (add_sums)
 #pragma unroll
             for (int r = 0; r < kConvRB; ++r) {
+                acc[r] = make_float2(0.f, 0.f);
                 win[r] = Qs[rb0 + r + 2 * PAD][lane];       // input row o - PAD - j at j = -PAD
                 if (PAIR) win2[r] = Qs2[rb0 + r][lane];     // input row o - PAD + j at j = -PAD
             }
@@ -2207,13 +2219,14 @@ __device__ __forceinline__ void wire_conv_tile(const float2* __restrict__ Qh, co
                     }
                 }
             }
+            add_sums<kConvRB>(sum, acc);
         }
     }
     if (fok) {
 #pragma unroll
         for (int r = 0; r < kConvRB; ++r) {
             const int o = o0 + rb0 + r;
-            if (o < nout) Vh[(size_t)o * M + f] = acc[r];
+            if (o < nout) Vh[(size_t)o * M + f] = sum[r];
         }
     }
 }
@@ -2336,9 +2349,9 @@ __device__ __forceinline__ void conv2_unit(const float2* __restrict__ Qh, const 
         }
         cp_async_commit();
     };
-    float2 acc[RB];
+    float2 sum[RB];
 #pragma unroll
-    for (int r = 0; r < RB; ++r) acc[r] = make_float2(0.f, 0.f);
+    for (int r = 0; r < RB; ++r) sum[r] = make_float2(0.f, 0.f);
     issue(0, 0);
     for (int gi = 0; gi < ng; ++gi) {
         if (gi + 1 < ng) {
@@ -2349,6 +2362,9 @@ __device__ __forceinline__ void conv2_unit(const float2* __restrict__ Qh, const 
             cp_async_wait<0>();
         __syncthreads();
         if (rb0 >= 0) {
+            float2 acc[RB];  // the group's sums (add_sums)
+#pragma unroll
+            for (int r = 0; r < RB; ++r) acc[r] = make_float2(0.f, 0.f);
             const float2* base = conv2_smem + (size_t)(gi & 1) * STAGE;
             const float2* Qs = base;
             const float2* Qs2 = base + SROWS * kConv2F;
@@ -2420,13 +2436,14 @@ __device__ __forceinline__ void conv2_unit(const float2* __restrict__ Qh, const 
                     }
                 }
             }
+            add_sums<RB>(sum, acc);
         }
         __syncthreads();  // buffer gi & 1 is refilled with group gi + 2 next
     }
     if (f < M && rb0 >= 0) {
 #pragma unroll
         for (int r = 0; r < RB; ++r)
-            if (mask >> r & 1) Vh[(size_t)(o0 + rb0 + r) * M + f] = acc[r];
+            if (mask >> r & 1) Vh[(size_t)(o0 + rb0 + r) * M + f] = sum[r];
     }
 }
 
@@ -3033,7 +3050,7 @@ void launch_rfft_batch(const BatchPlan* plan, const FftDesc* descs, float* Q, in
 // PAD < 0: run-time pad (bs.pl[ip].npad) without shared-memory staging.
 // Items of planes ip0 .. ip1-1 in order; within a plane, events in order.
 template <int PAD, bool PAIR>
-__global__ void __launch_bounds__(32 * kConvRG) k_conv_batch(const BatchPlan* __restrict__ plan, BatchStatic bs,
+__global__ void __launch_bounds__(32 * kConvRG, PAD < 0 ? 1 : 3) k_conv_batch(const BatchPlan* __restrict__ plan, BatchStatic bs,
                                                              int ip0, int ip1, const float2* const* __restrict__ spec,
                                                              const float* __restrict__ Q, float2* __restrict__ V)
 {

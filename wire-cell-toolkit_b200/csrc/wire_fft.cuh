@@ -322,7 +322,7 @@ __device__ __forceinline__ void spec_tile(const float2* __restrict__ taps, float
 // row, in 1e-7 of the row itself against 64 bits (full APA, 20k track depos; by
 // rms around the row / rms of the row): 1 to 2: 2.2, worst 3.0 in overlap-save
 // blocks; 2 to 4: 2.9, worst 8.1; 4 to 8: 9; 8 to 16: 19; over 64: 4500.  The
-// direct sum: 3.8 throughout, worst 5.1, with the row transforms of then, 3.4 now.
+// direct sum: 1.6 throughout, worst 2.6 (3.8 and 5.1 before the blocks).
 //
 // What it costs, and why this form: a launch that adds up the energies (9 us, a
 // block per 256 wires) and one that takes the list.  Rows are few on tracks (3 %
