@@ -317,7 +317,7 @@ def run_b200(args):
     achieved = bytes_per_launch / (ms_per_launch / 1e3) / 1e9 if ms_per_launch > 0 else 0.0
     traffic = None
     tp = os.path.join(ROOT, "profiles", "traffic.json")
-    if os.path.exists(tp):
+    if args.workload == "apa" and os.path.exists(tp):  # measured on that event
         try:
             traffic = json.load(open(tp))["stages"].get(dom)
         except Exception:

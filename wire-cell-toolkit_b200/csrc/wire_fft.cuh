@@ -330,9 +330,9 @@ __device__ __forceinline__ void spec_tile(const float2* __restrict__ taps, float
 // direct kernel's time a row decides, so the list keeps the shape of its blocks:
 // windows of sixteen groups of eight rows, staged once (one warp a group from L2:
 // 348 us against 146 for the three planes of 200k shower depos).  Events without
-// -> with this, us: plane 2k 267 -> 282, full APA on tracks 20k 523 -> 561, 520k
-// 1034 -> 1062, shower 200k 1665 -> 1744, fit step 20k 1443 -> 1518; 16 batched
-// events, kernels 4761 -> 5900.
+// -> with this, us: plane 2k 267 -> 282, full APA on tracks 20k 487 -> 528, 520k
+// 965 -> 1003, shower 200k 1624 -> 1715, fit step 20k 1409 -> 1496; 16 batched
+// events 4.25 -> 5.33 ms a call, 64 of 500-5000 depos 9.2 -> 12.4.
 // ---------------------------------------------------------------------------
 constexpr double kFaintEnergy = 9.0;
 
